@@ -1,0 +1,1288 @@
+// The linear recurrences of the decoder designs over long portions, 64 tokens at a time (the bfloat16 engine's steps; single
+// tokens, short portions and the 32-bit engine stay in the token-by-token kernels of decay_attention.cu, gated_recurrence.cu
+// and state_recurrence.cu).  Per head, with a 32-bit state S [dim, vdim]:
+//
+//   fixed     S_t = d S_(t-1) + k_t v_t^T                              linear attention with a fixed decay
+//   ssm       S_t = g_t S_(t-1) + k_t (w_t v_t)^T   (+ D v_t behind)   selective state space
+//   hgrn2     S_t = diag(f_t) S_(t-1) + (1 - f_t) v_t^T
+//   delta     S' = g_t S_(t-1);  u_t = w_t (v_t - S'^T k_t);  S_t = S' + k_t u_t^T
+//   channels  the same with a decay for every row of the state, S' = diag(g_t) S_(t-1)
+//   and always  o_t = S_t^T q_t
+//
+// With S0 the state before a chunk, G(j, i) the product of the decays of tokens j + 1 .. i and c_i = G(-1, i), one set of
+// formulas covers all five:
+//
+//   U = U' - W S0        o = Q S0 + A U        S = diag(c_63) S0 + K^T U
+//   Q_i = c_i q_i     K_j = G(j, 63) k_j     A_ij = sum_d q_id k_jd G(j, i)_d   (j <= i)
+//   delta:  (1 + L) [U' | W] = [w v | w c k],  L_ij = w_i sum_d k_id k_jd G(j, i)_d (j < i);   else U' = w v, no W
+//
+// Three launches.  First, every (chunk, head) by itself: K^T U (chunk_states_kernel), or W, U' and K (chunk_solve_kernel) for
+// the delta rules.  Then the states before all chunks, which is the only part that goes from chunk to chunk: a sum with decays
+// (chunk_scan_kernel), or two small products a chunk (chunk_walk_kernel).  Last, every (chunk, head) by itself again, the
+// outputs (chunk_outputs_kernel).  A walk token by token is a chain of 2048 dependent updates for a prompt of 2048 tokens; here
+// the chain has 32 links.
+//
+// Decays never appear as quotients or as exponentials of sums: every G is a running product of factors in [0, 1].  With a
+// decay for every row the chunk is cut into blocks of 16: pairs inside a block are formed one by one (their G is carried along
+// in registers), pairs of different blocks as (q_i G(block start, i)) . (k_j G(j, block start)).
+//
+// Everything is 32-bit.  The products run on the tensor cores as three TF32 products of operands split in two, x = hi + lo
+// with 11 bits each: what is dropped (lo * lo and the end of lo) is below 2^-21 of a term and has no direction.
+//
+// Measured (B200, one prompt of 2048 tokens, 16 heads of 128 x 128; all launches, token by token -> here): HGRN2 421 -> 127 us,
+// delta rule 801 -> 178 us (solve 46, walk 72, outputs 60); fixed decays, four prompts of 1654 tokens in all, 403 -> 112 us.
+// What bounds it: mma.sync issues one product of 16 x 8 x 8 every 8 cycles a scheduler on this GPU whatever its type, so the three
+// TF32 products of a term are worth 1.3 times the ordinary 32-bit pipes, about 30 us of the states and outputs; the rest is the
+// splitting of operands (two integer operations at half rate and one addition an element) and the phases of a CTA waiting for
+// one another.
+#include "common.cuh"
+#include "warp_mma.cuh"
+
+namespace lb {
+
+constexpr int CR_C = 64;                 // tokens a chunk
+constexpr int CR_PT = CR_C + 4;          // floats between rows of 64 places: 16-byte pieces of 8 rows lie in all banks
+constexpr int CR_VT = 64;                // value columns at a time
+constexpr int CR_PV = CR_VT + 8;         // and between their rows: 4 rows of 8 neighbours lie in all banks
+constexpr int CR_THREADS = 512;
+constexpr int CR_SCAN = 256, CR_WALK = 256;
+constexpr int CR_SEQS = 64;              // sequences a launch
+
+enum CrKind : int { CR_FIXED = 0, CR_SSM = 1, CR_DELTA = 2, CR_HGRN2 = 3, CR_CHANNELS = 4 };
+
+__host__ __device__ constexpr bool cr_delta(int kind) { return kind == CR_DELTA || kind == CR_CHANNELS; }
+__host__ __device__ constexpr bool cr_rows(int kind) { return kind == CR_HGRN2 || kind == CR_CHANNELS; }   // a decay for every row
+
+struct ChunkParams {
+  const float* q; const float* k; const float* v; const float* a; const float* b;    // hgrn2: k is the gate's input
+  long long q_ld, k_ld, v_ld, a_ld, b_ld;
+  const float* A_log; const float* dt_bias; const float* D; const float* bias; const float* lower; const float* decay;
+  float* state; float* out; long long out_ld;
+  const int* cu_tokens; const int* slots;
+  int heads, groups, dim, vdim, unit_norm, act;
+  float q_scale, unit_eps;
+  int vec, vecv, vec2;                   // rows of q, k, a and rows of v in whole aligned 16-byte pieces; rows of out in 8-byte ones
+  int slot0;                             // first chunk of this launch, counted over the sequences below
+  int num_seqs;
+  float* scratch;                        // per (chunk of this launch, head), the arrays at these offsets
+  long long per_head;
+  int off_w, off_k, off_u, off_g, v_ld_s;    // state (before the chunk; first K^T U) at 0: [KD][v_ld_s]; W [64][KD + 4]; K^T [KD][68]; U [64][v_ld_s]; c_63
+  int seq[CR_SEQS];                      // sequence of the step
+  int base[CR_SEQS + 1];                 // its first chunk
+};
+
+__device__ __forceinline__ float cr_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
+__device__ __forceinline__ float cr_sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
+__device__ __forceinline__ float cr_silu(float x) { return __fdividef(x, 1.f + expf(-x)); }
+__device__ __forceinline__ float cr_silu_fast(float x) { return __fdividef(x, 1.f + __expf(-x)); }    // as decay_chunk_kernel's, within 2 ulp
+template <typename F>
+__device__ __forceinline__ float4 cr_map(float4 x, F f) { return make_float4(f(x.x), f(x.y), f(x.z), f(x.w)); }
+__device__ __forceinline__ void cr_scale(float* x, float g) {
+  float4* y = reinterpret_cast<float4*>(x);
+  *y = make_float4(y->x * g, y->y * g, y->z * g, y->w * g);
+}
+
+// x as hi + lo: hi rounded to 11 significant bits, lo what is left, of which the product reads the first 11 (cut, but lo is as
+// often negative as positive, so the cut has no direction)
+__device__ __forceinline__ void cr_split(float x, uint32_t& hi, uint32_t& lo) {
+  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;   // (cvt.rna.tf32 does the same and is slower)
+  lo = __float_as_uint(x - __uint_as_float(hi));
+}
+
+__device__ __forceinline__ void mma_tf32(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// The 16 x 8 tile of a row-major 32-bit matrix at `tile` (shared address of its first element, `pitch` floats a row) as the
+// left operand of a TF32 product, split in two.
+__device__ __forceinline__ void cr_left(uint32_t tile, int pitch, int lane, uint32_t* hi, uint32_t* lo) {
+  uint32_t r[4];
+  ldmatrix_x4(tile + 4 * ((((lane >> 3) & 1) * 8 + (lane & 7)) * pitch + (lane >> 4) * 4), r[0], r[1], r[2], r[3]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) cr_split(__uint_as_float(r[i]), hi[i], lo[i]);
+}
+// The same of a matrix that lies transposed: [8 places][16 rows], rows 8 or 24 floats apart modulo 32.
+__device__ __forceinline__ void cr_left_t(const float* tile, int pitch, int lane, uint32_t* hi, uint32_t* lo) {
+  const float* x = tile + (lane & 3) * pitch + (lane >> 2);
+  cr_split(x[0], hi[0], lo[0]);
+  cr_split(x[8], hi[1], lo[1]);
+  cr_split(x[4 * pitch], hi[2], lo[2]);
+  cr_split(x[4 * pitch + 8], hi[3], lo[3]);
+}
+// An 8 x 8 right operand: from [8 columns][8 places] (ldmatrix), from [8 places][8 columns] (plain loads), both split; and two
+// of the first form that are split already.
+__device__ __forceinline__ void cr_right(uint32_t tile, int pitch, int lane, uint32_t* hi, uint32_t* lo) {
+  uint32_t r[2];
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1]) : "r"(tile + 4 * ((lane & 7) * pitch + ((lane >> 3) & 1) * 4)));
+  cr_split(__uint_as_float(r[0]), hi[0], lo[0]);
+  cr_split(__uint_as_float(r[1]), hi[1], lo[1]);
+}
+__device__ __forceinline__ void cr_right_t(const float* tile, int pitch, int lane, uint32_t* hi, uint32_t* lo) {
+  const float* x = tile + (lane & 3) * pitch + (lane >> 2);
+  cr_split(x[0], hi[0], lo[0]);
+  cr_split(x[4 * pitch], hi[1], lo[1]);
+}
+__device__ __forceinline__ void cr_right2(uint32_t tile, int pitch, int lane, uint32_t* r) {
+  ldmatrix_x4(tile + 4 * (((lane >> 4) * 8 + (lane & 7)) * pitch + ((lane >> 3) & 1) * 4), r[0], r[1], r[2], r[3]);
+}
+
+// MT x NT tiles of one step of 8 places.  The two cross terms go to `small`, so that the chains are short and their rounding
+// is; products on one accumulator stand as far apart as there are tiles.
+template <int MT, int NT>
+__device__ __forceinline__ void cr_step(float (*acc)[NT][4], float (*small)[NT][4], const uint32_t (*ah)[4], const uint32_t (*al)[4],
+                                        const uint32_t (*bh)[2], const uint32_t (*bl)[2]) {
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int t = 0; t < NT; ++t) mma_tf32(small[m][t], al[m], bh[t][0], bh[t][1]);
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int t = 0; t < NT; ++t) mma_tf32(acc[m][t], ah[m], bh[t][0], bh[t][1]);
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int t = 0; t < NT; ++t) mma_tf32(small[m][t], ah[m], bl[t][0], bl[t][1]);
+}
+
+// 16 rows of `left` times NT n-tiles of `right` (both row-major along the KS * 8 places summed over).
+template <int KS, int NT>
+__device__ __forceinline__ void cr_scores(uint32_t left, uint32_t right, int pitch, int lane, float (*acc)[NT][4], float (*small)[NT][4]) {
+#pragma unroll 2
+  for (int ks = 0; ks < KS; ++ks) {
+    uint32_t ah[1][4], al[1][4], bh[NT][2], bl[NT][2];
+    cr_left(left + 32 * ks, pitch, lane, ah[0], al[0]);
+#pragma unroll
+    for (int t = 0; t < NT; ++t) cr_right(right + 4 * (8 * t * pitch + 8 * ks), pitch, lane, bh[t], bl[t]);
+    cr_step<1, NT>(acc, small, ah, al, bh, bl);
+  }
+}
+
+// The scores of a chunk on and below its diagonal, in 20 tiles of 16 x 8 shared out over the warps, at most two a warp.
+// leave(r, n, tile): 16-row tile r, 8-column tile n.
+template <int KS, typename F>
+__device__ __forceinline__ void cr_triangle(uint32_t left, uint32_t right, int pitch, int warp, int lane, F leave) {
+  auto run = [&](int r, int n0, auto count) {
+    constexpr int NT = decltype(count)::value;
+    float acc[1][NT][4] = {}, small[1][NT][4] = {};
+    cr_scores<KS, NT>(left + 4 * 16 * r * pitch, right + 4 * 8 * n0 * pitch, pitch, lane, acc, small);
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[0][t][e] += small[0][t][e];
+      leave(r, n0 + t, acc[0][t]);
+    }
+  };
+  struct One { enum { value = 1 }; };
+  struct Two { enum { value = 2 }; };
+  if (warp < 8) run(3, warp, One());
+  else if (warp < 11) run(2, 2 * (warp - 8), Two());
+  else if (warp < 13) run(1, 2 * (warp - 11), Two());
+  else if (warp < 15) run(0, warp - 13, One());
+}
+
+// 64 rows of COLS floats into shared memory by asynchronous copies, PITCH floats apart; rows from m and columns from cols on
+// are zeros.
+template <int COLS, int PITCH>
+__device__ __forceinline__ void cr_fetch(float* dst, const float* src, long long ld, int m, int cols, bool vec, int tid) {
+  if (vec) {
+    constexpr int STEP = CR_THREADS / (COLS / 4);  // rows between two of a thread's pieces
+    const int t0 = tid / (COLS / 4), c = (tid % (COLS / 4)) * 4;
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + t0 * PITCH + c);
+    const float* x = src + (size_t)t0 * ld + c;
+    const int rows = c < cols ? m - t0 : 0;
+#pragma unroll
+    for (int i = 0; i < CR_C / STEP; ++i) {
+      const bool real = i * STEP < rows;
+      cp_async16(d + 4 * i * STEP * PITCH, real ? x : src, real);
+      x += (size_t)STEP * ld;
+    }
+  } else {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    for (int i = tid; i < CR_C * COLS; i += CR_THREADS) {
+      const int t = i / COLS, c = i % COLS;
+      const bool real = t < m && c < cols;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4 * (t * PITCH + c)), "l"(real ? src + (size_t)t * ld + c : src),
+                   "r"(real ? 4 : 0) : "memory");
+    }
+  }
+}
+
+struct ChunkPlace { int seq, first, m; };        // sequence, first token, tokens
+
+__device__ __forceinline__ ChunkPlace cr_place(const ChunkParams& p, int at) {
+  const int slot = p.slot0 + at;
+  int si = 0;
+  while (si + 1 < p.num_seqs && p.base[si + 1] <= slot) ++si;
+  ChunkPlace c;
+  c.seq = p.seq[si];
+  c.first = p.cu_tokens[c.seq] + (slot - p.base[si]) * CR_C;
+  c.m = min(CR_C, p.cu_tokens[c.seq + 1] - c.first);
+  return c;
+}
+
+// Decay and write strength of each token, one number a head (decay 1, strength 0 behind the last token).
+template <int KIND>
+__device__ __forceinline__ void cr_numbers(const ChunkParams& p, const ChunkPlace& c, int h, float* gs, float* ws, int tid) {
+  if (tid >= CR_C) return;
+  float g = 1.f, w = 0.f;
+  if (tid < c.m) {
+    w = 1.f;
+    if (KIND == CR_FIXED) g = p.decay[h];
+    if (KIND == CR_SSM || KIND == CR_DELTA) {
+      const float sp = cr_softplus(p.a[(size_t)(c.first + tid) * p.a_ld + h] + p.dt_bias[h]);
+      g = expf(-expf(p.A_log[h]) * sp);
+      w = sp;
+    }
+    if (cr_delta(KIND)) w = cr_sigmoid(p.b[(size_t)(c.first + tid) * p.b_ld + h]);
+  }
+  gs[tid] = g;
+  ws[tid] = w;
+}
+
+// What the fetched rows become, in place: k (and q) through their activation or to unit length, hgrn2's gate input (without q) to
+// decay and 1 - decay; decays behind the last token and row: 1.
+template <int KIND, int KD, int PITCH, bool WITH_Q>
+__device__ __forceinline__ void cr_form(const ChunkParams& p, const ChunkPlace& c, int h, float* Qs, float* Ks, float* Gs, int tid) {
+  constexpr int STEP = CR_THREADS / (KD / 4);
+  const int lane = tid & 31, warp = tid >> 5, t0 = tid / (KD / 4), d = (tid % (KD / 4)) * 4;
+  if (KIND == CR_FIXED && p.act) {
+#pragma unroll 4
+    for (int i = 0; i < CR_C / STEP; ++i) {
+      const int at = (t0 + i * STEP) * PITCH + d;
+      float4* k = reinterpret_cast<float4*>(Ks + at);
+      *k = cr_map(*k, cr_silu_fast);
+      if (WITH_Q) { float4* q = reinterpret_cast<float4*>(Qs + at); *q = cr_map(*q, cr_silu_fast); }
+    }
+  }
+  if (KIND == CR_HGRN2 && WITH_Q) {                // the decays follow block by block
+#pragma unroll 4
+    for (int i = 0; i < CR_C / STEP; ++i) {
+      float4* q = reinterpret_cast<float4*>(Qs + (t0 + i * STEP) * PITCH + d);
+      *q = cr_map(*q, cr_silu);
+    }
+  }
+  if (KIND == CR_HGRN2 && !WITH_Q) {
+    float low[4], bi[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      low[e] = d + e < p.dim ? p.lower[h * p.dim + d + e] : 1.f;          // rows beyond dim: decay 1
+      bi[e] = d + e < p.dim ? p.bias[h * p.dim + d + e] : 0.f;
+    }
+#pragma unroll 2
+    for (int i = 0; i < CR_C / STEP; ++i) {
+      const int t = t0 + i * STEP, at = t * PITCH + d;
+      float4* k = reinterpret_cast<float4*>(Ks + at);
+      float g[4] = {k->x, k->y, k->z, k->w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) g[e] = t < c.m ? low[e] + (1.f - low[e]) * __frcp_rn(1.f + expf(-(g[e] + bi[e]))) : 1.f;
+      *reinterpret_cast<float4*>(Gs + at) = make_float4(g[0], g[1], g[2], g[3]);
+      *k = make_float4(1.f - g[0], 1.f - g[1], 1.f - g[2], 1.f - g[3]);
+    }
+  }
+  if (cr_delta(KIND) && p.unit_norm) {
+#pragma unroll
+    for (int t = warp; t < CR_C; t += CR_THREADS / 32) {                  // rows behind the last token are zeros and stay so
+      float sq = 0.f, sk = 0.f, x[KD / 32], y[KD / 32];
+#pragma unroll
+      for (int u = 0; u < KD / 32; ++u) {
+        y[u] = Ks[t * PITCH + lane + 32 * u];
+        x[u] = WITH_Q ? Qs[t * PITCH + lane + 32 * u] : 0.f;
+        sq += x[u] * x[u]; sk += y[u] * y[u];
+      }
+      sk = warp_sum(sk);
+      const float fk = 1.f / sqrtf(sk + p.unit_eps);
+#pragma unroll
+      for (int u = 0; u < KD / 32; ++u) Ks[t * PITCH + lane + 32 * u] = y[u] * fk;
+      if (WITH_Q) {
+        sq = warp_sum(sq);
+        const float fq = p.q_scale / sqrtf(sq + p.unit_eps);
+#pragma unroll
+        for (int u = 0; u < KD / 32; ++u) Qs[t * PITCH + lane + 32 * u] = x[u] * fq;
+      }
+    }
+  }
+}
+
+// The decays of 16 tokens from `b0` on, a warp a token and a lane KD / 32 neighbouring channels: requested (channels), or formed
+// from the gate's input in Ks, which becomes 1 - decay (hgrn2); then left in Gb [16][PITCH].
+template <int KIND, int KD>
+__device__ __forceinline__ void cr_request_decays(const ChunkParams& p, const ChunkPlace& c, int h, int b0, int tid, float* g) {
+  const int t = b0 + tid / 32, d0 = (tid % 32) * (KD / 32);
+  const float* src = p.a + (size_t)(c.first + t) * p.a_ld + (size_t)h * p.dim + d0;
+#pragma unroll
+  for (int e = 0; e < KD / 32; ++e) g[e] = 1.f;
+  if (t < c.m && p.vec && KD == 128) {
+    if (d0 < p.dim) {
+      const float4 x = *reinterpret_cast<const float4*>(src);
+      g[0] = x.x; g[1] = x.y; g[KD / 32 - 2] = x.z; g[KD / 32 - 1] = x.w;
+    }
+  } else if (t < c.m) {
+#pragma unroll
+    for (int e = 0; e < KD / 32; ++e) if (d0 + e < p.dim) g[e] = src[e];
+  }
+}
+template <int KIND, int KD, int PITCH>
+__device__ __forceinline__ void cr_put_decays(const ChunkPlace& c, int b0, int tid, const float* g, const float* low, const float* bi, float* Ks, float* Gb) {
+  const int r = tid / 32, d0 = (tid % 32) * (KD / 32);
+  float x[KD / 32];
+  if (KIND == CR_HGRN2) {
+    float* k = Ks + (b0 + r) * PITCH + d0;
+#pragma unroll
+    for (int e = 0; e < KD / 32; ++e) x[e] = b0 + r < c.m ? low[e] + (1.f - low[e]) * __frcp_rn(1.f + expf(-(k[e] + bi[e]))) : 1.f;
+#pragma unroll
+    for (int e = 0; e < KD / 32; ++e) k[e] = 1.f - x[e];
+  } else {
+#pragma unroll
+    for (int e = 0; e < KD / 32; ++e) x[e] = g[e];
+  }
+#pragma unroll
+  for (int e = 0; e < KD / 32; ++e) Gb[r * PITCH + d0 + e] = x[e];
+}
+
+// The value rows of the lightning form pass silu as well.
+__device__ __forceinline__ void cr_form_values(float* Us, int tid) {
+  constexpr int STEP = CR_THREADS / (CR_VT / 4);
+#pragma unroll
+  for (int i = 0; i < CR_C / STEP; ++i) {
+    float4* x = reinterpret_cast<float4*>(Us + (tid / (CR_VT / 4) + i * STEP) * CR_PV + (tid % (CR_VT / 4)) * 4);
+    *x = cr_map(*x, cr_silu_fast);
+  }
+}
+
+// G(j, i) at [i][j] for one decay a token (zeros above the diagonal), and c_i: a thread eight rows of a column, from the product
+// of the decays between.
+__device__ __forceinline__ void cr_products(const float* gs, float* Ds, float* cs, int tid) {
+  static_assert(CR_THREADS == 8 * CR_C, "a thread eight rows of a column");
+  const int j = tid % CR_C, i0 = tid / CR_C * 8;
+  float g[8], d = 1.f, c = 1.f;
+#pragma unroll 8
+  for (int i = 0; i < i0; ++i) { const float x = gs[i]; if (i > j) d *= x; }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) g[i] = gs[i0 + i];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (i0 + i > j) d *= g[i];
+    Ds[(i0 + i) * CR_PT + j] = i0 + i >= j ? d : 0.f;
+  }
+  if (j == 0) {                                    // one thread a block of eight: c_i
+#pragma unroll 8
+    for (int i = 0; i < i0; ++i) c *= gs[i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { c *= g[i]; cs[i0 + i] = c; }
+  }
+}
+
+// sum_d x_id k_jd G(j, i)_d for one column j and the rows i of its block of 16 from j (SELF) or j + 1 on, a warp: a lane takes KD / 32
+// neighbouring channels and carries k_j G(j, i); four rows are added up together, in six shuffles.  store(i, sum).
+template <int KD, int PITCH, bool SELF, typename F>
+__device__ __forceinline__ void cr_pairs(const float* Xs, const float* Ks, const float* Gb, int b0, int j, int lane, F store) {
+  const int end = b0 + 16;
+  constexpr int N = KD / 32;
+  float kk[N];
+  auto load = [&](const float* x, float* to) {
+    if constexpr (N == 4) *reinterpret_cast<float4*>(to) = *reinterpret_cast<const float4*>(x + 4 * lane);
+    else *reinterpret_cast<float2*>(to) = *reinterpret_cast<const float2*>(x + 2 * lane);
+  };
+  load(Ks + j * PITCH, kk);
+  for (int i0 = SELF ? j : j + 1; i0 < end; i0 += 4) {
+    float s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u;
+      s[u] = 0.f;
+      if (i < end) {
+        float x[N], g[N];
+        load(Xs + i * PITCH, x);
+        if (i > j) {
+          load(Gb + (i - b0) * PITCH, g);
+#pragma unroll
+          for (int e = 0; e < N; ++e) kk[e] *= g[e];
+        }
+#pragma unroll
+        for (int e = 0; e < N; ++e) s[u] = fmaf(x[e], kk[e], s[u]);
+      }
+    }
+    const bool high = lane & 16, upper = lane & 8;
+    const float x0 = (high ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, high ? s[0] : s[2], 16);
+    const float x1 = (high ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, high ? s[1] : s[3], 16);
+    float x = (upper ? x1 : x0) + __shfl_xor_sync(0xffffffffu, upper ? x0 : x1, 8);
+    x += __shfl_xor_sync(0xffffffffu, x, 4);
+    x += __shfl_xor_sync(0xffffffffu, x, 2);
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    const int i = i0 + (high ? 2 : 0) + (upper ? 1 : 0);
+    if ((lane & 7) == 0 && i < end) store(i, x);
+  }
+}
+
+// ---- every chunk by itself: K^T U of the kinds without the delta rule --------------------------------------------------------
+// Reads k and v (64 KB a chunk and head of 128 x 128), writes 64 KB.
+__host__ __device__ constexpr int cr_states_floats(int kind, int kd) {
+  return CR_C * (kd + 8) * (cr_rows(kind) ? 2 : 1) + CR_C * CR_PV + 3 * CR_C + 4;
+}
+
+template <int KIND, int KD>
+__global__ void __launch_bounds__(CR_THREADS, 2) chunk_states_kernel(const __grid_constant__ ChunkParams p) {
+  constexpr int PD = KD + 8;
+  constexpr bool ROWS = cr_rows(KIND);
+  extern __shared__ __align__(16) float cr_smem[];
+  float* Ks = cr_smem;                             // [64][PD]
+  float* Us = Ks + CR_C * PD;                      // [64][PV]
+  float* gs = Us + CR_C * CR_PV;
+  float* ws = gs + CR_C;
+  float* ts = ws + CR_C;                           // w_j G(j, 63)
+  float* cs = ts + CR_C;                           // c_63
+  float* Gs = cs + 4;                              // [64][PD]
+  pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = blockIdx.y, grp = h / (p.heads / p.groups);
+  pdl_wait();
+  const ChunkPlace c = cr_place(p, blockIdx.x);
+  float* mine = p.scratch + ((size_t)blockIdx.x * p.heads + h) * p.per_head;
+  const float* vsrc = p.v + (size_t)c.first * p.v_ld + (size_t)h * p.vdim;
+  cr_fetch<KD, PD>(Ks, p.k + (size_t)c.first * p.k_ld + (size_t)grp * p.dim, p.k_ld, c.m, p.dim, p.vec, tid);
+  cr_fetch<CR_VT, CR_PV>(Us, vsrc, p.v_ld, c.m, min(CR_VT, p.vdim), p.vecv, tid);
+  cp_async_commit();
+  cr_numbers<KIND>(p, c, h, gs, ws, tid);
+  cp_async_wait<0>();
+  __syncthreads();
+  if (!ROWS && tid < CR_C) {
+    float d = 1.f;
+#pragma unroll 16
+    for (int i = 1; i < CR_C; ++i) { const float x = gs[i]; if (i > tid) d *= x; }
+    ts[tid] = d * ws[tid];
+    if (tid == 0) cs[0] = d * gs[0];
+  }
+  cr_form<KIND, KD, PD, false>(p, c, h, nullptr, Ks, Gs, tid);
+  __syncthreads();
+  if (!ROWS) {
+    if (tid < KD) mine[p.off_g + tid] = cs[0];
+    constexpr int STEP = CR_THREADS / (KD / 4);
+#pragma unroll
+    for (int i = 0; i < CR_C / STEP; ++i) {
+      const int t = tid / (KD / 4) + i * STEP;
+      cr_scale(Ks + t * PD + (tid % (KD / 4)) * 4, ts[t]);
+    }
+  } else {
+    // a thread a channel and a quarter of the chunk: k_j G(j, 63) from the last token back
+    const int d = tid % KD, part = tid / KD;
+    if (part < 4) {
+      float g = 1.f;
+#pragma unroll 8
+      for (int t = CR_C - 1; t >= 16 * part + 16; --t) g *= Gs[t * PD + d];
+      float x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) x[i] = Gs[(16 * part + i) * PD + d];
+#pragma unroll
+      for (int i = 15; i >= 0; --i) { Ks[(16 * part + i) * PD + d] *= g; g *= x[i]; }
+      if (part == 0) mine[p.off_g + d] = g;
+    }
+  }
+  constexpr int MT = KD / 64;
+  const int mt0 = (warp >> 2) * MT, n0 = (warp & 3) * 2;         // a warp: KD / 4 rows, 16 columns
+  for (int v0 = 0; v0 < p.vdim; v0 += CR_VT) {
+    if (v0 > 0) {
+      __syncthreads();
+      cr_fetch<CR_VT, CR_PV>(Us, vsrc + v0, p.v_ld, c.m, min(CR_VT, p.vdim - v0), p.vecv, tid);
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();
+    }
+    if (KIND == CR_FIXED && p.act) cr_form_values(Us, tid);
+    __syncthreads();
+    float acc[MT][2][4] = {}, small[MT][2][4] = {};
+#pragma unroll 4
+    for (int ks = 0; ks < CR_C / 8; ++ks) {
+      uint32_t ah[MT][4], al[MT][4], bh[2][2], bl[2][2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) cr_right_t(Us + 8 * ks * CR_PV + 8 * (n0 + t), CR_PV, lane, bh[t], bl[t]);
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) cr_left_t(Ks + 8 * ks * PD + 16 * (mt0 + mt), PD, lane, ah[mt], al[mt]);
+      cr_step<MT, 2>(acc, small, ah, al, bh, bl);
+    }
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int col = v0 + 8 * (n0 + t) + 2 * (lane & 3);
+        if (col >= p.v_ld_s) continue;
+        float* dst = mine + (16 * (mt0 + mt) + (lane >> 2)) * p.v_ld_s + col;
+        *reinterpret_cast<float2*>(dst) = make_float2(acc[mt][t][0] + small[mt][t][0], acc[mt][t][1] + small[mt][t][1]);
+        *reinterpret_cast<float2*>(dst + 8 * p.v_ld_s) = make_float2(acc[mt][t][2] + small[mt][t][2], acc[mt][t][3] + small[mt][t][3]);
+      }
+  }
+}
+
+// ---- the states before the chunks: S <- diag(c) S + K^T U, element by element --------------------------------------------------
+// A thread four neighbouring columns of one row; eight chunks are requested ahead.
+__global__ void __launch_bounds__(CR_SCAN) chunk_scan_kernel(const __grid_constant__ ChunkParams p, int nslots, int kd) {
+  pdl_trigger();
+  const int h = blockIdx.y, seq = p.seq[blockIdx.z], base = p.base[blockIdx.z];
+  const int c_lo = max(0, p.slot0 - base), c_hi = min(p.base[blockIdx.z + 1], p.slot0 + nslots) - base;
+  const int idx = blockIdx.x * CR_SCAN + threadIdx.x, per = p.v_ld_s / 4;
+  pdl_wait();
+  if (c_lo >= c_hi || idx >= kd * per) return;
+  const int d = idx / per, e = (idx - d * per) * 4;
+  float* S = p.state + ((size_t)p.slots[seq] * p.heads + h) * p.dim * p.vdim + (size_t)d * p.vdim + e;
+  const int have = d < p.dim ? min(4, p.vdim - e) : 0;           // columns of the state; the rest of the scratch is zeros
+  float s[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) s[i] = i < have ? S[i] : 0.f;
+  const size_t stride = (size_t)p.heads * p.per_head;
+  float* x = p.scratch + ((size_t)(base + c_lo - p.slot0) * p.heads + h) * p.per_head;
+  for (int c = c_lo; c < c_hi; c += 8) {
+    float4 ds[8];
+    float g[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (c + i < c_hi) {
+        ds[i] = *reinterpret_cast<const float4*>(x + i * stride + (size_t)d * p.v_ld_s + e);
+        g[i] = x[i * stride + p.off_g + d];
+      }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (c + i < c_hi) {
+        *reinterpret_cast<float4*>(x + i * stride + (size_t)d * p.v_ld_s + e) = make_float4(s[0], s[1], s[2], s[3]);
+        s[0] = fmaf(g[i], s[0], ds[i].x); s[1] = fmaf(g[i], s[1], ds[i].y);
+        s[2] = fmaf(g[i], s[2], ds[i].z); s[3] = fmaf(g[i], s[3], ds[i].w);
+      }
+    x += 8 * stride;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) if (i < have) S[i] = s[i];
+}
+
+// ---- every chunk by itself: W, U' and K of the delta rules ----------------------------------------------------------------------
+// (1 + L) X = B goes by blocks of 16 rows, X_I = (1 + L_II)^-1 (B_I - sum_(J < I) L_IJ X_J), on the tensor cores: the four inverses
+// are formed first (a thread a column), then a warp owns 16 columns of [U' | W] and needs nobody else's.  A thread a column
+// down all 64 rows took 2000 dependent multiply-adds, most of this kernel's time.
+constexpr int CR_XV = 128;               // value columns at a time
+constexpr int CR_PI = 20;                // floats between rows of an inverse
+
+__host__ __device__ constexpr int cr_solve_floats(int kind, int kd) {
+  const int mat = CR_C * (kd + 4);
+  const int x = CR_C * (CR_XV + 4);
+  return mat + 3 * CR_C + CR_C * CR_PT + 64 * CR_PI + (cr_rows(kind) ? (mat > x ? mat : x) + 32 * (kd + 4) + 5 * kd : CR_C * CR_PT + x);
+}
+
+template <int KIND, int KD>
+__global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid_constant__ ChunkParams p) {
+  constexpr int PK = KD + 4, MAT = CR_C * PK, KS = KD / 8;
+  constexpr bool ROWS = cr_rows(KIND);
+  extern __shared__ __align__(16) float cr_smem[];
+  float* Ks = cr_smem;                             // [64][PK]
+  float* gs = Ks + MAT;
+  float* ws = gs + CR_C;
+  float* cs = ws + CR_C;                           // c_i
+  float* Ls = cs + CR_C;                           // [64][PT]
+  constexpr int PX = CR_XV + 4;
+  float* Ti = Ls + CR_C * CR_PT;                   // [4][16][PI]: inverses of the diagonal blocks
+  float* Xv = Ti + 64 * CR_PI;                     // [64][PX]: w v, then U'; with a decay for every row it takes the place of Kr
+  float* Ds = Xv + CR_C * PX;                      // one decay a token: G(j, i) at [i][j]
+  float* Kr = Xv;                                  // a decay for every row: k_j G(j, start of the block at work)
+  float* Gb = Kr + (MAT > CR_C * PX ? MAT : CR_C * PX);    // [2][16][PK]: decays of the block at work and of the next
+  float* starts = Gb + 32 * PK;                    // [5][KD]: product of the decays before block I; [4]: over the block at work
+  pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = blockIdx.y, grp = h / (p.heads / p.groups);
+  pdl_wait();
+  const ChunkPlace c = cr_place(p, blockIdx.x);
+  float* mine = p.scratch + ((size_t)blockIdx.x * p.heads + h) * p.per_head;
+  float* oW = mine + p.off_w;
+  float* oK = mine + p.off_k;
+  float* oU = mine + p.off_u;
+  float* oG = mine + p.off_g;
+  cr_fetch<KD, PK>(Ks, p.k + (size_t)c.first * p.k_ld + (size_t)grp * p.dim, p.k_ld, c.m, p.dim, p.vec, tid);
+  const float* vsrc = p.v + (size_t)c.first * p.v_ld + (size_t)h * p.vdim;
+  if (!ROWS) cr_fetch<CR_XV, PX>(Xv, vsrc, p.v_ld, c.m, min(CR_XV, p.vdim), p.vecv, tid);
+  cp_async_commit();
+  float gn[KD / 32];
+  if (ROWS) cr_request_decays<KIND, KD>(p, c, h, 0, tid, gn);
+  cr_numbers<KIND>(p, c, h, gs, ws, tid);
+  cp_async_wait<0>();
+  __syncthreads();
+  cr_form<KIND, KD, PK, false>(p, c, h, nullptr, Ks, nullptr, tid);
+  if (ROWS) cr_put_decays<KIND, KD, PK>(c, 0, tid, gn, nullptr, nullptr, Ks, Gb);
+  if (!ROWS) cr_products(gs, Ds, cs, tid);
+  __syncthreads();
+  const uint32_t Ka = (uint32_t)__cvta_generic_to_shared(Ks);
+  auto keys_out = [&](const float* K, const float* scale) {      // keys to the state behind the chunk, a row of the state a row
+    for (int i = warp; i < 2 * (KD / 4); i += CR_THREADS / 32) {
+      const int t = (i & 1) * 32 + lane, d = (i >> 1) * 4;
+      const float g = scale ? scale[t] : 1.f;
+      const float4 x = *reinterpret_cast<const float4*>(K + t * PK + d);
+      oK[d * CR_PT + t] = x.x * g; oK[(d + 1) * CR_PT + t] = x.y * g; oK[(d + 2) * CR_PT + t] = x.z * g; oK[(d + 3) * CR_PT + t] = x.w * g;
+    }
+  };
+  if (!ROWS) {
+    cr_triangle<KS>(Ka, Ka, PK, warp, lane, [&](int r, int n, const float* s) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = 16 * r + (lane >> 2) + (e >> 1) * 8, j = 8 * n + 2 * (lane & 3) + (e & 1);
+        Ls[i * CR_PT + j] = j < i ? s[e] * ws[i] * Ds[i * CR_PT + j] : 0.f;
+      }
+    });
+    keys_out(Ks, Ds + (CR_C - 1) * CR_PT);
+    if (tid < KD) oG[tid] = cs[CR_C - 1];
+  } else {
+    const uint32_t Kra = (uint32_t)__cvta_generic_to_shared(Kr);
+    float c_start = 1.f;                           // of this thread's channel: product of the decays before the block
+    const int ch = tid % KD;
+    for (int I = 0; I < 4; ++I) {
+      const int b0 = 16 * I;
+      float* Gi = Gb + (I & 1) * 16 * PK;
+      if (I < 3) cr_request_decays<KIND, KD>(p, c, h, b0 + 16, tid, gn);
+      const int jj = b0 + warp;                    // pairs inside the block: a warp a column
+      cr_pairs<KD, PK, false>(Ks, Ks, Gi, b0, jj, lane, [&](int i, float x) { Ls[i * CR_PT + jj] = x * ws[i]; });
+      if (lane < 16 && b0 + lane <= jj) Ls[(b0 + lane) * CR_PT + jj] = 0.f;
+      __syncthreads();                             // the block's rows as they came are read (and the keys before it moved on)
+      if (tid < KD) {                              // times c_i from the block's start, in place; times G(i, block's end)
+        float g = 1.f, kb[16], gb[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { kb[i] = Ks[(b0 + i) * PK + ch]; gb[i] = Gi[i * PK + ch]; }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { g *= gb[i]; Ks[(b0 + i) * PK + ch] = kb[i] * g; }
+        starts[I * KD + ch] = c_start;
+        starts[4 * KD + ch] = g;
+        c_start *= g;
+        if (I == 3) oG[ch] = c_start;
+        g = 1.f;
+#pragma unroll
+        for (int i = 15; i >= 0; --i) { Kr[(b0 + i) * PK + ch] = kb[i] * g; g *= gb[i]; }
+      }
+      __syncthreads();
+      if (I < 3) cr_put_decays<KIND, KD, PK>(c, b0 + 16, tid, gn, nullptr, nullptr, Ks, Gb + (~I & 1) * 16 * PK);
+      if (I > 0) {                                 // the block's rows against all tokens before it
+        for (int n = warp; n < 2 * I; n += CR_THREADS / 32) {
+          float acc[1][1][4] = {}, small[1][1][4] = {};
+          cr_scores<KS, 1>(Ka + 4 * b0 * PK, Kra + 4 * 8 * n * PK, PK, lane, acc, small);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = b0 + (lane >> 2) + (e >> 1) * 8;
+            Ls[i * CR_PT + 8 * n + 2 * (lane & 3) + (e & 1)] = (acc[0][0][e] + small[0][0][e]) * ws[i];
+          }
+        }
+      }
+      __syncthreads();
+      if (I > 0) {
+        const float g = starts[4 * KD + ch];
+        for (int j = tid / KD; j < b0; j += CR_THREADS / KD) Kr[j * PK + ch] *= g;     // the keys move on to the block's end
+      }
+    }
+    __syncthreads();
+    keys_out(Kr, nullptr);
+  }
+  __syncthreads();                                 // L is complete, the keys are out
+  if (ROWS) {
+    cr_fetch<CR_XV, PX>(Xv, vsrc, p.v_ld, c.m, min(CR_XV, p.vdim), p.vecv, tid);
+    cp_async_commit();
+  }
+  if (tid < 64) {                                  // column tid % 16 of the inverse of block tid / 16
+    const float* L = Ls + (tid & ~15) * (CR_PT + 1);
+    const int col = tid & 15;
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float y0 = 0.f, y1 = 0.f;
+#pragma unroll
+      for (int j = 0; j < i; j += 2) {
+        y0 = fmaf(L[i * CR_PT + j], x[j], y0);
+        if (j + 1 < i) y1 = fmaf(L[i * CR_PT + j + 1], x[j + 1], y1);
+      }
+      x[i] = (i == col ? 1.f : 0.f) - (y0 + y1);
+      Ti[((tid & ~15) + i) * CR_PI + col] = x[i];
+    }
+  }
+  {                                                // w c k, in place
+    constexpr int STEP = CR_THREADS / (KD / 4);
+#pragma unroll
+    for (int i = 0; i < CR_C / STEP; ++i) {
+      const int t = tid / (KD / 4) + i * STEP, d = (tid % (KD / 4)) * 4;
+      float4* x = reinterpret_cast<float4*>(Ks + t * PK + d);
+      const float w = ws[t];
+      const float4 g = ROWS ? *reinterpret_cast<const float4*>(starts + (t / 16) * KD + d) : make_float4(cs[t], cs[t], cs[t], cs[t]);
+      *x = make_float4(x->x * g.x * w, x->y * g.y * w, x->z * g.z * w, x->w * g.w * w);
+    }
+  }
+  const uint32_t La = (uint32_t)__cvta_generic_to_shared(Ls), Ta = (uint32_t)__cvta_generic_to_shared(Ti);
+  // 16 columns of X [64][pitch] (a warp's own), solved in place and written out
+  auto solve = [&](float* X, int pitch, float* dst, int ld, bool stored0, bool stored1) {
+    for (int I = 0; I < 4; ++I) {
+      float acc[1][2][4] = {}, small[1][2][4] = {};
+      uint32_t ah[1][4], al[1][4], bh[2][2], bl[2][2];
+#pragma unroll 2
+      for (int ks = 0; ks < 2 * I; ++ks) {
+        cr_left(La + 4 * (16 * I * CR_PT + 8 * ks), CR_PT, lane, ah[0], al[0]);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) cr_right_t(X + 8 * ks * pitch + 8 * t, pitch, lane, bh[t], bl[t]);
+        cr_step<1, 2>(acc, small, ah, al, bh, bl);
+      }
+      float* mineX = X + (16 * I + (lane >> 2)) * pitch + 2 * (lane & 3);
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float* x = mineX + (e >> 1) * 8 * pitch + 8 * t + (e & 1);
+          *x -= acc[0][t][e] + small[0][t][e];
+          acc[0][t][e] = small[0][t][e] = 0.f;
+        }
+      __syncwarp();
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        cr_left(Ta + 4 * (16 * I * CR_PI + 8 * ks), CR_PI, lane, ah[0], al[0]);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) cr_right_t(X + (16 * I + 8 * ks) * pitch + 8 * t, pitch, lane, bh[t], bl[t]);
+        cr_step<1, 2>(acc, small, ah, al, bh, bl);
+      }
+      __syncwarp();
+      float* out = dst + (16 * I + (lane >> 2)) * ld + 2 * (lane & 3);
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e2 = 0; e2 < 2; ++e2) {
+          const float2 x = make_float2(acc[0][t][2 * e2] + small[0][t][2 * e2], acc[0][t][2 * e2 + 1] + small[0][t][2 * e2 + 1]);
+          *reinterpret_cast<float2*>(mineX + e2 * 8 * pitch + 8 * t) = x;
+          if (t ? stored1 : stored0) *reinterpret_cast<float2*>(out + e2 * 8 * ld + 8 * t) = x;
+        }
+      __syncwarp();
+    }
+  };
+  for (int v0 = 0; v0 < p.v_ld_s; v0 += CR_XV) {
+    if (v0 > 0) {
+      __syncthreads();
+      cr_fetch<CR_XV, PX>(Xv, vsrc + v0, p.v_ld, c.m, min(CR_XV, p.vdim - v0), p.vecv, tid);
+      cp_async_commit();
+    }
+    cp_async_wait<0>();
+    __syncthreads();                               // the inverses, w c k and the values are in place
+#pragma unroll
+    for (int i = 0; i < CR_C / 16; ++i) {          // this warp's values times w: they lie in columns that it owns
+      const int t = 16 * i + (lane >> 1);
+      if (warp < 8) { cr_scale(Xv + t * PX + 16 * warp + 8 * (lane & 1), ws[t]); cr_scale(Xv + t * PX + 16 * warp + 8 * (lane & 1) + 4, ws[t]); }
+    }
+    __syncwarp();
+    const int left = p.v_ld_s - v0;                // columns still to come, in whole tiles of eight
+    if (warp < 8) {
+      if (16 * warp < left) solve(Xv + 16 * warp, PX, oU + v0 + 16 * warp, p.v_ld_s, true, 16 * warp + 8 < left);
+    } else if (v0 == 0 && 16 * (warp - 8) < KD) {
+      solve(Ks + 16 * (warp - 8), PK, oW + 16 * (warp - 8), PK, true, true);
+    }
+  }
+}
+
+// ---- the states before the chunks of the delta rules: U = U' - W S, S <- diag(c) S + K^T U --------------------------------------
+// A CTA for every (NV value columns, head, sequence).  A chunk is two phases: the product with W (16 rows a pair of warps,
+// which share out the places summed over) and the one with K^T (16 rows a warp, whose part of the state stays in registers).
+// The right operands lie in shared memory already split.  W, K^T and U' of the next chunk are under way during both phases.
+__host__ __device__ constexpr int cr_walk_floats(int kd, int nv) {
+  return 2 * (CR_C * (kd + 4) + kd * CR_PT) + 2 * nv * (kd + 4) + 2 * nv * CR_PT + CR_C * (nv + 8);
+}
+
+template <int KD, int NV>
+__global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_constant__ ChunkParams p, int nslots) {
+  constexpr int PK = KD + 4, NT = NV / 8, MW = KD / 16, WK = CR_C * PK + KD * CR_PT;       // MW warps hold the state, 16 rows each
+  extern __shared__ __align__(16) float cr_smem[];
+  float* WK_s = cr_smem;                           // [2]: W [64][PK], K^T [KD][PT]
+  float* Sh = WK_s + 2 * WK;                       // [NV][PK] state, a column a row: high and low parts
+  float* Sl = Sh + NV * PK;
+  float* Uh = Sl + NV * PK;                        // [NV][PT]
+  float* Ul = Uh + NV * CR_PT;
+  float* Y = Ul + NV * CR_PT;                      // [64][NV + 8] the second half of the places' share of W S
+  constexpr int PY = NV + 8;
+  pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = blockIdx.y, seq = p.seq[blockIdx.z], base = p.base[blockIdx.z];
+  const int c_lo = max(0, p.slot0 - base), c_hi = min(p.base[blockIdx.z + 1], p.slot0 + nslots) - base;
+  const int col0 = blockIdx.x * NV, row = lane >> 2, cc = 2 * (lane & 3);
+  pdl_wait();
+  if (c_lo >= c_hi) return;
+  float* S = p.state + ((size_t)p.slots[seq] * p.heads + h) * p.dim * p.vdim;
+  const size_t stride = (size_t)p.heads * p.per_head;
+  float* mine = p.scratch + ((size_t)(base + c_lo - p.slot0) * p.heads + h) * p.per_head;
+  const uint32_t wk_a = (uint32_t)__cvta_generic_to_shared(WK_s);
+  const uint32_t sh_a = (uint32_t)__cvta_generic_to_shared(Sh), sl_a = (uint32_t)__cvta_generic_to_shared(Sl);
+  const uint32_t uh_a = (uint32_t)__cvta_generic_to_shared(Uh), ul_a = (uint32_t)__cvta_generic_to_shared(Ul);
+  const int r0 = (warp & 3) * 16 + row;            // a pair's token rows
+  auto fetch = [&](int buf, const float* src) {    // W and, right behind it, K^T
+    const uint32_t dst = wk_a + buf * WK * 4 + 16 * tid;
+    const float* x = src + p.off_w + 4 * tid;
+#pragma unroll
+    for (int i = 0; i < WK / 4 / CR_WALK; ++i) cp_async16(dst + i * 16 * CR_WALK, x + i * 4 * CR_WALK, true);
+    constexpr int left = WK / 4 % CR_WALK, done = WK / 4 - left;
+    if (tid < left) cp_async16(dst + done * 16, x + done * 4, true);
+    cp_async_commit();
+  };
+  float u_next[NT][4], g_next[2];
+  auto request = [&](const float* src) {
+    if (warp < 4) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e2 = 0; e2 < 2; ++e2) {
+          const int cl = col0 + nt * 8 + cc;       // v_ld_s is a multiple of eight
+          const float2 x = cl < p.v_ld_s ? *reinterpret_cast<const float2*>(src + p.off_u + (r0 + e2 * 8) * p.v_ld_s + cl) : make_float2(0.f, 0.f);
+          u_next[nt][2 * e2] = x.x; u_next[nt][2 * e2 + 1] = x.y;
+        }
+    }
+    if (warp < MW) {
+      g_next[0] = src[p.off_g + warp * 16 + row];
+      g_next[1] = src[p.off_g + warp * 16 + row + 8];
+    }
+  };
+  fetch(0, mine);
+  request(mine);
+
+  float s[NT][4];                                  // warps 0 .. MW - 1: the state at (16 warp + row + 8 (e / 2), 8 nt + cc + e % 2)
+  auto put_state = [&](float* keep) {              // split, for the next product; whole, for the outputs of the chunk it stands before
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        uint32_t hi, lo;
+        cr_split(s[nt][e], hi, lo);
+        const int at = (nt * 8 + cc + (e & 1)) * PK + warp * 16 + row + (e >> 1) * 8;
+        Sh[at] = __uint_as_float(hi);
+        Sl[at] = __uint_as_float(lo);
+      }
+      const int cl = col0 + nt * 8 + cc;
+      if (cl < p.v_ld_s) {
+#pragma unroll
+        for (int e2 = 0; e2 < 2; ++e2)
+          *reinterpret_cast<float2*>(keep + (warp * 16 + row + e2 * 8) * p.v_ld_s + cl) = make_float2(s[nt][2 * e2], s[nt][2 * e2 + 1]);
+      }
+    }
+  };
+  if (warp < MW) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int d = warp * 16 + row + (e >> 1) * 8, c = col0 + nt * 8 + cc + (e & 1);
+        s[nt][e] = (d < p.dim && c < p.vdim) ? S[(size_t)d * p.vdim + c] : 0.f;
+      }
+    put_state(mine);
+  }
+  // 16 rows of `left` times the split right operand [NV][pitch], over KSTEPS * 8 places
+  auto product = [&](uint32_t left, int pitch, uint32_t rh, uint32_t rl, auto ksteps, float (*acc)[4]) {
+    float x1[NT][4] = {}, x2[NT][4] = {};
+#pragma unroll
+    for (int ks = 0; ks < decltype(ksteps)::value; ++ks) {
+      uint32_t ah[4], al[4], bh[NT][2], bl[NT][2];
+      cr_left(left + 32 * ks, pitch, lane, ah, al);
+      if constexpr (NT == 1) {
+        const uint32_t at = 4 * ((lane & 7) * pitch + ((lane >> 3) & 1) * 4) + 32 * ks;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(bh[0][0]), "=r"(bh[0][1]) : "r"(rh + at));
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(bl[0][0]), "=r"(bl[0][1]) : "r"(rl + at));
+      } else {
+#pragma unroll
+        for (int n2 = 0; n2 < NT / 2; ++n2) {
+          cr_right2(rh + 4 * n2 * 16 * pitch + 32 * ks, pitch, lane, bh[2 * n2]);
+          cr_right2(rl + 4 * n2 * 16 * pitch + 32 * ks, pitch, lane, bl[2 * n2]);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t) mma_tf32(x1[t], al, bh[t][0], bh[t][1]);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) mma_tf32(acc[t], ah, bh[t][0], bh[t][1]);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) mma_tf32(x2[t], ah, bl[t][0], bl[t][1]);
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[nt][e] += x1[nt][e] + x2[nt][e];
+  };
+  struct HalfK { enum { value = KD / 16 }; };
+  struct Tokens { enum { value = CR_C / 8 }; };
+
+  for (int c = c_lo; c < c_hi; ++c) {
+    const int buf = (c - c_lo) & 1;
+    const uint32_t w_a = wk_a + buf * WK * 4, k_a = w_a + 4 * CR_C * PK;
+    float u[NT][4];
+    const float gam0 = g_next[0], gam1 = g_next[1];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) u[nt][e] = u_next[nt][e];
+    cp_async_wait<0>();
+    __syncthreads();                               // W and K have landed, the state is in place, the chunk before is through
+    if (c + 1 < c_hi) { fetch(buf ^ 1, mine + stride); request(mine + stride); }
+    float y[NT][4] = {};
+    const int k0 = (warp >> 2) * (KD / 2);         // this warp's half of the places
+    product(w_a + 4 * ((warp & 3) * 16 * PK + k0), PK, sh_a + 4 * k0, sl_a + 4 * k0, HalfK(), y);
+    if (warp >= 4) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e2 = 0; e2 < 2; ++e2) *reinterpret_cast<float2*>(Y + (r0 + e2 * 8) * PY + nt * 8 + cc) = make_float2(y[nt][2 * e2], y[nt][2 * e2 + 1]);
+    }
+    __syncthreads();                               // the state is read
+    if (warp < 4) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int cl = col0 + nt * 8 + cc;
+#pragma unroll
+        for (int e2 = 0; e2 < 2; ++e2) {
+          const float2 z = *reinterpret_cast<const float2*>(Y + (r0 + e2 * 8) * PY + nt * 8 + cc);
+          u[nt][2 * e2] -= y[nt][2 * e2] + z.x;
+          u[nt][2 * e2 + 1] -= y[nt][2 * e2 + 1] + z.y;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          uint32_t hi, lo;
+          cr_split(u[nt][e], hi, lo);
+          const int at = (nt * 8 + cc + (e & 1)) * CR_PT + r0 + (e >> 1) * 8;
+          Uh[at] = __uint_as_float(hi);
+          Ul[at] = __uint_as_float(lo);
+        }
+        if (cl < p.v_ld_s) {
+#pragma unroll
+          for (int e2 = 0; e2 < 2; ++e2)
+            *reinterpret_cast<float2*>(mine + p.off_u + (r0 + e2 * 8) * p.v_ld_s + cl) = make_float2(u[nt][2 * e2], u[nt][2 * e2 + 1]);
+        }
+      }
+    }
+    __syncthreads();                               // U is in place
+    mine += stride;
+    if (warp < MW) {
+      float x[NT][4] = {};
+      product(k_a + 4 * warp * 16 * CR_PT, CR_PT, uh_a, ul_a, Tokens(), x);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[nt][e] = fmaf(e < 2 ? gam0 : gam1, s[nt][e], x[nt][e]);
+      if (c + 1 < c_hi) put_state(mine);
+    }
+  }
+  if (warp < MW) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int d = warp * 16 + row + (e >> 1) * 8, c = col0 + nt * 8 + cc + (e & 1);
+        if (d < p.dim && c < p.vdim) S[(size_t)d * p.vdim + c] = s[nt][e];
+      }
+  }
+}
+
+// ---- every chunk by itself: the outputs ---------------------------------------------------------------------------------------
+// Two CTAs an SM: the state takes the place of k once the scores are formed, U that of the decays (two blocks' worth at a time).
+__host__ __device__ constexpr int cr_out_floats(int kind, int kd) {
+  const int mat = CR_C * (kd + 4), k = mat > kd * CR_PV ? mat : kd * CR_PV;
+  return mat + k + CR_C * CR_PV + CR_C * CR_PT + 3 * CR_C + (cr_rows(kind) ? 5 * kd : 0);
+}
+
+template <int KIND, int KD>
+__global__ void __launch_bounds__(CR_THREADS, 2) chunk_outputs_kernel(const __grid_constant__ ChunkParams p) {
+  constexpr int PK = KD + 4, MAT = CR_C * PK, KS = KD / 8, KBUF = MAT > KD * CR_PV ? MAT : KD * CR_PV;
+  constexpr bool ROWS = cr_rows(KIND), DELTA = cr_delta(KIND);
+  static_assert(32 * PK <= CR_C * CR_PV, "two blocks' decays lie where U does");
+  constexpr int STEP = CR_THREADS / (KD / 4);
+  extern __shared__ __align__(16) float cr_smem[];
+  float* Qs = cr_smem;                             // [64][PK]
+  float* Ks = Qs + MAT;                            // [64][PK]; then the state's columns at work [KD][PV]
+  float* Gb = Ks + KBUF;                           // a decay for every row: of two blocks [2][16][PK]; then (else from the start) U [64][PV]
+  float* As = Gb + CR_C * CR_PV;                         // [64][PT]: first G(j, i) of one decay a token
+  float* gs = As + CR_C * CR_PT;
+  float* ws = gs + CR_C;
+  float* cs = ws + CR_C;
+  float* starts = cs + CR_C;                       // [5][KD]: product of the decays before block I; [4]: over the block at work
+  float* Ss = Ks;
+  float* Us = Gb;
+  pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = blockIdx.y, grp = h / (p.heads / p.groups);
+  pdl_wait();
+  const ChunkPlace c = cr_place(p, blockIdx.x);
+  const float* mine = p.scratch + ((size_t)blockIdx.x * p.heads + h) * p.per_head;
+  const float* vsrc = p.v + (size_t)c.first * p.v_ld + (size_t)h * p.vdim;
+  cr_fetch<KD, PK>(Qs, p.q + (size_t)c.first * p.q_ld + (size_t)grp * p.dim, p.q_ld, c.m, p.dim, p.vec, tid);
+  cr_fetch<KD, PK>(Ks, p.k + (size_t)c.first * p.k_ld + (size_t)grp * p.dim, p.k_ld, c.m, p.dim, p.vec, tid);
+  cp_async_commit();
+  float gn[KD / 32], low[KD / 32], bi[KD / 32];
+  if (KIND == CR_CHANNELS) cr_request_decays<KIND, KD>(p, c, h, 0, tid, gn);
+  if (KIND == CR_HGRN2) {
+#pragma unroll
+    for (int e = 0; e < KD / 32; ++e) {
+      const int d = (tid % 32) * (KD / 32) + e;
+      low[e] = d < p.dim ? p.lower[h * p.dim + d] : 1.f;         // rows beyond dim: decay 1
+      bi[e] = d < p.dim ? p.bias[h * p.dim + d] : 0.f;
+    }
+  }
+  auto fetch_u = [&](int v0) {
+    if (DELTA) cr_fetch<CR_VT, CR_PV>(Us, mine + p.off_u + v0, p.v_ld_s, CR_C, min(CR_VT, p.v_ld_s - v0), true, tid);
+    else cr_fetch<CR_VT, CR_PV>(Us, vsrc + v0, p.v_ld, c.m, min(CR_VT, p.vdim - v0), p.vecv, tid);
+  };
+  auto fetch_s = [&](int v0) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(Ss);
+    const int r0 = tid / (CR_VT / 4), e = (tid % (CR_VT / 4)) * 4;
+    const bool real = v0 + e < p.v_ld_s;
+    const float* x = real ? mine + r0 * p.v_ld_s + v0 + e : mine;
+#pragma unroll
+    for (int i = 0; i < KD / 32; ++i) cp_async16(d + 4 * ((r0 + 32 * i) * CR_PV + e), x + (real ? 32 * i * p.v_ld_s : 0), real);
+  };
+  cr_numbers<KIND>(p, c, h, gs, ws, tid);
+  cp_async_wait<0>();
+  __syncthreads();
+  cr_form<KIND, KD, PK, true>(p, c, h, Qs, Ks, nullptr, tid);
+  if (ROWS) cr_put_decays<KIND, KD, PK>(c, 0, tid, gn, low, bi, Ks, Gb);
+  if (!ROWS) cr_products(gs, As, cs, tid);
+  else for (int i = tid; i < CR_C * CR_PT; i += CR_THREADS) As[i] = 0.f;
+  __syncthreads();
+  if (!ROWS) {
+    fetch_u(0);
+    cp_async_commit();
+  }
+  const uint32_t Qa = (uint32_t)__cvta_generic_to_shared(Qs), Ka = (uint32_t)__cvta_generic_to_shared(Ks), Aa = (uint32_t)__cvta_generic_to_shared(As);
+  if (!ROWS) {
+    cr_triangle<KS>(Qa, Ka, PK, warp, lane, [&](int r, int n, const float* s) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = 16 * r + (lane >> 2) + (e >> 1) * 8, j = 8 * n + 2 * (lane & 3) + (e & 1);
+        float* x = As + i * CR_PT + j;
+        *x = j <= i ? *x * s[e] * (KIND == CR_SSM ? ws[j] : 1.f) : 0.f;
+      }
+    });
+    __syncthreads();                               // q and k are read
+    fetch_s(0);
+    cp_async_commit();
+#pragma unroll
+    for (int i = 0; i < CR_C / STEP; ++i) {
+      const int t = tid / (KD / 4) + i * STEP;
+      cr_scale(Qs + t * PK + (tid % (KD / 4)) * 4, cs[t]);
+    }
+  } else {
+    float c_start = 1.f;                           // of this thread's channel: product of the decays before the block
+    const int ch = tid % KD;
+    for (int I = 0; I < 4; ++I) {
+      const int b0 = 16 * I;
+      const float* Gi = Gb + (I & 1) * 16 * PK;
+      if (KIND == CR_CHANNELS && I < 3) cr_request_decays<KIND, KD>(p, c, h, b0 + 16, tid, gn);
+      const int jj = b0 + warp;                    // pairs inside the block: a warp a column
+      cr_pairs<KD, PK, true>(Qs, Ks, Gi, b0, jj, lane, [&](int i, float x) { As[i * CR_PT + jj] = x; });
+      __syncthreads();                             // the block's rows as they came are read (and the keys before it moved on)
+      if (tid < KD) {
+        float g = 1.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { g *= Gi[i * PK + ch]; Qs[(b0 + i) * PK + ch] *= g; }
+        starts[I * KD + ch] = c_start;
+        starts[4 * KD + ch] = g;
+        c_start *= g;
+      }
+      if (tid >= CR_THREADS - KD) {
+        float g = 1.f;
+#pragma unroll
+        for (int i = 15; i >= 0; --i) { Ks[(b0 + i) * PK + ch] *= g; g *= Gi[i * PK + ch]; }
+      }
+      __syncthreads();
+      if (I < 3) cr_put_decays<KIND, KD, PK>(c, b0 + 16, tid, gn, low, bi, Ks, Gb + (~I & 1) * 16 * PK);
+      if (I > 0) {                                 // the block's rows against all tokens before it
+        for (int n = warp; n < 2 * I; n += CR_THREADS / 32) {
+          float acc[1][1][4] = {}, small[1][1][4] = {};
+          cr_scores<KS, 1>(Qa + 4 * b0 * PK, Ka + 4 * 8 * n * PK, PK, lane, acc, small);
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            As[(b0 + (lane >> 2) + (e >> 1) * 8) * CR_PT + 8 * n + 2 * (lane & 3) + (e & 1)] = acc[0][0][e] + small[0][0][e];
+        }
+      }
+      __syncthreads();
+      if (I > 0 && I < 3) {
+        const float g = starts[4 * KD + ch];
+        for (int j = tid / KD; j < b0; j += CR_THREADS / KD) Ks[j * PK + ch] *= g;     // the keys move on to the block's end
+      }
+    }
+    __syncthreads();                               // k and the decays are read
+    fetch_u(0);
+    fetch_s(0);
+    cp_async_commit();
+#pragma unroll
+    for (int i = 0; i < CR_C / STEP; ++i) {
+      const int t = tid / (KD / 4) + i * STEP, d = (tid % (KD / 4)) * 4;
+      float4* x = reinterpret_cast<float4*>(Qs + t * PK + d);
+      const float4 g = *reinterpret_cast<const float4*>(starts + (t / 16) * KD + d);
+      *x = make_float4(x->x * g.x, x->y * g.y, x->z * g.z, x->w * g.w);
+    }
+  }
+  const int m = warp >> 2, n0 = (warp & 3) * 2;    // a warp: 16 rows, 16 columns
+  for (int v0 = 0; v0 < p.vdim; v0 += CR_VT) {
+    if (v0 > 0) {
+      __syncthreads();
+      fetch_u(v0);
+      fetch_s(v0);
+      cp_async_commit();
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    if (KIND == CR_FIXED && p.act) {
+      cr_form_values(Us, tid);
+      __syncthreads();
+    }
+    float acc[1][2][4] = {}, small[1][2][4] = {};
+    auto add = [&](uint32_t left, int pitch, const float* right, int ksteps) {
+#pragma unroll 4
+      for (int ks = 0; ks < ksteps; ++ks) {
+        uint32_t ah[1][4], al[1][4], bh[2][2], bl[2][2];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) cr_right_t(right + 8 * ks * CR_PV + 8 * (n0 + t), CR_PV, lane, bh[t], bl[t]);
+        cr_left(left + 32 * ks, pitch, lane, ah[0], al[0]);
+        cr_step<1, 2>(acc, small, ah, al, bh, bl);
+      }
+    };
+    add(Qa + 4 * 16 * m * PK, PK, Ss, KS);
+    add(Aa + 4 * 16 * m * CR_PT, CR_PT, Us, 2 * m + 2);
+#pragma unroll
+    for (int e2 = 0; e2 < 2; ++e2) {
+      const int t = 16 * m + (lane >> 2) + 8 * e2;
+      if (t >= c.m) continue;
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const int col = v0 + 8 * (n0 + nt) + 2 * (lane & 3);
+        if (col >= p.vdim) continue;
+        float x = acc[0][nt][2 * e2] + small[0][nt][2 * e2], y = acc[0][nt][2 * e2 + 1] + small[0][nt][2 * e2 + 1];
+        if (p.D) {
+          x += p.D[h] * vsrc[(size_t)t * p.v_ld + col];
+          if (col + 1 < p.vdim) y += p.D[h] * vsrc[(size_t)t * p.v_ld + col + 1];
+        }
+        float* dst = p.out + (size_t)(c.first + t) * p.out_ld + (size_t)h * p.vdim + col;
+        if (p.vec2) *reinterpret_cast<float2*>(dst) = make_float2(x, y);
+        else { dst[0] = x; if (col + 1 < p.vdim) dst[1] = y; }
+      }
+    }
+  }
+}
+
+template <typename K>
+static cudaError_t cr_allow(K kernel, int floats) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, floats * (int)sizeof(float));
+}
+
+template <int KD, int NV>
+static cudaError_t launch_chunk_walk(const ChunkParams& p, int nslots, cudaStream_t stream) {
+  constexpr int floats = cr_walk_floats(KD, NV);
+  static const cudaError_t cfg = cr_allow(chunk_walk_kernel<KD, NV>, floats);
+  if (cfg != cudaSuccess) return cfg;
+  return launch(chunk_walk_kernel<KD, NV>, dim3((p.vdim + NV - 1) / NV, p.heads, p.num_seqs), dim3(CR_WALK), floats * sizeof(float), stream, p, nslots);
+}
+
+template <int KIND, int KD>
+static cudaError_t launch_chunks(const ChunkParams& p, int nslots, cudaStream_t stream) {
+  const dim3 grid(nslots, p.heads), block(CR_THREADS);
+  cudaError_t e;
+  if constexpr (cr_delta(KIND)) {
+    constexpr int floats = cr_solve_floats(KIND, KD);
+    static const cudaError_t cfg = cr_allow(chunk_solve_kernel<KIND, KD>, floats);
+    if (cfg != cudaSuccess) return cfg;
+    e = launch(chunk_solve_kernel<KIND, KD>, grid, block, floats * sizeof(float), stream, p);
+    if (e != cudaSuccess) return e;
+    count_launch();
+    int nv = 32;
+    while (nv > 8 && (long long)p.num_seqs * p.heads * ((p.vdim + nv - 1) / nv) < 100) nv /= 2;
+    e = nv == 32 ? launch_chunk_walk<KD, 32>(p, nslots, stream) : nv == 16 ? launch_chunk_walk<KD, 16>(p, nslots, stream)
+                                                                           : launch_chunk_walk<KD, 8>(p, nslots, stream);
+  } else {
+    constexpr int floats = cr_states_floats(KIND, KD);
+    static const cudaError_t cfg = cr_allow(chunk_states_kernel<KIND, KD>, floats);
+    if (cfg != cudaSuccess) return cfg;
+    e = launch(chunk_states_kernel<KIND, KD>, grid, block, floats * sizeof(float), stream, p);
+    if (e != cudaSuccess) return e;
+    count_launch();
+    e = launch(chunk_scan_kernel, dim3((KD * (p.v_ld_s / 4) + CR_SCAN - 1) / CR_SCAN, p.heads, p.num_seqs), dim3(CR_SCAN), 0, stream, p, nslots, KD);
+  }
+  if (e != cudaSuccess) return e;
+  count_launch();
+  constexpr int floats = cr_out_floats(KIND, KD);
+  static const cudaError_t cfg = cr_allow(chunk_outputs_kernel<KIND, KD>, floats);
+  if (cfg != cudaSuccess) return cfg;
+  return launch(chunk_outputs_kernel<KIND, KD>, grid, block, floats * sizeof(float), stream, p);
+}
+
+template <int KD>
+static cudaError_t launch_chunks_kind(int kind, const ChunkParams& p, int nslots, cudaStream_t stream) {
+  switch (kind) {
+    case CR_FIXED: return launch_chunks<CR_FIXED, KD>(p, nslots, stream);
+    case CR_SSM: return launch_chunks<CR_SSM, KD>(p, nslots, stream);
+    case CR_DELTA: return launch_chunks<CR_DELTA, KD>(p, nslots, stream);
+    case CR_HGRN2: return launch_chunks<CR_HGRN2, KD>(p, nslots, stream);
+    default: return launch_chunks<CR_CHANNELS, KD>(p, nslots, stream);
+  }
+}
+
+// floats of scratch a (chunk, head); the arrays' offsets, in whole 16-byte pieces
+static long long cr_layout(ChunkParams& p, int kind) {
+  const int kd = p.dim <= 64 ? 64 : 128;
+  p.v_ld_s = (p.vdim + 7) / 8 * 8;
+  int at = kd * p.v_ld_s;
+  p.off_w = at;
+  if (cr_delta(kind)) at += CR_C * (kd + 4);
+  p.off_k = at;
+  if (cr_delta(kind)) at += kd * CR_PT;
+  p.off_u = at;
+  if (cr_delta(kind)) at += CR_C * p.v_ld_s;
+  p.off_g = at;
+  p.per_head = at + kd;
+  return p.per_head;
+}
+
+}  // namespace lb
+
+// Floats of scratch that one chunk of 64 tokens takes (all heads); 0: sizes the kernels do not take.
+LB_EXPORT long long lb_chunk_recurrence_scratch(int kind, int heads, int dim, int vdim) {
+  if (kind < 0 || kind > lb::CR_CHANNELS || heads <= 0 || heads > 65535 || dim <= 0 || dim > 128 || vdim <= 0 || vdim > 4096) return 0;
+  lb::ChunkParams p;
+  p.dim = dim; p.vdim = vdim;
+  return lb::cr_layout(p, kind) * heads;
+}
+
+// The sequences seqs[0 .. num_long - 1] of the step (host array; with seq_tokens[i] tokens each, which must be what cu_tokens
+// says), all their tokens.  `scratch` holds scratch_chunks chunks; more are worked off in turns.  fixed: `decay`; ssm: a, A_log,
+// dt_bias, D; delta: a, b, A_log, dt_bias; hgrn2: k (the gate's input), bias, lower; channels: a (the decays), b.
+LB_EXPORT int lb_chunk_recurrence(int kind, const float* q, long long q_ld, const float* k, long long k_ld, const float* v, long long v_ld,
+                                  const float* a, long long a_ld, const float* b, long long b_ld, const float* A_log, const float* dt_bias,
+                                  const float* D, const float* bias, const float* lower, const float* decay, float* state, float* out,
+                                  long long out_ld, const int* cu_tokens, const int* slots, const int* seqs, const int* seq_tokens,
+                                  int num_long, int heads, int groups, int dim, int vdim, int unit_norm, float q_scale, float unit_eps,
+                                  int act, float* scratch, int scratch_chunks, cudaStream_t stream) {
+  LB_CHECK_ARG(lb_chunk_recurrence_scratch(kind, heads, dim, vdim) > 0, "chunk_recurrence: kind %d with %d heads of %d x %d", kind, heads, dim, vdim);
+  LB_CHECK_ARG(q && k && v && state && out && cu_tokens && slots && seqs && seq_tokens && scratch && scratch_chunks > 0, "chunk_recurrence: null argument");
+  LB_CHECK_ARG(groups > 0 && heads % groups == 0, "chunk_recurrence: %d heads are not a multiple of %d groups", heads, groups);
+  LB_CHECK_ARG(kind != lb::CR_FIXED || decay, "chunk_recurrence: no decays");
+  LB_CHECK_ARG((kind != lb::CR_SSM && kind != lb::CR_DELTA) || (a && A_log && dt_bias), "chunk_recurrence: null argument");
+  LB_CHECK_ARG(!lb::cr_delta(kind) || (a && b), "chunk_recurrence: null argument");
+  LB_CHECK_ARG(kind != lb::CR_HGRN2 || (bias && lower), "chunk_recurrence: null argument");
+  LB_CHECK_ARG(((uintptr_t)scratch & 15) == 0, "chunk_recurrence: scratch is not aligned");
+  for (int i = 0; i < num_long; ++i) LB_CHECK_ARG(seq_tokens[i] > 0, "chunk_recurrence: a sequence without tokens");
+  lb::ChunkParams p = {};
+  p.q = q; p.k = k; p.v = v; p.a = a; p.b = b; p.q_ld = q_ld; p.k_ld = k_ld; p.v_ld = v_ld; p.a_ld = a_ld; p.b_ld = b_ld;
+  p.A_log = A_log; p.dt_bias = dt_bias; p.D = D; p.bias = bias; p.lower = lower; p.decay = decay;
+  p.state = state; p.out = out; p.out_ld = out_ld; p.cu_tokens = cu_tokens; p.slots = slots;
+  p.heads = heads; p.groups = groups; p.dim = dim; p.vdim = vdim; p.unit_norm = unit_norm; p.act = act;
+  p.q_scale = q_scale; p.unit_eps = unit_eps; p.scratch = scratch;
+  auto aligned = [](const float* x, long long ld) { return (uintptr_t)x % 16 == 0 && ld % 4 == 0; };
+  p.vec = dim % 4 == 0 && aligned(q, q_ld) && aligned(k, k_ld) && (kind != lb::CR_CHANNELS || aligned(a, a_ld));
+  p.vecv = vdim % 4 == 0 && aligned(v, v_ld);
+  p.vec2 = vdim % 2 == 0 && out_ld % 2 == 0 && (uintptr_t)out % 8 == 0;
+  lb::cr_layout(p, kind);
+  for (int done = 0; done < num_long;) {
+    const int ns = num_long - done < lb::CR_SEQS ? num_long - done : lb::CR_SEQS;
+    p.num_seqs = ns;
+    p.base[0] = 0;
+    for (int i = 0; i < ns; ++i) {
+      p.seq[i] = seqs[done + i];
+      p.base[i + 1] = p.base[i] + (seq_tokens[done + i] + lb::CR_C - 1) / lb::CR_C;
+    }
+    const int total = p.base[ns], turns = (total + scratch_chunks - 1) / scratch_chunks;
+    for (int turn = 0; turn < turns; ++turn) {
+      const int lo = (int)((long long)total * turn / turns), hi = (int)((long long)total * (turn + 1) / turns);
+      p.slot0 = lo;
+      const cudaError_t e = dim <= 64 ? lb::launch_chunks_kind<64>(kind, p, hi - lo, stream) : lb::launch_chunks_kind<128>(kind, p, hi - lo, stream);
+      if (e != cudaSuccess) { lb::set_error("chunk_recurrence: %s", cudaGetErrorString(e)); return 2; }
+      LB_CHECK_LAUNCH("chunk_recurrence");
+    }
+    done += ns;
+  }
+  return 0;
+}

@@ -31,6 +31,7 @@ struct DecayRecurrenceParams {
   const int* cu_tokens; const int* slots;
   int heads, dim, vdim;
   int act;                              // 1: q, k, v pass silu; 0: they are taken as they come
+  int skip_from;                        // > 0: sequences with so many tokens or more belong to another kernel (chunk_recurrence.cu)
 };
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.f + expf(-x)); }
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(MAX_THREADS) decay_recurrence_kernel(DecayRecu
   float* st = p.state + (((size_t)p.slots[seq] * p.heads + h) * p.dim) * p.vdim;
   float s[DS];
   pdl_wait();
+  if (p.skip_from > 0 && n >= p.skip_from) return;
 #pragma unroll
   for (int i = 0; i < DS; ++i) {
     const int d = warp * DS + i;
@@ -372,7 +374,7 @@ LB_EXPORT int lb_decay_row_split(int num_seqs, int heads, int dim, int vdim, int
 LB_EXPORT int lb_decay_recurrence(const float* pre, long long ld, int q_col, int k_col, int v_col, const float* decay,
                                   float* state, float* out, const int* cu_tokens, const int* slots, int num_seqs,
                                   int heads, int dim, int vdim, int max_tokens_a_seq, int row_split, long long plane,
-                                  int act, cudaStream_t stream) {
+                                  int act, int skip_from, cudaStream_t stream) {
   LB_CHECK_ARG(pre && decay && state && out && cu_tokens && slots, "decay_recurrence: null argument");
   LB_CHECK_ARG(num_seqs >= 0 && heads > 0 && heads <= 65535 && dim > 0 && dim <= 1024 && vdim > 0 && num_seqs <= 65535,
                "decay_recurrence: bad sizes seqs=%d heads=%d dim=%d vdim=%d (dim at most 1024)", num_seqs, heads, dim, vdim);
@@ -381,6 +383,8 @@ LB_EXPORT int lb_decay_recurrence(const float* pre, long long ld, int q_col, int
   p.pre = pre; p.ld = ld; p.q_col = q_col; p.k_col = k_col; p.v_col = v_col; p.decay = decay;
   p.state = state; p.out = out; p.cu_tokens = cu_tokens; p.slots = slots; p.heads = heads; p.dim = dim; p.vdim = vdim;
   p.act = act ? 1 : 0;
+  p.skip_from = skip_from;
+  LB_CHECK_ARG(skip_from <= 0 || row_split == 0, "decay_recurrence: sequences are left out by the token-by-token kernel only");
   const bool few = max_tokens_a_seq > 0 && max_tokens_a_seq <= 4;
   cudaError_t e;
   if (row_split >= 1) {

@@ -34,6 +34,7 @@ struct GatedRecurrenceParams {
   float* out;                           // [T, heads * vdim]
   const int* cu_tokens; const int* slots;
   int heads, dim, vdim;
+  int skip_from;                        // > 0: sequences with so many tokens or more belong to another kernel (chunk_recurrence.cu)
 };
 
 __host__ __device__ inline int gr_chunk_tokens(int dimp) {
@@ -78,6 +79,7 @@ __global__ void gated_recurrence_kernel(GatedRecurrenceParams p) {
     vv[0] = vv[1] = 0.f;
   }
   pdl_wait();
+  if (p.skip_from > 0 && n >= p.skip_from) return;
   auto request = [&](int cs) {                        // the inputs of chunk cs, into registers
     const int c0 = cs * tc, cn = min(tc, n - c0);
 #pragma unroll
@@ -214,6 +216,7 @@ __global__ void __launch_bounds__(MAX_THREADS) gated_recurrence_short_kernel(Gat
   float* st = p.state + (((size_t)p.slots[seq] * p.heads + h) * p.dim) * p.vdim;
   float s[DS];
   pdl_wait();
+  if (p.skip_from > 0 && n >= p.skip_from) return;
 #pragma unroll
   for (int i = 0; i < DS; ++i) {
     const int d = warp * DS + i;
@@ -291,7 +294,7 @@ static cudaError_t launch_gated_recurrence_short(const GatedRecurrenceParams& p,
 
 LB_EXPORT int lb_gated_recurrence(const float* pre, long long ld, int q_col, int f_col, int v_col, const float* bias,
                                   const float* lower, float* state, float* out, const int* cu_tokens, const int* slots,
-                                  int num_seqs, int heads, int dim, int vdim, int max_tokens_a_seq, cudaStream_t stream) {
+                                  int num_seqs, int heads, int dim, int vdim, int max_tokens_a_seq, int skip_from, cudaStream_t stream) {
   LB_CHECK_ARG(pre && bias && lower && state && out && cu_tokens && slots, "gated_recurrence: null argument");
   LB_CHECK_ARG(num_seqs >= 0 && heads > 0 && heads <= 65535 && dim > 0 && dim <= 1024 && vdim > 0 && num_seqs <= 65535,
                "gated_recurrence: bad sizes seqs=%d heads=%d dim=%d vdim=%d (dim at most 1024)", num_seqs, heads, dim, vdim);
@@ -299,6 +302,7 @@ LB_EXPORT int lb_gated_recurrence(const float* pre, long long ld, int q_col, int
   lb::GatedRecurrenceParams p;
   p.pre = pre; p.ld = ld; p.q_col = q_col; p.f_col = f_col; p.v_col = v_col; p.bias = bias; p.lower = lower;
   p.state = state; p.out = out; p.cu_tokens = cu_tokens; p.slots = slots; p.heads = heads; p.dim = dim; p.vdim = vdim;
+  p.skip_from = skip_from;
   cudaError_t e;
   // rows of the state a warp keeps: as few as give at most 8 warps.  Heads of more than 256 rows: 32 rows a warp and
   // up to 32 warps, in the kernel without feeding warps whatever the step (the other would need more registers than a

@@ -43,6 +43,7 @@ struct StateRecurrenceParams {
   int vec;                       // q, k, v rows start on 16-byte boundaries and hold whole 16-byte pieces
   int svec;                      // so do the state's rows
   int avec;                      // with a decay for every state row: so do the rows of `a`
+  int skip_from;                 // > 0: sequences with so many tokens or more belong to another kernel (chunk_recurrence.cu)
 };
 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(SR_THREADS) state_recurrence_kernel(StateRecur
   }
   pdl_wait();
   const int first = p.cu_tokens[seq], n = p.cu_tokens[seq + 1] - first;
+  if (p.skip_from > 0 && n >= p.skip_from) return;
   float* S = p.state + ((size_t)p.slots[seq] * p.heads + h) * p.dim * p.vdim;
   const int shift = (TURN * sub) % COLS;     // a lane's column of the state's tile, turned so that a warp's lanes spread over the banks
 
@@ -338,7 +340,7 @@ LB_EXPORT int lb_state_recurrence(int delta, const float* q, long long q_ld, con
                                   const float* A_log, const float* dt_bias, const float* D, float* state, float* out,
                                   long long out_ld, const int* cu_tokens, const int* slots, int num_seqs, int heads, int groups,
                                   int dim, int vdim, int unit_norm, float q_scale, float unit_eps, int single_tokens, int rows_decay,
-                                  int wide_lanes, cudaStream_t stream) {
+                                  int wide_lanes, int skip_from, cudaStream_t stream) {
   LB_CHECK_ARG(!rows_decay || delta, "state_recurrence: a decay for every state row comes with the delta rule");
   LB_CHECK_ARG(q && k && v && a && A_log && dt_bias && state && out && cu_tokens && slots && (!delta || b),
                "state_recurrence: null argument");
@@ -350,7 +352,7 @@ LB_EXPORT int lb_state_recurrence(int delta, const float* q, long long q_ld, con
   p.q = q; p.k = k; p.v = v; p.a = a; p.b = b; p.q_ld = q_ld; p.k_ld = k_ld; p.v_ld = v_ld; p.a_ld = a_ld; p.b_ld = b_ld;
   p.A_log = A_log; p.dt_bias = dt_bias; p.D = D; p.state = state; p.out = out; p.out_ld = out_ld;
   p.cu_tokens = cu_tokens; p.slots = slots; p.heads = heads; p.groups = groups; p.dim = dim; p.vdim = vdim;
-  p.unit_norm = unit_norm; p.q_scale = q_scale; p.unit_eps = unit_eps;
+  p.unit_norm = unit_norm; p.q_scale = q_scale; p.unit_eps = unit_eps; p.skip_from = skip_from;
   auto aligned = [](const float* x, long long ld) { return ((uintptr_t)x % 16 == 0) && ld % 4 == 0; };
   p.vec = dim % 4 == 0 && vdim % 4 == 0 && aligned(q, q_ld) && aligned(k, k_ld) && aligned(v, v_ld);
   p.svec = vdim % 4 == 0 && (uintptr_t)state % 16 == 0;

@@ -40,7 +40,7 @@ _SIGNATURES = {
                          c_int, c_int, c_void_p],
     "lb_round_copy": [c_void_p, c_int, c_void_p, c_longlong, c_void_p],
     "lb_decay_recurrence": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                            c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_int, c_void_p],
+                            c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_int, c_int, c_void_p],
     "lb_rmsnorm_gated": [c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_float, c_float, c_int, c_int,
                          c_int, c_longlong, c_void_p],
     "lb_head_gate": [c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_longlong, c_float, c_int, c_int, c_int, c_void_p],
@@ -67,7 +67,7 @@ _SIGNATURES = {
     "lb_latent_norm": [c_int, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                        c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
     "lb_gated_recurrence": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                            c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                            c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "lb_gemm_heads_mma": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                           c_longlong, c_longlong, c_void_p, c_longlong, c_int, c_void_p],
     "lb_gemm_plain_batched": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_longlong,
@@ -87,7 +87,9 @@ _SIGNATURES = {
     "lb_short_conv_state": [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "lb_state_recurrence": [c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
                             c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
-                            c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_int, c_int, c_void_p],
+                            c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_int, c_int, c_int, c_void_p],
+    "lb_chunk_recurrence": [c_int] + [c_void_p, c_longlong] * 5 + [c_void_p] * 8 + [c_longlong] + [c_void_p] * 4
+                           + [c_int] * 6 + [c_float, c_float, c_int, c_void_p, c_int, c_void_p],
     "lb_channel_decay": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "lb_gated_group_norm": [c_void_p, c_int, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_int,
                             c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_longlong, c_void_p],
@@ -269,18 +271,26 @@ def latent_norm(pre: torch.Tensor, q_col: int, kv_col: int, q_rank: int, kv_rank
 
 def gated_recurrence(pre: torch.Tensor, q_col: int, f_col: int, v_col: int, bias: torch.Tensor, lower: torch.Tensor,
                      state: torch.Tensor, out: torch.Tensor, step, heads: int, dim: int, vdim: int, stream: int,
-                     max_tokens_a_seq: int = 0) -> None:
+                     max_tokens_a_seq: int = 0, by_shape: bool = False) -> None:
     """The HGRN2 recurrence over this step's tokens: per head S <- diag(f) S + (1 - f) v^T, out = S^T q with
     q = silu(pre[:, q_col..]), f = lower + (1 - lower) sigmoid(pre[:, f_col..] + bias), v = pre[:, v_col..];
     state [slots + 1, heads, dim, vdim] float32 is read and written at each sequence's slot; out [T, heads * vdim] float32.
     `max_tokens_a_seq`: the most tokens any sequence brings, if the host knows it (0: unknown); steps of a few tokens a
-    sequence run in a kernel made for them, with the same sums in the same order."""
+    sequence run in a kernel made for them, with the same sums in the same order.  `by_shape`: long portions go through the
+    chunked form (chunk_portions), which adds in another order."""
     _check(pre, "input projections", torch.float32); _check(bias, "gate bias", torch.float32)
     _check(lower, "lower bound", torch.float32); _check(state, "recurrent state", torch.float32)
     _check(out, "recurrence output", torch.float32)
+    long, skip = chunk_portions("hgrn2", step, heads, dim, vdim) if by_shape else ([], 0)
+    if long:
+        n, m = heads * dim, heads * vdim
+        _chunk_recurrence("hgrn2", pre[:, q_col:q_col + n], pre[:, f_col:f_col + n], pre[:, v_col:v_col + m], state, out, step, long, heads, heads, dim,
+                          vdim, stream, bias=bias, lower=lower)
+        if len(long) == step.num_seqs:
+            return
     _call("lb_gated_recurrence", pre.data_ptr(), pre.stride(0), q_col, f_col, v_col, bias.data_ptr(), lower.data_ptr(),
           state.data_ptr(), out.data_ptr(), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), step.num_seqs,
-          heads, dim, vdim, max_tokens_a_seq, stream)
+          heads, dim, vdim, max_tokens_a_seq, skip, stream)
 
 
 def gemm_heads(y: torch.Tensor, x: torch.Tensor, w: torch.Tensor, stream: int, gate: torch.Tensor | None = None) -> None:
@@ -574,6 +584,46 @@ def short_conv_state(state: torch.Tensor, x: torch.Tensor, taps: int, step, stre
           step.state_slots.data_ptr(), step.num_seqs, x.shape[1], taps, stream)
 
 
+# From how many tokens a sequence's recurrence goes through the chunked form (csrc/chunk_recurrence.cu): the walk token by token
+# costs its tokens times the rounds its CTAs need, the chunked form three launches of about 15 us and little a chunk.  Measured
+# (B200, heads of 128 x 128, us token by token / chunked; one sequence and 16 heads | four and 32): fixed decays 192 tokens 43 / 46 |
+# 64 tokens 73 / 60; state space 192: 31 / 29 | 96: 41 / 38; HGRN2 256: 53 / 57 | 128: 112 / 73; delta rule 128: 60 / 56 | 64: 80 / 74;
+# channel decays 192: 90 / 86 | 64: 124 / 98.
+CHUNK_FROM = {"fixed": 240, "ssm": 240, "hgrn2": 420, "delta": 160, "channels": 230}
+CHUNK_LEAST = 32
+# Scratch of the chunked form, in floats: more chunks are worked off in turns.
+CHUNK_SCRATCH = 32 << 20
+_CHUNK_KINDS = {"fixed": 0, "ssm": 1, "delta": 2, "hgrn2": 3, "channels": 4}
+
+
+def chunk_portions(kind: str, step, heads: int, dim: int, vdim: int) -> tuple[list[int], int]:
+    """The sequences of a step whose recurrence goes 64 tokens at a time, by the lengths the host knows, and from how many
+    tokens on they do (0: none does); states of up to 128 rows."""
+    if dim > 128 or vdim > 4096 or len(step.q_lens) != step.num_seqs or step.max_q_len < CHUNK_LEAST:
+        return [], 0
+    candidates = [i for i, n in enumerate(step.q_lens) if n >= CHUNK_LEAST]
+    start = max(CHUNK_LEAST, int(CHUNK_FROM[kind] / (1.0 + len(candidates) * heads / 64.0)))
+    long = [i for i in candidates if step.q_lens[i] >= start]
+    return long, start if long else 0
+
+
+def _chunk_recurrence(kind: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, out: torch.Tensor, step, long: list[int],
+                      heads: int, groups: int, dim: int, vdim: int, stream: int, a=None, b=None, A_log=None, dt_bias=None, D=None, bias=None,
+                      lower=None, decay=None, unit_norm: bool = False, q_scale: float = 1.0, unit_eps: float = 1e-6, act: bool = False) -> None:
+    """The sequences `long` of the step, all their tokens; operands as the callers have checked them."""
+    lib = library()
+    lib.lb_chunk_recurrence_scratch.argtypes, lib.lb_chunk_recurrence_scratch.restype = [c_int] * 4, c_longlong
+    code, n = _CHUNK_KINDS[kind], len(long)
+    lens = [step.q_lens[i] for i in long]
+    one = int(lib.lb_chunk_recurrence_scratch(code, heads, dim, vdim))
+    chunks = max(1, min(sum(-(-t // 64) for t in lens), CHUNK_SCRATCH // max(one, 1)))
+    scratch = torch.empty(chunks * one, dtype=torch.float32, device=q.device)
+    rows = lambda t: (t.data_ptr(), t.stride(0)) if t is not None else (None, 0)
+    _call("lb_chunk_recurrence", code, *rows(q), *rows(k), *rows(v), *rows(a), *rows(b), _ptr(A_log), _ptr(dt_bias), _ptr(D), _ptr(bias), _ptr(lower),
+          _ptr(decay), state.data_ptr(), out.data_ptr(), out.stride(0), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), (c_int * n)(*long),
+          (c_int * n)(*lens), n, heads, groups, dim, vdim, 1 if unit_norm else 0, q_scale, unit_eps, 1 if act else 0, scratch.data_ptr(), chunks, stream)
+
+
 def state_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tensor, b: torch.Tensor | None,
                      A_log: torch.Tensor, dt_bias: torch.Tensor, D: torch.Tensor | None, state: torch.Tensor, out: torch.Tensor,
                      step, heads: int, groups: int, dim: int, vdim: int, stream: int, delta: bool, unit_norm: bool = False,
@@ -587,7 +637,8 @@ def state_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
     form them again on the path from token to token).  `by_shape`: the kernel's layout may follow the step's shape (steps of
     single tokens keep sixteen state rows a lane, which issues fewer instructions; all others eight, which shortens the path
     from token to token); a column's terms are then added in an order that depends on the step.  Without it one layout
-    serves every step, so a 32-bit result does not depend on how a sequence was cut."""
+    serves every step, so a 32-bit result does not depend on how a sequence was cut.  Long portions then go through the
+    chunked form (chunk_portions)."""
     for t, w in ((q, "q"), (k, "k"), (v, "v"), (a, "a")) + (((b, "b"),) if b is not None else ()):
         _rows32(t, w)
     _rows32(out, "recurrence output")
@@ -601,11 +652,19 @@ def state_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
         raise KernelError("the recurrence's operands do not fit its head counts and sizes")
     if rows_decay:
         _call("lb_channel_decay", a.data_ptr(), a.stride(0), A_log.data_ptr(), dt_bias.data_ptr(), T, heads, dim, stream)
+    kind = "channels" if rows_decay else "delta" if delta else "ssm"
+    long, skip = chunk_portions(kind, step, heads, dim, vdim) if by_shape else ([], 0)
+    if long:
+        _chunk_recurrence(kind, q, k, v, state, out, step, long, heads, groups, dim, vdim, stream,
+                          a=a, b=b, A_log=A_log, dt_bias=dt_bias, D=D, unit_norm=unit_norm, q_scale=q_scale, unit_eps=unit_eps)
+        if len(long) == step.num_seqs:
+            return
     _call("lb_state_recurrence", 1 if delta else 0, q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
           a.data_ptr(), a.stride(0), _ptr(b), b.stride(0) if b is not None else 0, A_log.data_ptr(), dt_bias.data_ptr(), _ptr(D),
           state.data_ptr(), out.data_ptr(), out.stride(0), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), step.num_seqs,
           heads, groups, dim, vdim, 1 if unit_norm else 0, q_scale, unit_eps, 1 if T == step.num_seqs else 0, 1 if rows_decay else 0,
-          1 if (by_shape and (T == step.num_seqs or _recurrence_fills_sms(step.num_seqs, heads, dim, vdim))) else 0, stream)
+          1 if (by_shape and (T == step.num_seqs or _recurrence_fills_sms(step.num_seqs, heads, dim, vdim))) else 0,
+          skip, stream)
 
 
 def _recurrence_fills_sms(num_seqs: int, heads: int, dim: int, vdim: int, sms: int = 148) -> bool:
@@ -954,23 +1013,31 @@ def decay_row_split(num_seqs: int, heads: int, dim: int, vdim: int, max_tokens_a
 
 def decay_recurrence(pre: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.Tensor, state: torch.Tensor,
                      out: torch.Tensor, step, heads: int, dim: int, vdim: int, stream: int, max_tokens_a_seq: int = 0,
-                     row_split: int = 0, act: bool = True) -> None:
+                     row_split: int = 0, act: bool = True, by_shape: bool = False) -> None:
     """Linear attention with a fixed decay per head over this step's tokens: S <- decay_h S + k v^T, out = S^T q with
     q, k, v = silu of the columns of `pre` (float32, row-strided) at q_col, k_col, v_col (act=False: the columns as they are); state [slots + 1, heads, dim, vdim]
     float32 is read and written at each sequence's slot; out [T, heads * vdim] float32.
     `row_split` >= 1 (see decay_row_split): the outputs of 16 tokens at a time are formed from the state before them
     and the tokens' own scores (32-bit, outputs equal within rounding, several times faster), the state's rows shared out
     over row_split CTAs; out is then [row_split, T, heads * vdim] and the sum over its first dimension is meant.
-    With 0 every output's sum has one order however the sequence is cut."""
+    With 0 every output's sum has one order however the sequence is cut, unless `by_shape` sends long portions through the
+    chunked form (chunk_portions)."""
     _check(decay, "decay", torch.float32); _check(state, "recurrent state", torch.float32); _check(out, "recurrence output", torch.float32)
     if pre.dtype != torch.float32 or pre.stride(1) != 1 or not pre.is_cuda:
         raise KernelError("the input projections must be float32 on the GPU with unit column stride")
     T = pre.shape[0]
     if tuple(out.shape) != ((row_split, T, heads * vdim) if row_split >= 1 else (T, heads * vdim)):
         raise KernelError(f"the recurrence's output has the wrong shape {tuple(out.shape)}")
+    long, skip = chunk_portions("fixed", step, heads, dim, vdim) if by_shape and row_split == 0 else ([], 0)
+    if long:
+        n, m = heads * dim, heads * vdim
+        _chunk_recurrence("fixed", pre[:, q_col:q_col + n], pre[:, k_col:k_col + n], pre[:, v_col:v_col + m], state, out, step, long, heads, heads, dim,
+                          vdim, stream, decay=decay, act=act)
+        if len(long) == step.num_seqs:
+            return
     _call("lb_decay_recurrence", pre.data_ptr(), pre.stride(0), q_col, k_col, v_col, decay.data_ptr(), state.data_ptr(),
           out.data_ptr(), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), step.num_seqs, heads, dim, vdim,
-          max_tokens_a_seq, row_split, T * heads * vdim, 1 if act else 0, stream)
+          max_tokens_a_seq, row_split, T * heads * vdim, 1 if act else 0, skip, stream)
 
 
 def rmsnorm_gated(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, gate: torch.Tensor, scale: float, eps: float,

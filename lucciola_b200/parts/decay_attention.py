@@ -7,9 +7,9 @@
 The state is 32-bit, one slot a request, zero for a new request, and is all this mixer keeps of the past: prompts,
 portions and decoded tokens go through the same kernel, which walks a sequence's tokens of the step in order from the
 state the step before left.  W_q | W_k | W_v | W_g are one product with 32-bit output; the activations, the recurrence,
-the norm and the gate are computed in 32-bit.  In the bfloat16 engine steps with many tokens a sequence form the
-outputs of 16 tokens side by side (still 32-bit, the same state); the 32-bit engine walks every step token by token,
-so its results do not depend on how a prompt was cut.
+the norm and the gate are computed in 32-bit.  The bfloat16 engine takes long portions 64 tokens at a time and forms the
+outputs of shorter ones side by side (still 32-bit, the same state within rounding); the 32-bit engine walks every step
+token by token, so its results do not depend on how a prompt was cut.
 
 The form is a parameter, so that a relative of the design above can use the same part and kernels ("retention"):
 `act` ("silu", or None: q, k, v as projected), `position_encoding` (q and k are rotated in 32-bit, in place, after the
@@ -96,11 +96,13 @@ class DecayLinearAttention(Mixer):
             inv_freq, rot = self.position_encoding.rotary_table() if self.position_encoding is not None else (None, 0)
             ops.rotate_rows(pre, step.positions, inv_freq, self.dim, rot, [(0, self.heads, 1.0), (n, self.heads, self.k_scale)], rt.stream,
                             rot_scale=getattr(self.position_encoding, "magnitude", 1.0))
-        # the bfloat16 engine forms the outputs of long steps 16 tokens at a time, the rows of the state shared out over CTAs
-        split = ops.decay_row_split(step.num_seqs, self.heads, self.dim, self.vdim, step.max_q_len) if rt.fast_kernels else 0
+        # the bfloat16 engine takes long portions 64 tokens at a time; where there are none, it forms the outputs of up to 16
+        # tokens side by side, the rows of the state shared out over CTAs
+        chunked = rt.fast_kernels and bool(ops.chunk_portions("fixed", step, self.heads, self.dim, self.vdim)[0])
+        split = ops.decay_row_split(step.num_seqs, self.heads, self.dim, self.vdim, step.max_q_len) if rt.fast_kernels and not chunked else 0
         o = rt.empty((split, T, self.inner_size) if split else (T, self.inner_size), torch.float32)
         ops.decay_recurrence(pre, 0, n, 2 * n, self.decay, cache.state, o, step, self.heads, self.dim, self.vdim, rt.stream,
-                             max_tokens_a_seq=step.max_q_len, row_split=split, act=self.act is not None)
+                             max_tokens_a_seq=step.max_q_len, row_split=split, act=self.act is not None, by_shape=chunked)
         g0 = 2 * n + self.inner_size
         if self.head_norm or not self.norm_weight or self.gate_act != "sigmoid":
             ops.gated_group_norm(out, o, pre[:, g0:g0 + self.inner_size], self.norm_w, self.heads if self.head_norm else 1, self.eps,

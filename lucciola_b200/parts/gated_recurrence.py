@@ -7,7 +7,8 @@
 The state is 32-bit, one slot a request, zero for a new request, and is all this mixer keeps of the past:
 prompts, portions and decoded tokens go through the same kernel, which walks a sequence's tokens of the
 step in order from the state the step before left.  W_q | W_f | W_v are one product with 32-bit output; the
-gates, the recurrence and the output are computed in 32-bit.
+gates, the recurrence and the output are computed in 32-bit.  The bfloat16 engine takes long portions 64 tokens at a time
+(still 32-bit, the same state within rounding).
 """
 from __future__ import annotations
 
@@ -56,7 +57,7 @@ class GatedLinearRecurrence(Mixer):
         pre = self.qfv.forward(u, out_dtype=torch.float32)                    # [T, 2 * H * dim + H * vdim]
         o = rt.empty((T, H * self.vdim), torch.float32)
         ops.gated_recurrence(pre, 0, n, 2 * n, self.bias, self.lower, cache.state, o, step, H, self.dim, self.vdim, rt.stream,
-                             max_tokens_a_seq=step.max_q_len)
+                             max_tokens_a_seq=step.max_q_len, by_shape=rt.fast_kernels)
         normed = rt.empty((T * H, self.vdim))
         ops.add_rmsnorm(normed, o.view(T * H, self.vdim), None, self.norm_w, self.eps, rt.stream)
         return self.o.forward(normed.view(T, H * self.vdim))

@@ -1,0 +1,166 @@
+"""Long portions of the linear recurrences, 64 tokens at a time, against the plain recurrence in 64 bits and against the
+token-by-token kernels: every kind, portions around the edges of a block, a chunk and several, sizes that fill no tile, inputs
+that are column ranges, portions beside single tokens, and scratch for fewer chunks than there are (GPU)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def step_of(lens, slots):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    return SimpleNamespace(num_seqs=len(lens), cu_tokens=i32(cu), state_slots=i32(slots), q_lens=list(lens), max_q_len=max(lens))
+
+
+def columns(x):
+    """The same values as a column range of a wider matrix whose rows start on no 16-byte boundary."""
+    return torch.cat([torch.zeros(x.shape[0], 3, device=DEV), x, torch.zeros(x.shape[0], 2, device=DEV)], dim=1)[:, 3:3 + x.shape[1]]
+
+
+def operands(kind, T, heads, groups, dim, vdim):
+    rnd = lambda *s: torch.randn(*s, device=DEV)
+    o = dict(v=rnd(T, heads * vdim))
+    if kind == "fixed":
+        o.update(q=rnd(T, heads * dim), k=rnd(T, heads * dim), decay=torch.tensor([0.999, 0.5, 1.0, 0.97, 0.9, 0.0][:heads], device=DEV))
+    elif kind == "hgrn2":
+        o.update(q=rnd(T, heads * dim), k=2 * rnd(T, heads * dim), bias=rnd(heads * dim), lower=torch.rand(heads * dim, device=DEV))
+        o["lower"][::3] = 0.0
+        o["bias"][::5] = -30.0                                    # gates of next to nothing: products that leave the range of 32 bits
+    else:
+        o.update(q=rnd(T, groups * dim), k=rnd(T, groups * dim), a=rnd(T, heads), b=rnd(T, heads), A_log=torch.rand(heads, device=DEV) * 2,
+                 dt_bias=rnd(heads) - 2)
+        if kind == "ssm":
+            o.update(D=rnd(heads), b=None)
+        if kind == "channels":
+            o.update(a=3 * rnd(T, heads * dim), dt_bias=rnd(heads * dim) - 2)
+    return o
+
+
+def through_ops(kind, o, state, step, heads, groups, dim, vdim, by_shape):
+    from lucciola_b200 import ops
+    s = torch.cuda.current_stream().cuda_stream
+    T = o["v"].shape[0]
+    out = torch.full((T, heads * vdim), float("nan"), device=DEV)
+    n, m = heads * dim, heads * vdim
+    if kind == "fixed":
+        pre = columns(torch.cat([o["q"], o["k"], o["v"]], dim=1)) if vdim % 2 else torch.cat([o["q"], o["k"], o["v"]], dim=1)
+        ops.decay_recurrence(pre, 0, n, 2 * n, o["decay"], state, out, step, heads, dim, vdim, s, by_shape=by_shape)
+    elif kind == "hgrn2":
+        pre = torch.cat([o["q"], o["k"], o["v"]], dim=1)
+        ops.gated_recurrence(pre, 0, n, 2 * n, o["bias"], o["lower"], state, out, step, heads, dim, vdim, s, by_shape=by_shape)
+    else:
+        delta = kind != "ssm"
+        ops.state_recurrence(columns(o["q"]), o["k"], columns(o["v"]), o["a"].clone(), o["b"], o["A_log"], o["dt_bias"], o.get("D"), state, out, step, heads,
+                             groups, dim, vdim, s, delta=delta, unit_norm=delta, q_scale=dim ** -0.5 if delta else 1.0, rows_decay=kind == "channels",
+                             by_shape=by_shape)
+    return out
+
+
+def plain(kind, o, state, step, heads, groups, dim, vdim):
+    d = {k: (t.double() if t is not None else None) for k, t in o.items()}
+    T, silu, soft = d["v"].shape[0], torch.nn.functional.silu, torch.nn.functional.softplus
+    v = d["v"].view(T, heads, 1, vdim)
+    q, k = (d[x].view(T, -1, dim) for x in "qk")
+    g, w = torch.ones(T, heads, 1, 1, dtype=torch.float64, device=DEV), torch.ones(T, heads, 1, dtype=torch.float64, device=DEV)
+    if kind == "fixed":
+        q, k, v = silu(q), silu(k), silu(v)
+        g = g * d["decay"][:, None, None]
+    elif kind == "hgrn2":
+        low = d["lower"].view(heads, dim)
+        q, f = silu(q), low + (1 - low) * torch.sigmoid(k + d["bias"].view(heads, dim))
+        g, k = f[..., None], 1 - f
+    else:
+        x = soft(d["a"] + d["dt_bias"])
+        if kind == "channels":
+            g = torch.exp(-torch.exp(d["A_log"])[:, None] * x.view(T, heads, dim))[..., None]
+        else:
+            g = torch.exp(-torch.exp(d["A_log"]) * x)[..., None, None]
+        if kind == "ssm":
+            w = x[..., None]
+        else:
+            q, k = (y / torch.sqrt((y * y).sum(-1, keepdim=True) + 1e-6) for y in (q, k))
+            q, w = q * dim ** -0.5, torch.sigmoid(d["b"])[..., None]
+        q, k = (y.repeat_interleave(heads // groups, 1) for y in (q, k))
+    out, S, at = [], state.double().clone(), 0
+    for i, n in enumerate(step.q_lens):
+        slot = int(step.state_slots[i])
+        for t in range(at, at + n):
+            X = g[t] * S[slot]
+            seen = (X * k[t][..., None]).sum(1) if kind in ("delta", "channels") else 0.0
+            X = X + k[t][..., None] * (w[t] * (v[t, :, 0] - seen))[:, None]
+            S[slot] = X
+            y = (X * q[t][..., None]).sum(1)
+            out.append(y + d["D"][:, None] * v[t, :, 0] if kind == "ssm" else y)
+        at += n
+    return torch.stack(out).reshape(T, -1), S
+
+
+@pytest.fixture(autouse=True)
+def from_32_tokens(monkeypatch):
+    from lucciola_b200 import ops
+    monkeypatch.setattr(ops, "CHUNK_FROM", {k: 0 for k in ops.CHUNK_FROM})
+
+
+@pytest.mark.parametrize("heads,groups,dim,vdim,lens", [
+    (2, 1, 128, 128, [64]), (3, 3, 128, 128, [63, 65]), (2, 2, 64, 64, [32, 200]), (4, 2, 20, 40, [33, 1, 129]), (2, 1, 72, 33, [1, 2, 47, 130, 31]),
+    (1, 1, 128, 8, [256]), (6, 3, 100, 72, [300]), (5, 5, 8, 6, [80])])
+@pytest.mark.parametrize("kind", ["fixed", "ssm", "hgrn2", "delta", "channels"])
+def test_long_portions(kind, heads, groups, dim, vdim, lens):
+    """Outputs and states within 1e-5 of their largest value: a few hundred terms of 2^-24 relative error each, as for the
+    kernels that walk token by token; rows of the state that belong to nobody stay as they are."""
+    torch.manual_seed(3)
+    o = operands(kind, sum(lens), heads, groups, dim, vdim)
+    slots = list(range(len(lens), 0, -1))
+    step = step_of(lens, slots)
+    state = 0.3 * torch.randn(len(lens) + 2, heads, dim, vdim, device=DEV)
+    state[0] = state[-1] = float("nan")
+    want, S = plain(kind, o, state, step, heads, groups, dim, vdim)
+    for by_shape in (True, False):
+        got_state = state.clone()
+        got = through_ops(kind, o, got_state, step, heads, groups, dim, vdim, by_shape)
+        assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max(), by_shape
+        live = got_state[1:-1].double()
+        assert (live - S[1:-1]).abs().max() <= 1e-5 * S[1:-1].abs().max(), by_shape
+        assert torch.isnan(got_state[0]).all() and torch.isnan(got_state[-1]).all()
+
+
+@pytest.mark.parametrize("kind", ["fixed", "delta", "channels"])
+def test_scratch_for_fewer_chunks_and_more_sequences_than_a_launch(kind, monkeypatch):
+    """The chunks of three sequences in turns of two, the same bits as in one; more than 64 long sequences in a step."""
+    from lucciola_b200 import ops
+    heads, dim, vdim, lens = 2, 64, 40, [150, 64, 90]
+    torch.manual_seed(4)
+    o = operands(kind, sum(lens), heads, heads, dim, vdim)
+    state = torch.randn(5, heads, dim, vdim, device=DEV)
+    step = step_of(lens, [2, 0, 3])
+    whole_state = state.clone()
+    whole = through_ops(kind, o, whole_state, step, heads, heads, dim, vdim, True)
+    one = ops.library().lb_chunk_recurrence_scratch(ops._CHUNK_KINDS[kind], heads, dim, vdim)
+    monkeypatch.setattr(ops, "CHUNK_SCRATCH", 2 * one + 1)
+    turned = through_ops(kind, o, state, step, heads, heads, dim, vdim, True)
+    assert torch.equal(turned, whole) and torch.equal(state, whole_state)
+    lens = [32 + i % 3 for i in range(70)]
+    o = operands(kind, sum(lens), heads, heads, dim, vdim)
+    step = step_of(lens, list(range(70)))
+    state = torch.randn(71, heads, dim, vdim, device=DEV)
+    want, S = plain(kind, o, state, step, heads, heads, dim, vdim)
+    got = through_ops(kind, o, state, step, heads, heads, dim, vdim, True)
+    assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max() and (state.double() - S).abs().max() <= 1e-5 * S.abs().max()
+
+
+def test_which_portions_are_long(monkeypatch):
+    from lucciola_b200 import ops
+    monkeypatch.undo()
+    step = lambda *lens: SimpleNamespace(num_seqs=len(lens), q_lens=list(lens), max_q_len=max(lens))
+    first = int(ops.CHUNK_FROM["delta"] / (1 + 2 / 64))
+    assert ops.chunk_portions("delta", step(1, first, 31), 2, 128, 64) == ([1], first)
+    assert ops.chunk_portions("delta", step(1, first - 1, 31), 2, 128, 64) == ([], 0)
+    assert ops.chunk_portions("delta", step(32, 40, 31), 4096, 128, 64) == ([0, 1], 32)
+    assert ops.chunk_portions("delta", step(9999), 2, 129, 64) == ([], 0)                # more rows of the state than the kernels hold
+    assert ops.chunk_portions("delta", SimpleNamespace(num_seqs=3, q_lens=[], max_q_len=9999), 2, 64, 64) == ([], 0)      # lengths the host does not know
