@@ -340,6 +340,51 @@ __global__ void rmsnorm_gated_kernel(TO* __restrict__ out, long long out_ld, con
     o[j] = from_f32<TO>(value(j) * inv * weight[j] * (1.f / (1.f + expf(-g[j]))) * scale);
 }
 
+// The same for rows in whole 16-byte words, NV of them a thread, kept in registers between the sum and the output.
+template <typename TO, int NV>
+__global__ void __launch_bounds__(1024) rmsnorm_gated_x4_kernel(TO* __restrict__ out, long long out_ld, const float* __restrict__ x,
+                                                                const float* __restrict__ weight, const float* __restrict__ gate, long long gate_ld,
+                                                                float scale, float eps, int n, int planes, long long plane) {
+  __shared__ float scratch[33];
+  pdl_trigger();
+  pdl_wait();
+  const float* r = x + (size_t)blockIdx.x * n;
+  const float* g = gate + (size_t)blockIdx.x * gate_ld;
+  float4 v[NV], z[NV];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (threadIdx.x + i * blockDim.x) * 4;
+    v[i] = z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < n) {
+      v[i] = *reinterpret_cast<const float4*>(r + c);
+      z[i] = *reinterpret_cast<const float4*>(g + c);
+      for (int q = 1; q < planes; ++q) {
+        const float4 d = *reinterpret_cast<const float4*>(r + (size_t)q * plane + c);
+        v[i].x += d.x; v[i].y += d.y; v[i].z += d.z; v[i].w += d.w;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+  const float inv = rsqrtf(block_sum(ss, scratch) / (float)n + eps) * scale;
+  TO* o = out + (size_t)blockIdx.x * out_ld;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (threadIdx.x + i * blockDim.x) * 4;
+    if (c >= n) continue;
+    const float4 w = *reinterpret_cast<const float4*>(weight + c);
+    const float y[4] = {v[i].x * inv * w.x * (1.f / (1.f + expf(-z[i].x))), v[i].y * inv * w.y * (1.f / (1.f + expf(-z[i].y))),
+                        v[i].z * inv * w.z * (1.f / (1.f + expf(-z[i].z))), v[i].w * inv * w.w * (1.f / (1.f + expf(-z[i].w)))};
+    if constexpr (sizeof(TO) == 2) {
+      __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]), hi = __floats2bfloat162_rn(y[2], y[3]);
+      *reinterpret_cast<uint2*>(o + c) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    } else {
+      *reinterpret_cast<float4*>(o + c) = make_float4(y[0], y[1], y[2], y[3]);
+    }
+  }
+}
+
 // out[t, h, :] = x[t, h, :] * sigmoid(gate[t, h]) * scale: one number a head
 template <typename T>
 __global__ void head_gate_kernel(T* __restrict__ out, long long out_ld, const T* __restrict__ x, const float* __restrict__ gate,
@@ -425,6 +470,18 @@ LB_EXPORT int lb_rmsnorm_gated(void* out, int out_dtype, long long out_ld, const
   LB_CHECK_ARG(num_rows >= 0 && n > 0 && out_ld >= n && gate_ld >= n, "rmsnorm_gated: bad sizes rows=%d n=%d", num_rows, n);
   if (num_rows == 0) return 0;
   const int threads = n >= 2048 ? 512 : (n >= 512 ? 256 : 128);
+  const uintptr_t low = (uintptr_t)x | (uintptr_t)weight | (uintptr_t)gate;
+  const int nv = (n + 4 * threads - 1) / (4 * threads);
+  // one pass in 16-byte words (1654 rows of 2048: 16.6 us four bytes at a time and twice, 10.8 us here)
+  if (n % 4 == 0 && low % 16 == 0 && (uintptr_t)out % (out_dtype == LB_BF16 ? 8 : 16) == 0 && gate_ld % 4 == 0 && out_ld % 4 == 0 && plane % 4 == 0 && nv <= 4) {
+    LB_DISPATCH_DTYPE(out_dtype, TO, {
+      if (nv == 1) lb::launch(lb::rmsnorm_gated_x4_kernel<TO, 1>, dim3(num_rows), dim3(threads), 0, stream, (TO*)out, out_ld, x, weight, gate, gate_ld, scale, eps, n, planes, plane);
+      else if (nv == 2) lb::launch(lb::rmsnorm_gated_x4_kernel<TO, 2>, dim3(num_rows), dim3(threads), 0, stream, (TO*)out, out_ld, x, weight, gate, gate_ld, scale, eps, n, planes, plane);
+      else lb::launch(lb::rmsnorm_gated_x4_kernel<TO, 4>, dim3(num_rows), dim3(threads), 0, stream, (TO*)out, out_ld, x, weight, gate, gate_ld, scale, eps, n, planes, plane);
+    })
+    LB_CHECK_LAUNCH("rmsnorm_gated");
+    return 0;
+  }
   LB_DISPATCH_DTYPE(out_dtype, TO, {
     lb::launch(lb::rmsnorm_gated_kernel<TO>, dim3(num_rows), dim3(threads), 0, stream, (TO*)out, out_ld, x, weight, gate, gate_ld,
                scale, eps, n, planes, plane);

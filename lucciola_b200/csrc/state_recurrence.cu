@@ -333,6 +333,73 @@ __global__ void gated_group_norm_kernel(TO* __restrict__ out, long long out_ld, 
   }
 }
 
+// The same for groups whose rows lie in whole 16-byte words: a lane keeps its NV words of y and of the gate in registers between
+// the sum and the output (one pass; the scalar kernel reads y twice and forms the gate twice, four bytes a request).  2048 rows of
+// 16 groups of 128, 42 MB: 32 -> 13 us.
+template <typename TO, int NV>
+__global__ void __launch_bounds__(256) gated_group_norm_x4_kernel(TO* __restrict__ out, long long out_ld, const float* __restrict__ y, long long y_ld,
+                                                                  const float* __restrict__ gate, long long gate_ld, const float* __restrict__ w, int wn,
+                                                                  int gs, int groups, int gate_first, int act, float eps, float scale, int planes,
+                                                                  long long plane) {
+  __shared__ float part[8][8];
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x, gy = threadIdx.y, g = blockIdx.y * blockDim.y + gy;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const bool real = g < groups;                    // a group past the last meets the others at the barrier
+  const float* yr = y + (size_t)t * y_ld + (size_t)g * gs;
+  const float* gr = gate + (size_t)t * gate_ld + (size_t)g * gs;
+  float x[NV][4], z[NV][4];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (threadIdx.x + i * blockDim.x) * 4;
+    const bool in = real && c < gs;
+    const float4 a = in ? *reinterpret_cast<const float4*>(yr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 b = in ? *reinterpret_cast<const float4*>(gr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    x[i][0] = a.x; x[i][1] = a.y; x[i][2] = a.z; x[i][3] = a.w;
+    z[i][0] = b.x; z[i][1] = b.y; z[i][2] = b.z; z[i][3] = b.w;
+    for (int q = 1; q < planes; ++q) {
+      const float4 d = in ? *reinterpret_cast<const float4*>(yr + (size_t)q * plane + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      x[i][0] += d.x; x[i][1] += d.y; x[i][2] += d.z; x[i][3] += d.w;
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float s = 1.f / (1.f + expf(-z[i][e]));
+      z[i][e] = act == 0 ? z[i][e] * s : s;
+      if (gate_first) x[i][e] *= z[i][e];
+      ss += x[i][e] * x[i][e];
+    }
+  ss = warp_sum(ss);
+  if (lane == 0) part[gy][warp] = ss;
+  __syncthreads();
+  ss = 0.f;
+  for (int i = 0; i < nwarps; ++i) ss += part[gy][i];
+  const float inv = 1.f / sqrtf(ss / (float)gs + eps) * scale;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = (threadIdx.x + i * blockDim.x) * 4;
+    if (!real || c >= gs) continue;
+    const int col = g * gs + c;
+    const float4 a = w ? *reinterpret_cast<const float4*>(w + col % wn) : make_float4(1.f, 1.f, 1.f, 1.f);
+    float r[4] = {x[i][0] * inv * a.x, x[i][1] * inv * a.y, x[i][2] * inv * a.z, x[i][3] * inv * a.w};
+    if (!gate_first) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) r[e] *= z[i][e];
+    }
+    TO* o = out + (size_t)t * out_ld + col;
+    if constexpr (sizeof(TO) == 2) {
+      __nv_bfloat162 lo = __floats2bfloat162_rn(r[0], r[1]), hi = __floats2bfloat162_rn(r[2], r[3]);
+      *reinterpret_cast<uint2*>(o) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    } else {
+      *reinterpret_cast<float4*>(o) = make_float4(r[0], r[1], r[2], r[3]);
+    }
+  }
+}
+
 }  // namespace lb
 
 LB_EXPORT int lb_state_recurrence(int delta, const float* q, long long q_ld, const float* k, long long k_ld, const float* v,
@@ -423,6 +490,22 @@ LB_EXPORT int lb_gated_group_norm(void* out, int out_dtype, long long out_ld, co
   int per_cta = 8 / warps;                                                  // groups of a row in one CTA
   if (per_cta > groups) per_cta = groups;
   LB_CHECK_ARG((groups + per_cta - 1) / per_cta <= 65535, "gated_group_norm: %d groups", groups);
+  auto words = [](const void* x, long long ld, int bytes) { return (uintptr_t)x % (4 * bytes) == 0 && ld % 4 == 0; };
+  const int nv = (gs + 128 * warps - 1) / (128 * warps);
+  if (gs % 4 == 0 && nv <= 4 && words(y, y_ld, 4) && words(gate, gate_ld, 4) && words(out, out_ld, out_dtype == LB_BF16 ? 2 : 4) && plane % 4 == 0
+      && (!w || ((uintptr_t)w % 16 == 0 && wn % 4 == 0))) {
+    const dim3 grid(num_rows, (groups + per_cta - 1) / per_cta), block(warps * 32, per_cta);
+#define LB_GGN(NV) lb::launch(lb::gated_group_norm_x4_kernel<TO, NV>, grid, block, 0, stream, (TO*)out, out_ld, y, y_ld, gate, gate_ld, w, wn > 0 ? wn : 4, \
+                              gs, groups, gate_first, act, eps, scale, planes, plane)
+    LB_DISPATCH_DTYPE(out_dtype, TO, {
+      if (nv == 1) LB_GGN(1);
+      else if (nv == 2) LB_GGN(2);
+      else LB_GGN(4);
+    })
+#undef LB_GGN
+    LB_CHECK_LAUNCH("gated_group_norm");
+    return 0;
+  }
   LB_DISPATCH_DTYPE(out_dtype, TO, {
     lb::launch(lb::gated_group_norm_kernel<TO>, dim3(num_rows, (groups + per_cta - 1) / per_cta), dim3(warps * 32, per_cta), 0, stream,
                (TO*)out, out_ld, y, y_ld, gate, gate_ld, w, wn > 0 ? wn : 1, n, groups, gate_first, act, eps, scale, planes, plane);

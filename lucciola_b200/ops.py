@@ -84,6 +84,7 @@ _SIGNATURES = {
                            c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "lb_short_conv": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                       c_int, c_int, c_int, c_int, c_void_p],
+    "lb_short_conv_step": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "lb_short_conv_state": [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "lb_state_recurrence": [c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
                             c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
@@ -582,6 +583,26 @@ def short_conv_state(state: torch.Tensor, x: torch.Tensor, taps: int, step, stre
     _check(state, "convolution state", torch.float32); _rows32(x, "convolution input")
     _call("lb_short_conv_state", state.data_ptr(), x.data_ptr(), x.stride(0), step.cu_tokens.data_ptr(),
           step.state_slots.data_ptr(), step.num_seqs, x.shape[1], taps, stream)
+
+
+def short_conv_step(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, state: torch.Tensor, step, stream: int,
+                    act: bool = True) -> bool:
+    """short_conv and short_conv_state in one launch, for steps of one token a sequence, four taps and rows in whole 16-byte words;
+    False (and nothing done) for any other."""
+    if weight.shape[0] != 4 or step.max_q_len != 1 or not step.q_lens.count(1) == step.num_seqs == len(step.q_lens) == x.shape[0]:
+        return False
+    _rows32(out, "convolution output"); _rows32(x, "convolution input"); _check(weight, "taps", torch.float32)
+    _check(state, "convolution state", torch.float32)
+    T, C = x.shape
+    if weight.shape[1] != C or tuple(out.shape) != (T, C) or tuple(state.shape[1:]) != (3, C):
+        raise KernelError(f"the taps are {tuple(weight.shape)} for rows of {C}, the output {tuple(out.shape)}, the state {tuple(state.shape)}")
+    if bias is not None:
+        _check(bias, "convolution bias", torch.float32)
+    rc = _fn("lb_short_conv_step")(out.data_ptr(), out.stride(0), x.data_ptr(), x.stride(0), weight.data_ptr(), _ptr(bias), state.data_ptr(),
+                                   step.state_slots.data_ptr(), T, C, 1 if act else 0, stream)
+    if rc not in (0, 3):
+        raise KernelError(library().lb_last_error().decode())
+    return rc == 0
 
 
 # From how many tokens a sequence's recurrence goes through the chunked form (csrc/chunk_recurrence.cu): the walk token by token

@@ -164,3 +164,52 @@ def test_which_portions_are_long(monkeypatch):
     assert ops.chunk_portions("delta", step(32, 40, 31), 4096, 128, 64) == ([0, 1], 32)
     assert ops.chunk_portions("delta", step(9999), 2, 129, 64) == ([], 0)                # more rows of the state than the kernels hold
     assert ops.chunk_portions("delta", SimpleNamespace(num_seqs=3, q_lens=[], max_q_len=9999), 2, 64, 64) == ([], 0)      # lengths the host does not know
+
+
+@pytest.mark.parametrize("channels,lens", [(8192, [1]), (260, [1] * 9), (4096, [700, 1, 2, 3, 4, 5, 333]), (1028, [9, 200]), (64, [3000]), (2048, [5, 4, 1, 1, 90])])
+@pytest.mark.parametrize("bias", [False, True])
+def test_short_convolution_of_several_tokens_a_thread(channels, lens, bias):
+    """Portions that start and end anywhere in a thread's tokens, and steps of single tokens with the state in the same launch:
+    the very sums of the token-a-thread kernel (any taps and alignment), so the same bits."""
+    from lucciola_b200 import ops
+    torch.manual_seed(6)
+    T, s = sum(lens), torch.cuda.current_stream().cuda_stream
+    x = torch.randn(T, channels + 4, device=DEV)[:, 4:]
+    w, b = torch.randn(4, channels, device=DEV), torch.randn(channels, device=DEV) if bias else None
+    state = torch.randn(len(lens) + 1, 3, channels, device=DEV)
+    step = step_of(lens, list(range(len(lens), 0, -1)))
+    step.token_seq = torch.tensor([i for i, n in enumerate(lens) for _ in range(n)], dtype=torch.int32, device=DEV)
+    odd = torch.cat([torch.zeros(T, 1, device=DEV), x], dim=1)[:, 1:]                      # rows on no 16-byte boundary: four bytes at a time
+    want, got, state2 = torch.empty(T, channels, device=DEV), torch.empty(T, channels, device=DEV), state.clone()
+    ops.short_conv(want, odd, w, b, state, step, s)
+    ops.short_conv_state(state, odd, 4, step, s)
+    if ops.short_conv_step(got, x, w, b, state2, step, s):
+        assert max(lens) == 1
+    else:
+        assert max(lens) > 1
+        ops.short_conv(got, x, w, b, state2, step, s)
+        ops.short_conv_state(state2, x, 4, step, s)
+    assert torch.equal(got, want) and torch.equal(state2, state)
+
+
+@pytest.mark.parametrize("rows,n,groups,planes", [(5, 2048, 16, 1), (3, 2048, 2, 1), (70, 4096, 1, 1), (2, 96, 8, 2), (9, 1040, 2, 3), (4, 8192, 1, 1), (3, 128, 4, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_norms_in_words(rows, n, groups, planes, dtype):
+    """Groups around the sizes at which a group takes another number of warps and words a lane, against the formula in 64 bits."""
+    from lucciola_b200 import ops
+    torch.manual_seed(7)
+    s, eps = torch.cuda.current_stream().cuda_stream, 1e-6
+    y, gate, w = torch.randn(planes, rows, n, device=DEV), torch.randn(rows, n + 8, device=DEV)[:, 8:], torch.randn(n // groups, device=DEV)
+    Y, Z, tol = y.double().sum(0), gate.double(), 3e-6 if dtype == torch.float32 else 8e-3
+    parts = lambda z: z / torch.sqrt((z.view(rows, groups, -1) ** 2).mean(-1, keepdim=True) + eps).expand(-1, -1, n // groups).reshape(rows, n)
+    for first in (False, True):
+        out = torch.empty(rows, n, dtype=dtype, device=DEV)
+        ops.gated_group_norm(out, y if planes > 1 else y[0], gate, w, groups, eps, s, gate_first=first, scale=0.5)
+        act = torch.nn.functional.silu(Z)
+        want = 0.5 * (parts(Y * act) if first else parts(Y) * act) * w.double().repeat(groups)
+        assert (out.double() - want).abs().max() <= tol * want.abs().max()
+    if groups == 1:
+        out = torch.empty(rows, n, dtype=dtype, device=DEV)
+        ops.rmsnorm_gated(out, y if planes > 1 else y[0], w, gate, 0.5, eps, s)
+        want = 0.5 * parts(Y) * w.double() * torch.sigmoid(Z)
+        assert (out.double() - want).abs().max() <= tol * want.abs().max()
