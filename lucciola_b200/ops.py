@@ -8,6 +8,7 @@ other implementation behind these functions: without the library they raise.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_longlong, c_uint, c_ulonglong, c_void_p
 
 import torch
@@ -91,6 +92,8 @@ _SIGNATURES = {
                             c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_int, c_int, c_int, c_void_p],
     "lb_chunk_recurrence": [c_int] + [c_void_p, c_longlong] * 5 + [c_void_p] * 8 + [c_longlong] + [c_void_p] * 4
                            + [c_int] * 6 + [c_float, c_float, c_int, c_void_p, c_int, c_void_p],
+    "lb_state_step": [c_int] + [c_void_p, c_longlong] * 5 + [c_void_p] * 8 + [c_longlong, c_void_p, c_void_p] + [c_int] * 6
+                     + [c_float, c_float, c_int, c_void_p],
     "lb_channel_decay": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "lb_gated_group_norm": [c_void_p, c_int, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_int,
                             c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_longlong, c_void_p],
@@ -278,15 +281,17 @@ def gated_recurrence(pre: torch.Tensor, q_col: int, f_col: int, v_col: int, bias
     state [slots + 1, heads, dim, vdim] float32 is read and written at each sequence's slot; out [T, heads * vdim] float32.
     `max_tokens_a_seq`: the most tokens any sequence brings, if the host knows it (0: unknown); steps of a few tokens a
     sequence run in a kernel made for them, with the same sums in the same order.  `by_shape`: long portions go through the
-    chunked form (chunk_portions), which adds in another order."""
+    chunked form (chunk_portions), steps of single tokens through a kernel of their own (single_tokens); both add in another order."""
     _check(pre, "input projections", torch.float32); _check(bias, "gate bias", torch.float32)
     _check(lower, "lower bound", torch.float32); _check(state, "recurrent state", torch.float32)
     _check(out, "recurrence output", torch.float32)
+    q, f, v = _rows(pre, q_col), _rows(pre, f_col), _rows(pre, v_col)
+    if by_shape and single_tokens(step, dim, vdim, state):
+        _state_step("hgrn2", q, f, v, state, out, step, heads, heads, dim, vdim, stream, bias=bias, lower=lower)
+        return
     long, skip = chunk_portions("hgrn2", step, heads, dim, vdim) if by_shape else ([], 0)
     if long:
-        n, m = heads * dim, heads * vdim
-        _chunk_recurrence("hgrn2", pre[:, q_col:q_col + n], pre[:, f_col:f_col + n], pre[:, v_col:v_col + m], state, out, step, long, heads, heads, dim,
-                          vdim, stream, bias=bias, lower=lower)
+        _chunk_recurrence("hgrn2", q, f, v, state, out, step, long, heads, heads, dim, vdim, stream, bias=bias, lower=lower)
         if len(long) == step.num_seqs:
             return
     _call("lb_gated_recurrence", pre.data_ptr(), pre.stride(0), q_col, f_col, v_col, bias.data_ptr(), lower.data_ptr(),
@@ -628,21 +633,48 @@ def chunk_portions(kind: str, step, heads: int, dim: int, vdim: int) -> tuple[li
     return long, start if long else 0
 
 
-def _chunk_recurrence(kind: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, out: torch.Tensor, step, long: list[int],
-                      heads: int, groups: int, dim: int, vdim: int, stream: int, a=None, b=None, A_log=None, dt_bias=None, D=None, bias=None,
-                      lower=None, decay=None, unit_norm: bool = False, q_scale: float = 1.0, unit_eps: float = 1e-6, act: bool = False) -> None:
-    """The sequences `long` of the step, all their tokens; operands as the callers have checked them."""
-    lib = library()
-    lib.lb_chunk_recurrence_scratch.argtypes, lib.lb_chunk_recurrence_scratch.restype = [c_int] * 4, c_longlong
+def single_tokens(step, dim: int, vdim: int, state: torch.Tensor) -> bool:
+    """Whether a step is one token a sequence, by the lengths the host knows, and its states are of a form that the kernel for such
+    steps takes (csrc/state_step.cu): up to 128 rows, whole 16-byte words a row."""
+    return (step.max_q_len == 1 and dim <= 128 and vdim % 4 == 0 and step.q_lens.count(1) == step.num_seqs == len(step.q_lens)
+            and state.data_ptr() % 16 == 0)
+
+
+def _rows(t: torch.Tensor | None, col: int = 0) -> tuple:
+    """(address, row stride) of a float32 matrix from a column on."""
+    return (None, 0) if t is None else (t.data_ptr() + 4 * col, t.stride(0))
+
+
+def _state_step(kind: str, q: tuple, k: tuple, v: tuple, state: torch.Tensor, out: torch.Tensor, step, heads: int, groups: int, dim: int, vdim: int,
+                stream: int, a=(None, 0), b=(None, 0), A_log=None, dt_bias=None, D=None, bias=None, lower=None, decay=None, unit_norm: bool = False,
+                q_scale: float = 1.0, unit_eps: float = 1e-6, act: bool = False) -> None:
+    """One token a sequence; q, k, v, a, b as _rows gives them, operands as the callers have checked them."""
+    _call("lb_state_step", _CHUNK_KINDS[kind], *q, *k, *v, *a, *b, _ptr(A_log), _ptr(dt_bias), _ptr(D), _ptr(bias), _ptr(lower), _ptr(decay),
+          state.data_ptr(), out.data_ptr(), out.stride(0), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), step.num_seqs, heads, groups, dim,
+          vdim, unit_norm, q_scale, unit_eps, act, stream)
+
+
+def _chunk_recurrence(kind: str, q: tuple, k: tuple, v: tuple, state: torch.Tensor, out: torch.Tensor, step, long: list[int], heads: int, groups: int,
+                      dim: int, vdim: int, stream: int, a=(None, 0), b=(None, 0), A_log=None, dt_bias=None, D=None, bias=None, lower=None, decay=None,
+                      unit_norm: bool = False, q_scale: float = 1.0, unit_eps: float = 1e-6, act: bool = False) -> None:
+    """The sequences `long` of the step, all their tokens; operands as _state_step's."""
     code, n = _CHUNK_KINDS[kind], len(long)
     lens = [step.q_lens[i] for i in long]
-    one = int(lib.lb_chunk_recurrence_scratch(code, heads, dim, vdim))
+    one = _chunk_floats(code, heads, dim, vdim)
     chunks = max(1, min(sum(-(-t // 64) for t in lens), CHUNK_SCRATCH // max(one, 1)))
-    scratch = torch.empty(chunks * one, dtype=torch.float32, device=q.device)
-    rows = lambda t: (t.data_ptr(), t.stride(0)) if t is not None else (None, 0)
-    _call("lb_chunk_recurrence", code, *rows(q), *rows(k), *rows(v), *rows(a), *rows(b), _ptr(A_log), _ptr(dt_bias), _ptr(D), _ptr(bias), _ptr(lower),
-          _ptr(decay), state.data_ptr(), out.data_ptr(), out.stride(0), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), (c_int * n)(*long),
-          (c_int * n)(*lens), n, heads, groups, dim, vdim, 1 if unit_norm else 0, q_scale, unit_eps, 1 if act else 0, scratch.data_ptr(), chunks, stream)
+    scratch = torch.empty(chunks * one, dtype=torch.float32, device=out.device)
+    seqs, tokens = (c_int * n)(*long), (c_int * n)(*lens)
+    _call("lb_chunk_recurrence", code, *q, *k, *v, *a, *b, _ptr(A_log), _ptr(dt_bias), _ptr(D), _ptr(bias), _ptr(lower), _ptr(decay), state.data_ptr(),
+          out.data_ptr(), out.stride(0), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), ctypes.addressof(seqs), ctypes.addressof(tokens), n,
+          heads, groups, dim, vdim, unit_norm, q_scale, unit_eps, act, scratch.data_ptr(), chunks, stream)
+
+
+@functools.lru_cache(maxsize=256)
+def _chunk_floats(code: int, heads: int, dim: int, vdim: int) -> int:
+    """Floats of scratch a chunk of 64 tokens takes."""
+    f = library().lb_chunk_recurrence_scratch
+    f.argtypes, f.restype = [c_int] * 4, c_longlong
+    return int(f(code, heads, dim, vdim))
 
 
 def state_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tensor, b: torch.Tensor | None,
@@ -659,7 +691,7 @@ def state_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
     single tokens keep sixteen state rows a lane, which issues fewer instructions; all others eight, which shortens the path
     from token to token); a column's terms are then added in an order that depends on the step.  Without it one layout
     serves every step, so a 32-bit result does not depend on how a sequence was cut.  Long portions then go through the
-    chunked form (chunk_portions)."""
+    chunked form (chunk_portions), steps of single tokens through a kernel of their own (single_tokens)."""
     for t, w in ((q, "q"), (k, "k"), (v, "v"), (a, "a")) + (((b, "b"),) if b is not None else ()):
         _rows32(t, w)
     _rows32(out, "recurrence output")
@@ -674,10 +706,14 @@ def state_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
     if rows_decay:
         _call("lb_channel_decay", a.data_ptr(), a.stride(0), A_log.data_ptr(), dt_bias.data_ptr(), T, heads, dim, stream)
     kind = "channels" if rows_decay else "delta" if delta else "ssm"
+    if by_shape and single_tokens(step, dim, vdim, state):
+        _state_step(kind, _rows(q), _rows(k), _rows(v), state, out, step, heads, groups, dim, vdim, stream, a=_rows(a), b=_rows(b), A_log=A_log,
+                    dt_bias=dt_bias, D=D, unit_norm=unit_norm, q_scale=q_scale, unit_eps=unit_eps)
+        return
     long, skip = chunk_portions(kind, step, heads, dim, vdim) if by_shape else ([], 0)
     if long:
-        _chunk_recurrence(kind, q, k, v, state, out, step, long, heads, groups, dim, vdim, stream,
-                          a=a, b=b, A_log=A_log, dt_bias=dt_bias, D=D, unit_norm=unit_norm, q_scale=q_scale, unit_eps=unit_eps)
+        _chunk_recurrence(kind, _rows(q), _rows(k), _rows(v), state, out, step, long, heads, groups, dim, vdim, stream, a=_rows(a), b=_rows(b),
+                          A_log=A_log, dt_bias=dt_bias, D=D, unit_norm=unit_norm, q_scale=q_scale, unit_eps=unit_eps)
         if len(long) == step.num_seqs:
             return
     _call("lb_state_recurrence", 1 if delta else 0, q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
@@ -1042,18 +1078,21 @@ def decay_recurrence(pre: torch.Tensor, q_col: int, k_col: int, v_col: int, deca
     and the tokens' own scores (32-bit, outputs equal within rounding, several times faster), the state's rows shared out
     over row_split CTAs; out is then [row_split, T, heads * vdim] and the sum over its first dimension is meant.
     With 0 every output's sum has one order however the sequence is cut, unless `by_shape` sends long portions through the
-    chunked form (chunk_portions)."""
+    chunked form (chunk_portions) and steps of single tokens through a kernel of their own (single_tokens)."""
     _check(decay, "decay", torch.float32); _check(state, "recurrent state", torch.float32); _check(out, "recurrence output", torch.float32)
     if pre.dtype != torch.float32 or pre.stride(1) != 1 or not pre.is_cuda:
         raise KernelError("the input projections must be float32 on the GPU with unit column stride")
     T = pre.shape[0]
     if tuple(out.shape) != ((row_split, T, heads * vdim) if row_split >= 1 else (T, heads * vdim)):
         raise KernelError(f"the recurrence's output has the wrong shape {tuple(out.shape)}")
-    long, skip = chunk_portions("fixed", step, heads, dim, vdim) if by_shape and row_split == 0 else ([], 0)
+    by_shape = by_shape and row_split == 0
+    q, k, v = _rows(pre, q_col), _rows(pre, k_col), _rows(pre, v_col)
+    if by_shape and single_tokens(step, dim, vdim, state):
+        _state_step("fixed", q, k, v, state, out, step, heads, heads, dim, vdim, stream, decay=decay, act=act)
+        return
+    long, skip = chunk_portions("fixed", step, heads, dim, vdim) if by_shape else ([], 0)
     if long:
-        n, m = heads * dim, heads * vdim
-        _chunk_recurrence("fixed", pre[:, q_col:q_col + n], pre[:, k_col:k_col + n], pre[:, v_col:v_col + m], state, out, step, long, heads, heads, dim,
-                          vdim, stream, decay=decay, act=act)
+        _chunk_recurrence("fixed", q, k, v, state, out, step, long, heads, heads, dim, vdim, stream, decay=decay, act=act)
         if len(long) == step.num_seqs:
             return
     _call("lb_decay_recurrence", pre.data_ptr(), pre.stride(0), q_col, k_col, v_col, decay.data_ptr(), state.data_ptr(),

@@ -98,11 +98,12 @@ class DecayLinearAttention(Mixer):
                             rot_scale=getattr(self.position_encoding, "magnitude", 1.0))
         # the bfloat16 engine takes long portions 64 tokens at a time; where there are none, it forms the outputs of up to 16
         # tokens side by side, the rows of the state shared out over CTAs
-        chunked = rt.fast_kernels and bool(ops.chunk_portions("fixed", step, self.heads, self.dim, self.vdim)[0])
-        split = ops.decay_row_split(step.num_seqs, self.heads, self.dim, self.vdim, step.max_q_len) if rt.fast_kernels and not chunked else 0
+        single = rt.fast_kernels and ops.single_tokens(step, self.dim, self.vdim, cache.state)
+        chunked = rt.fast_kernels and not single and bool(ops.chunk_portions("fixed", step, self.heads, self.dim, self.vdim)[0])
+        split = ops.decay_row_split(step.num_seqs, self.heads, self.dim, self.vdim, step.max_q_len) if rt.fast_kernels and not (single or chunked) else 0
         o = rt.empty((split, T, self.inner_size) if split else (T, self.inner_size), torch.float32)
         ops.decay_recurrence(pre, 0, n, 2 * n, self.decay, cache.state, o, step, self.heads, self.dim, self.vdim, rt.stream,
-                             max_tokens_a_seq=step.max_q_len, row_split=split, act=self.act is not None, by_shape=chunked)
+                             max_tokens_a_seq=step.max_q_len, row_split=split, act=self.act is not None, by_shape=single or chunked)
         g0 = 2 * n + self.inner_size
         if self.head_norm or not self.norm_weight or self.gate_act != "sigmoid":
             ops.gated_group_norm(out, o, pre[:, g0:g0 + self.inner_size], self.norm_w, self.heads if self.head_norm else 1, self.eps,

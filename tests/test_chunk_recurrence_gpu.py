@@ -1,4 +1,4 @@
-"""Long portions of the linear recurrences, 64 tokens at a time, against the plain recurrence in 64 bits and against the
+"""Long portions of the linear recurrences, 64 tokens at a time, and steps of single tokens, against the plain recurrence in 64 bits and against the
 token-by-token kernels: every kind, portions around the edges of a block, a chunk and several, sizes that fill no tile, inputs
 that are column ranges, portions beside single tokens, and scratch for fewer chunks than there are (GPU)."""
 from types import SimpleNamespace
@@ -130,6 +130,29 @@ def test_long_portions(kind, heads, groups, dim, vdim, lens):
         assert torch.isnan(got_state[0]).all() and torch.isnan(got_state[-1]).all()
 
 
+@pytest.mark.parametrize("seqs,heads,groups,dim,vdim", [(1, 2, 1, 128, 128), (3, 4, 2, 64, 64), (80, 4, 4, 128, 128), (5, 64, 2, 128, 64), (40, 8, 4, 72, 40), (2, 3, 3, 5, 260),
+                                                        (150, 2, 1, 33, 132)])
+@pytest.mark.parametrize("kind", ["fixed", "ssm", "hgrn2", "delta", "channels"])
+def test_single_tokens(kind, seqs, heads, groups, dim, vdim):
+    """One token a sequence, in every width of CTA: the bounds of test_long_portions, and close to the kernels that walk tokens."""
+    from lucciola_b200 import ops
+    torch.manual_seed(5)
+    o = operands(kind, seqs, heads, groups, dim, vdim)
+    if kind == "fixed":
+        o["decay"] = torch.rand(heads, device=DEV)
+    step = step_of([1] * seqs, list(range(seqs, 0, -1)))
+    state = 0.3 * torch.randn(seqs + 2, heads, dim, vdim, device=DEV)
+    state[0] = state[-1] = float("nan")
+    assert ops.single_tokens(step, dim, vdim, state)
+    want, S = plain(kind, o, state, step, heads, groups, dim, vdim)
+    for by_shape in (True, False):
+        got_state = state.clone()
+        got = through_ops(kind, o, got_state, step, heads, groups, dim, vdim, by_shape)
+        assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max(), by_shape
+        assert (got_state[1:-1].double() - S[1:-1]).abs().max() <= 1e-5 * S[1:-1].abs().max(), by_shape
+        assert torch.isnan(got_state[0]).all() and torch.isnan(got_state[-1]).all()
+
+
 @pytest.mark.parametrize("kind", ["fixed", "delta", "channels"])
 def test_scratch_for_fewer_chunks_and_more_sequences_than_a_launch(kind, monkeypatch):
     """The chunks of three sequences in turns of two, the same bits as in one; more than 64 long sequences in a step."""
@@ -141,7 +164,7 @@ def test_scratch_for_fewer_chunks_and_more_sequences_than_a_launch(kind, monkeyp
     step = step_of(lens, [2, 0, 3])
     whole_state = state.clone()
     whole = through_ops(kind, o, whole_state, step, heads, heads, dim, vdim, True)
-    one = ops.library().lb_chunk_recurrence_scratch(ops._CHUNK_KINDS[kind], heads, dim, vdim)
+    one = ops._chunk_floats(ops._CHUNK_KINDS[kind], heads, dim, vdim)
     monkeypatch.setattr(ops, "CHUNK_SCRATCH", 2 * one + 1)
     turned = through_ops(kind, o, state, step, heads, heads, dim, vdim, True)
     assert torch.equal(turned, whole) and torch.equal(state, whole_state)
