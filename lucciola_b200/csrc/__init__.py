@@ -11,6 +11,10 @@ Where the library goes: `<this folder>/_build/` when that is writable (so the
 built file travels with the tree), else `$LUCCIOLA_B200_BUILD_DIR`, else a
 per-user folder under the system's temporary directory.
 
+Beside the library stands `lb_caller`, a small extension module in C through which Python calls the library's functions
+without ctypes' conversion of every argument; where it cannot be built (no Python headers, another machine than x86-64) the
+calls go through ctypes.
+
 There is no fallback: if the library cannot be built or loaded, `library()`
 raises, and every operation of the engine raises with it.
 """
@@ -22,6 +26,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -31,6 +36,7 @@ from pathlib import Path
 _HERE = Path(__file__).resolve().parent
 ABI_VERSION = 10
 LIB_NAME = "liblucciola_b200.so"
+_CALLER = _HERE / "lb_caller.c"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -79,7 +85,7 @@ def _digest(paths: list[Path], extra: str = "") -> str:
 
 
 def source_digest() -> str:
-    return _digest(sources() + _headers(), " ".join(NVCC_FLAGS) + f"|abi{ABI_VERSION}")
+    return _digest(sources() + _headers() + [_CALLER], " ".join(NVCC_FLAGS) + f"|abi{ABI_VERSION}")
 
 
 def _writable(d: Path) -> bool:
@@ -120,6 +126,41 @@ def _existing_library() -> Path | None:
         except OSError:
             continue
     return None
+
+
+def _caller_path(folder: Path) -> Path:
+    return folder / ("lb_caller" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+
+
+def _build_caller(out: Path) -> None:
+    """The extension module beside the library; left out where it cannot be built."""
+    path = _caller_path(out)
+    path.unlink(missing_ok=True)
+    include, cc = sysconfig.get_paths().get("include", ""), shutil.which("gcc") or shutil.which("cc")
+    if not cc or not (Path(include) / "Python.h").exists():
+        return
+    tmp = path.with_name(path.name + f".{os.getpid()}.tmp")
+    r = subprocess.run([cc, "-O2", "-fPIC", "-shared", "-I", include, "-o", str(tmp), str(_CALLER)], capture_output=True, text=True)
+    if r.returncode == 0:
+        os.replace(tmp, path)
+    else:
+        tmp.unlink(missing_ok=True)
+
+
+def caller():
+    """The module lb_caller of the loaded library, or None."""
+    import importlib.machinery
+    import importlib.util
+    path = _caller_path(Path(library()._name).parent)
+    if not path.exists():
+        return None
+    try:
+        loader = importlib.machinery.ExtensionFileLoader("lb_caller", str(path))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("lb_caller", str(path), loader=loader))
+        loader.exec_module(module)
+        return module
+    except ImportError:
+        return None
 
 
 def _compile_one(nvcc: str, src: Path, obj: Path) -> tuple[Path, float]:
@@ -181,6 +222,7 @@ def build(verbose: bool = True) -> Path:
         if r.returncode != 0:
             raise KernelLibraryError(f"linking the kernel library failed:\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, lib)
+        _build_caller(out)
         stamp.write_text(want + "\n")
         if verbose:
             _say(f"kernel library ready: {lib} ({time.time() - t0:.1f} s)")

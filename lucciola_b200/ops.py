@@ -13,7 +13,7 @@ from ctypes import c_float, c_int, c_longlong, c_uint, c_ulonglong, c_void_p
 
 import torch
 
-from .csrc import KernelLibraryError, library
+from .csrc import KernelLibraryError, caller, library
 
 F32, BF16 = 0, 1
 
@@ -127,6 +127,12 @@ _SIGNATURES = {
     "lb_latent_gather": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "lb_latent_prefill": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                           c_float, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_void_p],
+    "lb_gemm_tcgen05_heads_ok": [c_int] * 4,
+    "lb_gemm_tcgen05_addnorm_ok": [c_int] * 3,
+    "lb_gemm_tcgen05_addnorm_tiles": [c_int] * 3,
+    "lb_decay_row_split": [c_int] * 5,
+    "lb_expert_tile_rows": [c_int] * 1,
+    "lb_latent_flash_ok": [c_int] * 4,
     "lb_sample": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
 }
 
@@ -147,10 +153,41 @@ def _fn(name: str):
     return f
 
 
+# The exported functions through lb_caller, by name (bound at their first call); None: there is no such module.
+_native: dict[str, object] | None = {}
+_LETTERS = {c_void_p: "p", c_int: "i", c_longlong: "i", c_uint: "i", c_ulonglong: "i", c_float: "f"}
+
+
+def _bind_native(name: str):
+    global _native
+    module = caller()
+    if module is None:
+        _native = None
+        return None
+    address = ctypes.cast(_fn(name), c_void_p).value
+    f = _native[name] = module.bind(address, "".join(_LETTERS[t] for t in _SIGNATURES[name]))
+    return f
+
+
+def _invoke(name: str, *args) -> int:
+    """What the library's function returns."""
+    if _native is not None:
+        f = _native.get(name) or _bind_native(name)
+        if f is not None:
+            rc = f(*args)
+            if rc is not NotImplemented:
+                return rc
+    return _fn(name)(*args)          # arguments that only ctypes takes, or no such module
+
+
 def _call(name: str, *args) -> None:
-    rc = _fn(name)(*args)
-    if rc != 0:
+    if _invoke(name, *args) != 0:
         raise KernelError(library().lb_last_error().decode())
+
+
+def _address(c) -> int | None:
+    """Of a ctypes object that the caller keeps until the call has returned."""
+    return None if c is None else ctypes.addressof(c)
 
 
 def hash_uniform(key: int, counter: int, i: int) -> float:
@@ -603,8 +640,8 @@ def short_conv_step(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bi
         raise KernelError(f"the taps are {tuple(weight.shape)} for rows of {C}, the output {tuple(out.shape)}, the state {tuple(state.shape)}")
     if bias is not None:
         _check(bias, "convolution bias", torch.float32)
-    rc = _fn("lb_short_conv_step")(out.data_ptr(), out.stride(0), x.data_ptr(), x.stride(0), weight.data_ptr(), _ptr(bias), state.data_ptr(),
-                                   step.state_slots.data_ptr(), T, C, 1 if act else 0, stream)
+    rc = _invoke("lb_short_conv_step", out.data_ptr(), out.stride(0), x.data_ptr(), x.stride(0), weight.data_ptr(), _ptr(bias), state.data_ptr(),
+                 step.state_slots.data_ptr(), T, C, 1 if act else 0, stream)
     if rc not in (0, 3):
         raise KernelError(library().lb_last_error().decode())
     return rc == 0
@@ -665,7 +702,7 @@ def _chunk_recurrence(kind: str, q: tuple, k: tuple, v: tuple, state: torch.Tens
     scratch = torch.empty(chunks * one, dtype=torch.float32, device=out.device)
     seqs, tokens = (c_int * n)(*long), (c_int * n)(*lens)
     _call("lb_chunk_recurrence", code, *q, *k, *v, *a, *b, _ptr(A_log), _ptr(dt_bias), _ptr(D), _ptr(bias), _ptr(lower), _ptr(decay), state.data_ptr(),
-          out.data_ptr(), out.stride(0), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), ctypes.addressof(seqs), ctypes.addressof(tokens), n,
+          out.data_ptr(), out.stride(0), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), _address(seqs), _address(tokens), n,
           heads, groups, dim, vdim, unit_norm, q_scale, unit_eps, act, scratch.data_ptr(), chunks, stream)
 
 
@@ -769,7 +806,8 @@ def bias_rmsnorm_cols(x: torch.Tensor, ranges, eps: float, stream: int) -> None:
     sizes = (c_int * 3)(*[r[1] for r in ranges])
     biases = (c_void_p * 3)(*[_ptr(r[2]) for r in ranges])
     weights = (c_void_p * 3)(*[_ptr(r[3]) for r in ranges])
-    _call("lb_bias_rmsnorm_cols", x.data_ptr(), x.stride(0), x.shape[0], n, cols, sizes, biases, weights, eps, stream)
+    _call("lb_bias_rmsnorm_cols", x.data_ptr(), x.stride(0), x.shape[0], n, _address(cols), _address(sizes), _address(biases),
+          _address(weights), eps, stream)
 
 
 def pool_kv(k_cache: torch.Tensor, v_cache: torch.Tensor, table: torch.Tensor, pool_k: torch.Tensor, pool_v: torch.Tensor,
@@ -869,26 +907,28 @@ def sample(tokens: torch.Tensor, logits: torch.Tensor, stream: int, temperature:
 
 _WORKSPACE_ELEMS = 16 * 1024 * 1024      # float32 partials of split products (64 MB)
 _COUNTERS = 4096
-_scratch: dict[int, tuple[torch.Tensor, torch.Tensor]] = {}
+_scratch: dict[int, tuple[int, int, torch.Tensor, torch.Tensor]] = {}
 
 
-def _gemm_scratch(device: torch.device) -> tuple[torch.Tensor, torch.Tensor]:
-    """Per device: the workspace for partial sums of split products and the tile counters (zero between launches)."""
+def _gemm_scratch(device: torch.device) -> tuple[int, int]:
+    """Per device: the addresses of the workspace for partial sums of split products (_WORKSPACE_ELEMS floats) and of the tile
+    counters (_COUNTERS, zero between launches)."""
     key = device.index if device.index is not None else torch.cuda.current_device()
     s = _scratch.get(key)
     if s is None:
-        s = (torch.empty(_WORKSPACE_ELEMS, dtype=torch.float32, device=device),
-             torch.zeros(_COUNTERS, dtype=torch.int32, device=device))
-        _scratch[key] = s
-    return s
+        ws = torch.empty(_WORKSPACE_ELEMS, dtype=torch.float32, device=device)
+        counters = torch.zeros(_COUNTERS, dtype=torch.int32, device=device)
+        s = _scratch[key] = (ws.data_ptr(), counters.data_ptr(), ws, counters)
+    return s[:2]
 
 
 def gemm_tcgen05_ok(y: torch.Tensor, x: torch.Tensor, w: torch.Tensor) -> bool:
     """The conditions of the tensor-core kernel: bfloat16 operands, K a multiple of 8, 16-byte alignment."""
-    K = x.shape[1]
+    M, K = x.shape
+    row, col = x.stride()
     return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and y.dtype in (torch.bfloat16, torch.float32)
-            and K % 8 == 0 and (x.shape[0] == 1 or x.stride(0) % 8 == 0) and x.data_ptr() % 16 == 0
-            and w.data_ptr() % 16 == 0 and w.is_contiguous() and x.stride(1) == 1 and y.stride(1) == 1)
+            and K % 8 == 0 and (M == 1 or row % 8 == 0) and x.data_ptr() % 16 == 0
+            and w.data_ptr() % 16 == 0 and w.is_contiguous() and col == 1 and y.stride(1) == 1)
 
 
 class LbRowScale(ctypes.Structure):
@@ -896,17 +936,17 @@ class LbRowScale(ctypes.Structure):
     _fields_ = [("on", c_int), ("tiles", c_int), ("sumsq", c_void_p), ("inv_width", c_float), ("eps", c_float)]
 
 
-def _row_scale(sumsq: torch.Tensor | None, width: int, eps: float):
-    """The argument for rows that lack their norm's factor: None, or a reference to an LbRowScale."""
+def _row_scale(sumsq: torch.Tensor | None, width: int, eps: float) -> LbRowScale | None:
+    """What a product is told of rows that lack their norm's factor; None for rows that do not.  The call takes its address."""
     if sumsq is None:
         return None
     _check(sumsq, "partial sums of squares", torch.float32)
-    return ctypes.byref(LbRowScale(1, sumsq.shape[1], sumsq.data_ptr(), 1.0 / width, eps))
+    return LbRowScale(1, sumsq.shape[1], sumsq.data_ptr(), 1.0 / width, eps)
 
 
 def gemm_tcgen05(y: torch.Tensor, x: torch.Tensor, w: torch.Tensor, stream: int, force_bt: int = 0,
                  force_splits: int = 0, swiglu: bool = False, sumsq: torch.Tensor | None = None, eps: float = 0.0,
-                 act: str = "silu", limit: float = 0.0, post: str | None = None, post_c: float = 0.0) -> None:
+                 act: str = "silu", limit: float = 0.0, post: str | None = None, post_c: float = 0.0, looked_at: bool = False) -> None:
     """y[M, N] = x[M, K] . w[N, K]^T on the tensor cores (tcgen05, accumulators in tensor memory).
 
     With `swiglu` the rows of w alternate in blocks of 64 between gate rows and up rows of the same 64
@@ -914,17 +954,19 @@ def gemm_tcgen05(y: torch.Tensor, x: torch.Tensor, w: torch.Tensor, stream: int,
     (act: one of GATE_ACTS; `limit` is the clamp of "clamped_swish").
     With `sumsq` [M, tiles] the rows of x lack the factor of an RMSNorm over K values: row m of the product is
     multiplied by rsqrt(sum(sumsq[m]) / K + eps), before the activation if there is one (see gemm_tcgen05_addnorm).
-    `post`, `post_c` (without swiglu): an element operation in the epilogue, see POST_OPS."""
+    `post`, `post_c` (without swiglu): an element operation in the epilogue, see POST_OPS.  `looked_at`: gemm_tcgen05_ok has
+    said yes to these operands."""
     M, K = x.shape
     N = w.shape[0]
     if w.shape[1] != K or tuple(y.shape) != (M, N // 2 if swiglu else N):
         raise KernelError(f"gemm shapes do not fit: x {tuple(x.shape)}, w {tuple(w.shape)}, y {tuple(y.shape)}")
-    if not gemm_tcgen05_ok(y, x, w):
+    if not looked_at and not gemm_tcgen05_ok(y, x, w):
         raise KernelError("gemm_tcgen05 takes bfloat16 operands with K a multiple of 8, 16-byte aligned, unit column stride")
     ws, counters = _gemm_scratch(x.device)
+    scale = _row_scale(sumsq, K, eps)
     _call("lb_gemm_tcgen05", y.data_ptr(), dtype_code(y.dtype), x.data_ptr(), w.data_ptr(), M, N, K,
-          x.stride(0) if M > 1 else K, y.stride(0) if M > 1 else y.shape[1], ws.data_ptr(), ws.numel(), counters.data_ptr(),
-          counters.numel(), force_bt, force_splits, (1 + GATE_ACTS[act]) if swiglu else 0, _row_scale(sumsq, K, eps), limit,
+          x.stride(0) if M > 1 else K, y.stride(0) if M > 1 else y.shape[1], ws, _WORKSPACE_ELEMS, counters,
+          _COUNTERS, force_bt, force_splits, (1 + GATE_ACTS[act]) if swiglu else 0, _address(scale), limit,
           POST_OPS[post], float(post_c), stream)
 
 
@@ -938,43 +980,31 @@ class LbHeadEpilogue(ctypes.Structure):
 
 def gemm_tcgen05_heads_sizes_ok(M: int, N: int, K: int, head_dim: int) -> bool:
     """The sizes the q|k|v product with the head epilogue takes (heads of 128, at most 32 tokens, a split product)."""
-    lib = library()
-    lib.lb_gemm_tcgen05_heads_ok.argtypes = [c_int, c_int, c_int, c_int]
-    lib.lb_gemm_tcgen05_heads_ok.restype = c_int
-    return bool(lib.lb_gemm_tcgen05_heads_ok(M, N, K, head_dim))
+    return bool(_invoke("lb_gemm_tcgen05_heads_ok", M, N, K, head_dim))
 
 
 def gemm_tcgen05_heads_ok(x: torch.Tensor, w: torch.Tensor, head_dim: int, rot_dim: int | None) -> bool:
     """The conditions of the q|k|v product whose epilogue norms, rotates and stores the heads: bfloat16, heads of
     128 rotated whole (or not at all), at most 32 tokens, a product that is split over a cluster."""
-    lib = library()
-    lib.lb_gemm_tcgen05_heads_ok.argtypes = [c_int, c_int, c_int, c_int]
-    lib.lb_gemm_tcgen05_heads_ok.restype = c_int
     M, K = x.shape
     return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous() and x.stride(1) == 1
             and (M == 1 or x.stride(0) % 8 == 0) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-            and rot_dim in (None, head_dim) and bool(lib.lb_gemm_tcgen05_heads_ok(M, w.shape[0], K, head_dim)))
+            and rot_dim in (None, head_dim) and bool(_invoke("lb_gemm_tcgen05_heads_ok", M, w.shape[0], K, head_dim)))
 
 
 def gemm_tcgen05_addnorm_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
     """The conditions of the product whose epilogue adds to the residual stream: bfloat16, 16-byte alignment, and sizes
     for which the product is split over a thread-block cluster (few tokens, fewer output tiles than SMs)."""
-    lib = library()
-    lib.lb_gemm_tcgen05_addnorm_ok.argtypes = [c_int, c_int, c_int]
-    lib.lb_gemm_tcgen05_addnorm_ok.restype = c_int
     M, K = x.shape
     return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous() and x.stride(1) == 1
             and (M == 1 or x.stride(0) % 8 == 0) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-            and bool(lib.lb_gemm_tcgen05_addnorm_ok(M, w.shape[0], K)))
+            and bool(_invoke("lb_gemm_tcgen05_addnorm_ok", M, w.shape[0], K)))
 
 
 def gemm_tcgen05_addnorm_tiles(M: int, N: int, K: int) -> int:
     """Columns of the partial sums of squares that gemm_tcgen05_addnorm writes for these sizes: blocks of 128 features
     with few tokens, the feature tiles the many-token product chooses otherwise (0: sizes it does not take)."""
-    lib = library()
-    lib.lb_gemm_tcgen05_addnorm_tiles.argtypes = [c_int, c_int, c_int]
-    lib.lb_gemm_tcgen05_addnorm_tiles.restype = c_int
-    return int(lib.lb_gemm_tcgen05_addnorm_tiles(M, N, K))
+    return int(_invoke("lb_gemm_tcgen05_addnorm_tiles", M, N, K))
 
 
 def gemm_tcgen05_addnorm(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor, norm_w: torch.Tensor, out: torch.Tensor,
@@ -1013,8 +1043,9 @@ def gemm_tcgen05_heads(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, po
     he = LbHeadEpilogue(1, num_q_heads, num_kv_heads, page_size, block_table.shape[1], eps, positions.data_ptr(),
                         token_seq.data_ptr(), block_table.data_ptr(), _ptr(q_norm_w), _ptr(k_norm_w), _ptr(inv_freq),
                         q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr())
+    scale = _row_scale(sumsq, K, row_eps)
     _call("lb_gemm_tcgen05_heads", x.data_ptr(), w.data_ptr(), M, w.shape[0], K, x.stride(0) if M > 1 else K,
-          ctypes.byref(he), _row_scale(sumsq, K, row_eps), stream)
+          _address(he), _address(scale), stream)
 
 
 def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
@@ -1062,10 +1093,7 @@ def round_copy(out: torch.Tensor, x: torch.Tensor, stream: int) -> None:
 def decay_row_split(num_seqs: int, heads: int, dim: int, vdim: int, max_tokens_a_seq: int) -> int:
     """Into how many shares of rows the kernel that forms outputs side by side cuts a head's state for a step of this
     shape (0: the step runs token by token): as many as fill the SMs, with 32 to 256 rows a share."""
-    lib = library()
-    lib.lb_decay_row_split.argtypes = [c_int, c_int, c_int, c_int, c_int]
-    lib.lb_decay_row_split.restype = c_int
-    return int(lib.lb_decay_row_split(num_seqs, heads, dim, vdim, max_tokens_a_seq))
+    return int(_invoke("lb_decay_row_split", num_seqs, heads, dim, vdim, max_tokens_a_seq))
 
 
 def decay_recurrence(pre: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.Tensor, state: torch.Tensor,
@@ -1144,10 +1172,7 @@ def route_topk(ids: torch.Tensor, weights: torch.Tensor, logits: torch.Tensor, c
 
 def expert_tile_rows(few: int = 0) -> int:
     """Places of a row tile of the experts' products; `few`: of those for steps with a few pairs an expert (1), or some more (2)."""
-    lib = library()
-    lib.lb_expert_tile_rows.argtypes = [c_int]
-    lib.lb_expert_tile_rows.restype = c_int
-    return int(lib.lb_expert_tile_rows(int(few)))
+    return int(_invoke("lb_expert_tile_rows", int(few)))
 
 
 def expert_max_tiles(pairs: int, experts: int, few: int = 0) -> int:
@@ -1301,7 +1326,7 @@ def linear(y: torch.Tensor, x: torch.Tensor, w: torch.Tensor, stream: int, fast:
     """y = post(x . w^T), see POST_OPS.  `fast` allows the tensor-core kernel where its conditions hold (otherwise, and
     always on the 32-bit path, the product runs on the ordinary pipes)."""
     if fast and gemm_tcgen05_ok(y, x, w):
-        gemm_tcgen05(y, x, w, stream, post=post, post_c=post_c)
+        gemm_tcgen05(y, x, w, stream, post=post, post_c=post_c, looked_at=True)
     else:
         gemm_plain(y, x, w, stream, post=post, post_c=post_c)
 
@@ -1434,8 +1459,7 @@ def latent_flash_ok(dk: int, dv: int, group: int, page_size: int) -> bool:
     values (multiples of 8), at most 64 heads a tile, pages of 8 to 128 tokens."""
     lib = library()
     lib.lb_latent_flash_ok.restype = c_int
-    lib.lb_latent_flash_ok.argtypes = [c_int, c_int, c_int, c_int]
-    return bool(lib.lb_latent_flash_ok(dk, dv, group, page_size))
+    return bool(_invoke("lb_latent_flash_ok", dk, dv, group, page_size))
 
 
 def latent_flash_splits(num_tiles: int, head_groups: int, max_span: int, slots: int = 148) -> int:

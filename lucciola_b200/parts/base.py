@@ -70,9 +70,13 @@ class Runtime:
         self.act_dtype = act_dtype
         self.stream: int = 0        # raw handle, set by the step function before parts run
         self.fast_kernels = act_dtype == torch.bfloat16
+        self._like: dict[torch.dtype | None, torch.Tensor] = {}     # an empty tensor of each type: new_empty() is cheaper than torch.empty()
 
     def empty(self, shape: Sequence[int], dtype: torch.dtype | None = None) -> torch.Tensor:
-        return torch.empty(tuple(shape), dtype=dtype or self.act_dtype, device=self.device)
+        like = self._like.get(dtype)
+        if like is None:
+            like = self._like[dtype] = torch.empty(0, dtype=dtype or self.act_dtype, device=self.device)
+        return like.new_empty(shape)
 
 
 @dataclass
