@@ -238,37 +238,37 @@ __global__ void rope_kv_vec_kernel(RopeKvParams p) {
 
 // The same with eight elements a lane (16-byte words) and LPH = d / 8 lanes a head, so that a warp walks 32 / LPH heads side by
 // side: half the shuffles of the norm's sum a head of 128, and the rotation's partners travel as the four words they came in (the
-// norm's factor is the head's, the partner's weights are known).  One sine and cosine a pair and token for the whole CTA.
-// 2048 tokens of 48 heads of 128, 50 MB: bound by its instructions, 30 us with four elements a lane.
+// norm's factor is the head's, the partner's weights are known).  One sine and cosine a pair and token for the whole CTA, with
+// the norms' weights multiplied in: an element is inv * (x a + partner b).
+// 2048 tokens of 48 heads of 128, 50 MB: bound by its instructions, 30 us with four elements a lane, 17 us.
 template <int LPH>
 __global__ void __launch_bounds__(128) rope_kv_rows_kernel(RopeKvParams p) {
   constexpr int d = LPH * 8, HPW = 32 / LPH, HALF = d / 2;
-  __shared__ float2 turn[HALF];
+  __shared__ __align__(16) float tab[4][d];          // a and b of queries, of keys
   pdl_trigger();
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int sub = lane % LPH, hsel = lane / LPH;
   const int pos = p.positions[t];
   const int total_heads = p.num_q_heads + 2 * p.num_kv_heads;
-  if (p.inv_freq) {
-    for (int i = threadIdx.x; i < HALF; i += blockDim.x) {
-      float sn, cs;
+  for (int i = threadIdx.x; i < HALF; i += blockDim.x) {
+    float sn = 0.f, cs = 1.f;
+    if (p.inv_freq) {
       sincosf((float)pos * p.inv_freq[i], &sn, &cs);
-      turn[i] = make_float2(cs * p.rot_scale, sn * p.rot_scale);
+      sn *= p.rot_scale; cs *= p.rot_scale;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {                              // first half: x cos - y sin with y the partner; second half: x cos + y sin
+      const float* w = k == 0 ? p.q_norm_w : p.k_norm_w;
+      const float lo = w ? w[i] : 1.f, hi = w ? w[i + HALF] : 1.f;
+      tab[2 * k][i] = lo * cs; tab[2 * k + 1][i] = -hi * sn;
+      tab[2 * k][i + HALF] = hi * cs; tab[2 * k + 1][i + HALF] = lo * sn;
     }
   }
   // The token's page does not depend on the kernel ahead either (positions and block tables are the step's inputs).
   int page = -1;
   if (p.k_cache) page = p.block_table[(size_t)p.token_seq[t] * p.max_pages + pos / p.page_size];
   __syncthreads();
-  const bool first = sub < LPH / 2;
-  const int e0 = sub * 8, o0 = (sub ^ (LPH / 2)) * 8;          // this lane's elements, and their partners
-  float cs[8], sn[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float2 a = p.inv_freq ? turn[(sub % (LPH / 2)) * 8 + i] : make_float2(1.f, 0.f);
-    cs[i] = a.x; sn[i] = first ? -a.y : a.y;                   // first half: x cos - y sin; second half: y cos + x sin
-  }
   pdl_wait();                                                  // what follows reads the q|k|v product
   constexpr int UNR = 4;                                       // heads of a lane whose loads are issued together
   const int hstep = gridDim.y * nwarps * HPW;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(128) rope_kv_rows_kernel(RopeKvParams p) {
         if (dsts[u]) reinterpret_cast<uint4*>(dsts[u])[sub] = raw[u];
         continue;
       }
-      const float* w = kinds[u] == 0 ? p.q_norm_w : p.k_norm_w;
+      const int k = kinds[u] == 0 ? 0 : 1;
       uint4 far = raw[u];
       if (p.inv_freq) {
         far.x = __shfl_xor_sync(0xffffffffu, raw[u].x, LPH / 2); far.y = __shfl_xor_sync(0xffffffffu, raw[u].y, LPH / 2);
@@ -317,24 +317,22 @@ __global__ void __launch_bounds__(128) rope_kv_rows_kernel(RopeKvParams p) {
       }
       const bf16* e = reinterpret_cast<const bf16*>(&raw[u]);
       const bf16* f = reinterpret_cast<const bf16*>(&far);
-      float x[8], y[8], ss = 0.f;
+      const float4 a0 = *reinterpret_cast<const float4*>(&tab[2 * k][sub * 8]), a1 = *reinterpret_cast<const float4*>(&tab[2 * k][sub * 8 + 4]);
+      const float4 b0 = *reinterpret_cast<const float4*>(&tab[2 * k + 1][sub * 8]), b1 = *reinterpret_cast<const float4*>(&tab[2 * k + 1][sub * 8 + 4]);
+      const float ta[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, tb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      float x[8], ss = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { x[i] = __bfloat162float(e[i]); y[i] = __bfloat162float(f[i]); ss += x[i] * x[i]; }
+      for (int i = 0; i < 8; ++i) {
+        const float v = __bfloat162float(e[i]);
+        ss += v * v;
+        x[i] = p.inv_freq ? fmaf(v, ta[i], __bfloat162float(f[i]) * tb[i]) : v * ta[i];
+      }
       if (p.q_norm_w || p.k_norm_w) {
 #pragma unroll
         for (int m = LPH / 2; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
-        if (w) {
-          const float inv = rsqrtf(ss / (float)d + p.eps);
-          const float4 wa = *reinterpret_cast<const float4*>(w + e0), wb = *reinterpret_cast<const float4*>(w + e0 + 4);
-          const float4 fa = *reinterpret_cast<const float4*>(w + o0), fb = *reinterpret_cast<const float4*>(w + o0 + 4);
-          const float ww[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w}, fw[8] = {fa.x, fa.y, fa.z, fa.w, fb.x, fb.y, fb.z, fb.w};
+        const float inv = (k == 0 ? p.q_norm_w : p.k_norm_w) ? rsqrtf(ss / (float)d + p.eps) : 1.f;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) { x[i] = x[i] * inv * ww[i]; y[i] = y[i] * inv * fw[i]; }
-        }
-      }
-      if (p.inv_freq) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = x[i] * cs[i] + y[i] * sn[i];
+        for (int i = 0; i < 8; ++i) x[i] *= inv;
       }
       uint4 o;
       bf16* ob = reinterpret_cast<bf16*>(&o);
