@@ -56,6 +56,28 @@ __global__ void embedding_kernel(float* __restrict__ out, const int* __restrict_
   }
 }
 
+// The table's rows alone, times `scale`: four entries a thread, a CTA up to 1024 of a row (the kernel above takes a row a CTA and an
+// entry a request: 6 us for 8 rows of 2048, 13 us for 2048 of them).
+__device__ __forceinline__ float4 embedding_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 embedding_load4(const bf16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+  return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
+
+template <typename TW>
+__global__ void __launch_bounds__(256) embedding_x4_kernel(float* __restrict__ out, const int* __restrict__ ids, const TW* __restrict__ table,
+                                                           int hidden, int vocab, float scale) {
+  pdl_trigger();
+  const int t = blockIdx.x, i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  pdl_wait();
+  if (i >= hidden) return;
+  int id = ids[t];
+  if (id < 0 || id >= vocab) id = 0;
+  const float4 v = embedding_load4(table + (size_t)id * hidden + i);
+  *reinterpret_cast<float4*>(out + (size_t)t * hidden + i) = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+}
+
 template <typename TW>
 __global__ void embedding_sinusoid_kernel(float* __restrict__ out, const int* __restrict__ ids, const TW* __restrict__ table,
                                           int hidden, int vocab, const double* __restrict__ sin_freq,
@@ -101,6 +123,14 @@ LB_EXPORT int lb_embedding(float* out, const int* ids, const void* table, int ta
     LB_DISPATCH_DTYPE(table_dtype, TW, {
       lb::launch(lb::embedding_sinusoid_kernel<TW>, dim3(num_tokens), dim3(threads), 0, stream, out, ids, (const TW*)table, hidden,
                  vocab, sin_freq, positions);
+    })
+    LB_CHECK_LAUNCH("embedding");
+    return 0;
+  }
+  if (!pos_table && !out2 && hidden % 4 == 0 && hidden <= 65535 * 256 && (uintptr_t)out % 16 == 0 && (uintptr_t)table % (table_dtype == LB_BF16 ? 8 : 16) == 0) {
+    LB_DISPATCH_DTYPE(table_dtype, TW, {
+      lb::launch(lb::embedding_x4_kernel<TW>, dim3(num_tokens, (hidden / 4 + threads - 1) / threads), dim3(threads), 0, stream, out, ids,
+                 (const TW*)table, hidden, vocab, scale);
     })
     LB_CHECK_LAUNCH("embedding");
     return 0;

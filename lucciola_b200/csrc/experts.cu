@@ -607,6 +607,53 @@ __global__ void expert_combine_kernel(TO* __restrict__ out, const float* __restr
   }
 }
 
+__device__ __forceinline__ float4 combine_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 combine_load4(const bf16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+  return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
+
+// The same without a gate, for up to eight choices a token and rows in whole words: four neighbouring columns a thread, a CTA 1024
+// of them, and a thread's rows all requested at once (the kernel above asks for a value, adds it and asks for the next, one CTA a
+// token: 12 us for 8 tokens of four rows of 4096).  The same sums.
+template <typename TO, typename TA>
+__global__ void __launch_bounds__(256) expert_combine_x4_kernel(TO* __restrict__ out, const float* __restrict__ y, const float* __restrict__ weights,
+                                                                float weight, const int* __restrict__ place_of, const TA* __restrict__ always, int top,
+                                                                int width) {
+  pdl_trigger();
+  const int t = blockIdx.x, j = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  pdl_wait();
+  if (j >= width) return;
+  int places[8];
+  float w[8];
+  float4 r[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    places[k] = k < top ? place_of[(size_t)t * top + k] : 0;
+    w[k] = k < top && weights ? weights[(size_t)t * top + k] : weight;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (k < top) r[k] = *reinterpret_cast<const float4*>(y + (size_t)places[k] * width + j);
+  float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (always) b = combine_load4(always + (size_t)t * width + j);
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (k < top) {
+      acc.x = fmaf(w[k], r[k].x, acc.x); acc.y = fmaf(w[k], r[k].y, acc.y); acc.z = fmaf(w[k], r[k].z, acc.z); acc.w = fmaf(w[k], r[k].w, acc.w);
+    }
+  if (always) { acc.x += b.x; acc.y += b.y; acc.z += b.z; acc.w += b.w; }
+  TO* o = out + (size_t)t * width + j;
+  if constexpr (sizeof(TO) == 2) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
+    *reinterpret_cast<uint2*>(o) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  } else {
+    *reinterpret_cast<float4*>(o) = acc;
+  }
+}
+
 }  // namespace lb
 
 // ids [T, top] int32, weights [T, top] float32 from logits [T, ld] float32 and correction [experts] float32 (may be null)
@@ -754,6 +801,17 @@ LB_EXPORT int lb_expert_combine(void* out, int out_dtype, const float* y, const 
   LB_CHECK_ARG(lb::valid_dtype(out_dtype) && lb::valid_dtype(always_dtype) && out && y && place_of && top > 0 && width > 0, "expert_combine: bad arguments");
   if (num_tokens <= 0) return 0;
   const int threads = width >= 1024 ? 256 : 128;
+  auto words = [](const void* x, int dtype) { return (uintptr_t)x % (dtype == LB_BF16 ? 8 : 16) == 0; };
+  if (!gate && top <= 8 && width % 4 == 0 && width <= 65535 * 512 && (uintptr_t)y % 16 == 0 && words(out, out_dtype) && words(always, always_dtype)) {
+    const dim3 grid(num_tokens, (width / 4 + threads - 1) / threads);
+    LB_DISPATCH_DTYPE(out_dtype, TO, {
+      LB_DISPATCH_DTYPE(always_dtype, TA, {
+        lb::launch(lb::expert_combine_x4_kernel<TO, TA>, grid, dim3(threads), 0, stream, (TO*)out, y, weights, weight, place_of, (const TA*)always, top, width);
+      })
+    })
+    LB_CHECK_LAUNCH("expert_combine");
+    return 0;
+  }
   LB_DISPATCH_DTYPE(out_dtype, TO, {
     LB_DISPATCH_DTYPE(always_dtype, TA, {
       lb::launch(lb::expert_combine_kernel<TO, TA>, dim3(num_tokens), dim3(threads), 0, stream, (TO*)out, y, weights, weight, place_of,
