@@ -38,3 +38,50 @@ def test_embedding_rows(tokens, hidden, scale, dtype):
     ops.embedding(out, ids, table, stream(), scale=scale)
     want = table.float()[torch.where(ids < 50, ids, 0).long()] * scale
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("nq,nkv,d", [(1, 1, 64), (3, 1, 64), (5, 2, 128), (32, 8, 128), (2, 1, 256), (7, 3, 256)])
+@pytest.mark.parametrize("tokens", [1, 9, 700])
+@pytest.mark.parametrize("norm,rotate,pages,pad", [("qk", True, True, 0), ("k", True, False, 0), ("q", False, True, 8), ("", True, True, 0), ("qk", True, True, 4),
+                                                   ("qk", True, False, 2)])
+def test_rope_rows(nq, nkv, d, tokens, norm, rotate, pages, pad):
+    """Heads of whole 16-byte words (pad 0 and 8) and rows that are not: the result's rounding, 2^-9 of each, behind 32-bit sums."""
+    from lucciola_b200 import ops
+    torch.manual_seed(tokens + nq)
+    a, b, ps = nq * d, (nq + nkv) * d, 16
+    qkv = torch.randn(tokens, b + nkv * d + pad, device=DEV).bfloat16()
+    weight = lambda on: 1 + 0.2 * torch.randn(d, device=DEV) if on else None
+    qw, kw = weight("q" in norm), weight("k" in norm)
+    inv = 1e4 ** (-torch.arange(0, d, 2, device=DEV, dtype=torch.float32) / d) if rotate else None
+    pos = torch.arange(tokens, device=DEV, dtype=torch.int32) * 3 + 5
+    seq = torch.arange(tokens, device=DEV, dtype=torch.int32) % 3
+    table = torch.randperm(3 * (tokens * 3 // ps + 2), device=DEV).to(torch.int32).view(3, -1).contiguous()
+    q_out = torch.empty(tokens, nq, d, device=DEV, dtype=torch.bfloat16)
+    shape = (table.numel(), nkv, ps, d) if pages else (tokens, nkv, d)
+    k_to, v_to = torch.full(shape, 9.0, device=DEV).bfloat16(), torch.full(shape, 9.0, device=DEV).bfloat16()
+    into = dict(k_cache=k_to, v_cache=v_to, token_seq=seq, block_table=table, page_size=ps) if pages else dict(k_out=k_to, v_out=v_to)
+    ops.rope_kv(qkv[:, :a], qkv[:, a:b], qkv[:, b:b + nkv * d], q_out, pos, nq, nkv, d, 1e-6, stream(), q_norm_w=qw, k_norm_w=kw,
+                inv_freq=inv, rot_dim=d if rotate else 0, **into)
+
+    def plain(x, w):
+        x = x.double()
+        if w is not None:
+            x = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+        if inv is not None:
+            at = (pos.float()[:, None] * inv).double()[:, None]
+            lo, hi = x[..., :d // 2], x[..., d // 2:]
+            x = torch.cat([lo * at.cos() - hi * at.sin(), lo * at.sin() + hi * at.cos()], -1)
+        return x
+
+    def near(got, want):
+        return bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all())
+
+    assert near(q_out, plain(qkv[:, :a].reshape(tokens, nq, d), qw))
+    if pages:
+        page = table[seq.long(), (pos // ps).long()].long()
+        k_got, v_got = k_to[page, :, (pos % ps).long()], v_to[page, :, (pos % ps).long()]
+        assert (v_to != 9).any(-1).sum() == tokens * nkv                              # no other slot was written
+    else:
+        k_got, v_got = k_to, v_to
+    assert near(k_got, plain(qkv[:, a:b].reshape(tokens, nkv, d), kw))
+    assert torch.equal(v_got, qkv[:, b:b + nkv * d].reshape(tokens, nkv, d))
