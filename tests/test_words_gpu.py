@@ -85,3 +85,20 @@ def test_rope_rows(nq, nkv, d, tokens, norm, rotate, pages, pad):
         k_got, v_got = k_to, v_to
     assert near(k_got, plain(qkv[:, a:b].reshape(tokens, nkv, d), kw))
     assert torch.equal(v_got, qkv[:, b:b + nkv * d].reshape(tokens, nkv, d))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (8, 16, 4096), (7, 128, 2048), (9, 33, 5000), (16, 64, 2056), (3, 16, 8192)])
+@pytest.mark.parametrize("out_type,post", [(torch.float32, None), (torch.bfloat16, None), (torch.float32, "cap")])
+def test_product_of_few_features(M, N, K, out_type, post):
+    """K products of bfloat16 values summed in 32 bits; each feature is a CTA's, so the sizes around its words and tokens matter."""
+    from lucciola_b200 import ops
+    torch.manual_seed(M)
+    x, w = torch.randn(M, K + 8, device=DEV).bfloat16()[:, 8:], torch.randn(N, K, device=DEV).bfloat16()
+    y = torch.full((M, N + 1), 7.0, dtype=out_type, device=DEV)
+    ops.gemm_tcgen05(y[:, :N], x, w, stream(), post=post, post_c=5.0)
+    terms = x.double()[:, None] * w.double()
+    want = terms.sum(-1)
+    if post:
+        want = 5.0 * torch.tanh(want / 5.0)
+    bound = (K / 256 + 13) * 2.0 ** -24 * terms.abs().sum(-1) + (2.0 ** -8 * want.abs() if out_type == torch.bfloat16 else 0) + 1e-6 * (post is not None)
+    assert ((y[:, :N].double() - want).abs() <= bound).all() and (y[:, N] == 7).all()
