@@ -119,12 +119,24 @@ __global__ void __launch_bounds__(256) short_conv_x4_tokens_kernel(float* __rest
   }
 }
 
-// Steps of one token a sequence: the token's output and the state's move in one pass over the state.
+// Steps of one token a sequence: the token's output and the state's move in one pass over the state.  The CTAs from `round_from`
+// on round other columns of the same rows, which the next product wants in bfloat16, so that these need no launch of their own.
 __global__ void __launch_bounds__(256) short_conv_step_kernel(float* __restrict__ out, long long out_ld, const float* __restrict__ x, long long x_ld,
                                                               const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ state,
-                                                              const int* __restrict__ slots, int channels, int act) {
+                                                              const int* __restrict__ slots, int channels, int act, int round_from,
+                                                              bf16* __restrict__ rounded, const float* __restrict__ round_x, long long round_ld, int round_n) {
   pdl_trigger();
-  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4, s = blockIdx.x;
+  const int s = blockIdx.x;
+  if ((int)blockIdx.y >= round_from) {
+    const int c = ((blockIdx.y - round_from) * blockDim.x + threadIdx.x) * 4;
+    pdl_wait();
+    if (c >= round_n) return;
+    const float4 y = *reinterpret_cast<const float4*>(round_x + (size_t)s * round_ld + c);
+    __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
+    *reinterpret_cast<uint2*>(rounded + (size_t)s * round_n + c) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    return;
+  }
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (c >= channels) { pdl_wait(); return; }
   float4 f[4], v[4], b = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -208,16 +220,21 @@ LB_EXPORT int lb_short_conv(float* out, long long out_ld, const float* x, long l
 }
 
 // One token a sequence, four taps: the outputs, and the state moved on, in one launch.  Returns 3 (and launches nothing) for
-// operands that are not in whole 16-byte words.
+// operands that are not in whole 16-byte words.  `rounded` (may be null): [num_seqs, round_n] bfloat16 receives the columns at round_x.
 LB_EXPORT int lb_short_conv_step(float* out, long long out_ld, const float* x, long long x_ld, const float* w, const float* bias,
-                                 float* state, const int* slots, int num_seqs, int channels, int act, cudaStream_t stream) {
+                                 float* state, const int* slots, int num_seqs, int channels, int act, void* rounded, const float* round_x,
+                                 long long round_ld, int round_n, cudaStream_t stream) {
   LB_CHECK_ARG(out && x && w && state && slots && num_seqs >= 0 && channels > 0, "short_conv_step: bad arguments");
+  LB_CHECK_ARG(!rounded || (round_x && round_n > 0 && round_ld >= round_n), "short_conv_step: bad columns to round");
   LB_CHECK_ARG(out != x, "short_conv_step: the output must not be the input");
   auto a16 = [](const void* q) { return (uintptr_t)q % 16 == 0; };
   const int threads = 64, by = (channels / 4 + threads - 1) / threads;
-  if (channels % 4 || out_ld % 4 || x_ld % 4 || !a16(out) || !a16(x) || !a16(w) || !a16(bias) || !a16(state) || by > 65535) return 3;
+  if (rounded && (round_n % 4 || round_ld % 4 || !a16(round_x) || (uintptr_t)rounded % 8)) return 3;
+  const int more = rounded ? (round_n / 4 + threads - 1) / threads : 0;
+  if (channels % 4 || out_ld % 4 || x_ld % 4 || !a16(out) || !a16(x) || !a16(w) || !a16(bias) || !a16(state) || by + more > 65535) return 3;
   if (num_seqs == 0) return 0;
-  lb::launch(lb::short_conv_step_kernel, dim3(num_seqs, by), dim3(threads), 0, stream, out, out_ld, x, x_ld, w, bias, state, slots, channels, act);
+  lb::launch(lb::short_conv_step_kernel, dim3(num_seqs, by + more), dim3(threads), 0, stream, out, out_ld, x, x_ld, w, bias, state, slots, channels, act,
+             by, (lb::bf16*)rounded, round_x, round_ld, round_n);
   LB_CHECK_LAUNCH("short_conv_step");
   return 0;
 }

@@ -73,7 +73,10 @@ __global__ void __launch_bounds__(256, RPT == 16 ? 2 : RPT == 8 ? 3 : 4) state_s
     w = sp;
   }
   if (DELTA) w = ss_sigmoid(p.b[(size_t)t * p.b_ld + h]);
-  if (KIND == SS_CHANNELS && tid >= 128) gs[d] = d < p.dim ? p.a[(size_t)t * p.a_ld + (size_t)h * p.dim + d] : 1.f;
+  if (KIND == SS_CHANNELS && tid >= 128) {         // as channel_decay_kernel of state_recurrence.cu
+    gs[d] = 1.f;
+    if (d < p.dim) gs[d] = expf(-expf(p.A_log[h]) * ss_softplus(p.a[(size_t)t * p.a_ld + (size_t)h * p.dim + d] + p.dt_bias[h * p.dim + d]));
+  }
   if (KIND == SS_HGRN2) {
     if (tid < 128) x = ss_silu(x);
     else {
@@ -177,7 +180,8 @@ static cudaError_t launch_state_step_kind(const StateStepParams& p, int num_seqs
 
 }  // namespace lb
 
-// Every sequence of the step brings one token.  Operands as lb_chunk_recurrence's.
+// Every sequence of the step brings one token.  Operands as lb_chunk_recurrence's; channel decays are formed here from `a` as the
+// product left it (with 16 heads a CTA has 128 of them to form, and a launch less to wait for).
 LB_EXPORT int lb_state_step(int kind, const float* q, long long q_ld, const float* k, long long k_ld, const float* v, long long v_ld,
                             const float* a, long long a_ld, const float* b, long long b_ld, const float* A_log, const float* dt_bias,
                             const float* D, const float* bias, const float* lower, const float* decay, float* state, float* out,
@@ -189,8 +193,9 @@ LB_EXPORT int lb_state_step(int kind, const float* q, long long q_ld, const floa
   LB_CHECK_ARG(dim > 0 && dim <= 128 && vdim > 0 && vdim % 4 == 0 && ((uintptr_t)state & 15) == 0, "state_step: a state of %d x %d", dim, vdim);
   LB_CHECK_ARG(num_seqs >= 0 && num_seqs <= 65535, "state_step: %d sequences", num_seqs);
   LB_CHECK_ARG(kind != lb::SS_FIXED || decay, "state_step: no decays");
-  LB_CHECK_ARG((kind != lb::SS_SSM && kind != lb::SS_DELTA) || (a && A_log && dt_bias), "state_step: null argument");
-  LB_CHECK_ARG((kind != lb::SS_DELTA && kind != lb::SS_CHANNELS) || (a && b), "state_step: null argument");
+  const bool delta = kind == lb::SS_DELTA || kind == lb::SS_CHANNELS;
+  LB_CHECK_ARG((kind != lb::SS_SSM && !delta) || (a && A_log && dt_bias), "state_step: null argument");
+  LB_CHECK_ARG(!delta || b, "state_step: null argument");
   LB_CHECK_ARG(kind != lb::SS_HGRN2 || (bias && lower), "state_step: null argument");
   if (num_seqs == 0) return 0;
   lb::StateStepParams p;

@@ -85,7 +85,8 @@ _SIGNATURES = {
                            c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "lb_short_conv": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                       c_int, c_int, c_int, c_int, c_void_p],
-    "lb_short_conv_step": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "lb_short_conv_step": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
+                           c_longlong, c_int, c_void_p],
     "lb_short_conv_state": [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "lb_state_recurrence": [c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
                             c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
@@ -628,9 +629,9 @@ def short_conv_state(state: torch.Tensor, x: torch.Tensor, taps: int, step, stre
 
 
 def short_conv_step(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, state: torch.Tensor, step, stream: int,
-                    act: bool = True) -> bool:
+                    act: bool = True, rounded: tuple | None = None) -> bool:
     """short_conv and short_conv_state in one launch, for steps of one token a sequence, four taps and rows in whole 16-byte words;
-    False (and nothing done) for any other."""
+    False (and nothing done) for any other.  `rounded` = (out, x): round_cols(out, x) is done by the same launch (out bfloat16)."""
     if weight.shape[0] != 4 or step.max_q_len != 1 or not step.q_lens.count(1) == step.num_seqs == len(step.q_lens) == x.shape[0]:
         return False
     _rows32(out, "convolution output"); _rows32(x, "convolution input"); _check(weight, "taps", torch.float32)
@@ -640,8 +641,14 @@ def short_conv_step(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bi
         raise KernelError(f"the taps are {tuple(weight.shape)} for rows of {C}, the output {tuple(out.shape)}, the state {tuple(state.shape)}")
     if bias is not None:
         _check(bias, "convolution bias", torch.float32)
+    r_out, r_x = rounded if rounded is not None else (None, None)
+    if r_out is not None:
+        _check(r_out, "rounded copy", torch.bfloat16); _rows32(r_x, "rows to round")
+        if r_out.shape != r_x.shape or r_x.shape[0] != T:
+            raise KernelError("a rounded copy has its source's shape, a row a token")
     rc = _invoke("lb_short_conv_step", out.data_ptr(), out.stride(0), x.data_ptr(), x.stride(0), weight.data_ptr(), _ptr(bias), state.data_ptr(),
-                 step.state_slots.data_ptr(), T, C, 1 if act else 0, stream)
+                 step.state_slots.data_ptr(), T, C, 1 if act else 0, _ptr(r_out), _ptr(r_x), r_x.stride(0) if r_x is not None else 0,
+                 r_x.shape[1] if r_x is not None else 0, stream)
     if rc not in (0, 3):
         raise KernelError(library().lb_last_error().decode())
     return rc == 0
@@ -724,7 +731,7 @@ def state_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
     state [slots + 1, heads, dim, vdim] float32 is read and written at each sequence's slot; out [T, heads * vdim] float32.
     `rows_decay` (delta rule only): a decay for every row of the state; a is then [T, heads * dim] and dt_bias [heads * dim], and
     a is overwritten with the decays (one pass over it before the recurrence, so that the CTAs that share a head do not each
-    form them again on the path from token to token).  `by_shape`: the kernel's layout may follow the step's shape (steps of
+    form them again on the path from token to token; steps of single tokens with `by_shape` leave it as it is).  `by_shape`: the kernel's layout may follow the step's shape (steps of
     single tokens keep sixteen state rows a lane, which issues fewer instructions; all others eight, which shortens the path
     from token to token); a column's terms are then added in an order that depends on the step.  Without it one layout
     serves every step, so a 32-bit result does not depend on how a sequence was cut.  Long portions then go through the
@@ -740,13 +747,13 @@ def state_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
             or tuple(a.shape) != (T, heads * dim if rows_decay else heads) or dt_bias.numel() != (heads * dim if rows_decay else heads)
             or tuple(out.shape) != (T, heads * vdim) or tuple(state.shape[1:]) != (heads, dim, vdim)):
         raise KernelError("the recurrence's operands do not fit its head counts and sizes")
-    if rows_decay:
-        _call("lb_channel_decay", a.data_ptr(), a.stride(0), A_log.data_ptr(), dt_bias.data_ptr(), T, heads, dim, stream)
     kind = "channels" if rows_decay else "delta" if delta else "ssm"
     if by_shape and single_tokens(step, dim, vdim, state):
         _state_step(kind, _rows(q), _rows(k), _rows(v), state, out, step, heads, groups, dim, vdim, stream, a=_rows(a), b=_rows(b), A_log=A_log,
                     dt_bias=dt_bias, D=D, unit_norm=unit_norm, q_scale=q_scale, unit_eps=unit_eps)
         return
+    if rows_decay:
+        _call("lb_channel_decay", a.data_ptr(), a.stride(0), A_log.data_ptr(), dt_bias.data_ptr(), T, heads, dim, stream)
     long, skip = chunk_portions(kind, step, heads, dim, vdim) if by_shape else ([], 0)
     if long:
         _chunk_recurrence(kind, _rows(q), _rows(k), _rows(v), state, out, step, long, heads, groups, dim, vdim, stream, a=_rows(a), b=_rows(b),

@@ -128,7 +128,6 @@ class GatedDeltaRule(Mixer):
             raise ops.KernelError("a recurrent mixer has no cache another call could have written")
         rt, n, m = self.rt, self.qk_size, self.inner_size
         conv_cache, state = (cache[0], cache[1]) if len(cache) == 2 else (None, cache[0])
-        qkv = self.conv.forward(pre[:, :2 * n + m], step, conv_cache)
         T, H = pre.shape[0], self.heads
         c = 2 * n + m                                      # columns behind q | k | v
         gate = None
@@ -138,10 +137,10 @@ class GatedDeltaRule(Mixer):
         a = None
         if not self.decay_rank:
             a, c = pre[:, c:c + H], c + H
+        first = (rt.empty((T, self.low_rank)), pre[:, c:c + self.low_rank]) if self.low is not None else None
+        qkv = self.conv.forward(pre[:, :2 * n + m], step, conv_cache, rounded=first)
         if self.low is not None:
-            first = rt.empty((T, self.low_rank))
-            ops.round_cols(first, pre[:, c:c + self.low_rank], rt.stream)
-            second = self.low.forward(first, out_dtype=torch.float32)
+            second = self.low.forward(first[0], out_dtype=torch.float32)
             at = 0
             if self.decay_rank:
                 a, at = second[:, :H * self.dim], H * self.dim

@@ -47,13 +47,18 @@ class ShortConv(Part):
     def cache_request(self) -> Optional[StateSlot]:
         return StateSlot((self.taps - 1, self.channels), torch.float32) if self.taps > 1 else None
 
-    def forward(self, x: torch.Tensor, step: StepContext, cache: Optional[StateCacheView]) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, step: StepContext, cache: Optional[StateCacheView], rounded: Optional[tuple] = None) -> torch.Tensor:
         """x: float32 [T, channels] (may be a column range).  Returns y, float32 [T, channels]; the sequences' states
-        move on to the end of the step."""
+        move on to the end of the step.  `rounded` = (out, x'): x', float32 [T, n], is rounded into out on the way."""
         out = self.rt.empty(x.shape, torch.float32)
         state = cache.state if self.taps > 1 else None
-        if state is not None and ops.short_conv_step(out, x, self.weight, self.bias, state, step, self.rt.stream, act=self.act):
+        together = rounded if rounded is not None and rounded[0].dtype == torch.bfloat16 and rounded[0].shape[1] % 4 == 0 else None
+        if state is not None and ops.short_conv_step(out, x, self.weight, self.bias, state, step, self.rt.stream, act=self.act, rounded=together):
+            if rounded is not None and together is None:
+                ops.round_cols(*rounded, self.rt.stream)
             return out
+        if rounded is not None:
+            ops.round_cols(*rounded, self.rt.stream)
         ops.short_conv(out, x, self.weight, self.bias, state, step, self.rt.stream, act=self.act)
         if state is not None:
             ops.short_conv_state(state, x, self.taps, step, self.rt.stream)

@@ -102,3 +102,21 @@ def test_product_of_few_features(M, N, K, out_type, post):
         want = 5.0 * torch.tanh(want / 5.0)
     bound = (K / 256 + 13) * 2.0 ** -24 * terms.abs().sum(-1) + (2.0 ** -8 * want.abs() if out_type == torch.bfloat16 else 0) + 1e-6 * (post is not None)
     assert ((y[:, :N].double() - want).abs() <= bound).all() and (y[:, N] == 7).all()
+
+
+@pytest.mark.parametrize("T,channels,n", [(1, 4, 4), (5, 260, 128), (64, 6144, 124), (3, 512, 300)])
+def test_conv_step_rounds_on_the_way(T, channels, n):
+    """The convolution's step with columns to round: both as the launches that do one of them, to the bit."""
+    from types import SimpleNamespace
+    from lucciola_b200 import ops
+    torch.manual_seed(T)
+    x, w = torch.randn(T, channels + n + 4, device=DEV), torch.randn(4, channels, device=DEV)
+    state = torch.randn(T + 1, 3, channels, device=DEV)
+    step = SimpleNamespace(max_q_len=1, q_lens=[1] * T, num_seqs=T, state_slots=torch.arange(T, 0, -1, dtype=torch.int32, device=DEV))
+    want, state2 = torch.empty(T, channels, device=DEV), state.clone()
+    assert ops.short_conv_step(want, x[:, :channels], w, None, state, step, stream())
+    first, plain = (torch.empty(T, n, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    ops.round_cols(plain, x[:, channels:channels + n], stream())
+    got = torch.empty_like(want)
+    assert ops.short_conv_step(got, x[:, :channels], w, None, state2, step, stream(), rounded=(first, x[:, channels:channels + n]))
+    assert torch.equal(got, want) and torch.equal(state2, state) and torch.equal(first, plain)
