@@ -87,7 +87,9 @@ gemm_heads_mma_kernel(bf16* __restrict__ y, const bf16* __restrict__ x, const bf
 
 // The same for few rows: the launch is the latency of fetching each head's matrix once, so a CTA of four warps takes 32 output
 // columns over the whole of K, requests its weights in one go while the kernel ahead may still run, then its 16 MT rows of x,
-// and multiplies when all has landed (a warp eight columns, K in steps of 32, what is missing there zeros).
+// and multiplies when all has landed (a warp eight columns, K in steps of 32, what is missing there zeros).  Gates are fetched with
+// the rows and neighbours stored together.  64 rows of 32 heads, one launch behind the other: K 512 to N 128 with gates 11.6 -> 5.5 us
+// (64 rows a CTA left it one CTA an SM with 100 KB to wait for), K 128 to N 512 7.5 -> 4.9 us.
 __device__ __forceinline__ void gh_cp_async16(void* dst, const void* src, bool valid) {
   const int n = valid ? 16 : 0;             // 0: the 16 bytes are filled with zeros, nothing is read
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
@@ -104,7 +106,7 @@ template <int MT>
 __global__ void __launch_bounds__(128)
 gemm_heads_few_kernel(bf16* __restrict__ y, const bf16* __restrict__ x, const bf16* __restrict__ w, int M, int N, int K,
                       long long ldx, long long ldy, long long bx, long long bw, long long by,
-                      const float* __restrict__ gate, long long ldg, int gate_one) {
+                      const float* __restrict__ gate, long long ldg, int gate_one, int pairs) {
   extern __shared__ __align__(16) uint8_t gf_raw[];
   const int LD = gf_ld(K), pieces = (LD - 8) / 8;
   bf16* Ws = reinterpret_cast<bf16*>(gf_raw);               // [32][LD]
@@ -113,16 +115,37 @@ gemm_heads_few_kernel(bf16* __restrict__ y, const bf16* __restrict__ x, const bf
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n0 = blockIdx.x * GF_BN, m0 = blockIdx.y * 16 * MT, b = blockIdx.z;
   x += (size_t)b * bx; w += (size_t)b * bw; y += (size_t)b * by;
-  for (int i = tid; i < GF_BN * pieces; i += 128) {
-    const int r = i / pieces, c = (i - r * pieces) * 8;
+  // piece `at` of row `r`, 128 pieces further each time
+  const int r0 = tid / pieces, at0 = tid - r0 * pieces, dr = 128 / pieces, dat = 128 - dr * pieces;
+  for (int r = r0, at = at0; r < GF_BN;) {
+    const int c = at * 8;
     const bool ok = n0 + r < N && c < K;
     gh_cp_async16(Ws + r * LD + c, ok ? w + (size_t)(n0 + r) * K + c : w, ok);
+    r += dr; at += dat;
+    if (at >= pieces) { at -= pieces; ++r; }
   }
   pdl_wait();
-  for (int i = tid; i < 16 * MT * pieces; i += 128) {
-    const int r = i / pieces, c = (i - r * pieces) * 8;
+  for (int r = r0, at = at0; r < 16 * MT;) {
+    const int c = at * 8;
     const bool ok = m0 + r < M && c < K;
     gh_cp_async16(Xs + r * LD + c, ok ? x + (size_t)(m0 + r) * ldx + c : x, ok);
+    r += dr; at += dat;
+    if (at >= pieces) { at -= pieces; ++r; }
+  }
+  // the gates are on their way with the rows
+  const int nc = n0 + warp * 8 + 2 * (lane & 3);
+  float gates[MT][2][2];
+  if (gate) {
+    gate += gate_one ? (size_t)b : (size_t)b * N;
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int m = m0 + 16 * i + (lane >> 2) + 8 * half;
+          gates[i][half][j] = m < M && nc + j < N ? gate[(size_t)m * ldg + (gate_one ? 0 : nc + j)] : 0.f;
+        }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
@@ -144,20 +167,23 @@ gemm_heads_few_kernel(bf16* __restrict__ y, const bf16* __restrict__ x, const bf
       mma_bf16_16816(acc[i], a, hi);
     }
   }
-  if (gate) gate += gate_one ? (size_t)b : (size_t)b * N;
 #pragma unroll
   for (int i = 0; i < MT; ++i)
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int m = m0 + 16 * i + (lane >> 2) + 8 * half;
       if (m >= M) continue;
+      float v[2];
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const int n = n0 + warp * 8 + 2 * (lane & 3) + j;
-        if (n >= N) continue;
-        float v = acc[i][2 * half + j];
-        if (gate) v *= 1.f / (1.f + expf(-gate[(size_t)m * ldg + (gate_one ? 0 : n)]));
-        y[(size_t)m * ldy + n] = __float2bfloat16_rn(v);
+        v[j] = acc[i][2 * half + j];
+        if (gate) v[j] *= 1.f / (1.f + expf(-gates[i][half][j]));
+      }
+      bf16* dst = y + (size_t)m * ldy + nc;
+      if (pairs && nc + 1 < N) *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(v[0], v[1]);
+      else {
+        if (nc < N) dst[0] = __float2bfloat16_rn(v[0]);
+        if (nc + 1 < N) dst[1] = __float2bfloat16_rn(v[1]);
       }
     }
 }
@@ -167,12 +193,13 @@ static cudaError_t launch_heads_few(dim3 grid, int K, cudaStream_t stream, bf16*
                                     long long bx, long long bw, long long by, const float* gate, long long ldg, int gate_one) {
   static int configured = 0;
   const int smem = gf_smem(K, MT);
+  const int pairs = (uintptr_t)y % 4 == 0 && ldy % 2 == 0 && by % 2 == 0;       // two neighbours in one store
   if (smem > 48 * 1024 && smem > configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_heads_few_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     configured = smem;
   }
-  launch(gemm_heads_few_kernel<MT>, grid, dim3(128), smem, stream, y, x, w, M, N, K, ldx, ldy, bx, bw, by, gate, ldg, gate_one);
+  launch(gemm_heads_few_kernel<MT>, grid, dim3(128), smem, stream, y, x, w, M, N, K, ldx, ldy, bx, bw, by, gate, ldg, gate_one, pairs);
   return cudaSuccess;
 }
 
@@ -192,9 +219,14 @@ LB_EXPORT int lb_gemm_heads_mma(void* y, const void* x, const void* w, int batch
   LB_CHECK_ARG(gate == nullptr || ldg >= (long long)batches * (gate_one ? 1 : N), "gemm_heads_mma: the gate's rows are too short");
   LB_CHECK_ARG((M + lb::GH_BM - 1) / lb::GH_BM <= 65535, "gemm_heads_mma: too many rows (%d)", M);
   if (M == 0) return 0;
-  const int mt = M <= 16 ? 1 : (M <= 32 ? 2 : 4);
+  int mt = M <= 16 ? 1 : (M <= 32 ? 2 : 4);
+  // The tokens are shared out as far as all CTAs still run at once: a CTA's time is that of bringing in its rows.  (32 heads of K 512,
+  // N 128, 64 tokens a CTA 11 us, 32 tokens 6.7, 16 tokens 5.5; 64 heads, where 32 tokens a CTA would be a wave and a half, 9.6 / 11.9.)
+  const long long wide = (long long)batches * ((N + lb::GF_BN - 1) / lb::GF_BN);
+  auto at_once = [&](int t) { const int n = 227 * 1024 / (lb::gf_smem(K, t) + 1024); return 148ll * (n < 16 ? n : 16); };
+  while (mt > 1 && wide * ((M + 8 * mt - 1) / (8 * mt)) <= at_once(mt / 2)) mt /= 2;
   if (M <= 64 && lb::gf_smem(K, mt) <= 112 * 1024) {        // two CTAs an SM
-    dim3 few((N + lb::GF_BN - 1) / lb::GF_BN, 1, batches);
+    dim3 few((N + lb::GF_BN - 1) / lb::GF_BN, (M + 16 * mt - 1) / (16 * mt), batches);
     cudaError_t e;
 #define LB_GF(MT_) e = lb::launch_heads_few<MT_>(few, K, stream, (lb::bf16*)y, (const lb::bf16*)x, (const lb::bf16*)w, M, N, ldx, ldy, bx, bw, by, gate, ldg, gate_one)
     if (mt == 1) LB_GF(1); else if (mt == 2) LB_GF(2); else LB_GF(4);

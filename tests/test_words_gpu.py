@@ -120,3 +120,22 @@ def test_conv_step_rounds_on_the_way(T, channels, n):
     got = torch.empty_like(want)
     assert ops.short_conv_step(got, x[:, :channels], w, None, state2, step, stream(), rounded=(first, x[:, channels:channels + n]))
     assert torch.equal(got, want) and torch.equal(state2, state) and torch.equal(first, plain)
+
+
+@pytest.mark.parametrize("heads,M,N,K", [(32, 64, 128, 512), (32, 33, 512, 128), (3, 17, 33, 40), (70, 64, 128, 512), (1, 1, 2, 8), (5, 48, 34, 264)])
+@pytest.mark.parametrize("gates", [0, 1, 2])
+def test_heads_of_few_rows(heads, M, N, K, gates):
+    """The tokens' shares by the number of heads, odd widths (no pairs of stores), rows of longer heads: K products in 32 bits, then bfloat16."""
+    from lucciola_b200 import ops
+    torch.manual_seed(M + N)
+    x = torch.randn(M, heads, K + 8, device=DEV).bfloat16()[:, :, 8:]
+    w = torch.randn(heads, N, K, device=DEV).bfloat16()
+    gate = torch.randn(M, heads * (N if gates == 2 else 1), device=DEV) if gates else None
+    y = torch.full((M, heads, N + 1), 9.0, device=DEV).bfloat16()
+    ops.gemm_heads(y[:, :, :N], x, w, stream(), gate=gate)
+    xd, wd = x.double(), w.double()
+    want, size = torch.einsum("mhk,hnk->mhn", xd, wd), torch.einsum("mhk,hnk->mhn", xd.abs(), wd.abs())
+    if gates:
+        g = torch.sigmoid(gate.double()).view(M, heads, -1)
+        want, size = want * g, size * g
+    assert ((y[:, :, :N].double() - want).abs() <= 2.0 ** -8 * want.abs() + (K / 8 + 4) * 2.0 ** -24 * size).all() and (y[:, :, N] == 9).all()
