@@ -26,15 +26,17 @@
 // decay for every row the chunk is cut into blocks of 16: pairs inside a block are formed one by one (their G is carried along
 // in registers), pairs of different blocks as (q_i G(block start, i)) . (k_j G(j, block start)).
 //
-// Everything is 32-bit.  The products run on the tensor cores as three TF32 products of operands split in two, x = hi + lo
-// with 11 bits each: what is dropped (lo * lo and the end of lo) is below 2^-21 of a term and has no direction.
+// Everything is 32-bit.  The products run on the tensor cores as six bfloat16 products of operands cut in three, which hold all 24
+// bits, 16 places at a time, and the sums from one 16 to the next are ordinary additions (see cr_step).  Decays and strengths that
+// are one number a token come out of 64 bits, and their products carry what rounding drops.  Against 64 bits the outputs before
+// the norm are 0.2 to 0.98 times as far off as those of the kernels that walk token by token, over the layers' sizes.
 //
-// Measured (B200, one prompt of 2048 tokens, 16 heads of 128 x 128; all launches, token by token -> here): HGRN2 421 -> 127 us,
-// delta rule 801 -> 178 us (solve 46, walk 72, outputs 60); fixed decays, four prompts of 1654 tokens in all, 403 -> 112 us.
-// What bounds it: mma.sync issues one product of 16 x 8 x 8 every 8 cycles a scheduler on this GPU whatever its type, so the three
-// TF32 products of a term are worth 1.3 times the ordinary 32-bit pipes, about 30 us of the states and outputs; the rest is the
-// splitting of operands (two integer operations at half rate and one addition an element) and the phases of a CTA waiting for
-// one another.
+// Measured (B200, all launches, token by token -> here): HGRN2, one prompt of 2048 tokens and 16 heads of 128 x 128, 403 -> 148 us; the
+// delta rule 865 -> 209; fixed decays, four prompts of 1654 tokens in all, 341 -> 133.  (Operands in two TF32 parts and sums in the
+// accumulator alone took 127, 170 and 100 and were 1.2 to 6 times as far off.)
+// What bounds it: mma.sync issues one product every 8 cycles a scheduler on this GPU whatever its type, so the six products of 16
+// places are worth 1.3 times the ordinary 32-bit pipes, about 30 us of the states and outputs; the rest is the cutting of operands
+// (some five operations an element, half of them at half rate) and the phases of a CTA waiting for one another.
 #include "common.cuh"
 #include "warp_mma.cuh"
 
@@ -71,10 +73,17 @@ struct ChunkParams {
   int base[CR_SEQS + 1];                 // its first chunk
 };
 
-__device__ __forceinline__ float cr_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
-__device__ __forceinline__ float cr_sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
-__device__ __forceinline__ float cr_silu(float x) { return __fdividef(x, 1.f + expf(-x)); }
-__device__ __forceinline__ float cr_silu_fast(float x) { return __fdividef(x, 1.f + __expf(-x)); }    // as decay_chunk_kernel's, within 2 ulp
+__device__ __forceinline__ float cr_silu(float x) { return x / (1.f + expf(-x)); }
+__device__ __forceinline__ float cr_silu_r(float x) { return x * __frcp_rn(1.f + expf(-x)); }       // a rounding more, a third of the instructions
+
+// 1 / sqrt(x) as r + rest: a token's factor errs for the whole row at once.
+__device__ __forceinline__ void cr_unit(float x, float scale, float& r, float& rest) {
+  r = 1.f / sqrtf(x);
+  const float p = r * r;
+  rest = 0.5f * r * fmaf(-x, fmaf(r, r, -p), fmaf(-x, p, 1.f));
+  rest = fmaf(scale, rest, fmaf(scale, r, -(scale * r)));
+  r *= scale;
+}
 template <typename F>
 __device__ __forceinline__ float4 cr_map(float4 x, F f) { return make_float4(f(x.x), f(x.y), f(x.z), f(x.w)); }
 __device__ __forceinline__ void cr_scale(float* x, float g) {
@@ -82,84 +91,111 @@ __device__ __forceinline__ void cr_scale(float* x, float g) {
   *y = make_float4(y->x * g, y->y * g, y->z * g, y->w * g);
 }
 
-// x as hi + lo: hi rounded to 11 significant bits, lo what is left, of which the product reads the first 11 (cut, but lo is as
-// often negative as positive, so the cut has no direction)
-__device__ __forceinline__ void cr_split(float x, uint32_t& hi, uint32_t& lo) {
-  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;   // (cvt.rna.tf32 does the same and is slower)
-  lo = __float_as_uint(x - __uint_as_float(hi));
+// Two numbers (the places that share a register of an operand) as three bfloat16 each, x = h + m + l: rounded to 8 bits, the rest
+// rounded to 8, and what is left, which has no more than 8.
+struct Split { uint32_t h, m, l; };
+__device__ __forceinline__ Split cr_split(float x, float y) {
+  Split s;
+  s.h = pack_bf16(x, y);
+  x -= __uint_as_float(s.h << 16); y -= __uint_as_float(s.h & 0xffff0000u);
+  s.m = pack_bf16(x, y);
+  x -= __uint_as_float(s.m << 16); y -= __uint_as_float(s.m & 0xffff0000u);
+  s.l = pack_bf16(x, y);
+  return s;
 }
 
-__device__ __forceinline__ void mma_tf32(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  asm(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+__device__ __forceinline__ void cr_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// The 16 x 8 tile of a row-major 32-bit matrix at `tile` (shared address of its first element, `pitch` floats a row) as the
-// left operand of a TF32 product, split in two.
-__device__ __forceinline__ void cr_left(uint32_t tile, int pitch, int lane, uint32_t* hi, uint32_t* lo) {
-  uint32_t r[4];
-  ldmatrix_x4(tile + 4 * ((((lane >> 3) & 1) * 8 + (lane & 7)) * pitch + (lane >> 4) * 4), r[0], r[1], r[2], r[3]);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) cr_split(__uint_as_float(r[i]), hi[i], lo[i]);
-}
-// The same of a matrix that lies transposed: [8 places][16 rows], rows 8 or 24 floats apart modulo 32.
-__device__ __forceinline__ void cr_left_t(const float* tile, int pitch, int lane, uint32_t* hi, uint32_t* lo) {
-  const float* x = tile + (lane & 3) * pitch + (lane >> 2);
-  cr_split(x[0], hi[0], lo[0]);
-  cr_split(x[8], hi[1], lo[1]);
-  cr_split(x[4 * pitch], hi[2], lo[2]);
-  cr_split(x[4 * pitch + 8], hi[3], lo[3]);
-}
-// An 8 x 8 right operand: from [8 columns][8 places] (ldmatrix), from [8 places][8 columns] (plain loads), both split; and two
-// of the first form that are split already.
-__device__ __forceinline__ void cr_right(uint32_t tile, int pitch, int lane, uint32_t* hi, uint32_t* lo) {
-  uint32_t r[2];
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
-               : "=r"(r[0]), "=r"(r[1]) : "r"(tile + 4 * ((lane & 7) * pitch + ((lane >> 3) & 1) * 4)));
-  cr_split(__uint_as_float(r[0]), hi[0], lo[0]);
-  cr_split(__uint_as_float(r[1]), hi[1], lo[1]);
-}
-__device__ __forceinline__ void cr_right_t(const float* tile, int pitch, int lane, uint32_t* hi, uint32_t* lo) {
-  const float* x = tile + (lane & 3) * pitch + (lane >> 2);
-  cr_split(x[0], hi[0], lo[0]);
-  cr_split(x[4 * pitch], hi[1], lo[1]);
-}
-__device__ __forceinline__ void cr_right2(uint32_t tile, int pitch, int lane, uint32_t* r) {
-  ldmatrix_x4(tile + 4 * (((lane >> 4) * 8 + (lane & 7)) * pitch + ((lane >> 3) & 1) * 4), r[0], r[1], r[2], r[3]);
-}
+// Operands of a product over 16 places, split.  The order of the places within a product is free as long as both sides agree: a
+// lane's registers hold places q, q + 4 | q + 8, q + 12 (q = lane % 4), which is what 32-bit loads give it.
+struct Left { uint32_t h[4], m[4], l[4]; };
+struct Right { uint32_t h[2], m[2], l[2]; };
+__device__ __forceinline__ void cr_put(Left& a, int i, float x, float y) { const Split s = cr_split(x, y); a.h[i] = s.h; a.m[i] = s.m; a.l[i] = s.l; }
+__device__ __forceinline__ void cr_put(Right& b, int i, float x, float y) { const Split s = cr_split(x, y); b.h[i] = s.h; b.m[i] = s.m; b.l[i] = s.l; }
 
-// MT x NT tiles of one step of 8 places.  The two cross terms go to `small`, so that the chains are short and their rounding
-// is; products on one accumulator stand as far apart as there are tiles.
-template <int MT, int NT>
-__device__ __forceinline__ void cr_step(float (*acc)[NT][4], float (*small)[NT][4], const uint32_t (*ah)[4], const uint32_t (*al)[4],
-                                        const uint32_t (*bh)[2], const uint32_t (*bl)[2]) {
+// The 16 x 16 tile of a row-major 32-bit matrix at `tile` (shared address of its first element, `pitch` floats a row).
+__device__ __forceinline__ void cr_left(uint32_t tile, int pitch, int lane, Left& a) {
+  const uint32_t at = tile + 4 * ((((lane >> 3) & 1) * 8 + (lane & 7)) * pitch + (lane >> 4) * 4);
 #pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int t = 0; t < NT; ++t) mma_tf32(small[m][t], al[m], bh[t][0], bh[t][1]);
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int t = 0; t < NT; ++t) mma_tf32(acc[m][t], ah[m], bh[t][0], bh[t][1]);
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int t = 0; t < NT; ++t) mma_tf32(small[m][t], ah[m], bl[t][0], bl[t][1]);
-}
-
-// 16 rows of `left` times NT n-tiles of `right` (both row-major along the KS * 8 places summed over).
-template <int KS, int NT>
-__device__ __forceinline__ void cr_scores(uint32_t left, uint32_t right, int pitch, int lane, float (*acc)[NT][4], float (*small)[NT][4]) {
-#pragma unroll 2
-  for (int ks = 0; ks < KS; ++ks) {
-    uint32_t ah[1][4], al[1][4], bh[NT][2], bl[NT][2];
-    cr_left(left + 32 * ks, pitch, lane, ah[0], al[0]);
-#pragma unroll
-    for (int t = 0; t < NT; ++t) cr_right(right + 4 * (8 * t * pitch + 8 * ks), pitch, lane, bh[t], bl[t]);
-    cr_step<1, NT>(acc, small, ah, al, bh, bl);
+  for (int i = 0; i < 2; ++i) {
+    uint32_t r[4];
+    ldmatrix_x4(at + 32 * i, r[0], r[1], r[2], r[3]);
+    cr_put(a, 2 * i, __uint_as_float(r[0]), __uint_as_float(r[2]));
+    cr_put(a, 2 * i + 1, __uint_as_float(r[1]), __uint_as_float(r[3]));
   }
+}
+// The same of a matrix that lies transposed: [16 places][16 rows], rows 8 or 24 floats apart modulo 32.
+__device__ __forceinline__ void cr_left_t(const float* tile, int pitch, int lane, Left& a) {
+  const float* x = tile + (lane & 3) * pitch + (lane >> 2);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    cr_put(a, 2 * i, x[8 * i * pitch], x[(8 * i + 4) * pitch]);
+    cr_put(a, 2 * i + 1, x[8 * i * pitch + 8], x[(8 * i + 4) * pitch + 8]);
+  }
+}
+// A right operand of 8 columns: from [8 columns][16 places] (ldmatrix), from [16 places][8 columns] (plain loads).
+__device__ __forceinline__ void cr_right(uint32_t tile, int pitch, int lane, Right& b) {
+  uint32_t r[4];
+  ldmatrix_x4(tile + 4 * ((lane & 7) * pitch + (lane >> 3) * 4), r[0], r[1], r[2], r[3]);
+  cr_put(b, 0, __uint_as_float(r[0]), __uint_as_float(r[1]));
+  cr_put(b, 1, __uint_as_float(r[2]), __uint_as_float(r[3]));
+}
+__device__ __forceinline__ void cr_right_t(const float* tile, int pitch, int lane, Right& b) {
+  const float* x = tile + (lane & 3) * pitch + (lane >> 2);
+  cr_put(b, 0, x[0], x[4 * pitch]);
+  cr_put(b, 1, x[8 * pitch], x[12 * pitch]);
+}
+
+// 16 rows times NT tiles of 8 columns over 16 places: the six products of parts that matter (m * l and l * l are below 2^-25 of a
+// term), the smallest first, in accumulators of their own; their sum is then added to `acc` rounded to nearest.  The tensor core
+// cuts its sums: a chain through its accumulator over all places leaned towards zero and was 1.2 to 6 times as far from 64 bits
+// as the kernels that walk token by token.
+template <int NT>
+__device__ __forceinline__ void cr_step(float (*acc)[4], const Left& a, const Right* b) {
+  float t[NT][4] = {}, hh[NT][4] = {};
+#pragma unroll
+  for (int n = 0; n < NT; ++n) cr_mma(t[n], a.l, b[n].h[0], b[n].h[1]);
+#pragma unroll
+  for (int n = 0; n < NT; ++n) cr_mma(t[n], a.h, b[n].l[0], b[n].l[1]);
+#pragma unroll
+  for (int n = 0; n < NT; ++n) cr_mma(t[n], a.m, b[n].m[0], b[n].m[1]);
+#pragma unroll
+  for (int n = 0; n < NT; ++n) cr_mma(t[n], a.m, b[n].h[0], b[n].h[1]);
+#pragma unroll
+  for (int n = 0; n < NT; ++n) cr_mma(t[n], a.h, b[n].m[0], b[n].m[1]);
+#pragma unroll
+  for (int n = 0; n < NT; ++n) cr_mma(hh[n], a.h, b[n].h[0], b[n].h[1]);
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[n][e] += hh[n][e] + t[n][e];
+}
+
+// 16 rows of `left` times NT n-tiles of `right` (both row-major along the KS * 16 places summed over); two chains of half the
+// length, whose roundings are fewer.
+template <int KS, int NT>
+__device__ __forceinline__ void cr_scores(uint32_t left, uint32_t right, int pitch, int lane, float (*acc)[4]) {
+  float even[NT][4] = {};
+#pragma unroll 1
+  for (int ks = 0; ks < KS; ks += 2) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      Left a;
+      Right b[NT];
+      cr_left(left + 64 * (ks + u), pitch, lane, a);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) cr_right(right + 4 * (8 * t * pitch + 16 * (ks + u)), pitch, lane, b[t]);
+      cr_step<NT>(u ? acc : even, a, b);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[t][e] += even[t][e];
 }
 
 // The scores of a chunk on and below its diagonal, in 20 tiles of 16 x 8 shared out over the warps, at most two a warp.
@@ -168,14 +204,10 @@ template <int KS, typename F>
 __device__ __forceinline__ void cr_triangle(uint32_t left, uint32_t right, int pitch, int warp, int lane, F leave) {
   auto run = [&](int r, int n0, auto count) {
     constexpr int NT = decltype(count)::value;
-    float acc[1][NT][4] = {}, small[1][NT][4] = {};
-    cr_scores<KS, NT>(left + 4 * 16 * r * pitch, right + 4 * 8 * n0 * pitch, pitch, lane, acc, small);
+    float acc[NT][4] = {};
+    cr_scores<KS, NT>(left + 4 * 16 * r * pitch, right + 4 * 8 * n0 * pitch, pitch, lane, acc);
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[0][t][e] += small[0][t][e];
-      leave(r, n0 + t, acc[0][t]);
-    }
+    for (int t = 0; t < NT; ++t) leave(r, n0 + t, acc[t]);
   };
   struct One { enum { value = 1 }; };
   struct Two { enum { value = 2 }; };
@@ -225,7 +257,8 @@ __device__ __forceinline__ ChunkPlace cr_place(const ChunkParams& p, int at) {
   return c;
 }
 
-// Decay and write strength of each token, one number a head (decay 1, strength 0 behind the last token).
+// Decay and write strength of each token, one number a head (decay 1, strength 0 behind the last token).  In 64 bits: a handful of
+// values a token while its rows are on their way, and an error here stays in the state as long as the token does.
 template <int KIND>
 __device__ __forceinline__ void cr_numbers(const ChunkParams& p, const ChunkPlace& c, int h, float* gs, float* ws, int tid) {
   if (tid >= CR_C) return;
@@ -234,11 +267,12 @@ __device__ __forceinline__ void cr_numbers(const ChunkParams& p, const ChunkPlac
     w = 1.f;
     if (KIND == CR_FIXED) g = p.decay[h];
     if (KIND == CR_SSM || KIND == CR_DELTA) {
-      const float sp = cr_softplus(p.a[(size_t)(c.first + tid) * p.a_ld + h] + p.dt_bias[h]);
-      g = expf(-expf(p.A_log[h]) * sp);
-      w = sp;
+      const double x = (double)p.a[(size_t)(c.first + tid) * p.a_ld + h] + (double)p.dt_bias[h];
+      const double sp = x > 20.0 ? x : log1p(exp(x));
+      g = (float)exp(-exp((double)p.A_log[h]) * sp);
+      w = (float)sp;
     }
-    if (cr_delta(KIND)) w = cr_sigmoid(p.b[(size_t)(c.first + tid) * p.b_ld + h]);
+    if (cr_delta(KIND)) w = (float)(1.0 / (1.0 + exp(-(double)p.b[(size_t)(c.first + tid) * p.b_ld + h])));
   }
   gs[tid] = g;
   ws[tid] = w;
@@ -255,8 +289,8 @@ __device__ __forceinline__ void cr_form(const ChunkParams& p, const ChunkPlace& 
     for (int i = 0; i < CR_C / STEP; ++i) {
       const int at = (t0 + i * STEP) * PITCH + d;
       float4* k = reinterpret_cast<float4*>(Ks + at);
-      *k = cr_map(*k, cr_silu_fast);
-      if (WITH_Q) { float4* q = reinterpret_cast<float4*>(Qs + at); *q = cr_map(*q, cr_silu_fast); }
+      *k = cr_map(*k, cr_silu_r);
+      if (WITH_Q) { float4* q = reinterpret_cast<float4*>(Qs + at); *q = cr_map(*q, cr_silu_r); }
     }
   }
   if (KIND == CR_HGRN2 && WITH_Q) {                // the decays follow block by block
@@ -295,14 +329,15 @@ __device__ __forceinline__ void cr_form(const ChunkParams& p, const ChunkPlace& 
         sq += x[u] * x[u]; sk += y[u] * y[u];
       }
       sk = warp_sum(sk);
-      const float fk = 1.f / sqrtf(sk + p.unit_eps);
+      float f, rest;
+      cr_unit(sk + p.unit_eps, 1.f, f, rest);
 #pragma unroll
-      for (int u = 0; u < KD / 32; ++u) Ks[t * PITCH + lane + 32 * u] = y[u] * fk;
+      for (int u = 0; u < KD / 32; ++u) Ks[t * PITCH + lane + 32 * u] = fmaf(y[u], f, y[u] * rest);
       if (WITH_Q) {
         sq = warp_sum(sq);
-        const float fq = p.q_scale / sqrtf(sq + p.unit_eps);
+        cr_unit(sq + p.unit_eps, p.q_scale, f, rest);
 #pragma unroll
-        for (int u = 0; u < KD / 32; ++u) Qs[t * PITCH + lane + 32 * u] = x[u] * fq;
+        for (int u = 0; u < KD / 32; ++u) Qs[t * PITCH + lane + 32 * u] = fmaf(x[u], f, x[u] * rest);
       }
     }
   }
@@ -350,30 +385,43 @@ __device__ __forceinline__ void cr_form_values(float* Us, int tid) {
 #pragma unroll
   for (int i = 0; i < CR_C / STEP; ++i) {
     float4* x = reinterpret_cast<float4*>(Us + (tid / (CR_VT / 4) + i * STEP) * CR_PV + (tid % (CR_VT / 4)) * 4);
-    *x = cr_map(*x, cr_silu_fast);
+    *x = cr_map(*x, cr_silu_r);
   }
 }
+
+// A product of decays with what its roundings drop: the error of 63 roundings is the same in every chunk of a head whose decay
+// does not change, and adds up over a state that lives for thousands of tokens.
+struct Product {
+  float h = 1.f, l = 0.f;
+  __device__ __forceinline__ void times(float g) {
+    const float p = h * g;
+    l = fmaf(l, g, fmaf(h, g, -p));
+    h = p;
+  }
+  __device__ __forceinline__ float value() const { return h + l; }
+};
 
 // G(j, i) at [i][j] for one decay a token (zeros above the diagonal), and c_i: a thread eight rows of a column, from the product
 // of the decays between.
 __device__ __forceinline__ void cr_products(const float* gs, float* Ds, float* cs, int tid) {
   static_assert(CR_THREADS == 8 * CR_C, "a thread eight rows of a column");
   const int j = tid % CR_C, i0 = tid / CR_C * 8;
-  float g[8], d = 1.f, c = 1.f;
+  float g[8];
+  Product d, c;
 #pragma unroll 8
-  for (int i = 0; i < i0; ++i) { const float x = gs[i]; if (i > j) d *= x; }
+  for (int i = 0; i < i0; ++i) { const float x = gs[i]; if (i > j) d.times(x); }
 #pragma unroll
   for (int i = 0; i < 8; ++i) g[i] = gs[i0 + i];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    if (i0 + i > j) d *= g[i];
-    Ds[(i0 + i) * CR_PT + j] = i0 + i >= j ? d : 0.f;
+    if (i0 + i > j) d.times(g[i]);
+    Ds[(i0 + i) * CR_PT + j] = i0 + i >= j ? d.value() : 0.f;
   }
   if (j == 0) {                                    // one thread a block of eight: c_i
 #pragma unroll 8
-    for (int i = 0; i < i0; ++i) c *= gs[i];
+    for (int i = 0; i < i0; ++i) c.times(gs[i]);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { c *= g[i]; cs[i0 + i] = c; }
+    for (int i = 0; i < 8; ++i) { c.times(g[i]); cs[i0 + i] = c.value(); }
   }
 }
 
@@ -451,11 +499,11 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_states_kernel(const __gri
   cp_async_wait<0>();
   __syncthreads();
   if (!ROWS && tid < CR_C) {
-    float d = 1.f;
+    Product d;
 #pragma unroll 16
-    for (int i = 1; i < CR_C; ++i) { const float x = gs[i]; if (i > tid) d *= x; }
-    ts[tid] = d * ws[tid];
-    if (tid == 0) cs[0] = d * gs[0];
+    for (int i = 1; i < CR_C; ++i) { const float x = gs[i]; if (i > tid) d.times(x); }
+    ts[tid] = d.value() * ws[tid];
+    if (tid == 0) { d.times(gs[0]); cs[0] = d.value(); }
   }
   cr_form<KIND, KD, PD, false>(p, c, h, nullptr, Ks, Gs, tid);
   __syncthreads();
@@ -494,15 +542,18 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_states_kernel(const __gri
     }
     if (KIND == CR_FIXED && p.act) cr_form_values(Us, tid);
     __syncthreads();
-    float acc[MT][2][4] = {}, small[MT][2][4] = {};
-#pragma unroll 4
-    for (int ks = 0; ks < CR_C / 8; ++ks) {
-      uint32_t ah[MT][4], al[MT][4], bh[2][2], bl[2][2];
+    float acc[MT][2][4] = {};
+#pragma unroll 1
+    for (int ks = 0; ks < CR_C / 16; ++ks) {
+      Right b[2];
 #pragma unroll
-      for (int t = 0; t < 2; ++t) cr_right_t(Us + 8 * ks * CR_PV + 8 * (n0 + t), CR_PV, lane, bh[t], bl[t]);
+      for (int t = 0; t < 2; ++t) cr_right_t(Us + 16 * ks * CR_PV + 8 * (n0 + t), CR_PV, lane, b[t]);
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) cr_left_t(Ks + 8 * ks * PD + 16 * (mt0 + mt), PD, lane, ah[mt], al[mt]);
-      cr_step<MT, 2>(acc, small, ah, al, bh, bl);
+      for (int mt = 0; mt < MT; ++mt) {
+        Left a;
+        cr_left_t(Ks + 16 * ks * PD + 16 * (mt0 + mt), PD, lane, a);
+        cr_step<2>(acc[mt], a, b);
+      }
     }
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
@@ -511,8 +562,8 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_states_kernel(const __gri
         const int col = v0 + 8 * (n0 + t) + 2 * (lane & 3);
         if (col >= p.v_ld_s) continue;
         float* dst = mine + (16 * (mt0 + mt) + (lane >> 2)) * p.v_ld_s + col;
-        *reinterpret_cast<float2*>(dst) = make_float2(acc[mt][t][0] + small[mt][t][0], acc[mt][t][1] + small[mt][t][1]);
-        *reinterpret_cast<float2*>(dst + 8 * p.v_ld_s) = make_float2(acc[mt][t][2] + small[mt][t][2], acc[mt][t][3] + small[mt][t][3]);
+        *reinterpret_cast<float2*>(dst) = make_float2(acc[mt][t][0], acc[mt][t][1]);
+        *reinterpret_cast<float2*>(dst + 8 * p.v_ld_s) = make_float2(acc[mt][t][2], acc[mt][t][3]);
       }
   }
 }
@@ -571,7 +622,7 @@ __host__ __device__ constexpr int cr_solve_floats(int kind, int kd) {
 
 template <int KIND, int KD>
 __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid_constant__ ChunkParams p) {
-  constexpr int PK = KD + 4, MAT = CR_C * PK, KS = KD / 8;
+  constexpr int PK = KD + 4, MAT = CR_C * PK, KS = KD / 16;
   constexpr bool ROWS = cr_rows(KIND);
   extern __shared__ __align__(16) float cr_smem[];
   float* Ks = cr_smem;                             // [64][PK]
@@ -658,12 +709,12 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
       if (I < 3) cr_put_decays<KIND, KD, PK>(c, b0 + 16, tid, gn, nullptr, nullptr, Ks, Gb + (~I & 1) * 16 * PK);
       if (I > 0) {                                 // the block's rows against all tokens before it
         for (int n = warp; n < 2 * I; n += CR_THREADS / 32) {
-          float acc[1][1][4] = {}, small[1][1][4] = {};
-          cr_scores<KS, 1>(Ka + 4 * b0 * PK, Kra + 4 * 8 * n * PK, PK, lane, acc, small);
+          float acc[1][4] = {};
+          cr_scores<KS, 1>(Ka + 4 * b0 * PK, Kra + 4 * 8 * n * PK, PK, lane, acc);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int i = b0 + (lane >> 2) + (e >> 1) * 8;
-            Ls[i * CR_PT + 8 * n + 2 * (lane & 3) + (e & 1)] = (acc[0][0][e] + small[0][0][e]) * ws[i];
+            Ls[i * CR_PT + 8 * n + 2 * (lane & 3) + (e & 1)] = acc[0][e] * ws[i];
           }
         }
       }
@@ -709,17 +760,18 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
     }
   }
   const uint32_t La = (uint32_t)__cvta_generic_to_shared(Ls), Ta = (uint32_t)__cvta_generic_to_shared(Ti);
-  // 16 columns of X [64][pitch] (a warp's own), solved in place and written out
-  auto solve = [&](float* X, int pitch, float* dst, int ld, bool stored0, bool stored1) {
+  // 16 columns of X [64][pitch] (a warp's own; values still without their w), solved in place and written out
+  auto solve = [&](float* X, int pitch, float* dst, int ld, bool values, bool stored0, bool stored1) {
     for (int I = 0; I < 4; ++I) {
-      float acc[1][2][4] = {}, small[1][2][4] = {};
-      uint32_t ah[1][4], al[1][4], bh[2][2], bl[2][2];
-#pragma unroll 2
-      for (int ks = 0; ks < 2 * I; ++ks) {
-        cr_left(La + 4 * (16 * I * CR_PT + 8 * ks), CR_PT, lane, ah[0], al[0]);
+      float acc[2][4] = {};
+      Left a;
+      Right b[2];
+#pragma unroll 1
+      for (int ks = 0; ks < I; ++ks) {
+        cr_left(La + 4 * (16 * I * CR_PT + 16 * ks), CR_PT, lane, a);
 #pragma unroll
-        for (int t = 0; t < 2; ++t) cr_right_t(X + 8 * ks * pitch + 8 * t, pitch, lane, bh[t], bl[t]);
-        cr_step<1, 2>(acc, small, ah, al, bh, bl);
+        for (int t = 0; t < 2; ++t) cr_right_t(X + 16 * ks * pitch + 8 * t, pitch, lane, b[t]);
+        cr_step<2>(acc, a, b);
       }
       float* mineX = X + (16 * I + (lane >> 2)) * pitch + 2 * (lane & 3);
 #pragma unroll
@@ -727,24 +779,21 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           float* x = mineX + (e >> 1) * 8 * pitch + 8 * t + (e & 1);
-          *x -= acc[0][t][e] + small[0][t][e];
-          acc[0][t][e] = small[0][t][e] = 0.f;
+          *x = fmaf(values ? ws[16 * I + (lane >> 2) + (e >> 1) * 8] : 1.f, *x, -acc[t][e]);
+          acc[t][e] = 0.f;
         }
       __syncwarp();
+      cr_left(Ta + 4 * 16 * I * CR_PI, CR_PI, lane, a);
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        cr_left(Ta + 4 * (16 * I * CR_PI + 8 * ks), CR_PI, lane, ah[0], al[0]);
-#pragma unroll
-        for (int t = 0; t < 2; ++t) cr_right_t(X + (16 * I + 8 * ks) * pitch + 8 * t, pitch, lane, bh[t], bl[t]);
-        cr_step<1, 2>(acc, small, ah, al, bh, bl);
-      }
+      for (int t = 0; t < 2; ++t) cr_right_t(X + 16 * I * pitch + 8 * t, pitch, lane, b[t]);
+      cr_step<2>(acc, a, b);
       __syncwarp();
       float* out = dst + (16 * I + (lane >> 2)) * ld + 2 * (lane & 3);
 #pragma unroll
       for (int t = 0; t < 2; ++t)
 #pragma unroll
         for (int e2 = 0; e2 < 2; ++e2) {
-          const float2 x = make_float2(acc[0][t][2 * e2] + small[0][t][2 * e2], acc[0][t][2 * e2 + 1] + small[0][t][2 * e2 + 1]);
+          const float2 x = make_float2(acc[t][2 * e2], acc[t][2 * e2 + 1]);
           *reinterpret_cast<float2*>(mineX + e2 * 8 * pitch + 8 * t) = x;
           if (t ? stored1 : stored0) *reinterpret_cast<float2*>(out + e2 * 8 * ld + 8 * t) = x;
         }
@@ -759,17 +808,11 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
     }
     cp_async_wait<0>();
     __syncthreads();                               // the inverses, w c k and the values are in place
-#pragma unroll
-    for (int i = 0; i < CR_C / 16; ++i) {          // this warp's values times w: they lie in columns that it owns
-      const int t = 16 * i + (lane >> 1);
-      if (warp < 8) { cr_scale(Xv + t * PX + 16 * warp + 8 * (lane & 1), ws[t]); cr_scale(Xv + t * PX + 16 * warp + 8 * (lane & 1) + 4, ws[t]); }
-    }
-    __syncwarp();
     const int left = p.v_ld_s - v0;                // columns still to come, in whole tiles of eight
     if (warp < 8) {
-      if (16 * warp < left) solve(Xv + 16 * warp, PX, oU + v0 + 16 * warp, p.v_ld_s, true, 16 * warp + 8 < left);
+      if (16 * warp < left) solve(Xv + 16 * warp, PX, oU + v0 + 16 * warp, p.v_ld_s, true, true, 16 * warp + 8 < left);
     } else if (v0 == 0 && 16 * (warp - 8) < KD) {
-      solve(Ks + 16 * (warp - 8), PK, oW + 16 * (warp - 8), PK, true, true);
+      solve(Ks + 16 * (warp - 8), PK, oW + 16 * (warp - 8), PK, false, true, true);
     }
   }
 }
@@ -777,9 +820,9 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
 // ---- the states before the chunks of the delta rules: U = U' - W S, S <- diag(c) S + K^T U --------------------------------------
 // A CTA for every (NV value columns, head, sequence).  A chunk is two phases: the product with W (16 rows a pair of warps,
 // which share out the places summed over) and the one with K^T (16 rows a warp, whose part of the state stays in registers).
-// The right operands lie in shared memory already split.  W, K^T and U' of the next chunk are under way during both phases.
+// The right operands lie in shared memory already split, the places of a product in the order of the left operands' registers.  W, K^T and U' of the next chunk are under way during both phases.
 __host__ __device__ constexpr int cr_walk_floats(int kd, int nv) {
-  return 2 * (CR_C * (kd + 4) + kd * CR_PT) + 2 * nv * (kd + 4) + 2 * nv * CR_PT + CR_C * (nv + 8);
+  return 2 * (CR_C * (kd + 4) + kd * CR_PT) + 3 * nv * ((kd + 8) + (CR_C + 8)) / 2 + CR_C * (nv + 8);
 }
 
 template <int KD, int NV>
@@ -787,11 +830,10 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
   constexpr int PK = KD + 4, NT = NV / 8, MW = KD / 16, WK = CR_C * PK + KD * CR_PT;       // MW warps hold the state, 16 rows each
   extern __shared__ __align__(16) float cr_smem[];
   float* WK_s = cr_smem;                           // [2]: W [64][PK], K^T [KD][PT]
-  float* Sh = WK_s + 2 * WK;                       // [NV][PK] state, a column a row: high and low parts
-  float* Sl = Sh + NV * PK;
-  float* Uh = Sl + NV * PK;                        // [NV][PT]
-  float* Ul = Uh + NV * CR_PT;
-  float* Y = Ul + NV * CR_PT;                      // [64][NV + 8] the second half of the places' share of W S
+  constexpr int PS = KD + 8, PU = CR_C + 8;        // values between rows of the split operands: 8 rows' pieces lie in all banks
+  bf16* Ss = reinterpret_cast<bf16*>(WK_s + 2 * WK);             // [3][NV][PS] state, a column a row, its three parts
+  bf16* Us = Ss + 3 * NV * PS;                     // [3][NV][PU]
+  float* Y = reinterpret_cast<float*>(Us + 3 * NV * PU);         // [64][NV + 8] the second half of the places' share of W S
   constexpr int PY = NV + 8;
   pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -804,8 +846,7 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
   const size_t stride = (size_t)p.heads * p.per_head;
   float* mine = p.scratch + ((size_t)(base + c_lo - p.slot0) * p.heads + h) * p.per_head;
   const uint32_t wk_a = (uint32_t)__cvta_generic_to_shared(WK_s);
-  const uint32_t sh_a = (uint32_t)__cvta_generic_to_shared(Sh), sl_a = (uint32_t)__cvta_generic_to_shared(Sl);
-  const uint32_t uh_a = (uint32_t)__cvta_generic_to_shared(Uh), ul_a = (uint32_t)__cvta_generic_to_shared(Ul);
+  const uint32_t s_a = (uint32_t)__cvta_generic_to_shared(Ss), u_a = (uint32_t)__cvta_generic_to_shared(Us);
   const int r0 = (warp & 3) * 16 + row;            // a pair's token rows
   auto fetch = [&](int buf, const float* src) {    // W and, right behind it, K^T
     const uint32_t dst = wk_a + buf * WK * 4 + 16 * tid;
@@ -837,17 +878,21 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
   request(mine);
 
   float s[NT][4];                                  // warps 0 .. MW - 1: the state at (16 warp + row + 8 (e / 2), 8 nt + cc + e % 2)
+  // rows (places) r and r + 8 of the columns 8 nt + cc, + 1 of x, split: place q of eight lies at 2 q, place q + 4 behind it
+  auto put_split = [&](bf16* dst, int pitch, int plane, int r, int nt, const float* x) {
+    const int at = (nt * 8 + cc) * pitch + (r & ~7) + 2 * (r & 3) + ((r >> 2) & 1);
+    const Split lo = cr_split(x[0], x[1]), hi = cr_split(x[2], x[3]);
+    auto put = [&](bf16* d, uint32_t a, uint32_t b) {
+      uint16_t* y = reinterpret_cast<uint16_t*>(d) + at;
+      y[0] = (uint16_t)a; y[pitch] = (uint16_t)(a >> 16);
+      y[8] = (uint16_t)b; y[pitch + 8] = (uint16_t)(b >> 16);
+    };
+    put(dst, lo.h, hi.h); put(dst + plane, lo.m, hi.m); put(dst + 2 * plane, lo.l, hi.l);
+  };
   auto put_state = [&](float* keep) {              // split, for the next product; whole, for the outputs of the chunk it stands before
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        uint32_t hi, lo;
-        cr_split(s[nt][e], hi, lo);
-        const int at = (nt * 8 + cc + (e & 1)) * PK + warp * 16 + row + (e >> 1) * 8;
-        Sh[at] = __uint_as_float(hi);
-        Sl[at] = __uint_as_float(lo);
-      }
+      put_split(Ss, PS, NV * PS, warp * 16 + row, nt, s[nt]);
       const int cl = col0 + nt * 8 + cc;
       if (cl < p.v_ld_s) {
 #pragma unroll
@@ -866,38 +911,34 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
       }
     put_state(mine);
   }
-  // 16 rows of `left` times the split right operand [NV][pitch], over KSTEPS * 8 places
-  auto product = [&](uint32_t left, int pitch, uint32_t rh, uint32_t rl, auto ksteps, float (*acc)[4]) {
-    float x1[NT][4] = {}, x2[NT][4] = {};
+  // 16 rows of `left` times the split right operand [3][NV][rp], over KSTEPS * 16 places
+  auto product = [&](uint32_t left, int pitch, uint32_t right, int rp, auto ksteps, float (*acc)[4]) {
 #pragma unroll
     for (int ks = 0; ks < decltype(ksteps)::value; ++ks) {
-      uint32_t ah[4], al[4], bh[NT][2], bl[NT][2];
-      cr_left(left + 32 * ks, pitch, lane, ah, al);
-      if constexpr (NT == 1) {
-        const uint32_t at = 4 * ((lane & 7) * pitch + ((lane >> 3) & 1) * 4) + 32 * ks;
-        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(bh[0][0]), "=r"(bh[0][1]) : "r"(rh + at));
-        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(bl[0][0]), "=r"(bl[0][1]) : "r"(rl + at));
-      } else {
+      Left a;
+      Right b[NT];
+      cr_left(left + 64 * ks, pitch, lane, a);
+      auto part = [&](uint32_t plane, auto get) {
+        if constexpr (NT == 1) {
+          uint32_t* r = get(b[0]);
+          asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
+                       : "=r"(r[0]), "=r"(r[1]) : "r"(plane + 2 * ((lane & 7) * rp + ((lane >> 3) & 1) * 8) + 32 * ks));
+        } else {
 #pragma unroll
-        for (int n2 = 0; n2 < NT / 2; ++n2) {
-          cr_right2(rh + 4 * n2 * 16 * pitch + 32 * ks, pitch, lane, bh[2 * n2]);
-          cr_right2(rl + 4 * n2 * 16 * pitch + 32 * ks, pitch, lane, bl[2 * n2]);
+          for (int n2 = 0; n2 < NT / 2; ++n2) {
+            uint32_t *r = get(b[2 * n2]), *q = get(b[2 * n2 + 1]);
+            ldmatrix_x4(plane + 2 * ((16 * n2 + (lane >> 4) * 8 + (lane & 7)) * rp + ((lane >> 3) & 1) * 8) + 32 * ks, r[0], r[1], q[0], q[1]);
+          }
         }
-      }
-#pragma unroll
-      for (int t = 0; t < NT; ++t) mma_tf32(x1[t], al, bh[t][0], bh[t][1]);
-#pragma unroll
-      for (int t = 0; t < NT; ++t) mma_tf32(acc[t], ah, bh[t][0], bh[t][1]);
-#pragma unroll
-      for (int t = 0; t < NT; ++t) mma_tf32(x2[t], ah, bl[t][0], bl[t][1]);
+      };
+      part(right, [](Right& x) { return x.h; });
+      part(right + 2 * NV * rp, [](Right& x) { return x.m; });
+      part(right + 4 * NV * rp, [](Right& x) { return x.l; });
+      cr_step<NT>(acc, a, b);
     }
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[nt][e] += x1[nt][e] + x2[nt][e];
   };
-  struct HalfK { enum { value = KD / 16 }; };
-  struct Tokens { enum { value = CR_C / 8 }; };
+  struct HalfK { enum { value = KD / 32 }; };
+  struct Tokens { enum { value = CR_C / 16 }; };
 
   for (int c = c_lo; c < c_hi; ++c) {
     const int buf = (c - c_lo) & 1;
@@ -913,7 +954,7 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
     if (c + 1 < c_hi) { fetch(buf ^ 1, mine + stride); request(mine + stride); }
     float y[NT][4] = {};
     const int k0 = (warp >> 2) * (KD / 2);         // this warp's half of the places
-    product(w_a + 4 * ((warp & 3) * 16 * PK + k0), PK, sh_a + 4 * k0, sl_a + 4 * k0, HalfK(), y);
+    product(w_a + 4 * ((warp & 3) * 16 * PK + k0), PK, s_a + 2 * k0, PS, HalfK(), y);
     if (warp >= 4) {
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
@@ -931,14 +972,7 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
           u[nt][2 * e2] -= y[nt][2 * e2] + z.x;
           u[nt][2 * e2 + 1] -= y[nt][2 * e2 + 1] + z.y;
         }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          uint32_t hi, lo;
-          cr_split(u[nt][e], hi, lo);
-          const int at = (nt * 8 + cc + (e & 1)) * CR_PT + r0 + (e >> 1) * 8;
-          Uh[at] = __uint_as_float(hi);
-          Ul[at] = __uint_as_float(lo);
-        }
+        put_split(Us, PU, NV * PU, r0, nt, u[nt]);
         if (cl < p.v_ld_s) {
 #pragma unroll
           for (int e2 = 0; e2 < 2; ++e2)
@@ -950,7 +984,7 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
     mine += stride;
     if (warp < MW) {
       float x[NT][4] = {};
-      product(k_a + 4 * warp * 16 * CR_PT, CR_PT, uh_a, ul_a, Tokens(), x);
+      product(k_a + 4 * warp * 16 * CR_PT, CR_PT, u_a, PU, Tokens(), x);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -978,7 +1012,7 @@ __host__ __device__ constexpr int cr_out_floats(int kind, int kd) {
 
 template <int KIND, int KD>
 __global__ void __launch_bounds__(CR_THREADS, 2) chunk_outputs_kernel(const __grid_constant__ ChunkParams p) {
-  constexpr int PK = KD + 4, MAT = CR_C * PK, KS = KD / 8, KBUF = MAT > KD * CR_PV ? MAT : KD * CR_PV;
+  constexpr int PK = KD + 4, MAT = CR_C * PK, KS = KD / 16, KBUF = MAT > KD * CR_PV ? MAT : KD * CR_PV;
   constexpr bool ROWS = cr_rows(KIND), DELTA = cr_delta(KIND);
   static_assert(32 * PK <= CR_C * CR_PV, "two blocks' decays lie where U does");
   constexpr int STEP = CR_THREADS / (KD / 4);
@@ -1082,11 +1116,11 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_outputs_kernel(const __gr
       if (I < 3) cr_put_decays<KIND, KD, PK>(c, b0 + 16, tid, gn, low, bi, Ks, Gb + (~I & 1) * 16 * PK);
       if (I > 0) {                                 // the block's rows against all tokens before it
         for (int n = warp; n < 2 * I; n += CR_THREADS / 32) {
-          float acc[1][1][4] = {}, small[1][1][4] = {};
-          cr_scores<KS, 1>(Qa + 4 * b0 * PK, Ka + 4 * 8 * n * PK, PK, lane, acc, small);
+          float acc[1][4] = {};
+          cr_scores<KS, 1>(Qa + 4 * b0 * PK, Ka + 4 * 8 * n * PK, PK, lane, acc);
 #pragma unroll
           for (int e = 0; e < 4; ++e)
-            As[(b0 + (lane >> 2) + (e >> 1) * 8) * CR_PT + 8 * n + 2 * (lane & 3) + (e & 1)] = acc[0][0][e] + small[0][0][e];
+            As[(b0 + (lane >> 2) + (e >> 1) * 8) * CR_PT + 8 * n + 2 * (lane & 3) + (e & 1)] = acc[0][e];
         }
       }
       __syncthreads();
@@ -1121,19 +1155,26 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_outputs_kernel(const __gr
       cr_form_values(Us, tid);
       __syncthreads();
     }
-    float acc[1][2][4] = {}, small[1][2][4] = {};
-    auto add = [&](uint32_t left, int pitch, const float* right, int ksteps) {
-#pragma unroll 4
-      for (int ks = 0; ks < ksteps; ++ks) {
-        uint32_t ah[1][4], al[1][4], bh[2][2], bl[2][2];
+    float acc[2][4] = {};                          // three sums apart: short chains, fewer roundings
+    auto add = [&](uint32_t left, int pitch, const float* right, int from, int to) {
+      float sum[2][4] = {};
+#pragma unroll 1
+      for (int ks = from; ks < to; ++ks) {
+        Left a;
+        Right b[2];
 #pragma unroll
-        for (int t = 0; t < 2; ++t) cr_right_t(right + 8 * ks * CR_PV + 8 * (n0 + t), CR_PV, lane, bh[t], bl[t]);
-        cr_left(left + 32 * ks, pitch, lane, ah[0], al[0]);
-        cr_step<1, 2>(acc, small, ah, al, bh, bl);
+        for (int t = 0; t < 2; ++t) cr_right_t(right + 16 * ks * CR_PV + 8 * (n0 + t), CR_PV, lane, b[t]);
+        cr_left(left + 64 * ks, pitch, lane, a);
+        cr_step<2>(sum, a, b);
       }
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[t][e] += sum[t][e];
     };
-    add(Qa + 4 * 16 * m * PK, PK, Ss, KS);
-    add(Aa + 4 * 16 * m * CR_PT, CR_PT, Us, 2 * m + 2);
+    add(Qa + 4 * 16 * m * PK, PK, Ss, 0, KS / 2);
+    add(Qa + 4 * 16 * m * PK, PK, Ss, KS / 2, KS);
+    add(Aa + 4 * 16 * m * CR_PT, CR_PT, Us, 0, m + 1);
 #pragma unroll
     for (int e2 = 0; e2 < 2; ++e2) {
       const int t = 16 * m + (lane >> 2) + 8 * e2;
@@ -1142,7 +1183,7 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_outputs_kernel(const __gr
       for (int nt = 0; nt < 2; ++nt) {
         const int col = v0 + 8 * (n0 + nt) + 2 * (lane & 3);
         if (col >= p.vdim) continue;
-        float x = acc[0][nt][2 * e2] + small[0][nt][2 * e2], y = acc[0][nt][2 * e2 + 1] + small[0][nt][2 * e2 + 1];
+        float x = acc[nt][2 * e2], y = acc[nt][2 * e2 + 1];
         if (p.D) {
           x += p.D[h] * vsrc[(size_t)t * p.v_ld + col];
           if (col + 1 < p.vdim) y += p.D[h] * vsrc[(size_t)t * p.v_ld + col + 1];
