@@ -26,6 +26,10 @@
 // decay for every row the chunk is cut into blocks of 16: pairs inside a block are formed one by one (their G is carried along
 // in registers), pairs of different blocks as (q_i G(block start, i)) . (k_j G(j, block start)).
 //
+// Infinities and NaN stay where the walk would have them: a bad value of token t reaches no output before t and no other request
+// (the two products in which a row meets later tokens, with zeros, take what is not finite out and mark the rows from it on);
+// from t on the walk may leave an infinity where a NaN stands here.
+//
 // Everything is 32-bit.  The products run on the tensor cores as six bfloat16 products of operands cut in three, which hold all 24
 // bits, 16 places at a time, and the sums from one 16 to the next are ordinary additions (see cr_step).  Decays and strengths that
 // are one number a token come out of 64 bits, and their products carry what rounding drops.  Against 64 bits the outputs before
@@ -174,6 +178,9 @@ __device__ __forceinline__ void cr_step(float (*acc)[4], const Left& a, const Ri
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[n][e] += hh[n][e] + t[n][e];
 }
+
+// Whether a value is finite and stays so when it is split.
+__device__ __forceinline__ bool cr_finite(float x) { return fabsf(x) <= 3.38e38f; }
 
 // 16 rows of `left` times NT n-tiles of `right` (both row-major along the KS * 16 places summed over); two chains of half the
 // length, whose roundings are fewer.
@@ -774,14 +781,33 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
         cr_step<2>(acc, a, b);
       }
       float* mineX = X + (16 * I + (lane >> 2)) * pitch + 2 * (lane & 3);
+      bool finite = true;
 #pragma unroll
       for (int t = 0; t < 2; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           float* x = mineX + (e >> 1) * 8 * pitch + 8 * t + (e & 1);
-          *x = fmaf(values ? ws[16 * I + (lane >> 2) + (e >> 1) * 8] : 1.f, *x, -acc[t][e]);
+          const float y = fmaf(values ? ws[16 * I + (lane >> 2) + (e >> 1) * 8] : 1.f, *x, -acc[t][e]);
+          *x = y;
           acc[t][e] = 0.f;
+          finite &= cr_finite(y);
         }
+      if (!__all_sync(0xffffffffu, finite)) {      // rare: a column is bad from its first such row on, and no earlier
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int e1 = 0; e1 < 2; ++e1) {
+            float* x = mineX + 8 * t + e1;
+            const bool upper = !cr_finite(x[0]), lower = !cr_finite(x[8 * pitch]);
+            int from = upper ? lane >> 2 : lower ? (lane >> 2) + 8 : 16;
+#pragma unroll
+            for (int d = 4; d < 32; d <<= 1) from = min(from, __shfl_xor_sync(0xffffffffu, from, d));
+            if (upper) x[0] = 0.f;
+            if (lower) x[8 * pitch] = 0.f;
+            if ((lane >> 2) >= from) acc[t][e1] = __int_as_float(0x7fffffff);
+            if ((lane >> 2) + 8 >= from) acc[t][2 + e1] = __int_as_float(0x7fffffff);
+          }
+      }
       __syncwarp();
       cr_left(Ta + 4 * 16 * I * CR_PI, CR_PI, lane, a);
 #pragma unroll
@@ -1174,7 +1200,44 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_outputs_kernel(const __gr
     };
     add(Qa + 4 * 16 * m * PK, PK, Ss, 0, KS / 2);
     add(Qa + 4 * 16 * m * PK, PK, Ss, KS / 2, KS);
-    add(Aa + 4 * 16 * m * CR_PT, CR_PT, Us, 0, m + 1);
+    add(Aa + 4 * 16 * m * CR_PT, CR_PT, Us, 0, m);
+    {                                              // the diagonal tile, whose rows have tokens behind them on the right
+      float sum[2][4] = {}, x[2][4];
+      bool finite = true;
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          x[t][i] = Us[(16 * m + (lane & 3) + 4 * i) * CR_PV + 8 * (n0 + t) + (lane >> 2)];
+          finite &= cr_finite(x[t][i]);
+        }
+      if (!__all_sync(0xffffffffu, finite)) {      // rare: a column is bad from its first such token on, and no earlier
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          int from = 16;
+#pragma unroll
+          for (int i = 3; i >= 0; --i)
+            if (!cr_finite(x[t][i])) { from = (lane & 3) + 4 * i; x[t][i] = 0.f; }
+          from = min(from, __shfl_xor_sync(0xffffffffu, from, 1));
+          from = min(from, __shfl_xor_sync(0xffffffffu, from, 2));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int f = __shfl_sync(0xffffffffu, from, 4 * (2 * (lane & 3) + (e & 1)));
+            if ((lane >> 2) + 8 * (e >> 1) >= f) sum[t][e] = __int_as_float(0x7fffffff);
+          }
+        }
+      }
+      Left a;
+      Right b[2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) { cr_put(b[t], 0, x[t][0], x[t][1]); cr_put(b[t], 1, x[t][2], x[t][3]); }
+      cr_left(Aa + 4 * (16 * m * CR_PT + 16 * m), CR_PT, lane, a);
+      cr_step<2>(sum, a, b);
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[t][e] += sum[t][e];
+    }
 #pragma unroll
     for (int e2 = 0; e2 < 2; ++e2) {
       const int t = 16 * m + (lane >> 2) + 8 * e2;

@@ -159,6 +159,34 @@ def test_as_exact_as_token_by_token(kind, heads, groups, dim, vdim, lens):
     assert (off[True] <= 1.1 * off[False]).all(), off
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("where,token,column", [("v", 37, 5), ("v", 32, 9), ("v", 70 + 47, 70), ("k", 40, 7), ("k", 70 + 64, 3), ("q", 50, 1), ("a", 41, 0), ("b", 43, 1)])
+@pytest.mark.parametrize("kind", ["fixed", "ssm", "hgrn2", "delta", "channels"])
+def test_what_is_not_finite_stays_with_its_tokens(kind, where, token, column, bad):
+    """One infinity or NaN in the first or second of three portions: outputs and states are finite exactly where the kernels that
+    walk token by token have them finite, and there as close to 64 bits as ever."""
+    heads, groups, dim, vdim, lens = 2, 2, 64, 72, [70, 130, 40]
+    torch.manual_seed(9)
+    o = operands(kind, sum(lens), heads, groups, dim, vdim)
+    if kind == "fixed":
+        o["decay"] = torch.tensor([0.97, 0.9], device=DEV)
+    if o.get(where) is None:
+        pytest.skip("this recurrence has no such operand")
+    step = step_of(lens, [2, 0, 1])
+    state = 0.3 * torch.randn(4, heads, dim, vdim, device=DEV)
+    o[where][token, column] = bad
+    want, S = plain(kind, o, state, step, heads, groups, dim, vdim)
+    got_state, walked_state = state.clone(), state.clone()
+    got = through_ops(kind, o, got_state, step, heads, groups, dim, vdim, True)
+    walked = through_ops(kind, o, walked_state, step, heads, groups, dim, vdim, False)
+    for x, y, z in ((got, walked, want), (got_state[:3], walked_state[:3], S[:3])):
+        assert torch.equal(torch.isfinite(x), torch.isfinite(y))
+        same = torch.isfinite(y) & torch.isfinite(z)
+        assert (x.double() - z).abs()[same].max() <= 1e-5 * z[same].abs().max()
+    before = torch.arange(sum(lens), device=DEV) < token
+    assert torch.isfinite(got[before]).all() and torch.isfinite(got[sum(lens[:2]):]).all()
+
+
 @pytest.mark.parametrize("seqs,heads,groups,dim,vdim", [(1, 2, 1, 128, 128), (3, 4, 2, 64, 64), (80, 4, 4, 128, 128), (5, 64, 2, 128, 64), (40, 8, 4, 72, 40), (2, 3, 3, 5, 260),
                                                         (150, 2, 1, 33, 132)])
 @pytest.mark.parametrize("kind", ["fixed", "ssm", "hgrn2", "delta", "channels"])
