@@ -85,7 +85,7 @@ def _digest(paths: list[Path], extra: str = "") -> str:
 
 
 def source_digest() -> str:
-    return _digest(sources() + _headers() + [_CALLER], " ".join(NVCC_FLAGS) + f"|abi{ABI_VERSION}")
+    return _digest(sources() + _headers(), " ".join(NVCC_FLAGS) + f"|abi{ABI_VERSION}")
 
 
 def _writable(d: Path) -> bool:
@@ -129,38 +129,55 @@ def _existing_library() -> Path | None:
 
 
 def _caller_path(folder: Path) -> Path:
-    return folder / ("lb_caller" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+    """Named by its source and by the interpreter it is for: several interpreters may share a folder."""
+    return folder / f"lb_caller-{_digest([_CALLER])}{sysconfig.get_config_var('EXT_SUFFIX') or '.so'}"
 
 
 def _build_caller(out: Path) -> None:
-    """The extension module beside the library; left out where it cannot be built."""
+    """The extension module beside the library, for this interpreter; says why where it cannot be built."""
     path = _caller_path(out)
-    path.unlink(missing_ok=True)
+    if path.exists():
+        return
     include, cc = sysconfig.get_paths().get("include", ""), shutil.which("gcc") or shutil.which("cc")
     if not cc or not (Path(include) / "Python.h").exists():
+        _say(f"no lb_caller ({'no C compiler' if not cc else 'no Python.h in ' + include}): calls into the kernel library go through ctypes")
         return
     tmp = path.with_name(path.name + f".{os.getpid()}.tmp")
     r = subprocess.run([cc, "-O2", "-fPIC", "-shared", "-I", include, "-o", str(tmp), str(_CALLER)], capture_output=True, text=True)
-    if r.returncode == 0:
-        os.replace(tmp, path)
-    else:
+    if r.returncode != 0:
         tmp.unlink(missing_ok=True)
+        _say(f"lb_caller could not be built, calls into the kernel library go through ctypes:\n{r.stderr}")
+        return
+    for old in out.glob("lb_caller*" + path.name.removeprefix(path.name.split(".")[0])):
+        if old != path:
+            old.unlink(missing_ok=True)          # of an earlier source, for this interpreter
+    os.replace(tmp, path)
+
+
+_caller_module: list = []                      # what caller() has found, once it has looked
 
 
 def caller():
-    """The module lb_caller of the loaded library, or None."""
+    """The module lb_caller beside the loaded library, built first where only it is missing; or None."""
     import importlib.machinery
     import importlib.util
-    path = _caller_path(Path(library()._name).parent)
-    if not path.exists():
-        return None
-    try:
-        loader = importlib.machinery.ExtensionFileLoader("lb_caller", str(path))
-        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("lb_caller", str(path), loader=loader))
-        loader.exec_module(module)
+    folder = Path(library()._name).parent
+    with _lock:
+        if _caller_module:
+            return _caller_module[0]
+        path, module = _caller_path(folder), None
+        if not path.exists() and _writable(folder):
+            _build_caller(folder)
+        if path.exists():
+            try:
+                loader = importlib.machinery.ExtensionFileLoader("lb_caller", str(path))
+                module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("lb_caller", str(path), loader=loader))
+                loader.exec_module(module)
+            except ImportError as e:
+                _say(f"{path} cannot be loaded, calls into the kernel library go through ctypes: {e}")
+                module = None
+        _caller_module.append(module)
         return module
-    except ImportError:
-        return None
 
 
 def _compile_one(nvcc: str, src: Path, obj: Path) -> tuple[Path, float]:
@@ -183,6 +200,7 @@ def build(verbose: bool = True) -> Path:
     with open(out / ".lock", "w") as lockf:
         fcntl.flock(lockf, fcntl.LOCK_EX)
         if lib.exists() and stamp.exists() and stamp.read_text().strip() == want:
+            _build_caller(out)
             return lib
         hdr = _digest(_headers(), " ".join(NVCC_FLAGS))
         jobs, objs = [], []

@@ -161,19 +161,20 @@ _LETTERS = {c_void_p: "p", c_int: "i", c_longlong: "i", c_uint: "i", c_ulonglong
 
 def _bind_native(name: str):
     global _native
-    module = caller()
-    if module is None:
+    native, module = _native, caller()
+    if module is None or native is None:
         _native = None
         return None
     address = ctypes.cast(_fn(name), c_void_p).value
-    f = _native[name] = module.bind(address, "".join(_LETTERS[t] for t in _SIGNATURES[name]))
+    f = native[name] = module.bind(address, "".join(_LETTERS[t] for t in _SIGNATURES[name]))
     return f
 
 
 def _invoke(name: str, *args) -> int:
     """What the library's function returns."""
-    if _native is not None:
-        f = _native.get(name) or _bind_native(name)
+    native = _native                 # another thread may find meanwhile that there is no such module
+    if native is not None:
+        f = native.get(name) or _bind_native(name)
         if f is not None:
             rc = f(*args)
             if rc is not NotImplemented:
@@ -1464,8 +1465,6 @@ def attention_flash(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v
 def latent_flash_ok(dk: int, dv: int, group: int, page_size: int) -> bool:
     """The sizes of the kernel for many heads on one cached vector: keys of up to 576 entries whose first up to 512 are the
     values (multiples of 8), at most 64 heads a tile, pages of 8 to 128 tokens."""
-    lib = library()
-    lib.lb_latent_flash_ok.restype = c_int
     return bool(_invoke("lb_latent_flash_ok", dk, dv, group, page_size))
 
 
