@@ -42,21 +42,23 @@ def operands(kind, T, heads, groups, dim, vdim):
     return o
 
 
-def through_ops(kind, o, state, step, heads, groups, dim, vdim, by_shape):
+def through_ops(kind, o, state, step, heads, groups, dim, vdim, by_shape, shifted=True):
+    """`shifted`: the operands that may be column ranges start on no 16-byte boundary."""
     from lucciola_b200 import ops
     s = torch.cuda.current_stream().cuda_stream
     T = o["v"].shape[0]
     out = torch.full((T, heads * vdim), float("nan"), device=DEV)
     n, m = heads * dim, heads * vdim
+    at = columns if shifted else (lambda x: x)
     if kind == "fixed":
-        pre = columns(torch.cat([o["q"], o["k"], o["v"]], dim=1)) if vdim % 2 else torch.cat([o["q"], o["k"], o["v"]], dim=1)
+        pre = at(torch.cat([o["q"], o["k"], o["v"]], dim=1))
         ops.decay_recurrence(pre, 0, n, 2 * n, o["decay"], state, out, step, heads, dim, vdim, s, by_shape=by_shape)
     elif kind == "hgrn2":
-        pre = torch.cat([o["q"], o["k"], o["v"]], dim=1)
+        pre = at(torch.cat([o["q"], o["k"], o["v"]], dim=1))
         ops.gated_recurrence(pre, 0, n, 2 * n, o["bias"], o["lower"], state, out, step, heads, dim, vdim, s, by_shape=by_shape)
     else:
         delta = kind != "ssm"
-        ops.state_recurrence(columns(o["q"]), o["k"], columns(o["v"]), o["a"].clone(), o["b"], o["A_log"], o["dt_bias"], o.get("D"), state, out, step, heads,
+        ops.state_recurrence(at(o["q"]), o["k"], at(o["v"]), at(o["a"].clone()), o["b"], o["A_log"], o["dt_bias"], o.get("D"), state, out, step, heads,
                              groups, dim, vdim, s, delta=delta, unit_norm=delta, q_scale=dim ** -0.5 if delta else 1.0, rows_decay=kind == "channels",
                              by_shape=by_shape)
     return out
@@ -111,7 +113,8 @@ def from_32_tokens(monkeypatch):
     (2, 1, 128, 128, [64]), (3, 3, 128, 128, [63, 65]), (2, 2, 64, 64, [32, 200]), (4, 2, 20, 40, [33, 1, 129]), (2, 1, 72, 33, [1, 2, 47, 130, 31]),
     (1, 1, 128, 8, [256]), (6, 3, 100, 72, [300]), (5, 5, 8, 6, [80])])
 @pytest.mark.parametrize("kind", ["fixed", "ssm", "hgrn2", "delta", "channels"])
-def test_long_portions(kind, heads, groups, dim, vdim, lens):
+@pytest.mark.parametrize("shifted", [False, True])
+def test_long_portions(kind, heads, groups, dim, vdim, lens, shifted):
     """Outputs and states within 1e-5 of their largest value: a few hundred terms of 2^-24 relative error each, as for the
     kernels that walk token by token; rows of the state that belong to nobody stay as they are."""
     torch.manual_seed(3)
@@ -123,11 +126,31 @@ def test_long_portions(kind, heads, groups, dim, vdim, lens):
     want, S = plain(kind, o, state, step, heads, groups, dim, vdim)
     for by_shape in (True, False):
         got_state = state.clone()
-        got = through_ops(kind, o, got_state, step, heads, groups, dim, vdim, by_shape)
+        got = through_ops(kind, o, got_state, step, heads, groups, dim, vdim, by_shape, shifted)
         assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max(), by_shape
         live = got_state[1:-1].double()
         assert (live - S[1:-1]).abs().max() <= 1e-5 * S[1:-1].abs().max(), by_shape
         assert torch.isnan(got_state[0]).all() and torch.isnan(got_state[-1]).all()
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(16, 128, 128), (32, 128, 128), (16, 128, 120), (32, 100, 120), (16, 64, 128), (32, 64, 128), (32, 40, 120)])
+@pytest.mark.parametrize("kind", ["delta", "channels"])
+@pytest.mark.parametrize("shifted", [False, True])
+def test_walks_of_wider_columns(kind, heads, dim, vdim, shifted):
+    """The walk over the chunks takes 32 value columns a CTA where that makes 100 CTAs (here 32 heads), else 16 (here 16 heads), else 8
+    (test_long_portions); the bounds of test_long_portions."""
+    torch.manual_seed(10)
+    lens = [90, 70]
+    o = operands(kind, sum(lens), heads, heads // 2, dim, vdim)
+    for one in range(2):                                          # a sequence a step, so that its heads alone choose the width
+        n = lens[one]
+        mine = {k: (x[:n] if x is not None and x.shape[0] == sum(lens) else x) for k, x in o.items()}
+        step = step_of([n], [1])
+        state = 0.3 * torch.randn(2, heads, dim, vdim, device=DEV)
+        want, S = plain(kind, mine, state, step, heads, heads // 2, dim, vdim)
+        got = through_ops(kind, mine, state, step, heads, heads // 2, dim, vdim, True, shifted)
+        assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max()
+        assert (state[1].double() - S[1]).abs().max() <= 1e-5 * S[1].abs().max()
 
 
 @pytest.mark.parametrize("heads,groups,dim,vdim,lens", [(4, 2, 128, 128, [600]), (3, 3, 64, 128, [250, 90]), (4, 1, 128, 64, [40, 333])])
