@@ -54,7 +54,7 @@ def through_ops(kind, o, state, step, heads, groups, dim, vdim, by_shape, shifte
         pre = at(torch.cat([o["q"], o["k"], o["v"]], dim=1))
         ops.decay_recurrence(pre, 0, n, 2 * n, o["decay"], state, out, step, heads, dim, vdim, s, by_shape=by_shape)
     elif kind == "hgrn2":
-        pre = at(torch.cat([o["q"], o["k"], o["v"]], dim=1))
+        pre = torch.cat([o["q"], o["k"], o["v"]], dim=1)          # whole rows: their alignment follows from the sizes
         ops.gated_recurrence(pre, 0, n, 2 * n, o["bias"], o["lower"], state, out, step, heads, dim, vdim, s, by_shape=by_shape)
     else:
         delta = kind != "ssm"
