@@ -188,6 +188,7 @@ __global__ void __launch_bounds__(256) decay_chunk_kernel(DecayChunkParams pc) {
   const float* q_src = p.pre + p.q_col + h * p.dim + row0 + td;
   const float* k_src = p.pre + p.k_col + h * p.dim + row0 + td;
   pdl_wait();
+  if (p.skip_from > 0 && n >= p.skip_from) return;
   auto request = [&](int c0) {                        // the raw inputs of the chunk that starts at token c0
     const int cn = min(DC_C, n - c0);
 #pragma unroll
@@ -429,7 +430,7 @@ LB_EXPORT int lb_decay_recurrence(const float* pre, long long ld, int q_col, int
   p.state = state; p.out = out; p.cu_tokens = cu_tokens; p.slots = slots; p.heads = heads; p.dim = dim; p.vdim = vdim;
   p.act = act ? 1 : 0;
   p.skip_from = skip_from;
-  LB_CHECK_ARG(skip_from <= 0 || row_split == 0, "decay_recurrence: sequences are left out by the token-by-token kernel only");
+  LB_CHECK_ARG(skip_from <= 0 || row_split <= 1, "decay_recurrence: sequences are left out where the output is one plane");
   const bool few = max_tokens_a_seq > 0 && max_tokens_a_seq <= 4;
   cudaError_t e;
   if (row_split >= 1) {

@@ -333,6 +333,7 @@ def gated_recurrence(pre: torch.Tensor, q_col: int, f_col: int, v_col: int, bias
         _chunk_recurrence("hgrn2", q, f, v, state, out, step, long, heads, heads, dim, vdim, stream, bias=bias, lower=lower)
         if len(long) == step.num_seqs:
             return
+        _, max_tokens_a_seq = _shorter(step, skip)
     _call("lb_gated_recurrence", pre.data_ptr(), pre.stride(0), q_col, f_col, v_col, bias.data_ptr(), lower.data_ptr(),
           state.data_ptr(), out.data_ptr(), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), step.num_seqs,
           heads, dim, vdim, max_tokens_a_seq, skip, stream)
@@ -655,16 +656,45 @@ def short_conv_step(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bi
     return rc == 0
 
 
-# From how many tokens a sequence's recurrence goes through the chunked form (csrc/chunk_recurrence.cu): the walk token by token
-# costs its tokens times the rounds its CTAs need, the chunked form three launches of about 15 us and little a chunk.  Measured
-# (B200, heads of 128 x 128, us token by token / chunked; one sequence and 16 heads | four and 32): fixed decays 192 tokens 43 / 46 |
-# 64 tokens 73 / 60; state space 192: 31 / 29 | 96: 41 / 38; HGRN2 256: 53 / 57 | 128: 112 / 73; delta rule 128: 60 / 56 | 64: 80 / 74;
-# channel decays 192: 90 / 86 | 64: 124 / 98.
-CHUNK_FROM = {"fixed": 240, "ssm": 240, "hgrn2": 420, "delta": 160, "channels": 230}
+# Portions that may go through the chunked form of a recurrence (csrc/chunk_recurrence.cu).
 CHUNK_LEAST = 32
 # Scratch of the chunked form, in floats: more chunks are worked off in turns.
 CHUNK_SCRATCH = 32 << 20
 _CHUNK_KINDS = {"fixed": 0, "ssm": 1, "delta": 2, "hgrn2": 3, "channels": 4}
+
+# What a step's recurrence costs in us, all launches (B200; fitted to 1400 steps of 1 to 16 equal portions of 32 to 448 tokens or of one to
+# four portions beside up to 60 shorter ones, 8 to 64 heads and states of 64 and 128 rows, most weight where the two forms lie
+# close together; off by 5 to 12 %).
+#
+# Token by token (fixed decays: side by side, 16 at a time): the launch; what a token of the longest portion takes at 128 rows, and how
+# much of that is left at none; what a token takes a CTA on the fullest SM, and how much of that is left; what a CTA's start is worth
+# in tokens; value columns a CTA.
+# 16 heads of 128 x 128, one portion of 448 tokens | 16 of 128, us: fixed 98 | 269, HGRN2 91 | 203, delta 195 | 276, channels 201 | 386.
+_WALK_US = {"fixed": (2.9, 0.497, 0.18, 0.285, 0.15, 0, 32), "ssm": (4.0, 0.275, 0.14, 0.176, 0.2, 15, 32), "hgrn2": (4.5, 0.187, 0.34, 0.187, 0.34, 27, 32),
+            "delta": (4.0, 0.43, 0.4, 0.276, 0.4, 13, 32), "channels": (7.6, 0.44, 0.4, 0.205, 0.4, 12, 16)}
+# Chunked, from the chunks times heads, at 128 value columns: start and a CTA while all run at once (two an SM), start and a CTA
+# beyond; factors on the starts and on the CTAs up to 64 rows.  The same steps: fixed 64 | 160, HGRN2 70 | 171, delta 82 | 207, channels 110 | 269.
+_CHUNK_US = {"fixed": (51, 0.117, 12, 0.282, 0.7, 0.6), "ssm": (34, 0.066, 15, 0.24, 0.73, 0.65), "hgrn2": (59, 0.097, 19, 0.294, 0.7, 0.6),
+             "delta": (57, 0.21, 23, 0.37, 0.8, 0.63), "channels": (77, 0.245, 37, 0.47, 0.8, 0.63)}
+
+
+def _walk_us(kind: str, lens, heads: int, dim: int, vdim: int, split: int) -> float:
+    launch, alone, alone0, shared, shared0, start, cols = _WALK_US[kind]
+    longest, rows, ctas = max(lens), dim / split / 128, len(lens) * heads * -(-vdim // cols) * split
+    if longest <= 4:
+        start = 4                                                 # kernels made for a few tokens
+    elif kind == "fixed":
+        lens = [-(-n // 16) * 16 for n in lens]
+    others = (sum(lens) - max(lens)) / (len(lens) - 1) if len(lens) > 1 else 0
+    return launch + max(alone * (alone0 + (1 - alone0) * rows) * longest,
+                        shared * (shared0 + (1 - shared0) * rows) * (longest + (-(-ctas // 148) - 1) * (others + start)))
+
+
+def _chunk_us(kind: str, lens, heads: int, dim: int, vdim: int) -> float:
+    few, one, many, more, starts, each = _CHUNK_US[kind]
+    ctas, cols = sum(-(-n // 64) for n in lens) * heads, 0.3 + 0.7 * vdim / 128
+    starts, each = (starts, each) if dim <= 64 else (1.0, 1.0)
+    return few * starts + one * each * cols * ctas if ctas <= 296 else many * starts + more * each * cols * ctas
 
 
 def chunk_portions(kind: str, step, heads: int, dim: int, vdim: int) -> tuple[list[int], int]:
@@ -672,10 +702,25 @@ def chunk_portions(kind: str, step, heads: int, dim: int, vdim: int) -> tuple[li
     tokens on they do (0: none does); states of up to 128 rows."""
     if dim > 128 or vdim > 4096 or len(step.q_lens) != step.num_seqs or step.max_q_len < CHUNK_LEAST:
         return [], 0
-    candidates = [i for i, n in enumerate(step.q_lens) if n >= CHUNK_LEAST]
-    start = max(CHUNK_LEAST, int(CHUNK_FROM[kind] / (1.0 + len(candidates) * heads / 64.0)))
-    long = [i for i in candidates if step.q_lens[i] >= start]
-    return long, start if long else 0
+    return _chunk_portions(kind, tuple(step.q_lens), heads, dim, vdim)
+
+
+@functools.lru_cache(maxsize=512)
+def _chunk_portions(kind: str, lens: tuple, heads: int, dim: int, vdim: int) -> tuple[list[int], int]:
+    """For the step as a whole: once a portion pays for the chunked form's launches, all others of CHUNK_LEAST tokens go with it, and
+    only shorter ones are walked behind it.  A tenth is asked for, which is what the estimates are off by."""
+    split = (decay_row_split(len(lens), heads, dim, vdim, max(lens)) or 1) if kind == "fixed" else 1
+    short = [n for n in lens if n < CHUNK_LEAST]
+    chunked = _chunk_us(kind, [n for n in lens if n >= CHUNK_LEAST], heads, dim, vdim) + (_walk_us(kind, short, heads, dim, vdim, 1) if short else 0.0)
+    if chunked > 0.92 * _walk_us(kind, lens, heads, dim, vdim, split):
+        return [], 0
+    return [i for i, n in enumerate(lens) if n >= CHUNK_LEAST], CHUNK_LEAST
+
+
+def _shorter(step, skip: int) -> tuple[int, int]:
+    """How many sequences of a step are shorter than that, and the longest of them."""
+    lens = [n for n in step.q_lens if n < skip]
+    return len(lens), max(lens)
 
 
 def single_tokens(step, dim: int, vdim: int, state: torch.Tensor) -> bool:
@@ -756,16 +801,19 @@ def state_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
     if rows_decay:
         _call("lb_channel_decay", a.data_ptr(), a.stride(0), A_log.data_ptr(), dt_bias.data_ptr(), T, heads, dim, stream)
     long, skip = chunk_portions(kind, step, heads, dim, vdim) if by_shape else ([], 0)
+    seqs, ones = step.num_seqs, T == step.num_seqs
     if long:
         _chunk_recurrence(kind, _rows(q), _rows(k), _rows(v), state, out, step, long, heads, groups, dim, vdim, stream, a=_rows(a), b=_rows(b),
                           A_log=A_log, dt_bias=dt_bias, D=D, unit_norm=unit_norm, q_scale=q_scale, unit_eps=unit_eps)
         if len(long) == step.num_seqs:
             return
+        seqs, most = _shorter(step, skip)
+        ones = most == 1
     _call("lb_state_recurrence", 1 if delta else 0, q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
           a.data_ptr(), a.stride(0), _ptr(b), b.stride(0) if b is not None else 0, A_log.data_ptr(), dt_bias.data_ptr(), _ptr(D),
           state.data_ptr(), out.data_ptr(), out.stride(0), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), step.num_seqs,
-          heads, groups, dim, vdim, 1 if unit_norm else 0, q_scale, unit_eps, 1 if T == step.num_seqs else 0, 1 if rows_decay else 0,
-          1 if (by_shape and (T == step.num_seqs or _recurrence_fills_sms(step.num_seqs, heads, dim, vdim))) else 0,
+          heads, groups, dim, vdim, 1 if unit_norm else 0, q_scale, unit_eps, 1 if ones else 0, 1 if rows_decay else 0,
+          1 if (by_shape and (ones or _recurrence_fills_sms(seqs, heads, dim, vdim))) else 0,
           skip, stream)
 
 
@@ -1114,7 +1162,8 @@ def decay_recurrence(pre: torch.Tensor, q_col: int, k_col: int, v_col: int, deca
     and the tokens' own scores (32-bit, outputs equal within rounding, several times faster), the state's rows shared out
     over row_split CTAs; out is then [row_split, T, heads * vdim] and the sum over its first dimension is meant.
     With 0 every output's sum has one order however the sequence is cut, unless `by_shape` sends long portions through the
-    chunked form (chunk_portions) and steps of single tokens through a kernel of their own (single_tokens)."""
+    chunked form (chunk_portions; the portions beside them side by side) and steps of single tokens through a kernel of their
+    own (single_tokens)."""
     _check(decay, "decay", torch.float32); _check(state, "recurrent state", torch.float32); _check(out, "recurrence output", torch.float32)
     if pre.dtype != torch.float32 or pre.stride(1) != 1 or not pre.is_cuda:
         raise KernelError("the input projections must be float32 on the GPU with unit column stride")
@@ -1131,6 +1180,8 @@ def decay_recurrence(pre: torch.Tensor, q_col: int, k_col: int, v_col: int, deca
         _chunk_recurrence("fixed", q, k, v, state, out, step, long, heads, heads, dim, vdim, stream, decay=decay, act=act)
         if len(long) == step.num_seqs:
             return
+        _, max_tokens_a_seq = _shorter(step, skip)
+        row_split = 1 if max_tokens_a_seq > 8 else 0          # side by side in one plane, unless half of the 16 would be formed for nothing
     _call("lb_decay_recurrence", pre.data_ptr(), pre.stride(0), q_col, k_col, v_col, decay.data_ptr(), state.data_ptr(),
           out.data_ptr(), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), step.num_seqs, heads, dim, vdim,
           max_tokens_a_seq, row_split, T * heads * vdim, 1 if act else 0, skip, stream)

@@ -96,8 +96,8 @@ class DecayLinearAttention(Mixer):
             inv_freq, rot = self.position_encoding.rotary_table() if self.position_encoding is not None else (None, 0)
             ops.rotate_rows(pre, step.positions, inv_freq, self.dim, rot, [(0, self.heads, 1.0), (n, self.heads, self.k_scale)], rt.stream,
                             rot_scale=getattr(self.position_encoding, "magnitude", 1.0))
-        # the bfloat16 engine takes long portions 64 tokens at a time; where there are none, it forms the outputs of up to 16
-        # tokens side by side, the rows of the state shared out over CTAs
+        # the bfloat16 engine takes steps with long portions 64 tokens at a time; where there are none, it forms the outputs of up
+        # to 16 tokens side by side, the rows of the state shared out over CTAs
         single = rt.fast_kernels and ops.single_tokens(step, self.dim, self.vdim, cache.state)
         chunked = rt.fast_kernels and not single and bool(ops.chunk_portions("fixed", step, self.heads, self.dim, self.vdim)[0])
         split = ops.decay_row_split(step.num_seqs, self.heads, self.dim, self.vdim, step.max_q_len) if rt.fast_kernels and not (single or chunked) else 0

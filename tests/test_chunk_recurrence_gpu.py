@@ -105,8 +105,9 @@ def plain(kind, o, state, step, heads, groups, dim, vdim):
 
 @pytest.fixture(autouse=True)
 def from_32_tokens(monkeypatch):
+    """Whatever it costs: the chunked form for every portion that it may take."""
     from lucciola_b200 import ops
-    monkeypatch.setattr(ops, "CHUNK_FROM", {k: 0 for k in ops.CHUNK_FROM})
+    monkeypatch.setattr(ops, "chunk_portions", lambda kind, step, *sizes: ([i for i, n in enumerate(step.q_lens) if n >= 32], 32))
 
 
 @pytest.mark.parametrize("heads,groups,dim,vdim,lens", [
@@ -255,18 +256,6 @@ def test_scratch_for_fewer_chunks_and_more_sequences_than_a_launch(kind, monkeyp
     want, S = plain(kind, o, state, step, heads, heads, dim, vdim)
     got = through_ops(kind, o, state, step, heads, heads, dim, vdim, True)
     assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max() and (state.double() - S).abs().max() <= 1e-5 * S.abs().max()
-
-
-def test_which_portions_are_long(monkeypatch):
-    from lucciola_b200 import ops
-    monkeypatch.undo()
-    step = lambda *lens: SimpleNamespace(num_seqs=len(lens), q_lens=list(lens), max_q_len=max(lens))
-    first = int(ops.CHUNK_FROM["delta"] / (1 + 2 / 64))
-    assert ops.chunk_portions("delta", step(1, first, 31), 2, 128, 64) == ([1], first)
-    assert ops.chunk_portions("delta", step(1, first - 1, 31), 2, 128, 64) == ([], 0)
-    assert ops.chunk_portions("delta", step(32, 40, 31), 4096, 128, 64) == ([0, 1], 32)
-    assert ops.chunk_portions("delta", step(9999), 2, 129, 64) == ([], 0)                # more rows of the state than the kernels hold
-    assert ops.chunk_portions("delta", SimpleNamespace(num_seqs=3, q_lens=[], max_q_len=9999), 2, 64, 64) == ([], 0)      # lengths the host does not know
 
 
 @pytest.mark.parametrize("channels,lens", [(8192, [1]), (260, [1] * 9), (4096, [700, 1, 2, 3, 4, 5, 333]), (1028, [9, 200]), (64, [3000]), (2048, [5, 4, 1, 1, 90])])
