@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(MAX_THREADS) decay_recurrence_kernel(DecayRecu
   float* st = p.state + (((size_t)p.slots[seq] * p.heads + h) * p.dim) * p.vdim;
   float s[DS];
   pdl_wait();
-  if (p.skip_from > 0 && n >= p.skip_from) return;
+  if (left_out(p.skip_from, n)) return;
 #pragma unroll
   for (int i = 0; i < DS; ++i) {
     const int d = warp * DS + i;
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(256) decay_chunk_kernel(DecayChunkParams pc) {
   const float* q_src = p.pre + p.q_col + h * p.dim + row0 + td;
   const float* k_src = p.pre + p.k_col + h * p.dim + row0 + td;
   pdl_wait();
-  if (p.skip_from > 0 && n >= p.skip_from) return;
+  if (left_out(p.skip_from, n)) return;
   auto request = [&](int c0) {                        // the raw inputs of the chunk that starts at token c0
     const int cn = min(DC_C, n - c0);
 #pragma unroll

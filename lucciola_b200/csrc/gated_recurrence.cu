@@ -79,7 +79,7 @@ __global__ void gated_recurrence_kernel(GatedRecurrenceParams p) {
     vv[0] = vv[1] = 0.f;
   }
   pdl_wait();
-  if (p.skip_from > 0 && n >= p.skip_from) return;
+  if (left_out(p.skip_from, n)) return;
   auto request = [&](int cs) {                        // the inputs of chunk cs, into registers
     const int c0 = cs * tc, cn = min(tc, n - c0);
 #pragma unroll
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(MAX_THREADS) gated_recurrence_short_kernel(Gat
   float* st = p.state + (((size_t)p.slots[seq] * p.heads + h) * p.dim) * p.vdim;
   float s[DS];
   pdl_wait();
-  if (p.skip_from > 0 && n >= p.skip_from) return;
+  if (left_out(p.skip_from, n)) return;
 #pragma unroll
   for (int i = 0; i < DS; ++i) {
     const int d = warp * DS + i;

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(SR_THREADS) state_recurrence_kernel(StateRecur
   }
   pdl_wait();
   const int first = p.cu_tokens[seq], n = p.cu_tokens[seq + 1] - first;
-  if (p.skip_from > 0 && n >= p.skip_from) return;
+  if (left_out(p.skip_from, n)) return;
   float* S = p.state + ((size_t)p.slots[seq] * p.heads + h) * p.dim * p.vdim;
   const int shift = (TURN * sub) % COLS;     // a lane's column of the state's tile, turned so that a warp's lanes spread over the banks
 
