@@ -32,6 +32,14 @@ def test_the_faster_form(kind, lens, walk, chunk):
     assert bool(portions(kind, lens, heads, dim, vdim)[0]) == (chunk < walk)
 
 
+def test_single_tokens_of_small_states_are_walked():
+    from lucciola_b200 import ops
+    state = SimpleNamespace(data_ptr=lambda: 4096)
+    one = lambda lens, dim, vdim: ops.single_tokens(SimpleNamespace(num_seqs=len(lens), q_lens=lens, max_q_len=max(lens)), dim, vdim, state)
+    assert one([1], 64, 64) and one([1] * 200, 128, 68)
+    assert not one([1], 63, 64) and not one([1], 64, 60) and not one([1], 129, 64) and not one([1], 64, 66) and not one([1, 2], 64, 64)
+
+
 def test_what_the_kernels_do_not_take():
     assert portions("delta", [9999], dim=129) == ([], 0)                    # more rows of the state than the kernels hold
     assert portions("delta", [9999], vdim=5000) == ([], 0)
