@@ -787,7 +787,7 @@ int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p,
 // a cluster's reduction).  Here a CTA takes one feature of up to eight tokens: its weight row is in registers before the
 // kernel ahead has ended, then the tokens' rows, 16 bytes a thread and row, and one sum over the CTA in a fixed order.
 // 8 tokens, 16 features of 4096, one launch behind the other: 5.1 -> 2.5 us.
-constexpr int FF_THREADS = 256, FF_TOKENS = 8, FF_AHEAD = 2;
+constexpr int FF_THREADS = 256, FF_TOKENS = 8, FF_AHEAD = 2, FF_PLACES = 16384;
 
 __device__ __forceinline__ float ff_dot(uint4 a, uint4 b, float acc) {
   const uint32_t x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
@@ -1548,8 +1548,9 @@ LB_EXPORT int lb_gemm_tcgen05(void* y, int y_dtype, const void* x, const void* w
   }
   // A router's product: 16 tokens of 128 features are 256 CTAs, which still run at once.  One launch behind the other, us, with the
   // pipeline / here: 16 features of 2048, 1 token 3.7 / 1.7, 16 tokens 4.0 / 1.9; 128 features of 4096, 1 token 4.9 / 2.7, 16 tokens
-  // 5.3 / 3.9; of 8192, 16 tokens 7.6 / 6.6, which is where the tokens' rows, read again for every feature, begin to cost as much.
-  if (M <= 16 && N <= 128 && !swiglu && !row_scale && force_bt == 0 && force_splits == 0) {
+  // 5.3 / 3.9; of 8192, 16 tokens 7.9 / 6.8; of 16384, 12.4 / 12.4, and of 32768, 21.4 / 23.5 (8 tokens 21.1 / 21.6): the tokens' rows are
+  // read again for every feature.
+  if (M <= 16 && N <= 128 && K <= lb::FF_PLACES && !swiglu && !row_scale && force_bt == 0 && force_splits == 0) {
     lb::launch(lb::gemm_few_features_kernel, dim3(N, (M + lb::FF_TOKENS - 1) / lb::FF_TOKENS), dim3(lb::FF_THREADS), 0, stream, y, y_dtype,
                (const lb::bf16*)x, (const lb::bf16*)w, M, K, ldx, ldy, post, post_c);
     LB_CHECK_LAUNCH("gemm_few_features");

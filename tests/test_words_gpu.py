@@ -87,10 +87,11 @@ def test_rope_rows(nq, nkv, d, tokens, norm, rotate, pages, pad):
     assert torch.equal(v_got, qkv[:, b:b + nkv * d].reshape(tokens, nkv, d))
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (8, 16, 4096), (7, 128, 2048), (9, 33, 5000), (16, 64, 2056), (3, 16, 8192)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (8, 16, 4096), (7, 128, 2048), (9, 33, 5000), (16, 64, 2056), (3, 16, 8192), (16, 128, 16384), (16, 128, 16392)])
 @pytest.mark.parametrize("out_type,post", [(torch.float32, None), (torch.bfloat16, None), (torch.float32, "cap")])
 def test_product_of_few_features(M, N, K, out_type, post):
-    """K products of bfloat16 values summed in 32 bits; each feature is a CTA's, so the sizes around its words and tokens matter."""
+    """K products of bfloat16 values summed in 32 bits; each feature is a CTA's, so the sizes around its words and tokens matter;
+    from 16385 places on the pipeline for few tokens takes them, in chains no longer than the bound."""
     from lucciola_b200 import ops
     torch.manual_seed(M)
     x, w = torch.randn(M, K + 8, device=DEV).bfloat16()[:, 8:], torch.randn(N, K, device=DEV).bfloat16()
