@@ -4,12 +4,12 @@
     S_t = decay_h S_(t-1) + k_t v_t^T        o_t = S_t^T q_t
     out = W_o ( rmsnorm(concat_h o_t) * w * sigmoid(W_g x) )       (one norm over all heads, w [heads * vdim])
 
-The state is 32-bit, one slot a request, zero for a new request, and is all this mixer keeps of the past: prompts,
-portions and decoded tokens go through the same kernel, which walks a sequence's tokens of the step in order from the
-state the step before left.  W_q | W_k | W_v | W_g are one product with 32-bit output; the activations, the recurrence,
-the norm and the gate are computed in 32-bit.  The bfloat16 engine takes long portions 64 tokens at a time and forms the
-outputs of shorter ones side by side (still 32-bit, the same state within rounding); the 32-bit engine walks every step
-token by token, so its results do not depend on how a prompt was cut.
+The state is 32-bit, one slot a request, zero for a new request, and is all this mixer keeps of the past: every step
+goes on from the state the step before left.  W_q | W_k | W_v | W_g are one product with 32-bit output; the activations,
+the recurrence, the norm and the gate are computed in 32-bit.  The bfloat16 engine takes steps with long portions 64 tokens
+at a time, forms the outputs of shorter ones side by side and streams the states through registers in steps of single
+tokens (still 32-bit, the same state within rounding); the 32-bit engine walks every step token by token in one kernel, so
+its results do not depend on how a prompt was cut.
 
 The form is a parameter, so that a relative of the design above can use the same part and kernels ("retention"):
 `act` ("silu", or None: q, k, v as projected), `position_encoding` (q and k are rotated in 32-bit, in place, after the

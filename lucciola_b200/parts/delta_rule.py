@@ -8,9 +8,10 @@ writes, with a decay and a write strength per head and token.  Per head, with a 
     out = W_o concat_h( o / rms(o) * n * silu(W_g x)_h )                    (n [vdim], shared by the heads)
 
 q and k come in `kv_heads` heads that heads / kv_heads value heads share.  The state and the last taps - 1 inputs of
-the convolutions are all this mixer keeps of the past: prompts, portions and decoded tokens go through the same
-kernels, which walk a sequence's tokens of the step in order from what the step before left.  W_q | W_k | W_v | W_g |
-W_b | W_a are one product with 32-bit output; everything behind it up to the output product is computed in 32-bit.
+the convolutions are all this mixer keeps of the past: every step goes on from what the step before left.  W_q | W_k |
+W_v | W_g | W_b | W_a are one product with 32-bit output; everything behind it up to the output product is computed in
+32-bit.  The 32-bit engine walks a sequence's tokens of the step in order in one kernel; the bfloat16 engine takes steps
+with long portions 64 tokens at a time and streams the states through registers in steps of single tokens.
 
 Two variants, by constructor arguments.  `decay_rank` R > 0: a decay for every key channel instead of one a head,
 g[h, d] = exp(-exp(A_log_h) * softplus((W_a2 W_a1 x)[h, d] + dt_bias[h, d])) with W_a1 [R, width], W_a2 [heads * dim, R] and

@@ -5,10 +5,10 @@
     out = W_o concat_h( rmsnorm(o_t,h) * w )          (w [vdim], shared by the heads)
 
 The state is 32-bit, one slot a request, zero for a new request, and is all this mixer keeps of the past:
-prompts, portions and decoded tokens go through the same kernel, which walks a sequence's tokens of the
-step in order from the state the step before left.  W_q | W_f | W_v are one product with 32-bit output; the
-gates, the recurrence and the output are computed in 32-bit.  The bfloat16 engine takes long portions 64 tokens at a time
-(still 32-bit, the same state within rounding).
+every step goes on from the state the step before left.  W_q | W_f | W_v are one product with 32-bit output; the
+gates, the recurrence and the output are computed in 32-bit.  The 32-bit engine walks a sequence's tokens of the
+step in order in one kernel; the bfloat16 engine takes steps with long portions 64 tokens at a time and streams the states through
+registers in steps of single tokens (still 32-bit, the same state within rounding).
 """
 from __future__ import annotations
 

@@ -6,9 +6,9 @@ and silu.  Per head (head h uses group h / (heads / G)), with a 32-bit state S [
     S <- exp(-exp(A_log) dt) S + B (dt x)^T            y = S^T C + D x
     out = W_o ( rmsnorm_parts(y * silu(z)) * w )       (the gate comes BEFORE the norm; norm_groups equal parts of the row)
 
-The state and the last taps - 1 inputs of the convolution are all this mixer keeps of the past.  The recurrence is the
-kernel of the gated delta rule without the delta rule's correction (csrc/state_recurrence.cu); everything between the
-two products is computed in 32-bit.
+The state and the last taps - 1 inputs of the convolution are all this mixer keeps of the past.  The recurrence goes
+through the kernels of the gated delta rule without the delta rule's correction (csrc/state_recurrence.cu; in the bfloat16
+engine also csrc/chunk_recurrence.cu and csrc/state_step.cu); everything between the two products is computed in 32-bit.
 
 Beside forward(), the mixer offers its steps apart (in_names / in_sizes, inner, `o`).
 """
