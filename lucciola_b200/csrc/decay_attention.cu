@@ -137,8 +137,8 @@ static cudaError_t launch_decay_recurrence(const DecayRecurrenceParams& p, int n
 // The first term is C independent sums over the rows of S0 (no token waits for the one before), the second needs the
 // C x C scores of the chunk, which every thread of the CTA shares.  The state itself still moves token by token,
 // S <- decay S + k_j v_j^T, the very operations of the kernel above; only the order in which an output's terms are
-// added differs (32-bit throughout; silu by the fast exponential and reciprocal, 2 ulp).  The raw inputs of the next
-// chunk are requested before the work on the current one and turned into q, k, v after it.
+// added differs (32-bit throughout; silu by the fast exponential, off by 2 + |1.16 x| units in the last place, and a reciprocal rounded
+// to nearest).  The raw inputs of the next chunk are requested before the work on the current one and turned into q, k, v after it.
 //
 // Both terms are sums over the rows of the state (the scores are sums over the same rows of q and k), so the rows may
 // be shared out: with `row_split` R a CTA takes dim / R rows and writes its share of every output to plane r of `out`
