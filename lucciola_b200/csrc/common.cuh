@@ -55,15 +55,6 @@ extern int g_pdl_enabled;
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Whether a sequence of n tokens is left to another kernel (from > 0: those of so many tokens or more).  The asm keeps the
-// comparison behind the first condition: before it, every launch would wait for n, which has just been asked for, before it asks
-// for the state (decode steps of 32-bit decay attention, 64 requests of 16 heads of 128 x 128: 31 -> 35 us).
-__device__ __forceinline__ bool left_out(int from, int n) {
-  if (from <= 0) return false;
-  asm volatile("" : "+r"(n) :: "memory");
-  return n >= from;
-}
-
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                           Args&&... args) {

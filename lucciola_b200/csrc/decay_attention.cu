@@ -31,12 +31,13 @@ struct DecayRecurrenceParams {
   const int* cu_tokens; const int* slots;
   int heads, dim, vdim;
   int act;                              // 1: q, k, v pass silu; 0: they are taken as they come
-  int skip_from;                        // > 0: sequences with so many tokens or more belong to another kernel (chunk_recurrence.cu)
+  int skip_from;                        // > 0: sequences with so many tokens or more belong to another kernel (chunk_recurrence.cu); kernels of
+                                        // their own (SKIP), as a look at the length before the state costs every launch 0.2 us and more
 };
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.f + expf(-x)); }
 
-template <int DS, int TC, int MAX_THREADS>
+template <int DS, int TC, int MAX_THREADS, bool SKIP>
 __global__ void __launch_bounds__(MAX_THREADS) decay_recurrence_kernel(DecayRecurrenceParams p) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(MAX_THREADS) decay_recurrence_kernel(DecayRecu
   float* st = p.state + (((size_t)p.slots[seq] * p.heads + h) * p.dim) * p.vdim;
   float s[DS];
   pdl_wait();
-  if (left_out(p.skip_from, n)) return;
+  if (SKIP && n >= p.skip_from) return;
 #pragma unroll
   for (int i = 0; i < DS; ++i) {
     const int d = warp * DS + i;
@@ -121,11 +122,12 @@ static cudaError_t launch_decay_recurrence(const DecayRecurrenceParams& p, int n
   const size_t smem = (size_t)TC * (2 * nwarps * DS + 32 + nwarps * 32) * sizeof(float);
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
-    const cudaError_t e = cudaFuncSetAttribute(decay_recurrence_kernel<DS, TC, MAX_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(decay_recurrence_kernel<DS, TC, MAX_THREADS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_recurrence_kernel<DS, TC, MAX_THREADS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     allowed = smem;
   }
-  return launch(decay_recurrence_kernel<DS, TC, MAX_THREADS>, dim3((p.vdim + 31) / 32, p.heads, num_seqs), dim3(nwarps * 32), smem, stream, p);
+  return launch(p.skip_from > 0 ? decay_recurrence_kernel<DS, TC, MAX_THREADS, true> : decay_recurrence_kernel<DS, TC, MAX_THREADS, false>, dim3((p.vdim + 31) / 32, p.heads, num_seqs), dim3(nwarps * 32), smem, stream, p);
 }
 
 
@@ -154,7 +156,7 @@ struct DecayChunkParams {
 
 __device__ __forceinline__ float silu_fast(float x) { return x * __frcp_rn(1.f + __expf(-x)); }
 
-template <int DS, int NV>      // NV: values of v a thread holds for the next chunk, ceil(C * 32 / threads) rounded up to 2, 4, 8 or 16
+template <int DS, int NV, bool SKIP>      // NV: values of v a thread holds for the next chunk, ceil(C * 32 / threads) rounded up to 2, 4, 8 or 16
 __global__ void __launch_bounds__(256) decay_chunk_kernel(DecayChunkParams pc) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
@@ -188,7 +190,7 @@ __global__ void __launch_bounds__(256) decay_chunk_kernel(DecayChunkParams pc) {
   const float* q_src = p.pre + p.q_col + h * p.dim + row0 + td;
   const float* k_src = p.pre + p.k_col + h * p.dim + row0 + td;
   pdl_wait();
-  if (left_out(p.skip_from, n)) return;
+  if (SKIP && n >= p.skip_from) return;
   auto request = [&](int c0) {                        // the raw inputs of the chunk that starts at token c0
     const int cn = min(DC_C, n - c0);
 #pragma unroll
@@ -299,11 +301,12 @@ static cudaError_t launch_decay_chunk_nv(const DecayChunkParams& pc, int num_seq
   const size_t smem = (size_t)(2 * DC_C * (dimp + 4) + DC_C * 32 + DC_C * nwarps * 32 + DC_C * (DC_C + 1)) * sizeof(float);
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
-    const cudaError_t e = cudaFuncSetAttribute(decay_chunk_kernel<DS, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(decay_chunk_kernel<DS, NV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(decay_chunk_kernel<DS, NV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     allowed = smem;
   }
-  return launch(decay_chunk_kernel<DS, NV>, dim3(((pc.b.vdim + 31) / 32) * pc.row_split, pc.b.heads, num_seqs), dim3(nwarps * 32), smem, stream, pc);
+  return launch(pc.b.skip_from > 0 ? decay_chunk_kernel<DS, NV, true> : decay_chunk_kernel<DS, NV, false>, dim3(((pc.b.vdim + 31) / 32) * pc.row_split, pc.b.heads, num_seqs), dim3(nwarps * 32), smem, stream, pc);
 }
 
 template <int DS>

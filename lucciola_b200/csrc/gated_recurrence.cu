@@ -34,7 +34,7 @@ struct GatedRecurrenceParams {
   float* out;                           // [T, heads * vdim]
   const int* cu_tokens; const int* slots;
   int heads, dim, vdim;
-  int skip_from;                        // > 0: sequences with so many tokens or more belong to another kernel (chunk_recurrence.cu)
+  int skip_from;                        // > 0: sequences with so many tokens or more belong to another kernel (chunk_recurrence.cu; SKIP)
 };
 
 __host__ __device__ inline int gr_chunk_tokens(int dimp) {
@@ -42,7 +42,7 @@ __host__ __device__ inline int gr_chunk_tokens(int dimp) {
   return tc > GR_TC_MAX ? GR_TC_MAX : (tc < 1 ? 1 : tc);
 }
 
-template <int DS>
+template <int DS, bool SKIP>
 __global__ void gated_recurrence_kernel(GatedRecurrenceParams p) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
@@ -79,7 +79,7 @@ __global__ void gated_recurrence_kernel(GatedRecurrenceParams p) {
     vv[0] = vv[1] = 0.f;
   }
   pdl_wait();
-  if (left_out(p.skip_from, n)) return;
+  if (SKIP && n >= p.skip_from) return;
   auto request = [&](int cs) {                        // the inputs of chunk cs, into registers
     const int c0 = cs * tc, cn = min(tc, n - c0);
 #pragma unroll
@@ -187,11 +187,12 @@ static cudaError_t launch_gated_recurrence(const GatedRecurrenceParams& p, int n
   const size_t smem = (size_t)(2 * tc * (2 * nwarps * DS + 32) + 2 * tc * nwarps * 32) * sizeof(float);
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
-    const cudaError_t e = cudaFuncSetAttribute(gated_recurrence_kernel<DS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gated_recurrence_kernel<DS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gated_recurrence_kernel<DS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     allowed = smem;
   }
-  return launch(gated_recurrence_kernel<DS>, dim3((p.vdim + 31) / 32, p.heads, num_seqs), dim3((nwarps + GR_FEED) * 32), smem, stream, p);
+  return launch(p.skip_from > 0 ? gated_recurrence_kernel<DS, true> : gated_recurrence_kernel<DS, false>, dim3((p.vdim + 31) / 32, p.heads, num_seqs), dim3((nwarps + GR_FEED) * 32), smem, stream, p);
 }
 
 // The same for steps in which no sequence brings more than a few tokens (decoding): no feeding warps and few
@@ -200,7 +201,7 @@ static cudaError_t launch_gated_recurrence(const GatedRecurrenceParams& p, int n
 // warp order: the sums and their order are those of the kernel above, so both give the same bits.
 constexpr int GR_SHORT_TC = 4;
 
-template <int DS, int MAX_THREADS>
+template <int DS, int MAX_THREADS, bool SKIP>
 __global__ void __launch_bounds__(MAX_THREADS) gated_recurrence_short_kernel(GatedRecurrenceParams p) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(MAX_THREADS) gated_recurrence_short_kernel(Gat
   float* st = p.state + (((size_t)p.slots[seq] * p.heads + h) * p.dim) * p.vdim;
   float s[DS];
   pdl_wait();
-  if (left_out(p.skip_from, n)) return;
+  if (SKIP && n >= p.skip_from) return;
 #pragma unroll
   for (int i = 0; i < DS; ++i) {
     const int d = warp * DS + i;
@@ -283,11 +284,12 @@ static cudaError_t launch_gated_recurrence_short(const GatedRecurrenceParams& p,
   const size_t smem = (size_t)GR_SHORT_TC * (2 * nwarps * DS + 32 + nwarps * 32) * sizeof(float);      // up to 50 KB (32 warps)
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
-    const cudaError_t e = cudaFuncSetAttribute(gated_recurrence_short_kernel<DS, MAX_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gated_recurrence_short_kernel<DS, MAX_THREADS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gated_recurrence_short_kernel<DS, MAX_THREADS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     allowed = smem;
   }
-  return launch(gated_recurrence_short_kernel<DS, MAX_THREADS>, dim3((p.vdim + 31) / 32, p.heads, num_seqs), dim3(nwarps * 32), smem, stream, p);
+  return launch(p.skip_from > 0 ? gated_recurrence_short_kernel<DS, MAX_THREADS, true> : gated_recurrence_short_kernel<DS, MAX_THREADS, false>, dim3((p.vdim + 31) / 32, p.heads, num_seqs), dim3(nwarps * 32), smem, stream, p);
 }
 
 }  // namespace lb

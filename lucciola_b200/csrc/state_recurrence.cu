@@ -43,7 +43,7 @@ struct StateRecurrenceParams {
   int vec;                       // q, k, v rows start on 16-byte boundaries and hold whole 16-byte pieces
   int svec;                      // so do the state's rows
   int avec;                      // with a decay for every state row: so do the rows of `a`
-  int skip_from;                 // > 0: sequences with so many tokens or more belong to another kernel (chunk_recurrence.cu)
+  int skip_from;                 // > 0: sequences with so many tokens or more belong to another kernel (chunk_recurrence.cu; SKIP)
 };
 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
@@ -67,7 +67,7 @@ __host__ __device__ constexpr int sr_smem_floats(int rpl, int sub, int tokens, b
 // VG: the decay is a vector, one number for every row of the state (key channel) and token, S <- diag(g) S.  `a` then
 // holds the decays themselves, heads * dim numbers a token, as lb_channel_decay leaves them: formed once for all the
 // CTAs that share a head, and off the path from one token to the next.
-template <bool DELTA, int RPL, int SUB, int TOK, bool VG = false>
+template <bool DELTA, int RPL, int SUB, int TOK, bool VG, bool SKIP>
 __global__ void __launch_bounds__(SR_THREADS) state_recurrence_kernel(StateRecurrenceParams p) {
   constexpr int T = TOK, COLS = SR_THREADS / SUB, ROW = (RPL + 4) * SUB, DP = RPL * SUB;
   constexpr int TURN = 32 / SUB < 4 ? 4 : 32 / SUB;   // columns by which a lane's rows are turned in the state's tile: whole 16-byte words
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(SR_THREADS) state_recurrence_kernel(StateRecur
   }
   pdl_wait();
   const int first = p.cu_tokens[seq], n = p.cu_tokens[seq + 1] - first;
-  if (left_out(p.skip_from, n)) return;
+  if (SKIP && n >= p.skip_from) return;
   float* S = p.state + ((size_t)p.slots[seq] * p.heads + h) * p.dim * p.vdim;
   const int shift = (TURN * sub) % COLS;     // a lane's column of the state's tile, turned so that a warp's lanes spread over the banks
 
@@ -424,13 +424,13 @@ LB_EXPORT int lb_state_recurrence(int delta, const float* q, long long q_ld, con
   p.vec = dim % 4 == 0 && vdim % 4 == 0 && aligned(q, q_ld) && aligned(k, k_ld) && aligned(v, v_ld);
   p.svec = vdim % 4 == 0 && (uintptr_t)state % 16 == 0;
   p.avec = rows_decay && dim % 4 == 0 && aligned(a, a_ld);
-#define LB_SR1(RPL, SUB, TOK)                                                                                       \
+#define LB_SR2(RPL, SUB, TOK, SKIP)                                                                                 \
   do {                                                                                                              \
     const size_t smem = (size_t)lb::sr_smem_floats(RPL, SUB, TOK) * sizeof(float);                                  \
     static bool cfg = false;                                                                                        \
     if (!cfg) {                                                                                                     \
-      cudaFuncSetAttribute(lb::state_recurrence_kernel<true, RPL, SUB, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-      cudaFuncSetAttribute(lb::state_recurrence_kernel<false, RPL, SUB, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+      cudaFuncSetAttribute(lb::state_recurrence_kernel<true, RPL, SUB, TOK, false, SKIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+      cudaFuncSetAttribute(lb::state_recurrence_kernel<false, RPL, SUB, TOK, false, SKIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
       cfg = true;                                                                                                   \
     }                                                                                                               \
     dim3 grid((vdim + lb::SR_THREADS / SUB - 1) / (lb::SR_THREADS / SUB), heads, num_seqs), block(lb::SR_THREADS); \
@@ -438,12 +438,17 @@ LB_EXPORT int lb_state_recurrence(int delta, const float* q, long long q_ld, con
       const size_t smem_g = (size_t)lb::sr_smem_floats(RPL, SUB, TOK, true) * sizeof(float);                        \
       static bool cfg_g = false;                                                                                    \
       if (!cfg_g) {                                                                                                 \
-        cudaFuncSetAttribute(lb::state_recurrence_kernel<true, RPL, SUB, TOK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_g); \
+        cudaFuncSetAttribute(lb::state_recurrence_kernel<true, RPL, SUB, TOK, true, SKIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_g); \
         cfg_g = true;                                                                                               \
       }                                                                                                             \
-      lb::launch(lb::state_recurrence_kernel<true, RPL, SUB, TOK, true>, grid, block, smem_g, stream, p);           \
-    } else if (delta) lb::launch(lb::state_recurrence_kernel<true, RPL, SUB, TOK>, grid, block, smem, stream, p);          \
-    else lb::launch(lb::state_recurrence_kernel<false, RPL, SUB, TOK>, grid, block, smem, stream, p);               \
+      lb::launch(lb::state_recurrence_kernel<true, RPL, SUB, TOK, true, SKIP>, grid, block, smem_g, stream, p);           \
+    } else if (delta) lb::launch(lb::state_recurrence_kernel<true, RPL, SUB, TOK, false, SKIP>, grid, block, smem, stream, p);          \
+    else lb::launch(lb::state_recurrence_kernel<false, RPL, SUB, TOK, false, SKIP>, grid, block, smem, stream, p);               \
+  } while (0)
+#define LB_SR1(RPL, SUB, TOK)                                                                                       \
+  do {                                                                                                              \
+    if (skip_from > 0) LB_SR2(RPL, SUB, TOK, true);                                                                 \
+    else LB_SR2(RPL, SUB, TOK, false);                                                                              \
   } while (0)
   // a step of single tokens stages one token at a time: the same sums in the same order, a fifth of the shared memory
 #define LB_SR(RPL, SUB)                                                                                             \
@@ -460,6 +465,7 @@ LB_EXPORT int lb_state_recurrence(int delta, const float* q, long long q_ld, con
   else if (dim <= 64) { if (wide_lanes) LB_SR(16, 4); else LB_SR(8, 8); }
   else if (dim <= 128) { if (wide_lanes) LB_SR(16, 8); else LB_SR(8, 16); }
   else { if (wide_lanes) LB_SR(32, 8); else LB_SR(16, 16); }
+#undef LB_SR2
 #undef LB_SR1
 #undef LB_SR
   LB_CHECK_LAUNCH("state_recurrence");
