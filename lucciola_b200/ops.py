@@ -726,8 +726,8 @@ def _shorter(step, skip: int) -> tuple[int, int]:
 def single_tokens(step, dim: int, vdim: int, state: torch.Tensor) -> bool:
     """Whether a step is one token a sequence, by the lengths the host knows, and its states are of a form that the kernel for such
     steps takes (csrc/state_step.cu) and is faster for: up to 128 rows, whole 16-byte words a row, and enough of both for its 256
-    threads (64 requests of 64 heads, us token by token | there: fixed decays 16 x 32 7.4 | 15.1, HGRN2 7.4 | 12.3; 64 heads of
-    64 rows and 8 heads of 64 x 64 are the smallest that gain throughout)."""
+    threads (64 requests of 64 heads, us token by token | there: fixed decays 16 x 32 7.4 | 15.1, HGRN2 7.4 | 12.3; states of
+    64 x 64 are the smallest measured that do not lose at any number of heads and requests)."""
     return (step.max_q_len == 1 and 64 <= dim <= 128 and vdim >= 64 and vdim % 4 == 0 and step.q_lens.count(1) == step.num_seqs == len(step.q_lens)
             and state.data_ptr() % 16 == 0)
 
