@@ -859,6 +859,19 @@ constexpr int PF_STAGES = 4;
 // tile running fastest, the second kind after the first.
 struct PrefillPlan { int bn1, cols1, bn2; int mb = 16; };     // mb: token tiles of a block (the order of the tiles, see tile_of)
 
+// 32 bytes of a row: a lane's own sector in one store where it begins one (width 2), which it does not share with the store of the next
+// 16 bytes (a warp writes 32 rows: 2048 x 6144 sums of 2048 places in float32 54.4 -> 43.9 us).
+__device__ __forceinline__ void store_words(void* dst, const uint32_t* w, int width) {
+  if (width == 2) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+  } else {
+    uint4* d = reinterpret_cast<uint4*>(dst);
+    d[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    d[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
+
 // PAIR: two CTAs of a cluster work on one tile of 256 tokens x up to 256 features (tcgen05 cta_group::2): each holds its
 // own 128 tokens and half of the tile's weight rows in shared memory (two thirds of the bytes a stage of one CTA holds:
 // six stages instead of four), the first CTA of the pair issues the MMAs for both, and each CTA finds its 128 tokens x
@@ -1067,6 +1080,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
         const int tile_col = second ? plan.cols1 + (n0 - plan.cols1 * plan.bn1) / plan.bn2 : n0 / plan.bn1;
         const bool row_ok = m < p.M;
         const bool vec = (p.N & 7) == 0;
+        const int words = (p.N & 15) == 0 && (((uintptr_t)an.residual | (uintptr_t)an.out) & 31) == 0 ? 2 : 1;
         float* res_row = an.residual + (size_t)(row_ok ? m : 0) * p.N;
         bf16* out_row = an.out + (size_t)(row_ok ? m : 0) * p.N;
         float ss = 0.f;
@@ -1108,9 +1122,8 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
                 if (n + j < p.N) ss += v[j] * v[j];
               }
               if (vec && n + 16 <= p.N) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                  *reinterpret_cast<float4*>(res_row + n + 4 * j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                store_words(res_row + n, reinterpret_cast<const uint32_t*>(v), words);
+                store_words(res_row + n + 8, reinterpret_cast<const uint32_t*>(v) + 8, words);
                 uint32_t w[8];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -1119,9 +1132,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
                   __nv_bfloat162 hi = __floats2bfloat162_rn(v[4 * j + 2] * nw.z, v[4 * j + 3] * nw.w);
                   w[2 * j] = *reinterpret_cast<uint32_t*>(&lo); w[2 * j + 1] = *reinterpret_cast<uint32_t*>(&hi);
                 }
-                uint4* dst = reinterpret_cast<uint4*>(out_row + n);
-                dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                store_words(out_row + n, w, words);
               } else {
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
@@ -1151,19 +1162,17 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
             for (int j = 0; j < 16; ++j) v[j] = gated_mul(p.swiglu, p.act_limit, __uint_as_float(g[j]) * rf, __uint_as_float(u[j]) * rf);
             if (vec_store && feature + 16 <= (p.N >> 1)) {
               if (p.out_dtype == LB_F32) {
-                float4* dst = reinterpret_cast<float4*>((float*)p.y + (size_t)m * p.ldy + feature);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                float* dst = (float*)p.y + (size_t)m * p.ldy + feature;
+                store_words(dst, reinterpret_cast<const uint32_t*>(v), vec_store);
+                store_words(dst + 8, reinterpret_cast<const uint32_t*>(v) + 8, vec_store);
               } else {
-                uint4* dst = reinterpret_cast<uint4*>((bf16*)p.y + (size_t)m * p.ldy + feature);
                 uint32_t w[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                   __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
                   w[j] = *reinterpret_cast<uint32_t*>(&b2);
                 }
-                dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                store_words((bf16*)p.y + (size_t)m * p.ldy + feature, w, vec_store);
               }
             } else {
 #pragma unroll
@@ -1197,20 +1206,17 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
         if (m < p.M && n < p.N) {
           if (vec_store && n + 16 <= p.N) {
             if (p.out_dtype == LB_F32) {
-              float4* dst = reinterpret_cast<float4*>((float*)p.y + (size_t)m * p.ldy + n);
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                dst[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+              float* dst = (float*)p.y + (size_t)m * p.ldy + n;
+              store_words(dst, r, vec_store);
+              store_words(dst + 8, r + 8, vec_store);
             } else {
-              uint4* dst = reinterpret_cast<uint4*>((bf16*)p.y + (size_t)m * p.ldy + n);
               uint32_t w[8];
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
                 w[j] = *reinterpret_cast<uint32_t*>(&v);
               }
-              dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-              dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+              store_words((bf16*)p.y + (size_t)m * p.ldy + n, w, vec_store);
             }
           } else {
 #pragma unroll
@@ -1402,7 +1408,8 @@ static int launch_prefill(const void* y, int y_dtype, const void* x, const void*
   const int rest = N - plan.cols1 * plan.bn1;
   const int num_tiles = m_tiles * (plan.cols1 + (rest > 0 ? (rest + plan.bn2 - 1) / plan.bn2 : 0));
   const int el = y_dtype == LB_F32 ? 4 : 2;
-  const int vec_store = ((uintptr_t)y % 16 == 0) && ((ldy * el) % 16 == 0);
+  const uintptr_t lowest = (uintptr_t)y | (uintptr_t)(ldy * el);
+  const int vec_store = lowest % 32 == 0 ? 2 : lowest % 16 == 0;
   const int smem = (use_pair ? PrefillSmemT<true>::TOTAL : PrefillSmemT<false>::TOTAL) + 1024;
   static bool configured[2] = {false, false};
   if (!configured[use_pair]) {
