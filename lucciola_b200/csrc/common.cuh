@@ -68,6 +68,15 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// One lane of a whole warp.  A role that one thread plays is entered this way and not by `lane == 0`: the compiler then knows that a
+// single thread is in it, and the operands of copies and matrix products need no loop over the lanes on their way into uniform
+// registers (four tcgen05.mma with their commit, 128 x 64: 264 -> 196 cycles; with the waits and copies of a ring 640 -> 490).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+
 __device__ __forceinline__ float to_f32(float x) { return x; }
 __device__ __forceinline__ float to_f32(bf16 x) { return __bfloat162float(x); }
 

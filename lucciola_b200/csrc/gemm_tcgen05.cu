@@ -361,7 +361,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
   if (warp == 0) {
     // ---- producer --------------------------------------------------------------------------
-    if (lane == 0 && !p.skip_loads) {
+    if (elect_one() && !p.skip_loads) {
       int issued = 0;
       // The token tiles follow the early weight tiles when the kernel before this one has completed.
       pdl_wait();
@@ -390,7 +390,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
   } else if (warp == 1) {
     // ---- tensor-core issue ---------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc(BT);
       bool ok = true;
       for (int i = 0; i < num_kb && ok; ++i) {
@@ -978,7 +978,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
 
   if (warp == 0) {
     // ---- producer: one ring of stages across all tiles of this CTA -------------------------------------
-    if (lane == 0 && my_tiles > 0) {
+    if (elect_one() && my_tiles > 0) {
       long long it = 0;                       // stage uses so far
       bool ok = true;
       // The weights of the first tile do not depend on the kernel before this one.
@@ -1021,7 +1021,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
     }
   } else if (warp == 1) {
     // ---- tensor-core issue -----------------------------------------------------------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       bool ok = true;
       for (int t = 0; t < my_tiles && ok; ++t) {
         const int b = t & 1;
