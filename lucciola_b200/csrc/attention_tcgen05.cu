@@ -202,7 +202,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, TcAttnParams
   } else if (warp == 0 || warp == 10) {
     // ---- producers: warp 0 the queries (TMA) and the keys, warp 10 the values ---------------------------------
     const bool is_v = warp == 10;
-    if (!is_v && lane == 0) {
+    if (!is_v && elect_one()) {
       ta_mbar_expect_tx(q_full, (uint32_t)(ntiles * G * per) * 256u);      // a tile's box: G * per rows of 256 bytes, in two halves
       for (int t = 0; t < ntiles; ++t) {
         ta_tma_3d(sbase + TA_Q_OFF + t * TA_TILE_BYTES, &map_q, 0, kvh * G, t0 + t * per, q_full);
@@ -251,7 +251,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, TcAttnParams
   } else if (warp == 1 || warp == 11) {
     // ---- tensor-core issue, one thread per tile --------------------------------------------------------------
     const int t = warp == 1 ? 0 : 1;
-    if (lane == 0 && t < ntiles) {
+    if (t < ntiles && elect_one()) {
       constexpr uint32_t idesc_qk = ta_idesc(0, TA_KEYS), idesc_pv = ta_idesc(1, TA_D);
       const uint32_t s_col = tmem + (uint32_t)t * 128u, o_col = tmem + 256u + (uint32_t)t * 128u;
       const uint32_t qa = sbase + TA_Q_OFF + t * TA_TILE_BYTES;

@@ -126,7 +126,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_qu, const __grid_c
     }
   } else if (warp == 0 || warp == 10) {
     // ---- producers, a thread each: warp 0 the queries and the keys, warp 10 the values -----------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       const bool is_v = warp == 10;
       if (!is_v) {
         ta_mbar_expect_tx(q_full, (uint32_t)(ntiles * p.chunks) * TA_HALF_BYTES);
@@ -163,7 +163,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap map_qu, const __grid_c
   } else if (warp == 1 || warp == 11) {
     // ---- tensor-core issue, one thread per tile --------------------------------------------------------------
     const int t = warp == 1 ? 0 : 1;
-    if (lane == 0 && t < ntiles) {
+    if (t < ntiles && elect_one()) {
       constexpr uint32_t idesc_qk = ta_idesc(0, TA_KEYS), idesc_pv = ta_idesc(1, VC * 64);
       const uint32_t s_col = tmem + (uint32_t)t * 128u, o_col = tmem + 256u + (uint32_t)t * 128u;
       const uint32_t qa = sbase + t * LP_Q_TILE;
