@@ -333,7 +333,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
   pdl_trigger();
   const int early = num_kb < STAGES ? num_kb : STAGES;
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
     for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
@@ -852,7 +852,6 @@ __global__ void __launch_bounds__(FF_THREADS) gemm_few_features_kernel(void* __r
 // 64 tiles for 148 SMs), and the launcher picks the width with the smallest waves x width.
 constexpr int PF_BM = 128;       // tokens of a tile (lanes)
 constexpr int PF_BN = 256;       // the most features of a tile (columns of an accumulator)
-constexpr int PF_STAGES = 4;
 
 // The feature tiles of a launch: `cols1` columns of tiles `bn1` wide, then the features from cols1 * bn1 on in tiles
 // `bn2` wide (their weight boxes come through a second tensor map).  Tiles are numbered column by column, the token
@@ -876,17 +875,18 @@ __device__ __forceinline__ void store_words(void* dst, const uint32_t* w, int wi
 // own 128 tokens and half of the tile's weight rows in shared memory (two thirds of the bytes a stage of one CTA holds:
 // six stages instead of four), the first CTA of the pair issues the MMAs for both, and each CTA finds its 128 tokens x
 // all features of the tile in its own tensor memory.
+// A stage holds 64 places of the tile's tokens and of as many weight rows as the launch's widest tile has, and the ring as many stages as
+// fit: what is in flight, not how many stages there are, is what a short tile's loop waits for (a CTA alone on its SM; 128 x 64
+// tiles with four stages of 24 KB took 0.33 us a stage, as did 128 x 256 ones with four of 48).
 template <bool PAIR>
 struct PrefillSmemT {
-  static constexpr int STAGES = PAIR ? 6 : PF_STAGES;
+  static constexpr int STAGES = 10;        // at most
   static constexpr int A_BYTES = PF_BM * BK * 2;
-  static constexpr int B_BYTES = (PAIR ? PF_BN / 2 : PF_BN) * BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
+  static constexpr int RING_BYTES = 192 * 1024;
+  static constexpr int BAR_OFFSET = RING_BYTES;
   static constexpr int NUM_BARS = 2 * STAGES + 4;
   static constexpr int TOTAL = BAR_OFFSET + NUM_BARS * 8 + 16;
 };
-using PrefillSmem = PrefillSmemT<false>;
 
 // With PAIR, m_tiles counts pairs of token tiles, num_tiles tiles of 256 tokens, and the grid holds two CTAs a tile slot.
 template <bool PAIR>
@@ -895,7 +895,9 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
                             const __grid_constant__ CUtensorMap map_w2, GemmParams p, int m_tiles, int num_tiles,
                             PrefillPlan plan, int vec_store) {
   using L = PrefillSmemT<PAIR>;
-  constexpr int PF_STAGES = L::STAGES;
+  const int widest = plan.cols1 > 0 && plan.bn1 > plan.bn2 ? plan.bn1 : plan.bn2;
+  const int stage = L::A_BYTES + (PAIR ? widest / 2 : widest) * BK * 2;
+  const int stages = min(L::STAGES, L::RING_BYTES / stage);
   const uint32_t rank = PAIR ? cluster_rank() : 0u;          // 0: the CTA that issues the pair's MMAs
   const int slot_id = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, num_slots = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   extern __shared__ uint8_t smem_raw[];
@@ -903,9 +905,9 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_base = smem_base + L::BAR_OFFSET;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](int s) { return bar_base + 8u * (PF_STAGES + s); };
-  auto acc_full = [&](int b) { return bar_base + 8u * (2 * PF_STAGES + b); };
-  auto acc_empty = [&](int b) { return bar_base + 8u * (2 * PF_STAGES + 2 + b); };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (L::STAGES + s); };
+  auto acc_full = [&](int b) { return bar_base + 8u * (2 * L::STAGES + b); };
+  auto acc_empty = [&](int b) { return bar_base + 8u * (2 * L::STAGES + 2 + b); };
   uint32_t* tmem_slot = (uint32_t*)(smem + L::BAR_OFFSET + L::NUM_BARS * 8);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
@@ -955,7 +957,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w2) : "memory");
-    for (int s = 0; s < PF_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+    for (int s = 0; s < stages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     // an accumulator is free again when the four epilogue warps (of both CTAs of a pair) have read it
     for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), PAIR ? 8 : 4); }
     *abort_flag = 0;
@@ -980,41 +982,42 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
     // ---- producer: one ring of stages across all tiles of this CTA -------------------------------------
     if (elect_one() && my_tiles > 0) {
       long long it = 0;                       // stage uses so far
+      int s = 0;                              // the next use's stage, and what its barrier's parity was a turn ago
+      uint32_t before = 1;
       bool ok = true;
       // The weights of the first tile do not depend on the kernel before this one.
-      const int early = p.tile_group ? 0 : (num_kb < PF_STAGES ? num_kb : PF_STAGES);   // (which weights: known behind the wait only)
+      const int early = p.tile_group ? 0 : min(num_kb, stages);   // (which weights: known behind the wait only)
       {
         int m0, n0, bn;
         const CUtensorMap* mw = tile_of(slot_id, m0, n0, bn) ? &map_w2 : &map_w;
         for (int i = 0; i < early; ++i) {
           if (rank == 0) mbar_expect_tx(full_bar(i), stage_bytes(bn));
-          load(smem_base + i * L::STAGE_BYTES + L::A_BYTES, mw, i * BK, w_row(n0, bn, m0), full_bar(i));
+          load(smem_base + i * stage + L::A_BYTES, mw, i * BK, w_row(n0, bn, m0), full_bar(i));
         }
         pdl_wait();
         for (int i = 0; i < early; ++i)
-          load(smem_base + i * L::STAGE_BYTES, &map_x, i * BK, m0, full_bar(i));
+          load(smem_base + i * stage, &map_x, i * BK, m0, full_bar(i));
+        it = s = early;
+        if (s == stages) { s = 0; before ^= 1; }
       }
       for (int t = 0; t < my_tiles && ok; ++t) {
         int m0, n0, bn;
         const CUtensorMap* mw = tile_of(slot_id + t * num_slots, m0, n0, bn) ? &map_w2 : &map_w;
         const uint32_t stage_tx = stage_bytes(bn);
         for (int kb = (t == 0 ? early : 0); kb < num_kb; ++kb) {
-          const long long use = (long long)t * num_kb + kb;
-          const int s = (int)(use % PF_STAGES);
-          const uint32_t parity = (uint32_t)((use / PF_STAGES) & 1) ^ 1u;
-          if (!mbar_wait(empty_bar(s), parity, abort_flag, ERR_EMPTY_WAIT)) { ok = false; break; }
+          if (!mbar_wait(empty_bar(s), before, abort_flag, ERR_EMPTY_WAIT)) { ok = false; break; }
           if (rank == 0) mbar_expect_tx(full_bar(s), stage_tx);
-          const uint32_t dst = smem_base + s * L::STAGE_BYTES;
+          const uint32_t dst = smem_base + s * stage;
           load(dst, &map_x, kb * BK, m0, full_bar(s));
           load(dst + L::A_BYTES, mw, kb * BK, w_row(n0, bn, m0), full_bar(s));
-          it = use + 1;
+          ++it;
+          if (++s == stages) { s = 0; before ^= 1; }
         }
-        if (t == 0 && it < early) it = early;
       }
       if (*abort_flag) {
-        for (long long u = it > PF_STAGES ? it - PF_STAGES : 0; u < it; ++u) {
+        for (long long u = it > stages ? it - stages : 0; u < it; ++u) {
           const long long t0 = clock64();
-          while (!mbar_try_wait(full_bar((int)(u % PF_STAGES)), (uint32_t)((u / PF_STAGES) & 1)) &&
+          while (!mbar_try_wait(full_bar((int)(u % stages)), (uint32_t)((u / stages) & 1)) &&
                  (unsigned long long)(clock64() - t0) < WAIT_CYCLES / 8) {}
         }
       }
@@ -1023,6 +1026,8 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
     // ---- tensor-core issue -----------------------------------------------------------------------------------
     if (rank == 0 && elect_one()) {
       bool ok = true;
+      int s = 0;
+      uint32_t turn = 0;
       for (int t = 0; t < my_tiles && ok; ++t) {
         const int b = t & 1;
         int m0, n0, bn;
@@ -1034,12 +1039,10 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_base + (uint32_t)b * PF_BN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          const long long use = (long long)t * num_kb + kb;
-          const int s = (int)(use % PF_STAGES);
-          ok = mbar_wait(full_bar(s), (uint32_t)((use / PF_STAGES) & 1), abort_flag, ERR_FULL_WAIT);
+          ok = mbar_wait(full_bar(s), turn, abort_flag, ERR_FULL_WAIT);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_addr = smem_base + s * L::STAGE_BYTES;
+          const uint32_t a_addr = smem_base + s * stage;
           const uint64_t a_desc = umma_desc(a_addr), b_desc = umma_desc(a_addr + L::A_BYTES);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
@@ -1047,6 +1050,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
             else umma_f16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
           }
           if (PAIR) umma_commit_pair(empty_bar(s)); else umma_commit(empty_bar(s));
+          if (++s == stages) { s = 0; turn ^= 1; }
         }
         if (ok) { if (PAIR) umma_commit_pair(acc_full(b)); else umma_commit(acc_full(b)); }
       }
