@@ -1495,9 +1495,13 @@ LB_EXPORT int lb_gemm_tcgen05_plan(int M, int N, int K, int* bt) {
   else if (M > 64) t = 128;
   else if (M > 32) t = 64;
   else if (M > 16) t = 32;
+  // Few features: 33 to 128 tokens as two tiles of half as many each, where those and eight splits are 256 CTAs at most (a cluster's
+  // reduction takes half as long): 2048 features of 6144 places, us, 64 tokens 10.9 -> 9.8, 128 tokens 14.7 -> 12.1; of 4096, 9.4 -> 8.4 and
+  // 12.7 -> 10.2; 4096 features of 12288, where eight splits are too many, 128 tokens 26.3 | 28.5.
+  const int kb = (K + lb::BK - 1) / lb::BK;
+  if (M > 32 && M <= 128 && ((N + lb::BM - 1) / lb::BM) * 2 * 8 <= 256 && kb >= 32) t /= 2;
   if (bt) *bt = t;
   const int tiles = ((N + lb::BM - 1) / lb::BM) * ((M + t - 1) / t);
-  const int kb = (K + lb::BK - 1) / lb::BK;
   int splits = 1;
   if (tiles < 148 && M <= 256) {       // splitting pays only while the weights are what is streamed
     // The splits of a tile form a thread-block cluster that adds up through shared memory: any count up to 8.  As many
@@ -1535,15 +1539,15 @@ LB_EXPORT int lb_gemm_tcgen05(void* y, int y_dtype, const void* x, const void* w
   LB_CHECK_ARG(K % 8 == 0 && ldx % 8 == 0, "gemm_tcgen05: K=%d and the row stride %lld must be multiples of 8 (TMA strides are multiples of 16 bytes)", K, ldx);
   LB_CHECK_ARG(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0), "gemm_tcgen05: operands must be 16-byte aligned");
   if (M == 0) return 0;
-  // Which kernel: above 256 tokens the one with tokens on the lanes.  Below, it still wins where the product has many
-  // features for its inner size, so that its tiles fill the SMs without any cut along K: the gate|up product from 65
-  // tokens on (8B sizes, 128 tokens: 39 us against 46; 256 tokens: 58 against 92), other products with more features
-  // than inner size (q|k|v) from 129 tokens on (256 tokens: 26 us against 37).  The o and down products, few features
-  // and a long inner size, stay with the kernel that cuts K over a cluster (256 tokens, down: 37 us against 64).  The
-  // same at the sizes of every model of the family from 0.6B to 32B.  force_bt < 0 asks for the kernel with tokens on the
-  // lanes at any size; force_bt > 0 or a given split count for the other one.
-  const bool many = M > 256 ? force_bt <= 0
-                            : force_bt < 0 || (force_bt == 0 && force_splits == 0 && (swiglu ? M > 64 : (M > 128 && N > K)));
+  // Which kernel: above 256 tokens the one with tokens on the lanes.  Below, it still wins where the product has many features for its
+  // inner size, so that its tiles fill the SMs without any cut along K, the more tokens the sooner: from as many features as places
+  // on with 65 tokens, three for two places with 33, half as many with 129.  us, the kernel that cuts K over a cluster | here: 64 tokens,
+  // 3072 features of 2048 places 8.4 | 8.0, 8192 of 4096 18.8 | 16.5, 4096 of 4096 11.7 | 13.9; 128 tokens, 2048 of 2048 11.4 | 7.9, 12288 of 4096
+  // 38.2 | 22.9, 4096 of 4096 15.4 | 14.5, 2048 of 4096 10.2 | 12.7; 256 tokens, 4096 of 4096 21.3 | 15.2, 2048 of 4096 14.1 | 13.1, of 6144 16.4 | 18.4.
+  // The gated product from 65 tokens on (24576 of 4096, 64 tokens 40.8 | 47.0, 128 48.5 | 47.4).  force_bt < 0 asks for the kernel
+  // with tokens on the lanes at any size; force_bt > 0 or a given split count for the other one.
+  const bool wide = M > 128 ? 2ll * N >= K : M > 64 ? N >= K : M > 32 && 2ll * N >= 3ll * K;
+  const bool many = M > 256 ? force_bt <= 0 : force_bt < 0 || (force_bt == 0 && force_splits == 0 && (swiglu ? M > 64 : wide));
   if (many) {
     // force_bt: 0 chooses between one CTA a tile of 128 tokens and a pair of CTAs a tile of 256, -1 asks for the former,
     // -2 for the latter
@@ -1569,6 +1573,9 @@ LB_EXPORT int lb_gemm_tcgen05(void* y, int y_dtype, const void* x, const void* w
   }
   int bt = 16;
   int splits = lb_gemm_tcgen05_plan(M, N, K, &bt);
+  // A short product whose tiles fill more than half of the SMs gains less from two splits, of which some SMs hold two, than their
+  // reduction costs: 12288 features, 8 tokens, of 2048 places 13.5 -> 11.8 us; of 4096, 21.7 | 21.9.
+  if (splits == 2 && M <= 32 && K < 3072 && (N + lb::BM - 1) / lb::BM * 2 > 148) splits = 1;
   if (force_bt) {
     LB_CHECK_ARG(force_bt == 16 || force_bt == 32 || force_bt == 64 || force_bt == 128 || force_bt == 256,
                  "gemm_tcgen05: token tile %d is not one of 16, 32, 64, 128, 256", force_bt);

@@ -1,0 +1,52 @@
+"""Products on the tensor cores where one kernel, tile or store gives way to another: token counts and ratios of features to places
+on both sides of every line, rows that begin on 32-, 16- and 2-byte boundaries, and inner sizes that end inside a stage of a ring
+of any length, against the product in 64 bits (GPU)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def check(M, N, K, dtype, ldy, shift, force_bt=0, force_splits=0):
+    from lucciola_b200 import ops
+    torch.manual_seed(M * 7 + N + K)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    w = torch.randn(N, K, device=DEV).bfloat16()
+    whole = torch.full((M, ldy), 7.0, device=DEV, dtype=dtype)
+    y = whole[:, shift:shift + N]
+    ops.gemm_tcgen05(y, x, w, torch.cuda.current_stream().cuda_stream, force_bt=force_bt, force_splits=force_splits)
+    want = x.double() @ w.double().T
+    # sums of K products of 8-bit numbers: the accumulator drops less than 2^-22 of the largest partial sum each 16 places, the output rounds once
+    bound = K / 16 * 2.0 ** -22 * (x.double().abs() @ w.double().abs().T) + (2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -23) * want.abs()
+    assert ((y.double() - want).abs() <= bound + 1e-30).all()
+    rest = torch.cat([whole[:, :shift], whole[:, shift + N:]], dim=1)
+    assert (rest == 7.0).all(), "written outside the product's columns"
+
+
+@pytest.mark.parametrize("M", [32, 33, 64, 65, 128, 129, 256, 257])
+@pytest.mark.parametrize("N,K", [(384, 256), (376, 256), (256, 256), (248, 256), (128, 256), (120, 256), (2048, 2048), (2176, 2048), (264, 2056)])
+def test_on_both_sides_of_every_line(M, N, K):
+    check(M, N, K, torch.bfloat16, N, 0)
+
+
+@pytest.mark.parametrize("M", [1, 8, 32])
+@pytest.mark.parametrize("N,K", [(9472, 256), (9600, 256), (9601, 2048), (9600, 3072)])
+def test_few_tokens_of_many_features(M, N, K):
+    check(M, N, K, torch.float32, N, 0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("ldy,shift", [(320, 0), (328, 8), (324, 4), (321, 1), (336, 16)])
+@pytest.mark.parametrize("M", [130, 300, 1100])
+def test_rows_on_any_boundary(M, ldy, shift, dtype):
+    check(M, 300, 136, dtype, ldy, shift, force_bt=-1)
+
+
+@pytest.mark.parametrize("width", [16, 64, 96, 128, 160, 256])
+@pytest.mark.parametrize("K", [8, 64, 72, 520, 1032])
+@pytest.mark.parametrize("pairs", [False, True])
+def test_rings_of_any_length(width, K, pairs):
+    if pairs and width % 32:
+        pytest.skip("pairs take widths that are multiples of 32")
+    check(300, 1000, K, torch.float32, 1000, 0, force_bt=-2 if pairs else -1, force_splits=width)
