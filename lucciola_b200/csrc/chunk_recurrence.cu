@@ -31,82 +31,18 @@
 // from t on the walk may leave an infinity where a NaN stands here.
 //
 // Everything is 32-bit.  The products run on the tensor cores as six bfloat16 products of operands cut in three, which hold all 24
-// bits, 16 places at a time, and the sums from one 16 to the next are ordinary additions (see cr_step).  Decays and strengths that
-// are one number a token come out of 64 bits, and their products carry what rounding drops.  Against 64 bits the outputs before
-// the norm are 0.2 to 0.98 times as far off as those of the kernels that walk token by token, over the layers' sizes.
+// bits, 16 places at a time, and the sums from one 16 to the next are ordinary additions: those of single chunks in chunk_tcgen05.cu,
+// here the walk's and the triangular solve's, in which a product's operands come out of the one before it (see cr_step).  Decays
+// and strengths that are one number a token come out of 64 bits, and their products carry what rounding drops.  Against 64 bits the
+// outputs before the norm are 0.2 to 0.98 times as far off as those of the kernels that walk token by token, over the layers' sizes.
 //
-// Measured (B200, all launches, token by token -> here): HGRN2, one prompt of 2048 tokens and 16 heads of 128 x 128, 403 -> 148 us; the
-// delta rule 865 -> 209; fixed decays, four prompts of 1654 tokens in all, 341 -> 133.  (Operands in two TF32 parts and sums in the
-// accumulator alone took 127, 170 and 100 and were 1.2 to 6 times as far off.)
-// What bounds it: mma.sync issues one product every 8 cycles a scheduler on this GPU whatever its type, so the six products of 16
-// places are worth 1.3 times the ordinary 32-bit pipes, about 30 us of the states and outputs; the rest is the cutting of operands
-// (some five operations an element, half of them at half rate) and the phases of a CTA waiting for one another.
-#include "common.cuh"
-#include "warp_mma.cuh"
+// Measured (B200, all launches, token by token | every product by mma.sync | here): HGRN2, one prompt of 2048 tokens and 16 heads of
+// 128 x 128, 403 | 150 | 124 us; the delta rule 865 | 210 | 195; fixed decays, four prompts of 1654 tokens in all, 341 | 137 | 88.
+// What bounds the kernels here: mma.sync issues one product every 8 cycles a scheduler on this GPU whatever its type, so the six products
+// of 16 places are worth 1.3 times the ordinary 32-bit pipes; the walk is 32 links of two small products each.
+#include "chunk_recurrence.cuh"
 
 namespace lb {
-
-constexpr int CR_C = 64;                 // tokens a chunk
-constexpr int CR_PT = CR_C + 4;          // floats between rows of 64 places: 16-byte pieces of 8 rows lie in all banks
-constexpr int CR_VT = 64;                // value columns at a time
-constexpr int CR_PV = CR_VT + 8;         // and between their rows: 4 rows of 8 neighbours lie in all banks
-constexpr int CR_THREADS = 512;
-constexpr int CR_SCAN = 256, CR_WALK = 256;
-constexpr int CR_SEQS = 64;              // sequences a launch
-
-enum CrKind : int { CR_FIXED = 0, CR_SSM = 1, CR_DELTA = 2, CR_HGRN2 = 3, CR_CHANNELS = 4 };
-
-__host__ __device__ constexpr bool cr_delta(int kind) { return kind == CR_DELTA || kind == CR_CHANNELS; }
-__host__ __device__ constexpr bool cr_rows(int kind) { return kind == CR_HGRN2 || kind == CR_CHANNELS; }   // a decay for every row
-
-struct ChunkParams {
-  const float* q; const float* k; const float* v; const float* a; const float* b;    // hgrn2: k is the gate's input
-  long long q_ld, k_ld, v_ld, a_ld, b_ld;
-  const float* A_log; const float* dt_bias; const float* D; const float* bias; const float* lower; const float* decay;
-  float* state; float* out; long long out_ld;
-  const int* cu_tokens; const int* slots;
-  int heads, groups, dim, vdim, unit_norm, act;
-  float q_scale, unit_eps;
-  int vec, vecv, vec2;                   // rows of q, k, a and rows of v in whole aligned 16-byte pieces; rows of out in 8-byte ones
-  int slot0;                             // first chunk of this launch, counted over the sequences below
-  int num_seqs;
-  float* scratch;                        // per (chunk of this launch, head), the arrays at these offsets
-  long long per_head;
-  int off_w, off_k, off_u, off_g, v_ld_s;    // state (before the chunk; first K^T U) at 0: [KD][v_ld_s]; W [64][KD + 4]; K^T [KD][68]; U [64][v_ld_s]; c_63
-  int seq[CR_SEQS];                      // sequence of the step
-  int base[CR_SEQS + 1];                 // its first chunk
-};
-
-__device__ __forceinline__ float cr_silu(float x) { return x / (1.f + expf(-x)); }
-__device__ __forceinline__ float cr_silu_r(float x) { return x * __frcp_rn(1.f + expf(-x)); }       // a rounding more, a third of the instructions
-
-// 1 / sqrt(x) as r + rest: a token's factor errs for the whole row at once.
-__device__ __forceinline__ void cr_unit(float x, float scale, float& r, float& rest) {
-  r = 1.f / sqrtf(x);
-  const float p = r * r;
-  rest = 0.5f * r * fmaf(-x, fmaf(r, r, -p), fmaf(-x, p, 1.f));
-  rest = fmaf(scale, rest, fmaf(scale, r, -(scale * r)));
-  r *= scale;
-}
-template <typename F>
-__device__ __forceinline__ float4 cr_map(float4 x, F f) { return make_float4(f(x.x), f(x.y), f(x.z), f(x.w)); }
-__device__ __forceinline__ void cr_scale(float* x, float g) {
-  float4* y = reinterpret_cast<float4*>(x);
-  *y = make_float4(y->x * g, y->y * g, y->z * g, y->w * g);
-}
-
-// Two numbers (the places that share a register of an operand) as three bfloat16 each, x = h + m + l: rounded to 8 bits, the rest
-// rounded to 8, and what is left, which has no more than 8.
-struct Split { uint32_t h, m, l; };
-__device__ __forceinline__ Split cr_split(float x, float y) {
-  Split s;
-  s.h = pack_bf16(x, y);
-  x -= __uint_as_float(s.h << 16); y -= __uint_as_float(s.h & 0xffff0000u);
-  s.m = pack_bf16(x, y);
-  x -= __uint_as_float(s.m << 16); y -= __uint_as_float(s.m & 0xffff0000u);
-  s.l = pack_bf16(x, y);
-  return s;
-}
 
 __device__ __forceinline__ void cr_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -130,15 +66,6 @@ __device__ __forceinline__ void cr_left(uint32_t tile, int pitch, int lane, Left
     ldmatrix_x4(at + 32 * i, r[0], r[1], r[2], r[3]);
     cr_put(a, 2 * i, __uint_as_float(r[0]), __uint_as_float(r[2]));
     cr_put(a, 2 * i + 1, __uint_as_float(r[1]), __uint_as_float(r[3]));
-  }
-}
-// The same of a matrix that lies transposed: [16 places][16 rows], rows 8 or 24 floats apart modulo 32.
-__device__ __forceinline__ void cr_left_t(const float* tile, int pitch, int lane, Left& a) {
-  const float* x = tile + (lane & 3) * pitch + (lane >> 2);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    cr_put(a, 2 * i, x[8 * i * pitch], x[(8 * i + 4) * pitch]);
-    cr_put(a, 2 * i + 1, x[8 * i * pitch + 8], x[(8 * i + 4) * pitch + 8]);
   }
 }
 // A right operand of 8 columns: from [8 columns][16 places] (ldmatrix), from [16 places][8 columns] (plain loads).
@@ -178,9 +105,6 @@ __device__ __forceinline__ void cr_step(float (*acc)[4], const Left& a, const Ri
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[n][e] += hh[n][e] + t[n][e];
 }
-
-// Whether a value is finite and stays so when it is split.
-__device__ __forceinline__ bool cr_finite(float x) { return fabsf(x) <= 3.38e38f; }
 
 // 16 rows of `left` times NT n-tiles of `right` (both row-major along the KS * 16 places summed over); two chains of half the
 // length, whose roundings are fewer.
@@ -251,108 +175,29 @@ __device__ __forceinline__ void cr_fetch(float* dst, const float* src, long long
   }
 }
 
-struct ChunkPlace { int seq, first, m; };        // sequence, first token, tokens
-
-__device__ __forceinline__ ChunkPlace cr_place(const ChunkParams& p, int at) {
-  const int slot = p.slot0 + at;
-  int si = 0;
-  while (si + 1 < p.num_seqs && p.base[si + 1] <= slot) ++si;
-  ChunkPlace c;
-  c.seq = p.seq[si];
-  c.first = p.cu_tokens[c.seq] + (slot - p.base[si]) * CR_C;
-  c.m = min(CR_C, p.cu_tokens[c.seq + 1] - c.first);
-  return c;
-}
-
-// Decay and write strength of each token, one number a head (decay 1, strength 0 behind the last token).  In 64 bits: a handful of
-// values a token while its rows are on their way, and an error here stays in the state as long as the token does.
-template <int KIND>
-__device__ __forceinline__ void cr_numbers(const ChunkParams& p, const ChunkPlace& c, int h, float* gs, float* ws, int tid) {
-  if (tid >= CR_C) return;
-  float g = 1.f, w = 0.f;
-  if (tid < c.m) {
-    w = 1.f;
-    if (KIND == CR_FIXED) g = p.decay[h];
-    if (KIND == CR_SSM || KIND == CR_DELTA) {
-      const double x = (double)p.a[(size_t)(c.first + tid) * p.a_ld + h] + (double)p.dt_bias[h];
-      const double sp = x > 20.0 ? x : log1p(exp(x));
-      g = (float)exp(-exp((double)p.A_log[h]) * sp);
-      w = (float)sp;
-    }
-    if (cr_delta(KIND)) w = (float)(1.0 / (1.0 + exp(-(double)p.b[(size_t)(c.first + tid) * p.b_ld + h])));
-  }
-  gs[tid] = g;
-  ws[tid] = w;
-}
-
-// What the fetched rows become, in place: k (and q) through their activation or to unit length, hgrn2's gate input (without q) to
-// decay and 1 - decay; decays behind the last token and row: 1.
-template <int KIND, int KD, int PITCH, bool WITH_Q>
-__device__ __forceinline__ void cr_form(const ChunkParams& p, const ChunkPlace& c, int h, float* Qs, float* Ks, float* Gs, int tid) {
-  constexpr int STEP = CR_THREADS / (KD / 4);
-  const int lane = tid & 31, warp = tid >> 5, t0 = tid / (KD / 4), d = (tid % (KD / 4)) * 4;
-  if (KIND == CR_FIXED && p.act) {
-#pragma unroll 4
-    for (int i = 0; i < CR_C / STEP; ++i) {
-      const int at = (t0 + i * STEP) * PITCH + d;
-      float4* k = reinterpret_cast<float4*>(Ks + at);
-      *k = cr_map(*k, cr_silu_r);
-      if (WITH_Q) { float4* q = reinterpret_cast<float4*>(Qs + at); *q = cr_map(*q, cr_silu_r); }
-    }
-  }
-  if (KIND == CR_HGRN2 && WITH_Q) {                // the decays follow block by block
-#pragma unroll 4
-    for (int i = 0; i < CR_C / STEP; ++i) {
-      float4* q = reinterpret_cast<float4*>(Qs + (t0 + i * STEP) * PITCH + d);
-      *q = cr_map(*q, cr_silu);
-    }
-  }
-  if (KIND == CR_HGRN2 && !WITH_Q) {
-    float low[4], bi[4];
+// The fetched keys to unit length, in place.
+template <int KD, int PITCH>
+__device__ __forceinline__ void cr_form(const ChunkParams& p, float* Ks, int tid) {
+  const int lane = tid & 31, warp = tid >> 5;
+  if (!p.unit_norm) return;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      low[e] = d + e < p.dim ? p.lower[h * p.dim + d + e] : 1.f;          // rows beyond dim: decay 1
-      bi[e] = d + e < p.dim ? p.bias[h * p.dim + d + e] : 0.f;
+  for (int t = warp; t < CR_C; t += CR_THREADS / 32) {                    // rows behind the last token are zeros and stay so
+    float sk = 0.f, y[KD / 32];
+#pragma unroll
+    for (int u = 0; u < KD / 32; ++u) {
+      y[u] = Ks[t * PITCH + lane + 32 * u];
+      sk += y[u] * y[u];
     }
-#pragma unroll 2
-    for (int i = 0; i < CR_C / STEP; ++i) {
-      const int t = t0 + i * STEP, at = t * PITCH + d;
-      float4* k = reinterpret_cast<float4*>(Ks + at);
-      float g[4] = {k->x, k->y, k->z, k->w};
+    sk = warp_sum(sk);
+    float f, rest;
+    cr_unit(sk + p.unit_eps, 1.f, f, rest);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) g[e] = t < c.m ? low[e] + (1.f - low[e]) * __frcp_rn(1.f + expf(-(g[e] + bi[e]))) : 1.f;
-      *reinterpret_cast<float4*>(Gs + at) = make_float4(g[0], g[1], g[2], g[3]);
-      *k = make_float4(1.f - g[0], 1.f - g[1], 1.f - g[2], 1.f - g[3]);
-    }
-  }
-  if (cr_delta(KIND) && p.unit_norm) {
-#pragma unroll
-    for (int t = warp; t < CR_C; t += CR_THREADS / 32) {                  // rows behind the last token are zeros and stay so
-      float sq = 0.f, sk = 0.f, x[KD / 32], y[KD / 32];
-#pragma unroll
-      for (int u = 0; u < KD / 32; ++u) {
-        y[u] = Ks[t * PITCH + lane + 32 * u];
-        x[u] = WITH_Q ? Qs[t * PITCH + lane + 32 * u] : 0.f;
-        sq += x[u] * x[u]; sk += y[u] * y[u];
-      }
-      sk = warp_sum(sk);
-      float f, rest;
-      cr_unit(sk + p.unit_eps, 1.f, f, rest);
-#pragma unroll
-      for (int u = 0; u < KD / 32; ++u) Ks[t * PITCH + lane + 32 * u] = fmaf(y[u], f, y[u] * rest);
-      if (WITH_Q) {
-        sq = warp_sum(sq);
-        cr_unit(sq + p.unit_eps, p.q_scale, f, rest);
-#pragma unroll
-        for (int u = 0; u < KD / 32; ++u) Qs[t * PITCH + lane + 32 * u] = fmaf(x[u], f, x[u] * rest);
-      }
-    }
+    for (int u = 0; u < KD / 32; ++u) Ks[t * PITCH + lane + 32 * u] = fmaf(y[u], f, y[u] * rest);
   }
 }
 
-// The decays of 16 tokens from `b0` on, a warp a token and a lane KD / 32 neighbouring channels: requested (channels), or formed
-// from the gate's input in Ks, which becomes 1 - decay (hgrn2); then left in Gb [16][PITCH].
-template <int KIND, int KD>
+// The decays of 16 tokens from `b0` on, a warp a token and a lane KD / 32 neighbouring channels: requested, then left in Gb [16][PITCH].
+template <int KD>
 __device__ __forceinline__ void cr_request_decays(const ChunkParams& p, const ChunkPlace& c, int h, int b0, int tid, float* g) {
   const int t = b0 + tid / 32, d0 = (tid % 32) * (KD / 32);
   const float* src = p.a + (size_t)(c.first + t) * p.a_ld + (size_t)h * p.dim + d0;
@@ -368,73 +213,15 @@ __device__ __forceinline__ void cr_request_decays(const ChunkParams& p, const Ch
     for (int e = 0; e < KD / 32; ++e) if (d0 + e < p.dim) g[e] = src[e];
   }
 }
-template <int KIND, int KD, int PITCH>
-__device__ __forceinline__ void cr_put_decays(const ChunkPlace& c, int b0, int tid, const float* g, const float* low, const float* bi, float* Ks, float* Gb) {
-  const int r = tid / 32, d0 = (tid % 32) * (KD / 32);
-  float x[KD / 32];
-  if (KIND == CR_HGRN2) {
-    float* k = Ks + (b0 + r) * PITCH + d0;
+template <int KD, int PITCH>
+__device__ __forceinline__ void cr_put_decays(int tid, const float* g, float* Gb) {
 #pragma unroll
-    for (int e = 0; e < KD / 32; ++e) x[e] = b0 + r < c.m ? low[e] + (1.f - low[e]) * __frcp_rn(1.f + expf(-(k[e] + bi[e]))) : 1.f;
-#pragma unroll
-    for (int e = 0; e < KD / 32; ++e) k[e] = 1.f - x[e];
-  } else {
-#pragma unroll
-    for (int e = 0; e < KD / 32; ++e) x[e] = g[e];
-  }
-#pragma unroll
-  for (int e = 0; e < KD / 32; ++e) Gb[r * PITCH + d0 + e] = x[e];
+  for (int e = 0; e < KD / 32; ++e) Gb[tid / 32 * PITCH + tid % 32 * (KD / 32) + e] = g[e];
 }
 
-// The value rows of the lightning form pass silu as well.
-__device__ __forceinline__ void cr_form_values(float* Us, int tid) {
-  constexpr int STEP = CR_THREADS / (CR_VT / 4);
-#pragma unroll
-  for (int i = 0; i < CR_C / STEP; ++i) {
-    float4* x = reinterpret_cast<float4*>(Us + (tid / (CR_VT / 4) + i * STEP) * CR_PV + (tid % (CR_VT / 4)) * 4);
-    *x = cr_map(*x, cr_silu_r);
-  }
-}
-
-// A product of decays with what its roundings drop: the error of 63 roundings is the same in every chunk of a head whose decay
-// does not change, and adds up over a state that lives for thousands of tokens.
-struct Product {
-  float h = 1.f, l = 0.f;
-  __device__ __forceinline__ void times(float g) {
-    const float p = h * g;
-    l = fmaf(l, g, fmaf(h, g, -p));
-    h = p;
-  }
-  __device__ __forceinline__ float value() const { return h + l; }
-};
-
-// G(j, i) at [i][j] for one decay a token (zeros above the diagonal), and c_i: a thread eight rows of a column, from the product
-// of the decays between.
-__device__ __forceinline__ void cr_products(const float* gs, float* Ds, float* cs, int tid) {
-  static_assert(CR_THREADS == 8 * CR_C, "a thread eight rows of a column");
-  const int j = tid % CR_C, i0 = tid / CR_C * 8;
-  float g[8];
-  Product d, c;
-#pragma unroll 8
-  for (int i = 0; i < i0; ++i) { const float x = gs[i]; if (i > j) d.times(x); }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) g[i] = gs[i0 + i];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (i0 + i > j) d.times(g[i]);
-    Ds[(i0 + i) * CR_PT + j] = i0 + i >= j ? d.value() : 0.f;
-  }
-  if (j == 0) {                                    // one thread a block of eight: c_i
-#pragma unroll 8
-    for (int i = 0; i < i0; ++i) c.times(gs[i]);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { c.times(g[i]); cs[i0 + i] = c.value(); }
-  }
-}
-
-// sum_d x_id k_jd G(j, i)_d for one column j and the rows i of its block of 16 from j (SELF) or j + 1 on, a warp: a lane takes KD / 32
+// sum_d x_id k_jd G(j, i)_d for one column j and the rows i of its block of 16 from j + 1 on, a warp: a lane takes KD / 32
 // neighbouring channels and carries k_j G(j, i); four rows are added up together, in six shuffles.  store(i, sum).
-template <int KD, int PITCH, bool SELF, typename F>
+template <int KD, int PITCH, typename F>
 __device__ __forceinline__ void cr_pairs(const float* Xs, const float* Ks, const float* Gb, int b0, int j, int lane, F store) {
   const int end = b0 + 16;
   constexpr int N = KD / 32;
@@ -444,7 +231,7 @@ __device__ __forceinline__ void cr_pairs(const float* Xs, const float* Ks, const
     else *reinterpret_cast<float2*>(to) = *reinterpret_cast<const float2*>(x + 2 * lane);
   };
   load(Ks + j * PITCH, kk);
-  for (int i0 = SELF ? j : j + 1; i0 < end; i0 += 4) {
+  for (int i0 = j + 1; i0 < end; i0 += 4) {
     float s[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -453,13 +240,9 @@ __device__ __forceinline__ void cr_pairs(const float* Xs, const float* Ks, const
       if (i < end) {
         float x[N], g[N];
         load(Xs + i * PITCH, x);
-        if (i > j) {
-          load(Gb + (i - b0) * PITCH, g);
+        load(Gb + (i - b0) * PITCH, g);
 #pragma unroll
-          for (int e = 0; e < N; ++e) kk[e] *= g[e];
-        }
-#pragma unroll
-        for (int e = 0; e < N; ++e) s[u] = fmaf(x[e], kk[e], s[u]);
+        for (int e = 0; e < N; ++e) { kk[e] *= g[e]; s[u] = fmaf(x[e], kk[e], s[u]); }
       }
     }
     const bool high = lane & 16, upper = lane & 8;
@@ -471,107 +254,6 @@ __device__ __forceinline__ void cr_pairs(const float* Xs, const float* Ks, const
     x += __shfl_xor_sync(0xffffffffu, x, 1);
     const int i = i0 + (high ? 2 : 0) + (upper ? 1 : 0);
     if ((lane & 7) == 0 && i < end) store(i, x);
-  }
-}
-
-// ---- every chunk by itself: K^T U of the kinds without the delta rule --------------------------------------------------------
-// Reads k and v (64 KB a chunk and head of 128 x 128), writes 64 KB.
-__host__ __device__ constexpr int cr_states_floats(int kind, int kd) {
-  return CR_C * (kd + 8) * (cr_rows(kind) ? 2 : 1) + CR_C * CR_PV + 3 * CR_C + 4;
-}
-
-template <int KIND, int KD>
-__global__ void __launch_bounds__(CR_THREADS, 2) chunk_states_kernel(const __grid_constant__ ChunkParams p) {
-  constexpr int PD = KD + 8;
-  constexpr bool ROWS = cr_rows(KIND);
-  extern __shared__ __align__(16) float cr_smem[];
-  float* Ks = cr_smem;                             // [64][PD]
-  float* Us = Ks + CR_C * PD;                      // [64][PV]
-  float* gs = Us + CR_C * CR_PV;
-  float* ws = gs + CR_C;
-  float* ts = ws + CR_C;                           // w_j G(j, 63)
-  float* cs = ts + CR_C;                           // c_63
-  float* Gs = cs + 4;                              // [64][PD]
-  pdl_trigger();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int h = blockIdx.y, grp = h / (p.heads / p.groups);
-  pdl_wait();
-  const ChunkPlace c = cr_place(p, blockIdx.x);
-  float* mine = p.scratch + ((size_t)blockIdx.x * p.heads + h) * p.per_head;
-  const float* vsrc = p.v + (size_t)c.first * p.v_ld + (size_t)h * p.vdim;
-  cr_fetch<KD, PD>(Ks, p.k + (size_t)c.first * p.k_ld + (size_t)grp * p.dim, p.k_ld, c.m, p.dim, p.vec, tid);
-  cr_fetch<CR_VT, CR_PV>(Us, vsrc, p.v_ld, c.m, min(CR_VT, p.vdim), p.vecv, tid);
-  cp_async_commit();
-  cr_numbers<KIND>(p, c, h, gs, ws, tid);
-  cp_async_wait<0>();
-  __syncthreads();
-  if (!ROWS && tid < CR_C) {
-    Product d;
-#pragma unroll 16
-    for (int i = 1; i < CR_C; ++i) { const float x = gs[i]; if (i > tid) d.times(x); }
-    ts[tid] = d.value() * ws[tid];
-    if (tid == 0) { d.times(gs[0]); cs[0] = d.value(); }
-  }
-  cr_form<KIND, KD, PD, false>(p, c, h, nullptr, Ks, Gs, tid);
-  __syncthreads();
-  if (!ROWS) {
-    if (tid < KD) mine[p.off_g + tid] = cs[0];
-    constexpr int STEP = CR_THREADS / (KD / 4);
-#pragma unroll
-    for (int i = 0; i < CR_C / STEP; ++i) {
-      const int t = tid / (KD / 4) + i * STEP;
-      cr_scale(Ks + t * PD + (tid % (KD / 4)) * 4, ts[t]);
-    }
-  } else {
-    // a thread a channel and a quarter of the chunk: k_j G(j, 63) from the last token back
-    const int d = tid % KD, part = tid / KD;
-    if (part < 4) {
-      float g = 1.f;
-#pragma unroll 8
-      for (int t = CR_C - 1; t >= 16 * part + 16; --t) g *= Gs[t * PD + d];
-      float x[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) x[i] = Gs[(16 * part + i) * PD + d];
-#pragma unroll
-      for (int i = 15; i >= 0; --i) { Ks[(16 * part + i) * PD + d] *= g; g *= x[i]; }
-      if (part == 0) mine[p.off_g + d] = g;
-    }
-  }
-  constexpr int MT = KD / 64;
-  const int mt0 = (warp >> 2) * MT, n0 = (warp & 3) * 2;         // a warp: KD / 4 rows, 16 columns
-  for (int v0 = 0; v0 < p.vdim; v0 += CR_VT) {
-    if (v0 > 0) {
-      __syncthreads();
-      cr_fetch<CR_VT, CR_PV>(Us, vsrc + v0, p.v_ld, c.m, min(CR_VT, p.vdim - v0), p.vecv, tid);
-      cp_async_commit();
-      cp_async_wait<0>();
-      __syncthreads();
-    }
-    if (KIND == CR_FIXED && p.act) cr_form_values(Us, tid);
-    __syncthreads();
-    float acc[MT][2][4] = {};
-#pragma unroll 1
-    for (int ks = 0; ks < CR_C / 16; ++ks) {
-      Right b[2];
-#pragma unroll
-      for (int t = 0; t < 2; ++t) cr_right_t(Us + 16 * ks * CR_PV + 8 * (n0 + t), CR_PV, lane, b[t]);
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        Left a;
-        cr_left_t(Ks + 16 * ks * PD + 16 * (mt0 + mt), PD, lane, a);
-        cr_step<2>(acc[mt], a, b);
-      }
-    }
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int col = v0 + 8 * (n0 + t) + 2 * (lane & 3);
-        if (col >= p.v_ld_s) continue;
-        float* dst = mine + (16 * (mt0 + mt) + (lane >> 2)) * p.v_ld_s + col;
-        *reinterpret_cast<float2*>(dst) = make_float2(acc[mt][t][0], acc[mt][t][1]);
-        *reinterpret_cast<float2*>(dst + 8 * p.v_ld_s) = make_float2(acc[mt][t][2], acc[mt][t][3]);
-      }
   }
 }
 
@@ -592,6 +274,8 @@ __global__ void __launch_bounds__(CR_SCAN) chunk_scan_kernel(const __grid_consta
   for (int i = 0; i < 4; ++i) s[i] = i < have ? S[i] : 0.f;
   const size_t stride = (size_t)p.heads * p.per_head;
   float* x = p.scratch + ((size_t)(base + c_lo - p.slot0) * p.heads + h) * p.per_head;
+  uint8_t* keep = cr_state_at(p, x, kd, d, e);
+  const int part = 128 * cr_tile(p.vdim);
   for (int c = c_lo; c < c_hi; c += 8) {
     float4 ds[8];
     float g[8];
@@ -604,11 +288,16 @@ __global__ void __launch_bounds__(CR_SCAN) chunk_scan_kernel(const __grid_consta
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       if (c + i < c_hi) {
-        *reinterpret_cast<float4*>(x + i * stride + (size_t)d * p.v_ld_s + e) = make_float4(s[0], s[1], s[2], s[3]);
+        const Split lo = cr_split(s[0], s[1]), hi = cr_split(s[2], s[3]);
+        uint8_t* to = keep + i * stride * sizeof(float);
+        *reinterpret_cast<uint2*>(to) = make_uint2(lo.h, hi.h);
+        *reinterpret_cast<uint2*>(to + part) = make_uint2(lo.m, hi.m);
+        *reinterpret_cast<uint2*>(to + 2 * part) = make_uint2(lo.l, hi.l);
         s[0] = fmaf(g[i], s[0], ds[i].x); s[1] = fmaf(g[i], s[1], ds[i].y);
         s[2] = fmaf(g[i], s[2], ds[i].z); s[3] = fmaf(g[i], s[3], ds[i].w);
       }
     x += 8 * stride;
+    keep += 8 * stride * sizeof(float);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) if (i < have) S[i] = s[i];
@@ -654,17 +343,18 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
   float* oK = mine + p.off_k;
   float* oU = mine + p.off_u;
   float* oG = mine + p.off_g;
+  for (int i = tid; i < p.v_ld_s; i += CR_THREADS) reinterpret_cast<int*>(mine)[p.off_f + i] = CR_C;
   cr_fetch<KD, PK>(Ks, p.k + (size_t)c.first * p.k_ld + (size_t)grp * p.dim, p.k_ld, c.m, p.dim, p.vec, tid);
   const float* vsrc = p.v + (size_t)c.first * p.v_ld + (size_t)h * p.vdim;
   if (!ROWS) cr_fetch<CR_XV, PX>(Xv, vsrc, p.v_ld, c.m, min(CR_XV, p.vdim), p.vecv, tid);
   cp_async_commit();
   float gn[KD / 32];
-  if (ROWS) cr_request_decays<KIND, KD>(p, c, h, 0, tid, gn);
+  if (ROWS) cr_request_decays<KD>(p, c, h, 0, tid, gn);
   cr_numbers<KIND>(p, c, h, gs, ws, tid);
   cp_async_wait<0>();
   __syncthreads();
-  cr_form<KIND, KD, PK, false>(p, c, h, nullptr, Ks, nullptr, tid);
-  if (ROWS) cr_put_decays<KIND, KD, PK>(c, 0, tid, gn, nullptr, nullptr, Ks, Gb);
+  cr_form<KD, PK>(p, Ks, tid);
+  if (ROWS) cr_put_decays<KD, PK>(tid, gn, Gb);
   if (!ROWS) cr_products(gs, Ds, cs, tid);
   __syncthreads();
   const uint32_t Ka = (uint32_t)__cvta_generic_to_shared(Ks);
@@ -693,9 +383,9 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
     for (int I = 0; I < 4; ++I) {
       const int b0 = 16 * I;
       float* Gi = Gb + (I & 1) * 16 * PK;
-      if (I < 3) cr_request_decays<KIND, KD>(p, c, h, b0 + 16, tid, gn);
+      if (I < 3) cr_request_decays<KD>(p, c, h, b0 + 16, tid, gn);
       const int jj = b0 + warp;                    // pairs inside the block: a warp a column
-      cr_pairs<KD, PK, false>(Ks, Ks, Gi, b0, jj, lane, [&](int i, float x) { Ls[i * CR_PT + jj] = x * ws[i]; });
+      cr_pairs<KD, PK>(Ks, Ks, Gi, b0, jj, lane, [&](int i, float x) { Ls[i * CR_PT + jj] = x * ws[i]; });
       if (lane < 16 && b0 + lane <= jj) Ls[(b0 + lane) * CR_PT + jj] = 0.f;
       __syncthreads();                             // the block's rows as they came are read (and the keys before it moved on)
       if (tid < KD) {                              // times c_i from the block's start, in place; times G(i, block's end)
@@ -713,7 +403,7 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
         for (int i = 15; i >= 0; --i) { Kr[(b0 + i) * PK + ch] = kb[i] * g; g *= gb[i]; }
       }
       __syncthreads();
-      if (I < 3) cr_put_decays<KIND, KD, PK>(c, b0 + 16, tid, gn, nullptr, nullptr, Ks, Gb + (~I & 1) * 16 * PK);
+      if (I < 3) cr_put_decays<KD, PK>(tid, gn, Gb + (~I & 1) * 16 * PK);
       if (I > 0) {                                 // the block's rows against all tokens before it
         for (int n = warp; n < 2 * I; n += CR_THREADS / 32) {
           float acc[1][4] = {};
@@ -905,9 +595,18 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
 
   float s[NT][4];                                  // warps 0 .. MW - 1: the state at (16 warp + row + 8 (e / 2), 8 nt + cc + e % 2)
   // rows (places) r and r + 8 of the columns 8 nt + cc, + 1 of x, split: place q of eight lies at 2 q, place q + 4 behind it
+  const int part = 128 * cr_tile(p.vdim);
+  int s_off[NT], u_off[NT];                        // bytes from the chunk's scratch to this thread's places of the state and of U
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    s_off[nt] = (int)(cr_state_at(p, mine, KD, warp * 16 + row, col0 + nt * 8 + cc) - reinterpret_cast<uint8_t*>(mine));
+    u_off[nt] = (int)(cr_u_at(p, mine, r0, col0 + nt * 8 + cc) - reinterpret_cast<uint8_t*>(mine));
+  }
+  Split lo, hi;
   auto put_split = [&](bf16* dst, int pitch, int plane, int r, int nt, const float* x) {
     const int at = (nt * 8 + cc) * pitch + (r & ~7) + 2 * (r & 3) + ((r >> 2) & 1);
-    const Split lo = cr_split(x[0], x[1]), hi = cr_split(x[2], x[3]);
+    lo = cr_split(x[0], x[1]);
+    hi = cr_split(x[2], x[3]);
     auto put = [&](bf16* d, uint32_t a, uint32_t b) {
       uint16_t* y = reinterpret_cast<uint16_t*>(d) + at;
       y[0] = (uint16_t)a; y[pitch] = (uint16_t)(a >> 16);
@@ -915,15 +614,15 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
     };
     put(dst, lo.h, hi.h); put(dst + plane, lo.m, hi.m); put(dst + 2 * plane, lo.l, hi.l);
   };
-  auto put_state = [&](float* keep) {              // split, for the next product; whole, for the outputs of the chunk it stands before
+  auto put_state = [&](float* keep) {              // for the next product, and for the outputs of the chunk it stands before
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       put_split(Ss, PS, NV * PS, warp * 16 + row, nt, s[nt]);
       const int cl = col0 + nt * 8 + cc;
       if (cl < p.v_ld_s) {
-#pragma unroll
-        for (int e2 = 0; e2 < 2; ++e2)
-          *reinterpret_cast<float2*>(keep + (warp * 16 + row + e2 * 8) * p.v_ld_s + cl) = make_float2(s[nt][2 * e2], s[nt][2 * e2 + 1]);
+        uint8_t* to = reinterpret_cast<uint8_t*>(keep) + s_off[nt];
+        cr_put(to, part, lo);
+        cr_put(to + 8 * 128, part, hi);
       }
     }
   };
@@ -1000,9 +699,19 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
         }
         put_split(Us, PU, NV * PU, r0, nt, u[nt]);
         if (cl < p.v_ld_s) {
+          if (!(cr_finite(u[nt][0]) && cr_finite(u[nt][1]) && cr_finite(u[nt][2]) && cr_finite(u[nt][3]))) {
+            float x[4];                            // rare: the outputs' product meets it with the zeros of earlier tokens
 #pragma unroll
-          for (int e2 = 0; e2 < 2; ++e2)
-            *reinterpret_cast<float2*>(mine + p.off_u + (r0 + e2 * 8) * p.v_ld_s + cl) = make_float2(u[nt][2 * e2], u[nt][2 * e2 + 1]);
+            for (int e = 0; e < 4; ++e) {
+              x[e] = cr_finite(u[nt][e]) ? u[nt][e] : 0.f;
+              if (!cr_finite(u[nt][e])) atomicMin(reinterpret_cast<int*>(mine) + p.off_f + cl + (e & 1), r0 + 8 * (e >> 1));
+            }
+            lo = cr_split(x[0], x[1]);
+            hi = cr_split(x[2], x[3]);
+          }
+          uint8_t* to = reinterpret_cast<uint8_t*>(mine) + u_off[nt];
+          cr_put(to, part, lo);
+          cr_put(to + 8 * 128, part, hi);
         }
       }
     }
@@ -1029,236 +738,6 @@ __global__ void __launch_bounds__(CR_WALK) chunk_walk_kernel(const __grid_consta
   }
 }
 
-// ---- every chunk by itself: the outputs ---------------------------------------------------------------------------------------
-// Two CTAs an SM: the state takes the place of k once the scores are formed, U that of the decays (two blocks' worth at a time).
-__host__ __device__ constexpr int cr_out_floats(int kind, int kd) {
-  const int mat = CR_C * (kd + 4), k = mat > kd * CR_PV ? mat : kd * CR_PV;
-  return mat + k + CR_C * CR_PV + CR_C * CR_PT + 3 * CR_C + (cr_rows(kind) ? 5 * kd : 0);
-}
-
-template <int KIND, int KD>
-__global__ void __launch_bounds__(CR_THREADS, 2) chunk_outputs_kernel(const __grid_constant__ ChunkParams p) {
-  constexpr int PK = KD + 4, MAT = CR_C * PK, KS = KD / 16, KBUF = MAT > KD * CR_PV ? MAT : KD * CR_PV;
-  constexpr bool ROWS = cr_rows(KIND), DELTA = cr_delta(KIND);
-  static_assert(32 * PK <= CR_C * CR_PV, "two blocks' decays lie where U does");
-  constexpr int STEP = CR_THREADS / (KD / 4);
-  extern __shared__ __align__(16) float cr_smem[];
-  float* Qs = cr_smem;                             // [64][PK]
-  float* Ks = Qs + MAT;                            // [64][PK]; then the state's columns at work [KD][PV]
-  float* Gb = Ks + KBUF;                           // a decay for every row: of two blocks [2][16][PK]; then (else from the start) U [64][PV]
-  float* As = Gb + CR_C * CR_PV;                         // [64][PT]: first G(j, i) of one decay a token
-  float* gs = As + CR_C * CR_PT;
-  float* ws = gs + CR_C;
-  float* cs = ws + CR_C;
-  float* starts = cs + CR_C;                       // [5][KD]: product of the decays before block I; [4]: over the block at work
-  float* Ss = Ks;
-  float* Us = Gb;
-  pdl_trigger();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int h = blockIdx.y, grp = h / (p.heads / p.groups);
-  pdl_wait();
-  const ChunkPlace c = cr_place(p, blockIdx.x);
-  const float* mine = p.scratch + ((size_t)blockIdx.x * p.heads + h) * p.per_head;
-  const float* vsrc = p.v + (size_t)c.first * p.v_ld + (size_t)h * p.vdim;
-  cr_fetch<KD, PK>(Qs, p.q + (size_t)c.first * p.q_ld + (size_t)grp * p.dim, p.q_ld, c.m, p.dim, p.vec, tid);
-  cr_fetch<KD, PK>(Ks, p.k + (size_t)c.first * p.k_ld + (size_t)grp * p.dim, p.k_ld, c.m, p.dim, p.vec, tid);
-  cp_async_commit();
-  float gn[KD / 32], low[KD / 32], bi[KD / 32];
-  if (KIND == CR_CHANNELS) cr_request_decays<KIND, KD>(p, c, h, 0, tid, gn);
-  if (KIND == CR_HGRN2) {
-#pragma unroll
-    for (int e = 0; e < KD / 32; ++e) {
-      const int d = (tid % 32) * (KD / 32) + e;
-      low[e] = d < p.dim ? p.lower[h * p.dim + d] : 1.f;         // rows beyond dim: decay 1
-      bi[e] = d < p.dim ? p.bias[h * p.dim + d] : 0.f;
-    }
-  }
-  auto fetch_u = [&](int v0) {
-    if (DELTA) cr_fetch<CR_VT, CR_PV>(Us, mine + p.off_u + v0, p.v_ld_s, CR_C, min(CR_VT, p.v_ld_s - v0), true, tid);
-    else cr_fetch<CR_VT, CR_PV>(Us, vsrc + v0, p.v_ld, c.m, min(CR_VT, p.vdim - v0), p.vecv, tid);
-  };
-  auto fetch_s = [&](int v0) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(Ss);
-    const int r0 = tid / (CR_VT / 4), e = (tid % (CR_VT / 4)) * 4;
-    const bool real = v0 + e < p.v_ld_s;
-    const float* x = real ? mine + r0 * p.v_ld_s + v0 + e : mine;
-#pragma unroll
-    for (int i = 0; i < KD / 32; ++i) cp_async16(d + 4 * ((r0 + 32 * i) * CR_PV + e), x + (real ? 32 * i * p.v_ld_s : 0), real);
-  };
-  cr_numbers<KIND>(p, c, h, gs, ws, tid);
-  cp_async_wait<0>();
-  __syncthreads();
-  cr_form<KIND, KD, PK, true>(p, c, h, Qs, Ks, nullptr, tid);
-  if (ROWS) cr_put_decays<KIND, KD, PK>(c, 0, tid, gn, low, bi, Ks, Gb);
-  if (!ROWS) cr_products(gs, As, cs, tid);
-  else for (int i = tid; i < CR_C * CR_PT; i += CR_THREADS) As[i] = 0.f;
-  __syncthreads();
-  if (!ROWS) {
-    fetch_u(0);
-    cp_async_commit();
-  }
-  const uint32_t Qa = (uint32_t)__cvta_generic_to_shared(Qs), Ka = (uint32_t)__cvta_generic_to_shared(Ks), Aa = (uint32_t)__cvta_generic_to_shared(As);
-  if (!ROWS) {
-    cr_triangle<KS>(Qa, Ka, PK, warp, lane, [&](int r, int n, const float* s) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = 16 * r + (lane >> 2) + (e >> 1) * 8, j = 8 * n + 2 * (lane & 3) + (e & 1);
-        float* x = As + i * CR_PT + j;
-        *x = j <= i ? *x * s[e] * (KIND == CR_SSM ? ws[j] : 1.f) : 0.f;
-      }
-    });
-    __syncthreads();                               // q and k are read
-    fetch_s(0);
-    cp_async_commit();
-#pragma unroll
-    for (int i = 0; i < CR_C / STEP; ++i) {
-      const int t = tid / (KD / 4) + i * STEP;
-      cr_scale(Qs + t * PK + (tid % (KD / 4)) * 4, cs[t]);
-    }
-  } else {
-    float c_start = 1.f;                           // of this thread's channel: product of the decays before the block
-    const int ch = tid % KD;
-    for (int I = 0; I < 4; ++I) {
-      const int b0 = 16 * I;
-      const float* Gi = Gb + (I & 1) * 16 * PK;
-      if (KIND == CR_CHANNELS && I < 3) cr_request_decays<KIND, KD>(p, c, h, b0 + 16, tid, gn);
-      const int jj = b0 + warp;                    // pairs inside the block: a warp a column
-      cr_pairs<KD, PK, true>(Qs, Ks, Gi, b0, jj, lane, [&](int i, float x) { As[i * CR_PT + jj] = x; });
-      __syncthreads();                             // the block's rows as they came are read (and the keys before it moved on)
-      if (tid < KD) {
-        float g = 1.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { g *= Gi[i * PK + ch]; Qs[(b0 + i) * PK + ch] *= g; }
-        starts[I * KD + ch] = c_start;
-        starts[4 * KD + ch] = g;
-        c_start *= g;
-      }
-      if (tid >= CR_THREADS - KD) {
-        float g = 1.f;
-#pragma unroll
-        for (int i = 15; i >= 0; --i) { Ks[(b0 + i) * PK + ch] *= g; g *= Gi[i * PK + ch]; }
-      }
-      __syncthreads();
-      if (I < 3) cr_put_decays<KIND, KD, PK>(c, b0 + 16, tid, gn, low, bi, Ks, Gb + (~I & 1) * 16 * PK);
-      if (I > 0) {                                 // the block's rows against all tokens before it
-        for (int n = warp; n < 2 * I; n += CR_THREADS / 32) {
-          float acc[1][4] = {};
-          cr_scores<KS, 1>(Qa + 4 * b0 * PK, Ka + 4 * 8 * n * PK, PK, lane, acc);
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            As[(b0 + (lane >> 2) + (e >> 1) * 8) * CR_PT + 8 * n + 2 * (lane & 3) + (e & 1)] = acc[0][e];
-        }
-      }
-      __syncthreads();
-      if (I > 0 && I < 3) {
-        const float g = starts[4 * KD + ch];
-        for (int j = tid / KD; j < b0; j += CR_THREADS / KD) Ks[j * PK + ch] *= g;     // the keys move on to the block's end
-      }
-    }
-    __syncthreads();                               // k and the decays are read
-    fetch_u(0);
-    fetch_s(0);
-    cp_async_commit();
-#pragma unroll
-    for (int i = 0; i < CR_C / STEP; ++i) {
-      const int t = tid / (KD / 4) + i * STEP, d = (tid % (KD / 4)) * 4;
-      float4* x = reinterpret_cast<float4*>(Qs + t * PK + d);
-      const float4 g = *reinterpret_cast<const float4*>(starts + (t / 16) * KD + d);
-      *x = make_float4(x->x * g.x, x->y * g.y, x->z * g.z, x->w * g.w);
-    }
-  }
-  const int m = warp >> 2, n0 = (warp & 3) * 2;    // a warp: 16 rows, 16 columns
-  for (int v0 = 0; v0 < p.vdim; v0 += CR_VT) {
-    if (v0 > 0) {
-      __syncthreads();
-      fetch_u(v0);
-      fetch_s(v0);
-      cp_async_commit();
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-    if (KIND == CR_FIXED && p.act) {
-      cr_form_values(Us, tid);
-      __syncthreads();
-    }
-    float acc[2][4] = {};                          // three sums apart: short chains, fewer roundings
-    auto add = [&](uint32_t left, int pitch, const float* right, int from, int to) {
-      float sum[2][4] = {};
-#pragma unroll 1
-      for (int ks = from; ks < to; ++ks) {
-        Left a;
-        Right b[2];
-#pragma unroll
-        for (int t = 0; t < 2; ++t) cr_right_t(right + 16 * ks * CR_PV + 8 * (n0 + t), CR_PV, lane, b[t]);
-        cr_left(left + 64 * ks, pitch, lane, a);
-        cr_step<2>(sum, a, b);
-      }
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[t][e] += sum[t][e];
-    };
-    add(Qa + 4 * 16 * m * PK, PK, Ss, 0, KS / 2);
-    add(Qa + 4 * 16 * m * PK, PK, Ss, KS / 2, KS);
-    add(Aa + 4 * 16 * m * CR_PT, CR_PT, Us, 0, m);
-    {                                              // the diagonal tile, whose rows have tokens behind them on the right
-      float sum[2][4] = {}, x[2][4];
-      bool finite = true;
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          x[t][i] = Us[(16 * m + (lane & 3) + 4 * i) * CR_PV + 8 * (n0 + t) + (lane >> 2)];
-          finite &= cr_finite(x[t][i]);
-        }
-      if (!__all_sync(0xffffffffu, finite)) {      // rare: a column is bad from its first such token on, and no earlier
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          int from = 16;
-#pragma unroll
-          for (int i = 3; i >= 0; --i)
-            if (!cr_finite(x[t][i])) { from = (lane & 3) + 4 * i; x[t][i] = 0.f; }
-          from = min(from, __shfl_xor_sync(0xffffffffu, from, 1));
-          from = min(from, __shfl_xor_sync(0xffffffffu, from, 2));
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int f = __shfl_sync(0xffffffffu, from, 4 * (2 * (lane & 3) + (e & 1)));
-            if ((lane >> 2) + 8 * (e >> 1) >= f) sum[t][e] = __int_as_float(0x7fffffff);
-          }
-        }
-      }
-      Left a;
-      Right b[2];
-#pragma unroll
-      for (int t = 0; t < 2; ++t) { cr_put(b[t], 0, x[t][0], x[t][1]); cr_put(b[t], 1, x[t][2], x[t][3]); }
-      cr_left(Aa + 4 * (16 * m * CR_PT + 16 * m), CR_PT, lane, a);
-      cr_step<2>(sum, a, b);
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[t][e] += sum[t][e];
-    }
-#pragma unroll
-    for (int e2 = 0; e2 < 2; ++e2) {
-      const int t = 16 * m + (lane >> 2) + 8 * e2;
-      if (t >= c.m) continue;
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        const int col = v0 + 8 * (n0 + nt) + 2 * (lane & 3);
-        if (col >= p.vdim) continue;
-        float x = acc[nt][2 * e2], y = acc[nt][2 * e2 + 1];
-        if (p.D) {
-          x += p.D[h] * vsrc[(size_t)t * p.v_ld + col];
-          if (col + 1 < p.vdim) y += p.D[h] * vsrc[(size_t)t * p.v_ld + col + 1];
-        }
-        float* dst = p.out + (size_t)(c.first + t) * p.out_ld + (size_t)h * p.vdim + col;
-        if (p.vec2) *reinterpret_cast<float2*>(dst) = make_float2(x, y);
-        else { dst[0] = x; if (col + 1 < p.vdim) dst[1] = y; }
-      }
-    }
-  }
-}
-
 template <typename K>
 static cudaError_t cr_allow(K kernel, int floats) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, floats * (int)sizeof(float));
@@ -1273,14 +752,18 @@ static cudaError_t launch_chunk_walk(const ChunkParams& p, int nslots, cudaStrea
 }
 
 template <int KIND, int KD>
-static cudaError_t launch_chunks(const ChunkParams& p, int nslots, cudaStream_t stream) {
-  const dim3 grid(nslots, p.heads), block(CR_THREADS);
+static cudaError_t launch_solve(const ChunkParams& p, int nslots, cudaStream_t stream) {
+  constexpr int floats = cr_solve_floats(KIND, KD);
+  static const cudaError_t cfg = cr_allow(chunk_solve_kernel<KIND, KD>, floats);
+  if (cfg != cudaSuccess) return cfg;
+  return launch(chunk_solve_kernel<KIND, KD>, dim3(nslots, p.heads), dim3(CR_THREADS), floats * sizeof(float), stream, p);
+}
+
+template <int KD>
+static cudaError_t launch_chunks(int kind, const ChunkParams& p, int nslots, cudaStream_t stream) {
   cudaError_t e;
-  if constexpr (cr_delta(KIND)) {
-    constexpr int floats = cr_solve_floats(KIND, KD);
-    static const cudaError_t cfg = cr_allow(chunk_solve_kernel<KIND, KD>, floats);
-    if (cfg != cudaSuccess) return cfg;
-    e = launch(chunk_solve_kernel<KIND, KD>, grid, block, floats * sizeof(float), stream, p);
+  if (cr_delta(kind)) {
+    e = kind == CR_DELTA ? launch_solve<CR_DELTA, KD>(p, nslots, stream) : launch_solve<CR_CHANNELS, KD>(p, nslots, stream);
     if (e != cudaSuccess) return e;
     count_launch();
     int nv = 32;
@@ -1288,44 +771,33 @@ static cudaError_t launch_chunks(const ChunkParams& p, int nslots, cudaStream_t 
     e = nv == 32 ? launch_chunk_walk<KD, 32>(p, nslots, stream) : nv == 16 ? launch_chunk_walk<KD, 16>(p, nslots, stream)
                                                                            : launch_chunk_walk<KD, 8>(p, nslots, stream);
   } else {
-    constexpr int floats = cr_states_floats(KIND, KD);
-    static const cudaError_t cfg = cr_allow(chunk_states_kernel<KIND, KD>, floats);
-    if (cfg != cudaSuccess) return cfg;
-    e = launch(chunk_states_kernel<KIND, KD>, grid, block, floats * sizeof(float), stream, p);
+    e = cr_launch_states(kind, p, nslots, stream);
     if (e != cudaSuccess) return e;
     count_launch();
     e = launch(chunk_scan_kernel, dim3((KD * (p.v_ld_s / 4) + CR_SCAN - 1) / CR_SCAN, p.heads, p.num_seqs), dim3(CR_SCAN), 0, stream, p, nslots, KD);
   }
   if (e != cudaSuccess) return e;
   count_launch();
-  constexpr int floats = cr_out_floats(KIND, KD);
-  static const cudaError_t cfg = cr_allow(chunk_outputs_kernel<KIND, KD>, floats);
-  if (cfg != cudaSuccess) return cfg;
-  return launch(chunk_outputs_kernel<KIND, KD>, grid, block, floats * sizeof(float), stream, p);
-}
-
-template <int KD>
-static cudaError_t launch_chunks_kind(int kind, const ChunkParams& p, int nslots, cudaStream_t stream) {
-  switch (kind) {
-    case CR_FIXED: return launch_chunks<CR_FIXED, KD>(p, nslots, stream);
-    case CR_SSM: return launch_chunks<CR_SSM, KD>(p, nslots, stream);
-    case CR_DELTA: return launch_chunks<CR_DELTA, KD>(p, nslots, stream);
-    case CR_HGRN2: return launch_chunks<CR_HGRN2, KD>(p, nslots, stream);
-    default: return launch_chunks<CR_CHANNELS, KD>(p, nslots, stream);
-  }
+  return cr_launch_outputs(kind, p, nslots, stream);
 }
 
 // floats of scratch a (chunk, head); the arrays' offsets, in whole 16-byte pieces
 static long long cr_layout(ChunkParams& p, int kind) {
-  const int kd = p.dim <= 64 ? 64 : 128;
+  const int kd = p.dim <= 64 ? 64 : 128, vt = cr_tile(p.vdim), tiles = (p.vdim + vt - 1) / vt;
   p.v_ld_s = (p.vdim + 7) / 8 * 8;
-  int at = kd * p.v_ld_s;
+  int at = cr_delta(kind) ? 0 : kd * p.v_ld_s;
   p.off_w = at;
   if (cr_delta(kind)) at += CR_C * (kd + 4);
   p.off_k = at;
   if (cr_delta(kind)) at += kd * CR_PT;
   p.off_u = at;
   if (cr_delta(kind)) at += CR_C * p.v_ld_s;
+  p.off_s = at;
+  at += tiles * kd * vt * 3 / 2;
+  p.off_up = at;
+  at += tiles * CR_C * vt * 3 / 2;
+  p.off_f = at;
+  at += tiles * vt;
   p.off_g = at;
   p.per_head = at + kd;
   return p.per_head;
@@ -1368,7 +840,6 @@ LB_EXPORT int lb_chunk_recurrence(int kind, const float* q, long long q_ld, cons
   auto aligned = [](const float* x, long long ld) { return (uintptr_t)x % 16 == 0 && ld % 4 == 0; };
   p.vec = dim % 4 == 0 && aligned(q, q_ld) && aligned(k, k_ld) && (kind != lb::CR_CHANNELS || aligned(a, a_ld));
   p.vecv = vdim % 4 == 0 && aligned(v, v_ld);
-  p.vec2 = vdim % 2 == 0 && out_ld % 2 == 0 && (uintptr_t)out % 8 == 0;
   lb::cr_layout(p, kind);
   for (int done = 0; done < num_long;) {
     const int ns = num_long - done < lb::CR_SEQS ? num_long - done : lb::CR_SEQS;
@@ -1382,7 +853,7 @@ LB_EXPORT int lb_chunk_recurrence(int kind, const float* q, long long q_ld, cons
     for (int turn = 0; turn < turns; ++turn) {
       const int lo = (int)((long long)total * turn / turns), hi = (int)((long long)total * (turn + 1) / turns);
       p.slot0 = lo;
-      const cudaError_t e = dim <= 64 ? lb::launch_chunks_kind<64>(kind, p, hi - lo, stream) : lb::launch_chunks_kind<128>(kind, p, hi - lo, stream);
+      const cudaError_t e = dim <= 64 ? lb::launch_chunks<64>(kind, p, hi - lo, stream) : lb::launch_chunks<128>(kind, p, hi - lo, stream);
       if (e != cudaSuccess) { lb::set_error("chunk_recurrence: %s", cudaGetErrorString(e)); return 2; }
       LB_CHECK_LAUNCH("chunk_recurrence");
     }

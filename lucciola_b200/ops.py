@@ -659,7 +659,7 @@ def short_conv_step(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bi
 # Portions that may go through the chunked form of a recurrence (csrc/chunk_recurrence.cu).
 CHUNK_LEAST = 32
 # Scratch of the chunked form, in floats: more chunks are worked off in turns.
-CHUNK_SCRATCH = 32 << 20
+CHUNK_SCRATCH = 64 << 20
 _CHUNK_KINDS = {"fixed": 0, "ssm": 1, "delta": 2, "hgrn2": 3, "channels": 4}
 
 # What a step's recurrence costs in us, all launches (B200; fitted to 1400 steps of 1 to 16 equal portions of 32 to 448 tokens or of one to
@@ -672,10 +672,16 @@ _CHUNK_KINDS = {"fixed": 0, "ssm": 1, "delta": 2, "hgrn2": 3, "channels": 4}
 # 16 heads of 128 x 128, one portion of 448 tokens | 16 of 128, us: fixed 98 | 269, HGRN2 91 | 203, delta 195 | 276, channels 201 | 386.
 _WALK_US = {"fixed": (2.9, 0.497, 0.18, 0.285, 0.15, 0, 32), "ssm": (4.0, 0.275, 0.14, 0.176, 0.2, 15, 32), "hgrn2": (4.5, 0.187, 0.34, 0.187, 0.34, 27, 32),
             "delta": (4.0, 0.43, 0.4, 0.276, 0.4, 13, 32), "channels": (7.6, 0.44, 0.4, 0.205, 0.4, 12, 16)}
-# Chunked, from the chunks times heads, at 128 value columns: start and a CTA while all run at once (two an SM), start and a CTA
-# beyond; factors on the starts and on the CTAs up to 64 rows.  The same steps: fixed 64 | 160, HGRN2 70 | 171, delta 82 | 207, channels 110 | 269.
-_CHUNK_US = {"fixed": (51, 0.117, 12, 0.282, 0.7, 0.6), "ssm": (34, 0.066, 15, 0.24, 0.73, 0.65), "hgrn2": (59, 0.097, 19, 0.294, 0.7, 0.6),
-             "delta": (57, 0.21, 23, 0.37, 0.8, 0.63), "channels": (77, 0.245, 37, 0.47, 0.8, 0.63)}
+# Chunked, from the chunks times heads, at 128 value columns: start and a CTA while all run at once (one an SM), start and a CTA
+# beyond; factors on the starts and on the CTAs up to 64 rows.
+_CHUNK_US = {"fixed": (23, 0.093, 15, 0.166, 0.74, 0.59), "ssm": (20.6, 0.073, 12.6, 0.189, 0.83, 0.78), "hgrn2": (29.3, 0.085, 16.3, 0.234, 0.74, 0.55),
+             "delta": (35, 0.259, 28, 0.318, 0.8, 0.63), "channels": (60, 0.173, 35, 0.464, 0.8, 0.63)}
+# Those of the chunked form while its products were mma.sync's, two CTAs an SM.  Whatever they send to it goes there still, so that no step
+# turns to sums that are further from 64 bits than those that its callers have had; steps whose longest portion is shorter than
+# _CHUNK_SHORT go by them alone and stay where they were.
+_CHUNK_SHORT = {"fixed": 97, "ssm": 97, "hgrn2": 193, "delta": 97, "channels": 97}
+_CHUNK_SHORT_US = {"fixed": (51, 0.117, 12, 0.282, 0.7, 0.6), "ssm": (34, 0.066, 15, 0.24, 0.73, 0.65), "hgrn2": (59, 0.097, 19, 0.294, 0.7, 0.6),
+                   "delta": (57, 0.21, 23, 0.37, 0.8, 0.63), "channels": (77, 0.245, 37, 0.47, 0.8, 0.63)}
 
 
 def _walk_us(kind: str, lens, heads: int, dim: int, vdim: int, split: int) -> float:
@@ -691,10 +697,14 @@ def _walk_us(kind: str, lens, heads: int, dim: int, vdim: int, split: int) -> fl
 
 
 def _chunk_us(kind: str, lens, heads: int, dim: int, vdim: int) -> float:
-    few, one, many, more, starts, each = _CHUNK_US[kind]
     ctas, cols = sum(-(-n // 64) for n in lens) * heads, 0.3 + 0.7 * vdim / 128
-    starts, each = (starts, each) if dim <= 64 else (1.0, 1.0)
-    return few * starts + one * each * cols * ctas if ctas <= 296 else many * starts + more * each * cols * ctas
+
+    def us(few, one, many, more, starts, each, at_once):
+        starts, each = (starts, each) if dim <= 64 else (1.0, 1.0)
+        return few * starts + one * each * cols * ctas if ctas <= at_once else many * starts + more * each * cols * ctas
+
+    before = us(*_CHUNK_SHORT_US[kind], 296)
+    return before if max(lens) < _CHUNK_SHORT[kind] else min(before, us(*_CHUNK_US[kind], 148))
 
 
 def chunk_portions(kind: str, step, heads: int, dim: int, vdim: int) -> tuple[list[int], int]:
@@ -1378,9 +1388,10 @@ def device_error() -> int:
     lib.lb_attention_flash_device_error.restype = c_int
     lib.lb_latent_flash_device_error.restype = c_int
     lib.lb_latent_prefill_device_error.restype = c_int
+    lib.lb_chunk_device_error.restype = c_int
     return (int(lib.lb_device_error()) or int(lib.lb_attention_tcgen05_device_error())
             or int(lib.lb_attention_flash_device_error()) or int(lib.lb_latent_flash_device_error())
-            or int(lib.lb_latent_prefill_device_error()))
+            or int(lib.lb_latent_prefill_device_error()) or int(lib.lb_chunk_device_error()))
 
 
 def linear(y: torch.Tensor, x: torch.Tensor, w: torch.Tensor, stream: int, fast: bool, post: str | None = None, post_c: float = 0.0) -> None:
