@@ -31,13 +31,13 @@
 // from t on the walk may leave an infinity where a NaN stands here.
 //
 // Everything is 32-bit.  The products run on the tensor cores as six bfloat16 products of operands cut in three, which hold all 24
-// bits, 16 places at a time, and the sums from one 16 to the next are ordinary additions: those of single chunks in chunk_tcgen05.cu,
-// here the walk's and the triangular solve's, in which a product's operands come out of the one before it (see cr_step).  Decays
+// bits, 16 places at a time, and the sums from one 16 to the next are ordinary additions: those of single chunks, and the walk where its
+// CTAs run at once, in chunk_tcgen05.cu; here the triangular solve's and the walk in several rounds (see cr_step).  Decays
 // and strengths that are one number a token come out of 64 bits, and their products carry what rounding drops.  Against 64 bits the
 // outputs before the norm are 0.2 to 0.98 times as far off as those of the kernels that walk token by token, over the layers' sizes.
 //
 // Measured (B200, all launches, token by token | every product by mma.sync | here): HGRN2, one prompt of 2048 tokens and 16 heads of
-// 128 x 128, 403 | 150 | 124 us; the delta rule 865 | 210 | 195; fixed decays, four prompts of 1654 tokens in all, 341 | 137 | 88.
+// 128 x 128, 403 | 150 | 124 us; the delta rule 865 | 210 | 177; fixed decays, four prompts of 1654 tokens in all, 341 | 137 | 88.
 // What bounds the kernels here: mma.sync issues one product every 8 cycles a scheduler on this GPU whatever its type, so the six products
 // of 16 places are worth 1.3 times the ordinary 32-bit pipes; the walk is 32 links of two small products each.
 #include "chunk_recurrence.cuh"
@@ -358,12 +358,27 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
   if (!ROWS) cr_products(gs, Ds, cs, tid);
   __syncthreads();
   const uint32_t Ka = (uint32_t)__cvta_generic_to_shared(Ks);
-  auto keys_out = [&](const float* K, const float* scale) {      // keys to the state behind the chunk, a row of the state a row
-    for (int i = warp; i < 2 * (KD / 4); i += CR_THREADS / 32) {
-      const int t = (i & 1) * 32 + lane, d = (i >> 1) * 4;
-      const float g = scale ? scale[t] : 1.f;
-      const float4 x = *reinterpret_cast<const float4*>(K + t * PK + d);
-      oK[d * CR_PT + t] = x.x * g; oK[(d + 1) * CR_PT + t] = x.y * g; oK[(d + 2) * CR_PT + t] = x.z * g; oK[(d + 3) * CR_PT + t] = x.w * g;
+  // Keys to the state behind the chunk: cut, as the wide walk's products read them, or a row of the state a row.
+  const bool wide = KD == 128 && p.wide;
+  auto keys_out = [&](const float* K, const float* scale) {
+    if (wide) {
+      for (int i = tid; i < CR_C * KD / 4; i += CR_THREADS) {
+        const int t = i / (KD / 4), d = i % (KD / 4) * 4;
+        const float g = scale ? scale[t] : 1.f;
+        const float4 x = *reinterpret_cast<const float4*>(K + t * PK + d);
+        const Split a = cr_split(x.x * g, x.y * g), b = cr_split(x.z * g, x.w * g);
+        uint8_t* to = reinterpret_cast<uint8_t*>(oK) + cr_at(t, d, CR_C);
+        *reinterpret_cast<uint2*>(to) = make_uint2(a.h, b.h);
+        *reinterpret_cast<uint2*>(to + CR_C * KD * 2) = make_uint2(a.m, b.m);
+        *reinterpret_cast<uint2*>(to + 2 * CR_C * KD * 2) = make_uint2(a.l, b.l);
+      }
+    } else {
+      for (int i = warp; i < 2 * (KD / 4); i += CR_THREADS / 32) {
+        const int t = (i & 1) * 32 + lane, d = (i >> 1) * 4;
+        const float g = scale ? scale[t] : 1.f;
+        const float4 x = *reinterpret_cast<const float4*>(K + t * PK + d);
+        oK[d * CR_PT + t] = x.x * g; oK[(d + 1) * CR_PT + t] = x.y * g; oK[(d + 2) * CR_PT + t] = x.z * g; oK[(d + 3) * CR_PT + t] = x.w * g;
+      }
     }
   };
   if (!ROWS) {
@@ -511,7 +526,9 @@ __global__ void __launch_bounds__(CR_THREADS, 2) chunk_solve_kernel(const __grid
         for (int e2 = 0; e2 < 2; ++e2) {
           const float2 x = make_float2(acc[t][2 * e2], acc[t][2 * e2 + 1]);
           *reinterpret_cast<float2*>(mineX + e2 * 8 * pitch + 8 * t) = x;
-          if (t ? stored1 : stored0) *reinterpret_cast<float2*>(out + e2 * 8 * ld + 8 * t) = x;
+          if (wide && !values)
+            cr_put(reinterpret_cast<uint8_t*>(oW) + cr_at(16 * I + (lane >> 2) + 8 * e2, (int)(dst - oW) + 8 * t + 2 * (lane & 3), CR_C), CR_C * KD * 2, cr_split(x.x, x.y));
+          else if (t ? stored1 : stored0) *reinterpret_cast<float2*>(out + e2 * 8 * ld + 8 * t) = x;
         }
       __syncwarp();
     }
@@ -766,10 +783,14 @@ static cudaError_t launch_chunks(int kind, const ChunkParams& p, int nslots, cud
     e = kind == CR_DELTA ? launch_solve<CR_DELTA, KD>(p, nslots, stream) : launch_solve<CR_CHANNELS, KD>(p, nslots, stream);
     if (e != cudaSuccess) return e;
     count_launch();
-    int nv = 32;
-    while (nv > 8 && (long long)p.num_seqs * p.heads * ((p.vdim + nv - 1) / nv) < 100) nv /= 2;
-    e = nv == 32 ? launch_chunk_walk<KD, 32>(p, nslots, stream) : nv == 16 ? launch_chunk_walk<KD, 16>(p, nslots, stream)
-                                                                           : launch_chunk_walk<KD, 8>(p, nslots, stream);
+    if (p.wide) {
+      e = cr_launch_walk(p, nslots, stream);
+    } else {
+      int nv = 32;
+      while (nv > 8 && (long long)p.num_seqs * p.heads * ((p.vdim + nv - 1) / nv) < 100) nv /= 2;
+      e = nv == 32 ? launch_chunk_walk<KD, 32>(p, nslots, stream) : nv == 16 ? launch_chunk_walk<KD, 16>(p, nslots, stream)
+                                                                             : launch_chunk_walk<KD, 8>(p, nslots, stream);
+    }
   } else {
     e = cr_launch_states(kind, p, nslots, stream);
     if (e != cudaSuccess) return e;
@@ -787,9 +808,9 @@ static long long cr_layout(ChunkParams& p, int kind) {
   p.v_ld_s = (p.vdim + 7) / 8 * 8;
   int at = cr_delta(kind) ? 0 : kd * p.v_ld_s;
   p.off_w = at;
-  if (cr_delta(kind)) at += CR_C * (kd + 4);
+  if (cr_delta(kind)) at += kd == 128 ? CR_C * kd * 3 / 2 : CR_C * (kd + 4);       // of 128 rows: of either walk's form
   p.off_k = at;
-  if (cr_delta(kind)) at += kd * CR_PT;
+  if (cr_delta(kind)) at += kd == 128 ? CR_C * kd * 3 / 2 : kd * CR_PT;
   p.off_u = at;
   if (cr_delta(kind)) at += CR_C * p.v_ld_s;
   p.off_s = at;
@@ -844,6 +865,11 @@ LB_EXPORT int lb_chunk_recurrence(int kind, const float* q, long long q_ld, cons
   for (int done = 0; done < num_long;) {
     const int ns = num_long - done < lb::CR_SEQS ? num_long - done : lb::CR_SEQS;
     p.num_seqs = ns;
+    // The walk on tcgen05 has a CTA for 16 columns and one CTA an SM: where all of them run at once it is the faster (16 heads of 128 x 128,
+    // one prompt of 2048 tokens, 92 -> 68 us), in more than one round the one with 32 columns a CTA is (32 heads, two rounds, 136 | 125).
+    p.wide = lb::cr_delta(kind) && dim > 64 && (long long)ns * heads * ((vdim + 15) / 16) <= 148;
+    if (!p.wide) p.off_k = p.off_w + lb::CR_C * ((dim <= 64 ? 64 : 128) + 4);      // right behind W: one copy
+    else p.off_k = p.off_w + lb::CR_C * 128 * 3 / 2;
     p.base[0] = 0;
     for (int i = 0; i < ns; ++i) {
       p.seq[i] = seqs[done + i];

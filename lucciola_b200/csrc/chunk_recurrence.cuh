@@ -29,11 +29,12 @@ struct ChunkParams {
   int vec, vecv;                         // rows of q, k, a and rows of v in whole aligned 16-byte pieces
   int slot0;                             // first chunk of this launch, counted over the sequences below
   int num_seqs;
+  int wide;                              // delta rules: the walk of chunk_tcgen05.cu, which wants W and K cut
   float* scratch;                        // per (chunk of this launch, head), the arrays at these offsets
   long long per_head;
-  // [KD][v_ld_s] K^T U at 0; or W [64][KD + 4], K^T [KD][68], U' [64][v_ld_s]; the state before the chunk and U as the outputs' products
-  // take them, of a tile of columns after the other (columns behind the last one are not written); the first token whose U is not
-  // finite, of every column; c_63
+  // [KD][v_ld_s] K^T U at 0; or W and K [64][KD] in three parts (wide), or W [64][KD + 4] and K^T [KD][68], then U' [64][v_ld_s]; the
+  // state before the chunk and U as the outputs' products take them, of a tile of columns after the other (columns behind the last one
+  // are not written); the first token whose U is not finite, of every column; c_63
   int off_w, off_k, off_u, off_s, off_up, off_f, off_g, v_ld_s;
   int seq[CR_SEQS];                      // sequence of the step
   int base[CR_SEQS + 1];                 // its first chunk
@@ -175,7 +176,8 @@ __device__ __forceinline__ void cr_put(uint8_t* at, int part, const Split& x) {
   *reinterpret_cast<uint32_t*>(at + 2 * part) = x.l;
 }
 
-// chunk_tcgen05.cu: K^T U of the kinds without the delta rule; the outputs.
+// chunk_tcgen05.cu: the states before the chunks of the delta rules; K^T U of the other kinds; the outputs.
+cudaError_t cr_launch_walk(const ChunkParams& p, int nslots, cudaStream_t stream);       // delta rules, `wide`
 cudaError_t cr_launch_states(int kind, const ChunkParams& p, int nslots, cudaStream_t stream);
 cudaError_t cr_launch_outputs(int kind, const ChunkParams& p, int nslots, cudaStream_t stream);
 

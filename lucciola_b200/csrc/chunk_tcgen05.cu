@@ -859,6 +859,220 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
   if (warp == 0) ct_free<512>(tmem);
 }
 
+// ---- the states before the chunks of the delta rules, 128 rows: U = U' - W S, S <- diag(c) S + K^T U -----------------------------
+// A CTA for every (16 value columns, head, sequence); the state's 128 x 16 numbers stay in registers, a row's eight columns a thread.  Both
+// products of a chunk have W or K^T on the lanes and the three parts of S or U side by side, [h | m | l] of 16 columns each: a product with
+// 16 columns takes the tensor cores as long as one with 48 (their left side's 4 KB from shared memory bound both), so three
+// products a step of 16 places form all six: W_h [h | m | l], W_m [h | m], W_l h, 8 sums of 16 places apart.  W and K, which the solve
+// leaves cut, are copied two chunks deep.  What bounds it is the path from chunk to chunk, 2.1 us (mma.sync, which cut W and K in every CTA, 2.9
+// where it leaves the states cut as here): products 0.55 and 0.3 us at their rate, twice the read-out of tensor memory, cutting and handing
+// over, and 96 KB a chunk and CTA out of L2, 5.7 TB/s over all CTAs.
+constexpr int CW_COLS = 16, CW_THREADS = 256;        // that compute; and a warp for the products and one for the copies
+constexpr int CW_PART = CR_C * 128 * 2;              // bytes of a part of W or K
+constexpr int CW_STAGE = 6 * CW_PART;                // W, K
+constexpr int CW_BYTES = 1024 + 2 * CW_STAGE + 128 * 128 + CR_C * 128;
+enum CwBar : int { CW_READY_S, CW_READY_U, CW_WS, CW_KU, CW_FULL_W, CW_FULL_W1, CW_FULL_K, CW_FULL_K1, CW_FREE_W, CW_FREE_W1, CW_FREE_K, CW_FREE_K1, CW_BARS };
+
+// The first 16 lanes of the warp's quarter x 8 columns: x[e] is lane l / 4 + 8 (e / 2), column 2 (l % 4) + e % 2.
+__device__ __forceinline__ void ct_ld8_half(uint32_t at, float* x) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(x);
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+// Sums of STEPS steps (48 columns each: large | small | small) of N values a step: the large ones pairwise, the small ones behind them.
+template <int STEPS, int N, typename F>
+__device__ __forceinline__ void cw_sums(uint32_t at, float* out, F load) {
+  float x[STEPS][N], y[STEPS][2][N];
+#pragma unroll
+  for (int k = 0; k < STEPS; ++k) {
+    load(at + 48 * k, x[k]);
+    load(at + 48 * k + 16, y[k][0]);
+    load(at + 48 * k + 32, y[k][1]);
+  }
+  ct_wait_ld();
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    float small = 0.f;
+#pragma unroll
+    for (int k = 0; k < STEPS; ++k) small += y[k][0][i] + y[k][1][i];
+#pragma unroll
+    for (int n = STEPS / 2; n >= 1; n /= 2)
+#pragma unroll
+      for (int k = 0; k < n; ++k) x[k][i] += x[k + n][i];
+    out[i] = x[0][i] + small;
+  }
+}
+
+__global__ void __launch_bounds__(CW_THREADS + 64, 1) chunk_walk_wide_kernel(const __grid_constant__ ChunkParams p, int nslots) {
+  extern __shared__ uint8_t ct_raw[];
+  __shared__ uint64_t bars_s[CW_BARS];
+  __shared__ uint32_t tmem_s;
+  __shared__ int abort_s;
+  uint8_t* base = ct_raw + ((1024u - (ta_smem_u32(ct_raw) & 1023u)) & 1023u);
+  uint8_t* Sp = base + 2 * CW_STAGE;                 // [128 rows of the state][3][16 columns], 128 bytes a row
+  uint8_t* Up = Sp + 128 * 128;                      // [64 tokens][3][16 columns]
+  pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = blockIdx.y, seq = p.seq[blockIdx.z], first = p.base[blockIdx.z];
+  const int c_lo = max(0, p.slot0 - first), c_hi = min(p.base[blockIdx.z + 1], p.slot0 + nslots) - first;
+  const uint32_t bar = ta_smem_u32(bars_s);
+  if (c_lo >= c_hi) return;                          // the whole CTA
+  if (tid == 0) {
+    abort_s = 0;
+    for (int i = 0; i < CW_BARS; ++i) ta_mbar_init(bar + 8 * i, i <= CW_READY_U ? CW_THREADS / 32 : 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) ct_alloc<512>(ta_smem_u32(&tmem_s));
+  ct_before_sync();
+  __syncthreads();
+  ct_after_sync();
+  const uint32_t tmem = tmem_s;
+  pdl_wait();
+  const size_t stride = (size_t)p.heads * p.per_head;
+  float* mine = p.scratch + ((size_t)(first + c_lo - p.slot0) * p.heads + h) * p.per_head;
+  uint32_t phases = 0;                               // parities, as in the outputs
+  auto wait = [&](int b) {
+    ta_mbar_wait(bar + 8 * b, (phases >> b) & 1u, &abort_s, CT_ERR_OUT + CT_BARS + b);
+    phases ^= 1u << b;
+  };
+
+  if (warp == CW_THREADS / 32) {
+    if (elect_one()) {
+      const uint32_t s_at = ta_smem_u32(Sp), u_at = ta_smem_u32(Up);
+      auto step = [&](uint32_t d, const CtOperand& left, int ks, uint64_t right, int m) {
+        ta_umma(d, ct_desc(left, 0, ks), right, ct_idesc(left.mn, 1, m, 48), 0);
+        ta_umma(d + 16, ct_desc(left, 1, ks), right, ct_idesc(left.mn, 1, m, 32), 1);
+        ta_umma(d + 32, ct_desc(left, 2, ks), right, ct_idesc(left.mn, 1, m, 16), 1);
+      };
+      for (int c = c_lo; c < c_hi; ++c) {
+        const int buf = (c - c_lo) & 1;
+        const uint32_t w_at = ta_smem_u32(base) + buf * CW_STAGE;
+        const CtOperand W = {w_at, CW_PART, CR_C * 128, CR_C, 0}, K = {w_at + 3 * CW_PART, CW_PART, 0, CR_C, 1};
+        wait(CW_FULL_W + buf);
+        wait(CW_READY_S);
+        ct_after_sync();
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) step(tmem + 48 * ks, W, ks, ta_desc_mnmajor(s_at + ks * 2048, 128 * 128), 64);
+        ta_commit(bar + 8 * CW_WS);
+        ta_commit(bar + 8 * (CW_FREE_W + buf));
+        wait(CW_FULL_K + buf);
+        wait(CW_READY_U);
+        ct_after_sync();
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) step(tmem + 48 * ks, K, ks, ta_desc_mnmajor(u_at + ks * 2048, CR_C * 128), 128);
+        ta_commit(bar + 8 * CW_KU);
+        ta_commit(bar + 8 * (CW_FREE_K + buf));
+      }
+    }
+    __syncwarp();
+  } else if (warp == CW_THREADS / 32 + 1) {
+    if (elect_one()) {
+      const float* from = mine;
+      for (int c = c_lo; c < c_hi; ++c, from += stride) {
+        const int buf = (c - c_lo) & 1;
+        const uint32_t to = ta_smem_u32(base) + buf * CW_STAGE;
+        if (c >= c_lo + 2) wait(CW_FREE_W + buf);
+        ta_mbar_expect_tx(bar + 8 * (CW_FULL_W + buf), 3 * CW_PART);
+        ct_bulk_in(to, from + p.off_w, 3 * CW_PART, bar + 8 * (CW_FULL_W + buf));
+        if (c >= c_lo + 2) wait(CW_FREE_K + buf);
+        ta_mbar_expect_tx(bar + 8 * (CW_FULL_K + buf), 3 * CW_PART);
+        ct_bulk_in(to + 3 * CW_PART, from + p.off_k, 3 * CW_PART, bar + 8 * (CW_FULL_K + buf));
+      }
+    }
+    __syncwarp();
+  } else {
+    const int quad = warp & 3, hf = (warp >> 2) * 8;             // 32 rows of the state or 16 tokens; eight columns
+    const int col0 = blockIdx.x * CW_COLS + hf;
+    const uint32_t at = tmem + ((uint32_t)(32 * quad) << 16) + hf;
+    const int part = 128 * cr_tile(p.vdim);
+    const int d = 32 * quad + lane, t = 16 * quad + (lane >> 2), cc = 2 * (lane & 3);
+    const bool there = col0 < p.v_ld_s;                          // a multiple of eight
+    const int s_off = there ? (int)(cr_state_at(p, mine, 128, d, col0) - reinterpret_cast<uint8_t*>(mine)) : 0;
+    const int u_off = there ? (int)(cr_u_at(p, mine, t, col0 + cc) - reinterpret_cast<uint8_t*>(mine)) : 0;
+    auto arrive = [&](int b) {
+      ct_publish();
+      ct_before_sync();
+      __syncwarp();
+      if (lane == 0) ta_mbar_arrive(bar + 8 * b);
+    };
+    float s[8], g = 1.f;
+    float2 u_next[2];
+    auto request = [&](const float* src) {                       // U' and the row's decay over the chunk
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        u_next[e] = there ? *reinterpret_cast<const float2*>(src + p.off_u + (t + 8 * e) * p.v_ld_s + col0 + cc) : make_float2(0.f, 0.f);
+      g = src[p.off_g + d];
+    };
+    auto put_state = [&](float* keep) {              // for the next product, and for the outputs of the chunk it stands before
+      Split x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = cr_split(s[2 * i], s[2 * i + 1]);
+      const uint4 hi = make_uint4(x[0].h, x[1].h, x[2].h, x[3].h), mi = make_uint4(x[0].m, x[1].m, x[2].m, x[3].m), lo = make_uint4(x[0].l, x[1].l, x[2].l, x[3].l);
+      *reinterpret_cast<uint4*>(Sp + cr_at(d, hf, 128)) = hi;
+      *reinterpret_cast<uint4*>(Sp + cr_at(d, 16 + hf, 128)) = mi;
+      *reinterpret_cast<uint4*>(Sp + cr_at(d, 32 + hf, 128)) = lo;
+      arrive(CW_READY_S);
+      if (there) {
+        uint8_t* to = reinterpret_cast<uint8_t*>(keep) + s_off;
+        *reinterpret_cast<uint4*>(to) = hi;
+        *reinterpret_cast<uint4*>(to + part) = mi;
+        *reinterpret_cast<uint4*>(to + 2 * part) = lo;
+      }
+    };
+    float* S = p.state + ((size_t)p.slots[seq] * p.heads + h) * p.dim * p.vdim + (size_t)d * p.vdim + col0;
+    const int have = d < p.dim ? min(8, p.vdim - col0) : 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = i < have ? S[i] : 0.f;
+    put_state(mine);
+    request(mine);
+    for (int c = c_lo; c < c_hi; ++c) {
+      const float2 u0 = u_next[0], u1 = u_next[1];
+      const float decay = g;
+      float* const keep = mine;
+      mine += stride;
+      if (c + 1 < c_hi) request(mine);
+      wait(CW_WS);
+      ct_after_sync();
+      float y[4];
+      cw_sums<8, 4>(at, y, [](uint32_t a, float* x) { ct_ld8_half(a, x); });
+      y[0] = u0.x - y[0]; y[1] = u0.y - y[1]; y[2] = u1.x - y[2]; y[3] = u1.y - y[3];
+      Split a = cr_split(y[0], y[1]), b = cr_split(y[2], y[3]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const Split& x = e ? b : a;
+        *reinterpret_cast<uint32_t*>(Up + cr_at(t + 8 * e, hf + cc, CR_C)) = x.h;
+        *reinterpret_cast<uint32_t*>(Up + cr_at(t + 8 * e, 16 + hf + cc, CR_C)) = x.m;
+        *reinterpret_cast<uint32_t*>(Up + cr_at(t + 8 * e, 32 + hf + cc, CR_C)) = x.l;
+      }
+      arrive(CW_READY_U);
+      if (there) {
+        if (!(cr_finite(y[0]) && cr_finite(y[1]) && cr_finite(y[2]) && cr_finite(y[3]))) {      // rare: the outputs' product meets it with the zeros of earlier tokens
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (!cr_finite(y[e])) { atomicMin(reinterpret_cast<int*>(keep) + p.off_f + col0 + cc + (e & 1), t + 8 * (e >> 1)); y[e] = 0.f; }
+          a = cr_split(y[0], y[1]);
+          b = cr_split(y[2], y[3]);
+        }
+        uint8_t* to = reinterpret_cast<uint8_t*>(keep) + u_off;
+        cr_put(to, part, a);
+        cr_put(to + 8 * 128, part, b);
+      }
+      wait(CW_KU);
+      ct_after_sync();
+      float x[8];
+      cw_sums<4, 8>(at, x, [](uint32_t a, float* z) { ct_ld8(a, z); });
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s[i] = fmaf(decay, s[i], x[i]);
+      if (c + 1 < c_hi) put_state(mine);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) if (i < have) S[i] = s[i];
+  }
+  ct_before_sync();
+  __syncthreads();
+  ct_after_sync();
+  if (warp == 0) ct_free<512>(tmem);
+}
+
 template <typename K>
 static cudaError_t ct_allow(K kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); }
 
@@ -880,6 +1094,12 @@ static cudaError_t launch_outputs(const ChunkParams& p, int nslots, cudaStream_t
   if (e != cudaSuccess) return e;
   const int units = nslots * p.heads;
   return launch(chunk_outputs_kernel<KIND, KD, VT>, dim3(units < sms ? units : sms), dim3(CT_OUT_THREADS), bytes, stream, p, units);
+}
+
+cudaError_t cr_launch_walk(const ChunkParams& p, int nslots, cudaStream_t stream) {
+  static const cudaError_t cfg = ct_allow(chunk_walk_wide_kernel, CW_BYTES);
+  if (cfg != cudaSuccess) return cfg;
+  return launch(chunk_walk_wide_kernel, dim3((p.vdim + CW_COLS - 1) / CW_COLS, p.heads, p.num_seqs), dim3(CW_THREADS + 64), CW_BYTES, stream, p, nslots);
 }
 
 // Value columns up to 64 take tiles of 64, more than that of 128.

@@ -675,7 +675,7 @@ _WALK_US = {"fixed": (2.9, 0.497, 0.18, 0.285, 0.15, 0, 32), "ssm": (4.0, 0.275,
 # Chunked, from the chunks times heads, at 128 value columns: start and a CTA while all run at once (one an SM), start and a CTA
 # beyond; factors on the starts and on the CTAs up to 64 rows.
 _CHUNK_US = {"fixed": (23, 0.093, 15, 0.166, 0.74, 0.59), "ssm": (20.6, 0.073, 12.6, 0.189, 0.83, 0.78), "hgrn2": (29.3, 0.085, 16.3, 0.234, 0.74, 0.55),
-             "delta": (35, 0.259, 28, 0.318, 0.8, 0.63), "channels": (60, 0.173, 35, 0.464, 0.8, 0.63)}
+             "delta": (36, 0.25, 25, 0.334, 0.8, 0.63), "channels": (60, 0.174, 31, 0.483, 0.8, 0.63)}
 # Those of the chunked form while its products were mma.sync's, two CTAs an SM.  Whatever they send to it goes there still, so that no step
 # turns to sums that are further from 64 bits than those that its callers have had; steps whose longest portion is shorter than
 # _CHUNK_SHORT go by them alone and stay where they were.
