@@ -13,7 +13,24 @@
 
 namespace lb {
 
-__device__ __forceinline__ float silu_exact(float x) { return x / (1.f + expf(-x)); }
+// x / (1 + e^-x) as the approximate reciprocal and one step on the remainder, which leaves half an ulp as a division does at a third of its
+// instructions; a division only where the reciprocal would be no normal number or the remainder no number.
+__device__ __forceinline__ bool silu_plain(float x) { return fabsf(x) < 80.f; }
+__device__ __forceinline__ float silu_divided(float x) { return x / (1.f + expf(-x)); }
+__device__ __forceinline__ float silu_near(float x) {
+  const float d = 1.f + expf(-x);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float y = x * r;
+  return fmaf(fmaf(-y, d, x), r, y);
+}
+__device__ __forceinline__ float silu_exact(float x) { return silu_plain(x) ? silu_near(x) : silu_divided(x); }
+__device__ __forceinline__ void silu_exact(float4& a) {
+  if (silu_plain(a.x) && silu_plain(a.y) && silu_plain(a.z) && silu_plain(a.w))
+    a = make_float4(silu_near(a.x), silu_near(a.y), silu_near(a.z), silu_near(a.w));
+  else
+    a = make_float4(silu_exact(a.x), silu_exact(a.y), silu_exact(a.z), silu_exact(a.w));
+}
 
 __global__ void short_conv_kernel(float* __restrict__ out, long long out_ld, const float* __restrict__ x, long long x_ld,
                                   const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ state,
@@ -62,16 +79,17 @@ __global__ void short_conv_x4_kernel(float* __restrict__ out, long long out_ld, 
       const float4 b = *reinterpret_cast<const float4*>(bias + c);
       acc.x += b.x; acc.y += b.y; acc.z += b.z; acc.w += b.w;
     }
-    if (act) { acc.x = silu_exact(acc.x); acc.y = silu_exact(acc.y); acc.z = silu_exact(acc.z); acc.w = silu_exact(acc.w); }
+    if (act) silu_exact(acc);
     *reinterpret_cast<float4*>(out + (size_t)t * out_ld + c) = acc;
   }
 }
 
 // Four taps, four channels a thread and TT neighbouring tokens: the inputs of the last three tokens slide through registers, so an
 // input is read once and three eighths of it once again (four times with a token a thread), and the weights once.  At a portion's
-// start the window comes from the state.  2048 tokens of 4096 channels, 67 MB: 29 us with a token a thread, 22 us with eight.
+// start the window comes from the state.  2048 tokens of 4096 channels, 67 MB: 29 us with a token a thread, 22 us with eight, 16 us with
+// the silu's reciprocal, one look at the portion for all eight and CTAs of 64 threads (of 256: 18.5); what it moves takes 10.
 template <int TT>
-__global__ void __launch_bounds__(256) short_conv_x4_tokens_kernel(float* __restrict__ out, long long out_ld, const float* __restrict__ x, long long x_ld,
+__global__ void __launch_bounds__(64) short_conv_x4_tokens_kernel(float* __restrict__ out, long long out_ld, const float* __restrict__ x, long long x_ld,
                                                                    const float* __restrict__ w, const float* __restrict__ bias,
                                                                    const float* __restrict__ state, const int* __restrict__ token_seq,
                                                                    const int* __restrict__ cu_tokens, const int* __restrict__ slots, int num_tokens,
@@ -85,27 +103,25 @@ __global__ void __launch_bounds__(256) short_conv_x4_tokens_kernel(float* __rest
   if (bias) b = *reinterpret_cast<const float4*>(bias + c);
   pdl_wait();
   float4 v[TT + 3];                                // v[i]: the input of token t0 + i - 3
-  int seqs[TT], firsts[TT];
 #pragma unroll
-  for (int i = 0; i < TT; ++i) {
-    v[i + 3] = t0 + i < num_tokens ? *reinterpret_cast<const float4*>(x + (size_t)(t0 + i) * x_ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    seqs[i] = t0 + i < num_tokens ? token_seq[t0 + i] : 0;
-  }
+  for (int i = 0; i < TT; ++i) v[i + 3] = t0 + i < num_tokens ? *reinterpret_cast<const float4*>(x + (size_t)(t0 + i) * x_ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < 3; ++i) v[i] = t0 + i >= 3 ? *reinterpret_cast<const float4*>(x + (size_t)(t0 + i - 3) * x_ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < TT; ++i) firsts[i] = cu_tokens[seqs[i]];
+  const int last = min(t0 + TT, num_tokens) - 1, seq = token_seq[t0];
+  const bool inside = token_seq[last] == seq && t0 - cu_tokens[seq] >= 3;      // one portion's, and none of its first three tokens
 #pragma unroll
   for (int i = 0; i < TT; ++i) {
     const int t = t0 + i;
-    if (t >= num_tokens) break;
-    const int idx = t - firsts[i];                 // place of the token in its portion
+    if (t > last) break;
     float4 h[3] = {v[i], v[i + 1], v[i + 2]};
-    if (idx < 3) {
-      const float* st = state + (size_t)slots[seqs[i]] * 3 * channels + c;
+    if (!inside) {
+      const int s = token_seq[t], idx = t - cu_tokens[s];                        // place of the token in its portion
+      if (idx < 3) {
+        const float* st = state + (size_t)slots[s] * 3 * channels + c;
 #pragma unroll
-      for (int j = 0; j < 3; ++j)                  // tap j: the input 3 - j tokens back
-        if (idx < 3 - j) h[j] = *reinterpret_cast<const float4*>(st + (size_t)(idx + j) * channels);
+        for (int j = 0; j < 3; ++j)                // tap j: the input 3 - j tokens back
+          if (idx < 3 - j) h[j] = *reinterpret_cast<const float4*>(st + (size_t)(idx + j) * channels);
+      }
     }
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -114,7 +130,7 @@ __global__ void __launch_bounds__(256) short_conv_x4_tokens_kernel(float* __rest
       a.x = fmaf(f[j].x, y.x, a.x); a.y = fmaf(f[j].y, y.y, a.y); a.z = fmaf(f[j].z, y.z, a.z); a.w = fmaf(f[j].w, y.w, a.w);
     }
     if (bias) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
-    if (act) { a.x = silu_exact(a.x); a.y = silu_exact(a.y); a.z = silu_exact(a.z); a.w = silu_exact(a.w); }
+    if (act) silu_exact(a);
     *reinterpret_cast<float4*>(out + (size_t)t * out_ld + c) = a;
   }
 }
@@ -153,7 +169,7 @@ __global__ void __launch_bounds__(256) short_conv_step_kernel(float* __restrict_
     a.x = fmaf(f[j].x, v[j].x, a.x); a.y = fmaf(f[j].y, v[j].y, a.y); a.z = fmaf(f[j].z, v[j].z, a.z); a.w = fmaf(f[j].w, v[j].w, a.w);
   }
   if (bias) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
-  if (act) { a.x = silu_exact(a.x); a.y = silu_exact(a.y); a.z = silu_exact(a.z); a.w = silu_exact(a.w); }
+  if (act) silu_exact(a);
   *reinterpret_cast<float4*>(out + (size_t)s * out_ld + c) = a;
 #pragma unroll
   for (int j = 0; j < 3; ++j) *reinterpret_cast<float4*>(st + (size_t)j * channels) = v[j + 1];
@@ -188,12 +204,13 @@ LB_EXPORT int lb_short_conv(float* out, long long out_ld, const float* x, long l
   if (num_tokens == 0) return 0;
   auto a16 = [](const void* q) { return (uintptr_t)q % 16 == 0; };
   if (channels % 4 == 0 && out_ld % 4 == 0 && x_ld % 4 == 0 && a16(out) && a16(x) && a16(w) && a16(bias) && a16(state)) {
-    const int threads4 = channels >= 1024 ? 256 : 64;
+    const int threads4 = 64;
     const int by = (channels / 4 + threads4 - 1) / threads4;
     if (taps == 4 && by <= 65535 && num_tokens >= 8) {
-      // as many tokens a thread as leave every SM a few CTAs
+      // as many tokens a thread as leave every SM a few CTAs; these are small, so that the last ones leave no SM idle for long (2048 tokens
+      // of 12288 channels, cold: 71.7 us with 256 threads and a division, 59 with the reciprocal, 51.2 with 64 threads)
       const long long ctas = (long long)num_tokens * by;
-      const int tt = ctas >= 8 * 148 * 4 ? 8 : ctas >= 4 * 148 * 2 ? 4 : ctas >= 2 * 148 * 2 ? 2 : 1;
+      const int tt = ctas >= 8 * 148 * 16 ? 8 : ctas >= 4 * 148 * 8 ? 4 : ctas >= 2 * 148 * 8 ? 2 : 1;
       const dim3 grid((num_tokens + tt - 1) / tt, by), block(threads4);
       if (tt == 8) lb::launch(lb::short_conv_x4_tokens_kernel<8>, grid, block, 0, stream, out, out_ld, x, x_ld, w, bias, state, token_seq, cu_tokens, slots, num_tokens, channels, act);
       else if (tt == 4) lb::launch(lb::short_conv_x4_tokens_kernel<4>, grid, block, 0, stream, out, out_ld, x, x_ld, w, bias, state, token_seq, cu_tokens, slots, num_tokens, channels, act);
