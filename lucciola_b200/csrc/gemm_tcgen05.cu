@@ -21,7 +21,7 @@
 // to) the partials go through a workspace in global memory and the CTA that finishes last for a
 // tile adds them, again in the order of the splits.  Either way the result does not depend on timing.
 //
-// With more than 256 tokens (and from 65 or 129 tokens on for products with many features, see lb_gemm_tcgen05) a second
+// With more than 256 tokens (and from 33, 65 or 129 tokens on for products with many features, see lb_gemm_tcgen05) a second
 // kernel takes over (gemm_tcgen05_prefill_kernel): tokens on the lanes, features on
 // the columns, persistent CTAs over tiles of 128 tokens x up to 256 features with two accumulators, so that the epilogue
 // of a tile runs under the MMAs of the next; from 1024 tokens on as pairs of CTAs on tiles of 256 x 256 (tcgen05
@@ -1544,9 +1544,12 @@ LB_EXPORT int lb_gemm_tcgen05(void* y, int y_dtype, const void* x, const void* w
   // on with 65 tokens, three for two places with 33, half as many with 129.  us, the kernel that cuts K over a cluster | here: 64 tokens,
   // 3072 features of 2048 places 8.4 | 8.0, 8192 of 4096 18.8 | 16.5, 4096 of 4096 11.7 | 13.9; 128 tokens, 2048 of 2048 11.4 | 7.9, 12288 of 4096
   // 38.2 | 22.9, 4096 of 4096 15.4 | 14.5, 2048 of 4096 10.2 | 12.7; 256 tokens, 4096 of 4096 21.3 | 15.2, 2048 of 4096 14.1 | 13.1, of 6144 16.4 | 18.4.
-  // The gated product from 65 tokens on (24576 of 4096, 64 tokens 40.8 | 47.0, 128 48.5 | 47.4).  force_bt < 0 asks for the kernel
-  // with tokens on the lanes at any size; force_bt > 0 or a given split count for the other one.
-  const bool wide = M > 128 ? 2ll * N >= K : M > 64 ? N >= K : M > 32 && 2ll * N >= 3ll * K;
+  // The gated product from 65 tokens on (24576 of 4096, 64 tokens 40.8 | 47.0, 128 48.5 | 47.4).  Sums that stay 32-bit numbers (what a
+  // recurrence reads) keep their cut along K up to 128 tokens, and to 256 unless there are more features than places: the accumulator drops
+  // what lies below its sums at every 16 places, so that one chain over 4096 places is 1.5 to 2 times as far from 64 bits as the sum
+  // of a cluster's shorter ones, which 16-bit outputs don't show.  force_bt < 0 asks for the kernel with tokens on the lanes at
+  // any size; force_bt > 0 or a given split count for the other one.
+  const bool wide = y_dtype == LB_F32 ? M > 128 && N > K : M > 128 ? 2ll * N >= K : M > 64 ? N >= K : M > 32 && 2ll * N >= 3ll * K;
   const bool many = M > 256 ? force_bt <= 0 : force_bt < 0 || (force_bt == 0 && force_splits == 0 && (swiglu ? M > 64 : wide));
   if (many) {
     // force_bt: 0 chooses between one CTA a tile of 128 tokens and a pair of CTAs a tile of 256, -1 asks for the former,
@@ -1574,8 +1577,8 @@ LB_EXPORT int lb_gemm_tcgen05(void* y, int y_dtype, const void* x, const void* w
   int bt = 16;
   int splits = lb_gemm_tcgen05_plan(M, N, K, &bt);
   // A short product whose tiles fill more than half of the SMs gains less from two splits, of which some SMs hold two, than their
-  // reduction costs: 12288 features, 8 tokens, of 2048 places 13.5 -> 11.8 us; of 4096, 21.7 | 21.9.
-  if (splits == 2 && M <= 32 && K < 3072 && (N + lb::BM - 1) / lb::BM * 2 > 148) splits = 1;
+  // reduction costs: 12288 features, 8 tokens, of 2048 places 13.5 -> 11.8 us; of 4096, 21.7 | 21.9.  32-bit outputs keep the shorter chains.
+  if (y_dtype != LB_F32 && splits == 2 && M <= 32 && K < 3072 && (N + lb::BM - 1) / lb::BM * 2 > 148) splits = 1;
   if (force_bt) {
     LB_CHECK_ARG(force_bt == 16 || force_bt == 32 || force_bt == 64 || force_bt == 128 || force_bt == 256,
                  "gemm_tcgen05: token tile %d is not one of 16, 32, 64, 128, 256", force_bt);

@@ -60,3 +60,28 @@ def test_a_bad_value_in_any_tile_of_columns(kind, token, column):
     beside = torch.arange(heads * vdim, device=DEV) != column
     assert torch.equal(got[:, beside], good[:, beside])
     assert torch.isnan(got[token:, column]).all() and torch.isnan(after[0, 0, :, column]).all()
+
+
+@pytest.mark.parametrize("tokens,channels", [(1, 64), (8, 64), (4096, 260), (1200, 1024)])
+def test_silu_of_the_short_convolution(tokens, channels):
+    """Where the activation changes from the reciprocal to the division (80), around the largest and smallest results and at what is no
+    number, alone and four in a word, for every number of tokens a thread: x / (1 + e^-x) within two units in the last place for the
+    exponential, one half for the sum and one half for the quotient, 3.6e-7, and 3e-37 where the exponential is infinite in 32 bits
+    (from -88.7 on)."""
+    from lucciola_b200 import ops
+    v = [0.0, -0.0, 1e-30, -1e-38, 79.99, -79.99, 80.0, -80.0, 87.0, -87.5, -88.5, -103.0, -200.0, 200.0, 3e38, -3e38, float("inf"), float("-inf"), float("nan"), -1.2785, 0.5]
+    x = torch.linspace(-90, 90, tokens * channels, device=DEV).view(tokens, channels)
+    x[0, : len(v)] = torch.tensor(v, device=DEV)
+    w = torch.zeros(4, channels, device=DEV)
+    w[3] = 1
+    step, s = step_of([tokens], [0]), torch.cuda.current_stream().cuda_stream
+    step.token_seq = torch.zeros(tokens, dtype=torch.int32, device=DEV)
+    out = torch.empty_like(x)
+    ops.short_conv(out, x, w, None, torch.zeros(1, 3, channels, device=DEV), step, s)
+    X = x.double()
+    want = X / (1 + torch.exp(-X))
+    ok = torch.ones_like(x, dtype=torch.bool)
+    ok[:4] = torch.isfinite(x[0])                # a tap of nothing times what is no number is no number in the three tokens behind it
+    assert ((out.double() - want).abs()[ok] <= 3.6e-7 * want.abs()[ok] + 3e-37).all()
+    inf = float("inf")
+    assert out[0, v.index(inf)] == inf and out[0, v.index(-inf)].isnan() and out[0, 18].isnan()

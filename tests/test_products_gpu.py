@@ -30,6 +30,26 @@ def test_on_both_sides_of_every_line(M, N, K):
     check(M, N, K, torch.bfloat16, N, 0)
 
 
+@pytest.mark.parametrize("M", [59, 93, 128, 200])
+@pytest.mark.parametrize("N,K", [(12288, 4096), (4096, 4096), (2048, 4096)])
+def test_32_bit_sums_in_short_chains(M, N, K):
+    """32-bit outputs of up to 256 tokens are no further from 64 bits than with the kernel that cuts K over a cluster and the cut that
+    it takes by itself (a quarter more than that for another order of the same sums); with more features than places from 129 tokens on, one
+    chain, which the bound of `check` holds."""
+    from lucciola_b200 import ops
+    torch.manual_seed(M + N)
+    x, w, s = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16(), torch.cuda.current_stream().cuda_stream
+    want = x.double() @ w.double().T
+    def off(**kw):
+        y = torch.empty(M, N, device=DEV)
+        ops.gemm_tcgen05(y, x, w, s, **kw)
+        return ((y.double() - want) ** 2).mean().sqrt()
+    if M > 128 and N > K:
+        check(M, N, K, torch.float32, N, 0)
+    else:
+        assert off() <= 1.25 * off(force_bt=128 if M > 64 else 64)
+
+
 @pytest.mark.parametrize("M", [1, 8, 32])
 @pytest.mark.parametrize("N,K", [(9472, 256), (9600, 256), (9601, 2048), (9600, 3072)])
 def test_few_tokens_of_many_features(M, N, K):
