@@ -54,6 +54,16 @@ extern int g_pdl_enabled;
 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The same for pointers to what other kernels write.  Loads through a `const __restrict__` parameter count as loads of constants: they may
+// become ld.global.nc, which takes no part in what the wait makes visible, and may be moved in front of it, where the kernel before is
+// still writing.  A pointer that comes out of the wait is nobody's constant, and cannot be read before it.
+template <typename P>
+__device__ __forceinline__ void pdl_from_here(P& from) { asm volatile("" : "+l"(from) : : "memory"); }
+template <typename... P>
+__device__ __forceinline__ void pdl_wait(P&... from) {
+  pdl_wait();
+  (pdl_from_here(from), ...);
+}
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

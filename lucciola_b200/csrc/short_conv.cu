@@ -37,7 +37,7 @@ __global__ void short_conv_kernel(float* __restrict__ out, long long out_ld, con
                                   const int* __restrict__ token_seq, const int* __restrict__ cu_tokens,
                                   const int* __restrict__ slots, int channels, int taps, int act) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, state, token_seq, cu_tokens, slots);
   const int t = blockIdx.x;
   const int s = token_seq[t];
   const int idx = t - cu_tokens[s];                       // place of the token in its portion
@@ -61,7 +61,7 @@ __global__ void short_conv_x4_kernel(float* __restrict__ out, long long out_ld, 
                                      const int* __restrict__ token_seq, const int* __restrict__ cu_tokens,
                                      const int* __restrict__ slots, int channels, int taps, int act) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, state, token_seq, cu_tokens, slots);
   const int t = blockIdx.x;
   const int s = token_seq[t];
   const int idx = t - cu_tokens[s];
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(64) short_conv_x4_tokens_kernel(float* __restr
 #pragma unroll
   for (int j = 0; j < 4; ++j) f[j] = *reinterpret_cast<const float4*>(w + (size_t)j * channels + c);
   if (bias) b = *reinterpret_cast<const float4*>(bias + c);
-  pdl_wait();
+  pdl_wait(x, state, token_seq, cu_tokens, slots);
   float4 v[TT + 3];                                // v[i]: the input of token t0 + i - 3
 #pragma unroll
   for (int i = 0; i < TT; ++i) v[i + 3] = t0 + i < num_tokens ? *reinterpret_cast<const float4*>(x + (size_t)(t0 + i) * x_ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256) short_conv_step_kernel(float* __restrict_
   const int s = blockIdx.x;
   if ((int)blockIdx.y >= round_from) {
     const int c = ((blockIdx.y - round_from) * blockDim.x + threadIdx.x) * 4;
-    pdl_wait();
+    pdl_wait(round_x);
     if (c >= round_n) return;
     const float4 y = *reinterpret_cast<const float4*>(round_x + (size_t)s * round_ld + c);
     __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256) short_conv_step_kernel(float* __restrict_
 #pragma unroll
   for (int j = 0; j < 4; ++j) f[j] = *reinterpret_cast<const float4*>(w + (size_t)j * channels + c);
   if (bias) b = *reinterpret_cast<const float4*>(bias + c);
-  pdl_wait();
+  pdl_wait(x, slots);
   float* st = state + (size_t)slots[s] * 3 * channels + c;
   v[3] = *reinterpret_cast<const float4*>(x + (size_t)s * x_ld + c);
 #pragma unroll
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(256) short_conv_step_kernel(float* __restrict_
 __global__ void short_conv_state_kernel(float* __restrict__ state, const float* __restrict__ x, long long x_ld,
                                         const int* __restrict__ cu_tokens, const int* __restrict__ slots, int channels, int taps) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, cu_tokens, slots);
   const int s = blockIdx.x;
   const int first = cu_tokens[s], n = cu_tokens[s + 1] - first;
   float* st = state + (size_t)slots[s] * (taps - 1) * channels;
