@@ -253,6 +253,19 @@ __device__ __forceinline__ float row_factor_warp(const RowScale& rs, int m, int 
   return rsqrtf(warp_sum(part) * rs.inv_width + rs.eps);
 }
 
+// The same by eight neighbouring lanes: lane `sub` adds every eighth tile, then the eight add up in a fixed pattern; 0 for a row behind the last.
+__device__ __forceinline__ float row_factor_eight(const RowScale& rs, int m, int M, int sub) {
+  float part = 0.f;
+  if (m < M) {
+    const float* src = rs.sumsq + (size_t)m * rs.tiles;
+    for (int i = sub; i < rs.tiles; i += 8) part += __ldcg(src + i);
+  }
+  part += __shfl_xor_sync(0xffffffffu, part, 4);
+  part += __shfl_xor_sync(0xffffffffu, part, 2);
+  part += __shfl_xor_sync(0xffffffffu, part, 1);
+  return m < M ? rsqrtf(part * rs.inv_width + rs.eps) : 0.f;
+}
+
 struct GemmParams {
   HeadEpilogue he = {};   // off unless a caller fills it in
   AddNormEpilogue an = {};
@@ -274,6 +287,9 @@ struct GemmParams {
   const int* tile_group = nullptr;   // many-token kernel only: w holds several matrices of N rows one below the other, and token
                                      // tile i (128 tokens) is multiplied with matrix tile_group[i] (tokens sorted into runs by
                                      // group, each run padded to whole tiles: the experts of a routed feed-forward)
+  int chains = 0;       // > 0: sums and rows' factors as a launch of gemm_tcgen05_kernel with that many splits forms them, K in as many
+                        // ranges, summed one behind the other in columns of their own and added in their order; with tokens on the
+                        // lanes not for the gated product
   unsigned long long wait_cycles = WAIT_CYCLES;   // after this many clock cycles a wait on a barrier gives up
   int skip_loads = 0;   // tests of the give-up path only: the producer requests nothing, so the first wait runs out
 };
@@ -295,8 +311,9 @@ __device__ __forceinline__ float gated_mul(int act, float limit, float g, float 
   return silu_mul(g, u);
 }
 
+// Up to 32 tokens: two sums of the tile (GemmParams::chains).
 template <int BT>
-__host__ __device__ constexpr int tmem_cols() { return BT < 32 ? 32 : BT; }
+__host__ __device__ constexpr int tmem_cols() { return BT <= 32 ? 2 * BT : BT; }
 
 template <int BT, int STAGES>
 struct SmemLayout {
@@ -393,19 +410,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc(BT);
       bool ok = true;
-      for (int i = 0; i < num_kb && ok; ++i) {
-        const int s = i % STAGES;
-        ok = mbar_wait(full_bar(s), (i / STAGES) & 1, abort_flag, ERR_FULL_WAIT, p.wait_cycles);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a_addr = smem_base + s * L::STAGE_BYTES;
-        const uint64_t a_desc = umma_desc(a_addr), b_desc = umma_desc(a_addr + L::W_BYTES);
+      for (int chain = p.chains == 2 ? 0 : 1, i = 0; ok && chain < 2; ++chain) {
+        const uint32_t acc = p.chains == 2 ? tmem_acc + chain * BT : tmem_acc;
+        const int begin = i, end = chain == 0 ? num_kb / 2 : num_kb;
+        for (; i < end; ++i) {
+          const int s = i % STAGES;
+          ok = mbar_wait(full_bar(s), (i / STAGES) & 1, abort_flag, ERR_FULL_WAIT, p.wait_cycles);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a_addr = smem_base + s * L::STAGE_BYTES;
+          const uint64_t a_desc = umma_desc(a_addr), b_desc = umma_desc(a_addr + L::W_BYTES);
 #pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k) {
-          // 16 bfloat16 = 32 bytes further along k inside the swizzled row: +2 in the address field
-          umma_f16(tmem_acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (i | k) != 0);
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            // 16 bfloat16 = 32 bytes further along k inside the swizzled row: +2 in the address field
+            umma_f16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, ((i - begin) | k) != 0);
+          }
+          umma_commit(empty_bar(s));
         }
-        umma_commit(empty_bar(s));
       }
       if (ok) umma_commit(accum_bar);
     }
@@ -445,7 +466,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       float* part = (direct || via_cluster) ? nullptr : p.workspace + (size_t)split * p.M * p.N;
       float* part_smem = reinterpret_cast<float*>(smem);          // [BT][128]; the stages are drained by now
       float* row_f = part_smem + BT * BM;                         // the rows' norm factors, when the input lacks them
-      if (p.rs.on && direct) {
+      if (p.rs.on && direct && p.chains > 1) {
+        // As where the splits of a cluster are added up, so that the sums are the same either way.
+        pdl_wait();
+        if (p.swiglu) {
+          const int j = threadIdx.x - 64;
+          if (j < BT) row_f[j] = m0 + j < p.M ? row_factor(p.rs, m0 + j) : 0.f;
+        } else {
+          for (int j = quarter; j < BT && m0 + j < p.M; j += 4) {
+            const float f = row_factor_warp(p.rs, m0 + j, lane);
+            if (lane == 0) row_f[j] = f;
+          }
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+      } else if (p.rs.on && direct) {
         // Eight threads a token, each adds every eighth block of the row (its loads are in flight together), then the
         // eight add up in a fixed pattern: one round trip to the L2 for 16 tokens.  (Waiting for the kernel before this
         // one any earlier, while the main loop runs, made the step slower, not faster: see the residual-add epilogue.)
@@ -453,15 +487,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const int t = threadIdx.x - 64, sub = t & 7;
         for (int jb = 0; jb < BT && m0 + jb < p.M; jb += 16) {
           const int j = jb + (t >> 3);
-          float part_sum = 0.f;
-          if (m0 + j < p.M) {
-            const float* src = p.rs.sumsq + (size_t)(m0 + j) * p.rs.tiles;
-            for (int i = sub; i < p.rs.tiles; i += 8) part_sum += __ldcg(src + i);
-          }
-          part_sum += __shfl_xor_sync(0xffffffffu, part_sum, 4);
-          part_sum += __shfl_xor_sync(0xffffffffu, part_sum, 2);
-          part_sum += __shfl_xor_sync(0xffffffffu, part_sum, 1);
-          if (sub == 0 && j < BT) row_f[j] = m0 + j < p.M ? rsqrtf(part_sum * p.rs.inv_width + p.rs.eps) : 0.f;
+          const float f = row_factor_eight(p.rs, m0 + j, p.M, sub);
+          if (sub == 0 && j < BT) row_f[j] = f;
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
       }
@@ -469,7 +496,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       for (int c = 0; c < BT; c += 16) {
         uint32_t r[16];
         tmem_ld16(taddr + c, r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (p.chains > 1) {
+          uint32_t r2[16];
+          tmem_ld16(taddr + BT + c, r2);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+        } else {
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        }
         if (via_cluster) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) part_smem[(c + j) * BM + quarter * 32 + lane] = __uint_as_float(r[j]);
@@ -1028,6 +1063,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
       bool ok = true;
       int s = 0;
       uint32_t turn = 0;
+      const int chains = !PAIR && p.chains > 1 ? p.chains : 1;
       for (int t = 0; t < my_tiles && ok; ++t) {
         const int b = t & 1;
         int m0, n0, bn;
@@ -1037,27 +1073,30 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
         ok = mbar_wait(acc_empty(b), (uint32_t)((t >> 1) & 1) ^ 1u, abort_flag, ERR_ACCUM_WAIT);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t acc = tmem_base + (uint32_t)b * PF_BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          ok = mbar_wait(full_bar(s), turn, abort_flag, ERR_FULL_WAIT);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_addr = smem_base + s * stage;
-          const uint64_t a_desc = umma_desc(a_addr), b_desc = umma_desc(a_addr + L::A_BYTES);
+        uint32_t acc = tmem_base + (uint32_t)b * PF_BN;
+        for (int chain = 1, kb = 0; ok && chain <= chains; ++chain, acc += bn) {
+          const int begin = kb, end = chain == chains ? num_kb : num_kb * chain / chains;
+          for (; kb < end; ++kb) {
+            ok = mbar_wait(full_bar(s), turn, abort_flag, ERR_FULL_WAIT);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a_addr = smem_base + s * stage;
+            const uint64_t a_desc = umma_desc(a_addr), b_desc = umma_desc(a_addr + L::A_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            if (PAIR) umma_f16_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
-            else umma_f16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              if (PAIR) umma_f16_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, ((kb - begin) | k) != 0);
+              else umma_f16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, ((kb - begin) | k) != 0);
+            }
+            if (PAIR) umma_commit_pair(empty_bar(s)); else umma_commit(empty_bar(s));
+            if (++s == stages) { s = 0; turn ^= 1; }
           }
-          if (PAIR) umma_commit_pair(empty_bar(s)); else umma_commit(empty_bar(s));
-          if (++s == stages) { s = 0; turn ^= 1; }
         }
         if (ok) { if (PAIR) umma_commit_pair(acc_full(b)); else umma_commit(acc_full(b)); }
       }
     }
   } else {
     // ---- epilogue: warp w reads lanes (w % 4) * 32 .. + 31, i.e. 32 tokens, 16 features at a time -------------
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, chains = p.chains > 1 ? p.chains : 1;
     bool ok = true;
     for (int t = 0; t < my_tiles && ok; ++t) {
       int m0, n0, bn;
@@ -1073,7 +1112,21 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
       float rf = 1.f;
       if (p.rs.on) {
         pdl_wait();
-        rf = m < p.M ? row_factor(p.rs, m) : 0.f;
+        const int first = m0 + quarter * 32;
+        if (!PAIR && p.chains > 1) {          // where the splits of a cluster are added up: a warp a token
+          for (int i = 0; i < 32 && first + i < p.M; ++i) {
+            const float f = row_factor_warp(p.rs, first + i, lane);
+            if (lane == i) rf = f;
+          }
+        } else if (!PAIR && p.chains == 1) {  // in one split: eight threads a token
+          for (int i = 0; i < 32 && first + i < p.M; i += 4) {
+            const float f = row_factor_eight(p.rs, first + i + (lane >> 3), p.M, lane & 7);
+            const float mine = __shfl_sync(0xffffffffu, f, (lane & 3) * 8);
+            if (lane >> 2 == i >> 2) rf = mine;
+          }
+        } else {
+          rf = m < p.M ? row_factor(p.rs, m) : 0.f;
+        }
       }
       if (p.an.on) {
         // The residual add and the first half of the norm that follows (AddNormEpilogue): this thread holds one token's
@@ -1194,7 +1247,24 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
       for (int c = 0; c < bn; c += 16) {
         uint32_t r[16];
         tmem_ld16(taddr + c, r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (PAIR || chains == 1) {
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        } else {
+          uint32_t more[4][16];                                  // four sums on their way at a time, added one by one
+#pragma unroll 1
+          for (int z = 0; z < chains; z += 4) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (z + i > 0 && z + i < chains) tmem_ld16(taddr + (z + i) * bn + c, more[i]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (z + i > 0 && z + i < chains) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(more[i][j]));
+              }
+          }
+        }
         const int n = n0 + c;
         if (p.rs.on) {
 #pragma unroll
@@ -1385,13 +1455,23 @@ static int prefill_feature_tiles(const PrefillPlan& plan, int N) {
   return plan.cols1 + (rest > 0 ? (rest + plan.bn2 - 1) / plan.bn2 : 0);
 }
 
+// What launch_prefill returns, and nothing is launched, where the tiles of its plan leave no room for that many sums in tensor memory.
+constexpr int PREFILL_CHAINS = -1;
+
 static int launch_prefill(const void* y, int y_dtype, const void* x, const void* w, int M, int N, int K, long long ldx,
                           long long ldy, int swiglu, int force_bn, int pair, cudaStream_t stream,
                           const AddNormEpilogue* an = nullptr, const RowScale* rs = nullptr, float act_limit = 0.f,
-                          const int* tile_group = nullptr, int groups = 1, int post = POST_NONE, float post_c = 0.f) {
+                          const int* tile_group = nullptr, int groups = 1, int post = POST_NONE, float post_c = 0.f, int chains = 0) {
   bool use_pair; int m_tiles, slots; PrefillPlan plan;
   if (tile_group) pair = 1;               // a group's run of tokens is padded to tiles of 128, not to pairs of them
+  if (chains > 0 && rs) pair = 1;         // pairs add the rows' factors in another order
   prefill_choose(M, N, K, swiglu, force_bn, pair, &use_pair, &m_tiles, &slots, &plan);
+  if (chains > 1) {
+    // the sums of a tile side by side: in one of the two accumulators, or in both where a CTA has one tile
+    const int widest = plan.cols1 > 0 && plan.bn1 > plan.bn2 ? plan.bn1 : plan.bn2;
+    const bool one_tile = (long long)m_tiles * prefill_feature_tiles(plan, N) <= slots;
+    if (use_pair || swiglu || an || chains * widest > (one_tile ? 2 : 1) * PF_BN) return PREFILL_CHAINS;
+  }
   if (use_pair && (plan.bn1 % 32 || plan.bn2 % 32)) { set_error("gemm_tcgen05: pairs of CTAs take tile widths that are multiples of 32"); return 1; }
   const int box1 = use_pair ? plan.bn1 / 2 : plan.bn1, box2 = use_pair ? plan.bn2 / 2 : plan.bn2;
   CUtensorMap mx, mw, mw2;
@@ -1403,7 +1483,7 @@ static int launch_prefill(const void* y, int y_dtype, const void* x, const void*
   GemmParams p;
   p.y = const_cast<void*>(y); p.workspace = nullptr; p.counters = nullptr; p.M = M; p.N = N; p.K = K; p.ldy = ldy;
   p.out_dtype = y_dtype; p.cluster = 0; p.swiglu = swiglu; p.act_limit = act_limit; p.tile_group = tile_group;
-  p.post = post; p.post_c = post_c;
+  p.post = post; p.post_c = post_c; p.chains = chains;
   if (an) {
     p.an = *an; p.an.on = 1;
     if (p.an.tiles != prefill_feature_tiles(plan, N)) { set_error("gemm_tcgen05: %d columns of partial sums, the plan has %d feature tiles", p.an.tiles, prefill_feature_tiles(plan, N)); return 1; }
@@ -1540,18 +1620,22 @@ LB_EXPORT int lb_gemm_tcgen05(void* y, int y_dtype, const void* x, const void* w
   LB_CHECK_ARG(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0), "gemm_tcgen05: operands must be 16-byte aligned");
   if (M == 0) return 0;
   // Which kernel: above 256 tokens the one with tokens on the lanes.  Below, it still wins where the product has many features for its
-  // inner size, so that its tiles fill the SMs without any cut along K, the more tokens the sooner: from as many features as places
-  // on with 65 tokens, three for two places with 33, half as many with 129.  us, the kernel that cuts K over a cluster | here: 64 tokens,
-  // 3072 features of 2048 places 8.4 | 8.0, 8192 of 4096 18.8 | 16.5, 4096 of 4096 11.7 | 13.9; 128 tokens, 2048 of 2048 11.4 | 7.9, 12288 of 4096
-  // 38.2 | 22.9, 4096 of 4096 15.4 | 14.5, 2048 of 4096 10.2 | 12.7; 256 tokens, 4096 of 4096 21.3 | 15.2, 2048 of 4096 14.1 | 13.1, of 6144 16.4 | 18.4.
-  // The gated product from 65 tokens on (24576 of 4096, 64 tokens 40.8 | 47.0, 128 48.5 | 47.4).  Sums that stay 32-bit numbers (what a
-  // recurrence reads) keep their cut along K up to 128 tokens, and to 256 unless there are more features than places: the accumulator drops
-  // what lies below its sums at every 16 places, so that one chain over 4096 places is 1.5 to 2 times as far from 64 bits as the sum
-  // of a cluster's shorter ones, which 16-bit outputs don't show.  force_bt < 0 asks for the kernel with tokens on the lanes at
-  // any size; force_bt > 0 or a given split count for the other one.
-  const bool wide = y_dtype == LB_F32 ? M > 128 && N > K : M > 128 ? 2ll * N >= K : M > 64 ? N >= K : M > 32 && 2ll * N >= 3ll * K;
-  const bool many = M > 256 ? force_bt <= 0 : force_bt < 0 || (force_bt == 0 && force_splits == 0 && (swiglu ? M > 64 : wide));
-  if (many) {
+  // inner size, so that its tiles fill the SMs, the more tokens the sooner.  The accumulator drops what lies below its sums at every 16 places:
+  // one chain over 4096 places is 1.5 to 2 times as far from 64 bits as the sum of a cluster's shorter ones.  So a product of up to 256
+  // tokens that a cluster would cut keeps the cut (`chains`: the same sums, added in the same order, the same bits), but for the gated
+  // one and that of more features than places from 129 tokens on, which have always been one chain.  Every further sum of a tile is read out of
+  // tensor memory for 0.25 us, so the lines ask for fewer of them or for more features.  us, the kernel that cuts K over a cluster | here:
+  //   64 tokens   2048 x 1024, 4 splits 8.2 | 5.8, 3072 x 2048, 8 8.1 | 9.7, 8192 x 4096, 4 20.1 | 18.0, 6144 x 4096, 5 15.5 | 16.8
+  //   128 tokens  2048 x 2048, 8 8.4 | 9.6, 2560 x 2048, 8 10.6 | 9.7, 4096 x 4096, 8 14.8 | 15.3, 6144 x 6144, 5 24.3 | 23.0, 12288 x 4096, 2 40.5 | 25.6
+  //   256 tokens  2048 x 4096, 8 13.8 | 14.3, 3072 x 4096, 5 17.6 | 15.1, 2048 x 2048, 8 11.6 | 9.7, 4096 x 4096, 4 20.8 | 15.4, 4608 x 6144, 3 30.7 | 21.4
+  // The gated product from 65 tokens on (24576 of 4096, 64 tokens 40.8 | 47.0, 128 48.5 | 47.4).  32-bit outputs stay with the cluster's
+  // kernel: the lines were measured for 16-bit ones.  force_bt < 0 asks for the kernel with tokens on the lanes, K in one
+  // chain, at any size; force_bt > 0 or a given split count for the other one.
+  const bool whole = M > 256 ? force_bt <= 0 : force_bt < 0 || (force_bt == 0 && force_splits == 0 && (swiglu ? M > 64 : M > 128 && N > K));
+  const int chains = M > 32 && M <= 256 ? lb_gemm_tcgen05_plan(M, N, K, nullptr) : 0;
+  const bool cut = !whole && chains > 0 && force_bt == 0 && force_splits == 0 && !swiglu && y_dtype != LB_F32 &&
+                   (M > 128 ? 2ll * N >= K && (4ll * N >= 3ll * K || chains <= 5) : M > 64 ? N >= K && (4ll * N >= 5ll * K || chains <= 5) : 2ll * N >= 3ll * K && chains <= 4);
+  if (whole || cut) {
     // force_bt: 0 chooses between one CTA a tile of 128 tokens and a pair of CTAs a tile of 256, -1 asks for the former,
     // -2 for the latter
     // with many tokens force_splits stands for the feature width of the tiles (0: choose; -(c * 1024 + w): c columns of
@@ -1560,9 +1644,13 @@ LB_EXPORT int lb_gemm_tcgen05(void* y, int y_dtype, const void* x, const void* w
     LB_CHECK_ARG(force_splits == 0 || (fw >= 16 && fw <= lb::PF_BN && fw % 16 == 0 && (!swiglu || fw % 128 == 0)),
                  "gemm_tcgen05: tile width %d is no multiple of 16 (128 with SwiGLU) up to 256", fw);
     LB_CHECK_ARG(force_bt >= -2, "gemm_tcgen05: token tile %d is not one of 16, 32, 64, 128, 256", force_bt);
-    if (int rc = lb::launch_prefill(y, y_dtype, x, w, M, N, K, ldx, ldy, swiglu, force_splits, -force_bt, stream, nullptr, row_scale, act_limit, nullptr, 1, post, post_c)) return rc;
-    LB_CHECK_LAUNCH("gemm_tcgen05 (many tokens)");
-    return 0;
+    const int rc = lb::launch_prefill(y, y_dtype, x, w, M, N, K, ldx, ldy, swiglu, force_splits, -force_bt, stream, nullptr, row_scale, act_limit, nullptr, 1,
+                                      post, post_c, cut ? chains : 0);
+    if (rc == 0) {
+      LB_CHECK_LAUNCH("gemm_tcgen05 (many tokens)");
+      return 0;
+    }
+    if (rc != lb::PREFILL_CHAINS) return rc;
   }
   // A router's product: 16 tokens of 128 features are 256 CTAs, which still run at once.  One launch behind the other, us, with the
   // pipeline / here: 16 features of 2048, 1 token 3.7 / 1.7, 16 tokens 4.0 / 1.9; 128 features of 4096, 1 token 4.9 / 2.7, 16 tokens
@@ -1577,8 +1665,15 @@ LB_EXPORT int lb_gemm_tcgen05(void* y, int y_dtype, const void* x, const void* w
   int bt = 16;
   int splits = lb_gemm_tcgen05_plan(M, N, K, &bt);
   // A short product whose tiles fill more than half of the SMs gains less from two splits, of which some SMs hold two, than their
-  // reduction costs: 12288 features, 8 tokens, of 2048 places 13.5 -> 11.8 us; of 4096, 21.7 | 21.9.  32-bit outputs keep the shorter chains.
-  if (y_dtype != LB_F32 && splits == 2 && M <= 32 && K < 3072 && (N + lb::BM - 1) / lb::BM * 2 > 148) splits = 1;
+  // reduction costs; one CTA then forms both splits' sums.  12288 features, us, two CTAs | one: 8 tokens of 1024 places 8.6 | 8.3, of 2048 13.8 | 12.7,
+  // of 2560 15.6 | 15.0, of 3008 17.7 | 17.4, of 3584 21.0 | 21.0, of 4096 23.0 | 23.5; one token, gated, of 2048 12.1 | 11.5, of 2560 13.6 | 13.9, not gated,
+  // of 1024 6.9 | 7.5, of 2048 11.9 | 12.1, of 3008 15.7 | 16.9 (16384 and 18816 features alike).
+  int sums = 0;
+  if (y_dtype != LB_F32 && force_bt == 0 && force_splits == 0 && splits == 2 && M <= 32 && (M >= 8 ? K < 3072 : swiglu && K <= 2048) &&
+      (N + lb::BM - 1) / lb::BM * 2 > 148) {
+    splits = 1;
+    sums = 2;
+  }
   if (force_bt) {
     LB_CHECK_ARG(force_bt == 16 || force_bt == 32 || force_bt == 64 || force_bt == 128 || force_bt == 256,
                  "gemm_tcgen05: token tile %d is not one of 16, 32, 64, 128, 256", force_bt);
@@ -1607,7 +1702,7 @@ LB_EXPORT int lb_gemm_tcgen05(void* y, int y_dtype, const void* x, const void* w
   // Clusters when the split count allows it and the caller did not ask for the workspace path
   // (force_splits < 0 asks for -force_splits splits through the workspace).
   p.cluster = (!workspace_path && splits > 1 && splits <= 8) ? splits : 0;
-  p.swiglu = swiglu; p.act_limit = act_limit; p.post = post; p.post_c = post_c;
+  p.swiglu = swiglu; p.act_limit = act_limit; p.post = post; p.post_c = post_c; p.chains = sums;
   LB_CHECK_ARG(!row_scale || splits == 1 || p.cluster > 0,
                "gemm_tcgen05: a row scale is not taken by a product that is split through the workspace (M=%d, %d splits)", M, splits);
   if (row_scale) { p.rs = *row_scale; p.rs.on = 1; }

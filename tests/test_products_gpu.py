@@ -50,10 +50,54 @@ def test_32_bit_sums_in_short_chains(M, N, K):
         assert off() <= 1.25 * off(force_bt=128 if M > 64 else 64)
 
 
-@pytest.mark.parametrize("M", [1, 8, 32])
-@pytest.mark.parametrize("N,K", [(9472, 256), (9600, 256), (9601, 2048), (9600, 3072)])
-def test_few_tokens_of_many_features(M, N, K):
-    check(M, N, K, torch.float32, N, 0)
+def plan(M, N, K):
+    """(splits, token tile) of the kernel that cuts K over a cluster."""
+    import ctypes
+    from lucciola_b200.csrc import library
+    bt = ctypes.c_int()
+    f = library().lb_gemm_tcgen05_plan
+    f.argtypes, f.restype = [ctypes.c_int] * 3 + [ctypes.c_void_p], ctypes.c_int
+    return f(M, N, K, ctypes.addressof(bt)), bt.value
+
+
+def as_the_cluster_adds(M, N, K, dtype, swiglu=False):
+    """Whichever kernel takes it: the bits of the kernel that cuts K over a cluster, as many ranges as it takes by itself, with rows that lack
+    their norm's factor (17 partial sums a row: more than one round of the loads that add them up), and without, and with an element operation."""
+    from lucciola_b200 import ops
+    torch.manual_seed(M + N + K)
+    x, w, s = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16(), torch.cuda.current_stream().cuda_stream
+    splits, bt = plan(M, N, K)
+    sumsq = K / 17 * (0.5 + torch.rand(M, 17, device=DEV))
+    for kw in (dict(), dict(sumsq=sumsq, eps=1e-6)) + (() if swiglu else (dict(post="gelu"),)):
+        got, want = (torch.empty(M, N // 2 if swiglu else N, device=DEV, dtype=dtype) for _ in range(2))
+        ops.gemm_tcgen05(got, x, w, s, swiglu=swiglu, **kw)
+        ops.gemm_tcgen05(want, x, w, s, swiglu=swiglu, force_bt=bt, force_splits=splits, **kw)
+        assert torch.equal(got, want), kw
+    assert ops.device_error() == 0
+    return splits
+
+
+# features and places, and the splits of 33 to 128 | 129 to 256 tokens, on both sides of the lines; widths that are no multiple of a tile, and sums
+# that fill tensor memory (eight of 64 columns)
+@pytest.mark.parametrize("M", [33, 64, 65, 93, 128, 129, 200, 256])
+@pytest.mark.parametrize("N,K,splits", [(4096, 2048, (8, 4)), (2048, 2048, (8, 8)), (2600, 2056, (8, 6)), (3000, 4104, (8, 5)), (4800, 3200, (6, 3)), (6144, 4096, (5, 2)),
+                                        (8192, 4096, (4, 2)), (4100, 4104, (7, 3)), (1000, 2000, (8, 8)), (12288, 4096, (2, 1)), (17000, 2048, (2, 1)), (600, 384, (1, 1)),
+                                        (1600, 1032, (4, 4))])
+def test_16_bit_sums_keep_the_cut(M, N, K, splits):
+    if M > 128 and N > K:
+        pytest.skip("one chain")
+    assert as_the_cluster_adds(M, N, K, torch.bfloat16) == splits[M > 128]
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 16, 17, 32])
+@pytest.mark.parametrize("N,K", [(12288, 2048), (12289, 512), (12288, 2056), (16384, 3064), (16384, 3072), (18816, 1024)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_few_tokens_of_many_features(M, N, K, dtype):
+    """Two splits, by two CTAs or, on the one side of the lines in tokens, places and types, by one."""
+    assert as_the_cluster_adds(M, N, K, dtype) == 2
+    check(M, N, K, dtype, N, 0)
+    if N % 128 == 0:
+        assert as_the_cluster_adds(M, N, K, dtype, swiglu=True) == 2
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
