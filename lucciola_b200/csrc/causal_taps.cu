@@ -18,7 +18,7 @@ __global__ void causal_taps_kernel(T* __restrict__ out, const T* __restrict__ h,
                                    const T* __restrict__ state, const int* __restrict__ token_seq,
                                    const int* __restrict__ cu_tokens, const int* __restrict__ slots, int width, int taps) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(h, state, token_seq, cu_tokens, slots);
   const int t = blockIdx.x;
   const int s = token_seq[t];
   const int idx = t - cu_tokens[s];                       // place of the token in its portion
@@ -43,7 +43,7 @@ __global__ void causal_taps_bf16x8_kernel(bf16* __restrict__ out, const bf16* __
                                           const bf16* __restrict__ state, const int* __restrict__ token_seq,
                                           const int* __restrict__ cu_tokens, const int* __restrict__ slots, int width, int taps) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(h, state, token_seq, cu_tokens, slots);
   const int t = blockIdx.x;
   const int s = token_seq[t];
   const int idx = t - cu_tokens[s];
@@ -80,7 +80,7 @@ template <typename T>
 __global__ void causal_taps_state_kernel(T* __restrict__ state, const T* __restrict__ h, const int* __restrict__ cu_tokens,
                                          const int* __restrict__ slots, int width, int taps) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(h, cu_tokens, slots);
   const int s = blockIdx.x;
   const int first = cu_tokens[s], n = cu_tokens[s + 1] - first;
   T* st = state + (size_t)slots[s] * (taps - 1) * width;

@@ -328,7 +328,7 @@ __global__ void rmsnorm_gated_kernel(TO* __restrict__ out, long long out_ld, con
                                      float scale, float eps, int n, int planes, long long plane) {
   __shared__ float scratch[33];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, gate);
   const float* r = x + (size_t)blockIdx.x * n;
   const float* g = gate + (size_t)blockIdx.x * gate_ld;
   auto value = [&](int j) {
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_gated_x4_kernel(TO* __restrict__
                                                                 float scale, float eps, int n, int planes, long long plane) {
   __shared__ float scratch[33];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, gate);
   const float* r = x + (size_t)blockIdx.x * n;
   const float* g = gate + (size_t)blockIdx.x * gate_ld;
   float4 v[NV], z[NV];
@@ -394,7 +394,7 @@ template <typename T>
 __global__ void head_gate_kernel(T* __restrict__ out, long long out_ld, const T* __restrict__ x, const float* __restrict__ gate,
                                  long long gate_ld, float scale, int heads, int vdim) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, gate);
   const int t = blockIdx.x, n = heads * vdim;
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
     const float g = gate[(size_t)t * gate_ld + j / vdim];

@@ -24,7 +24,7 @@ __global__ void embedding_kernel(float* __restrict__ out, const int* __restrict_
                                  const TW* __restrict__ pos_table, const int* __restrict__ positions, int max_positions,
                                  float scale, void* __restrict__ out2, int out2_dtype) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(ids, positions);
   const int t = blockIdx.x;
   int id = ids[t];
   if (id < 0 || id >= vocab) id = 0;
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256) embedding_x4_kernel(float* __restrict__ o
                                                            int hidden, int vocab, float scale) {
   pdl_trigger();
   const int t = blockIdx.x, i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
-  pdl_wait();
+  pdl_wait(ids);
   if (i >= hidden) return;
   int id = ids[t];
   if (id < 0 || id >= vocab) id = 0;
@@ -83,7 +83,7 @@ __global__ void embedding_sinusoid_kernel(float* __restrict__ out, const int* __
                                           int hidden, int vocab, const double* __restrict__ sin_freq,
                                           const int* __restrict__ positions) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(ids, positions);
   const int t = blockIdx.x;
   int id = ids[t];
   if (id < 0 || id >= vocab) id = 0;

@@ -38,7 +38,7 @@ __global__ void route_topk_kernel(int* __restrict__ ids, float* __restrict__ wei
                                   int groups, int keep, float scale, int softmax) {
   extern __shared__ float smem[];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(logits);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int t = blockIdx.x * nwarps + warp;
   if (t >= num_tokens) return;
@@ -117,7 +117,7 @@ __global__ void expert_dispatch_kernel(const int* __restrict__ ids, const int* _
                                        int* __restrict__ place_of, int* __restrict__ meta) {
   extern __shared__ int ism[];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(ids, tokens);
   int* count = ism;                 // [experts]
   int* start = ism + experts;       // [experts + 1]
   int* tile0 = start + experts + 1; // [experts + 1]
@@ -159,7 +159,7 @@ __global__ void expert_dispatch_padded_kernel(const int* __restrict__ ids, const
                                               int* __restrict__ pair_at, int* __restrict__ place_of, int* __restrict__ tile_group) {
   extern __shared__ int ism[];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(ids, tokens);
   int* count = ism;                 // [experts]
   int* start = ism + experts;       // [experts + 1]
   for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
@@ -187,7 +187,7 @@ __global__ void expert_dispatch_padded_kernel(const int* __restrict__ ids, const
 __global__ void expert_gather_rows_kernel(uint4* __restrict__ xs, const uint4* __restrict__ x, const int* __restrict__ pair_at,
                                           int top, int row_words) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, pair_at);
   const int place = blockIdx.x, pair = pair_at[place];
   uint4* dst = xs + (size_t)place * row_words;
   if (pair < 0) {
@@ -589,7 +589,7 @@ __global__ void expert_combine_kernel(TO* __restrict__ out, const float* __restr
                                       int x_bf16, const float* __restrict__ gate, int top, int width) {
   __shared__ float scratch[33];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(y, weights, place_of, always, x, gate);
   const int t = blockIdx.x;
   float g = 1.f;
   if (gate) {
@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(256) expert_combine_x4_kernel(TO* __restrict__
                                                                 int width) {
   pdl_trigger();
   const int t = blockIdx.x, j = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
-  pdl_wait();
+  pdl_wait(y, weights, place_of, always);
   if (j >= width) return;
   int places[8];
   float w[8];

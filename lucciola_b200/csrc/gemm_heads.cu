@@ -23,7 +23,7 @@ gemm_heads_mma_kernel(bf16* __restrict__ y, const bf16* __restrict__ x, const bf
   __shared__ __align__(16) bf16 As[GH_BM][GH_LD];
   __shared__ __align__(16) bf16 Bs[GH_BN][GH_LD];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, gate);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
   const int m0 = blockIdx.y * GH_BM, n0 = blockIdx.x * GH_BN, b = blockIdx.z;
@@ -124,7 +124,7 @@ gemm_heads_few_kernel(bf16* __restrict__ y, const bf16* __restrict__ x, const bf
     r += dr; at += dat;
     if (at >= pieces) { at -= pieces; ++r; }
   }
-  pdl_wait();
+  pdl_wait(x, gate);
   for (int r = r0, at = at0; r < 16 * MT;) {
     const int c = at * 8;
     const bool ok = m0 + r < M && c < K;

@@ -29,7 +29,7 @@ gemm_plain_kernel(TY* __restrict__ y, const TX* __restrict__ x, const TW* __rest
   __shared__ float xs[PG_BK][PG_BM + 4];
   __shared__ float ws[PG_BK][PG_BN + 4];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, gate);
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * PG_BM, n0 = blockIdx.x * PG_BN;
   x += (size_t)blockIdx.z * bx; w += (size_t)blockIdx.z * bw; y += (size_t)blockIdx.z * by;

@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(FF_THREADS) gemm_few_features_kernel(void* __r
   uint4 first[FF_AHEAD];
 #pragma unroll
   for (int i = 0; i < FF_AHEAD; ++i) first[i] = tid + i * FF_THREADS < words ? wr[tid + i * FF_THREADS] : zero;
-  pdl_wait();
+  pdl_wait(x);
   float acc[FF_TOKENS] = {};
   auto add = [&](uint4 ww, int at) {
     uint4 v[FF_TOKENS];

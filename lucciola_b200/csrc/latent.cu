@@ -17,7 +17,7 @@ __global__ void latent_norm_kernel(const float* __restrict__ pre, long long ld, 
                                    int page_size, int max_pages, float eps) {
   __shared__ float scratch[33];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(pre, positions, token_seq, block_table);
   const int t = blockIdx.x;
   const bool is_q = blockIdx.y == 0;
   const int n = is_q ? q_rank : kv_rank;

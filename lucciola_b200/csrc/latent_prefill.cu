@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(uint4* __restrict__ 
   const int j = row - en.y;
   int page = -1;
   if (row < total_rows && e < num_entries && j < context_lens[en.x]) page = block_table[(size_t)en.x * max_pages + j / page_size];
-  pdl_wait();
+  pdl_wait(pool);                                // the entries and tables were written before the step began
   if (row >= total_rows) return;
   const uint4* src = page >= 0 ? pool + ((size_t)page * page_size + j % page_size) * words : nullptr;
   for (int i = lane; i < words; i += 32) out[(size_t)row * words + i] = src ? src[i] : make_uint4(0u, 0u, 0u, 0u);

@@ -18,7 +18,7 @@ __global__ void layernorm_kernel(TO* __restrict__ out, const float* __restrict__
                                  const int* __restrict__ rows, int hidden, float eps) {
   __shared__ float scratch[33];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x, rows);
   const int i = blockIdx.x;
   const float* r = x + (size_t)(rows ? rows[i] : i) * hidden;
   float s = 0.f;
@@ -37,7 +37,7 @@ __global__ void layernorm_add_kernel(float* __restrict__ residual, const TY* __r
                                      TC* __restrict__ copy, int hidden) {
   __shared__ float scratch[33];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(a, b);
   const size_t row = (size_t)blockIdx.x * hidden;
   const TY* ra = a + row;
   const TY* rb = b ? b + row : nullptr;
@@ -59,7 +59,7 @@ __global__ void layernorm_add_kernel(float* __restrict__ residual, const TY* __r
 template <typename TC>
 __global__ void round_copy_kernel(TC* __restrict__ out, const float* __restrict__ x, long long n) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     out[i] = from_f32<TC>(x[i]);
 }

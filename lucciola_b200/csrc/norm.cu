@@ -20,7 +20,7 @@ __global__ void add_rmsnorm_kernel(TO* __restrict__ out, float* __restrict__ res
                                    const int* __restrict__ rows, int hidden, float eps) {
   __shared__ float scratch[33];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(delta, rows);
   const int i = blockIdx.x;
   const int src = rows ? rows[i] : i;
   float* r = residual + (size_t)src * hidden;
@@ -84,7 +84,7 @@ __global__ void add_rmsnorm_row_kernel(TO* __restrict__ out, float* __restrict__
   float4 w[PER / 4], v[PER / 4];
 #pragma unroll
   for (int q = 0; q < PER / 4; ++q) w[q] = load4(weight + 4 * (q * nt + tid));
-  pdl_wait();
+  pdl_wait(delta, rows);
   const int i = blockIdx.x;
   const int src = rows ? rows[i] : i;
   float* r = residual + (size_t)src * hidden;
@@ -118,7 +118,7 @@ template <typename TO>
 __global__ void rmsnorm_short_rows_kernel(TO* __restrict__ out, const float* __restrict__ x, const float* __restrict__ weight,
                                           int num_rows, int hidden, float eps) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x);
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= num_rows) return;
@@ -144,7 +144,7 @@ __global__ void add_group_rmsnorm_kernel(TO* __restrict__ out, float* __restrict
   // (all loads issued before any is used); EPL == 0: any size, the row is read again (from cache) for the output.
   __shared__ float part[32];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(delta_a, delta_b, rows);
   const int i = blockIdx.x;
   const int src = rows ? rows[i] : i;
   float* r = residual + (size_t)src * hidden;
@@ -275,7 +275,7 @@ namespace lb {
 template <typename TD>
 __global__ void add_into_kernel(float* __restrict__ residual, const TD* __restrict__ delta, long long n) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(delta);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     residual[i] += to_f32(delta[i]);
 }
@@ -367,7 +367,7 @@ __global__ void add_rmsnorm_pair_kernel(TO* __restrict__ out_a, TO* __restrict__
                                         const float* __restrict__ w_a, const float* __restrict__ w_b, int hidden, float eps) {
   __shared__ float scratch[33];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(delta_a, delta_b);
   const size_t base = (size_t)blockIdx.x * hidden;
   float ss = 0.f;
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
@@ -391,7 +391,7 @@ __global__ void rmsnorm_mix2_kernel(float* __restrict__ out, const float* __rest
                                     float eps) {
   __shared__ float scratch[33];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(a, b);
   const size_t base = (size_t)blockIdx.x * hidden;
   float ssa = 0.f, ssb = 0.f;
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) {

@@ -46,7 +46,7 @@ __global__ void pool_kv_kernel(const T* __restrict__ k_cache, const T* __restric
                                int pool_max_pages, const int* __restrict__ cu_tokens, const int* __restrict__ context_lens,
                                int num_kv_heads, int d, int dv, int page_size, int P) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(k_cache, v_cache, table, pool_table, cu_tokens, context_lens);
   const int s = blockIdx.y, kvh = blockIdx.z;
   const int ctx = context_lens[s];
   const int start = ctx - (cu_tokens[s + 1] - cu_tokens[s]);

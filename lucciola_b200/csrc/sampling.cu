@@ -40,7 +40,7 @@ __global__ void sample_kernel(int* __restrict__ tokens, const float* __restrict_
   __shared__ float best_v[32];
   __shared__ int best_i[32];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(logits, temperature, keys, counters);
   const int r = blockIdx.x;
   const float* row = logits + (size_t)r * vocab;
   const float temp = temperature ? temperature[r] : 0.f;

@@ -11,7 +11,7 @@ namespace lb {
 __global__ void zero_rows_kernel(unsigned char* __restrict__ base, long long row_bytes,
                                  const int* __restrict__ slots, int num_rows) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(slots);
   const int slot = slots[blockIdx.x];
   if (slot < 0 || slot >= num_rows) return;
   unsigned char* row = base + (size_t)slot * (size_t)row_bytes;

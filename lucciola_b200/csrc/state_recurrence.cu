@@ -296,7 +296,7 @@ __global__ void gated_group_norm_kernel(TO* __restrict__ out, long long out_ld, 
                                         int n, int groups, int gate_first, int act, float eps, float scale, int planes, long long plane) {
   __shared__ float part[8][8];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(y, gate);
   const int t = blockIdx.x, gy = threadIdx.y, g = blockIdx.y * blockDim.y + gy;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int gs = g < groups ? n / groups : 0;      // a group past the last has no columns, but meets the others at the barrier
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_x4_kernel(TO* __restrict
                                                                   long long plane) {
   __shared__ float part[8][8];
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(y, gate);
   const int t = blockIdx.x, gy = threadIdx.y, g = blockIdx.y * blockDim.y + gy;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const bool real = g < groups;                    // a group past the last meets the others at the barrier

@@ -24,7 +24,7 @@ __global__ void swiglu_kernel(T* __restrict__ out, const T* __restrict__ gate,
                               const T* __restrict__ up, long long in_stride, int inter,
                               long long total, int act, float limit) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(gate, up);
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const long long t = idx / inter;
@@ -40,7 +40,7 @@ __global__ void swiglu_bf16x8_kernel(bf16* __restrict__ out, const bf16* __restr
                                      const bf16* __restrict__ up, long long in_stride, int inter,
                                      long long total8, int act, float limit) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(gate, up);
   const int per_row = inter >> 3;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total8;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -106,7 +106,7 @@ template <typename T>
 __global__ void activation_kernel(T* __restrict__ out, const T* __restrict__ x, long long in_stride, int n, long long total,
                                   int act, float p0, float p1) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x);
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
     const long long t = idx / n;
     const int c = (int)(idx - t * n);
@@ -118,7 +118,7 @@ __global__ void activation_kernel(T* __restrict__ out, const T* __restrict__ x, 
 __global__ void activation_bf16x8_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, long long in_stride, int n8,
                                          long long total8, int act, float p0, float p1) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x);
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total8; idx += (long long)gridDim.x * blockDim.x) {
     const long long t = idx / n8;
     const int c = (int)(idx - t * n8) * 8;
@@ -167,7 +167,7 @@ namespace lb {
 template <typename TO>
 __global__ void round_cols_kernel(TO* __restrict__ out, const float* __restrict__ x, long long x_ld, int n, long long total) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(x);
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
     const long long t = idx / n;
     out[idx] = from_f32<TO>(x[t * x_ld + (idx - t * n)]);
