@@ -34,14 +34,15 @@ __device__ __forceinline__ bool ta_mbar_try_wait(uint32_t bar, uint32_t parity) 
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool ta_mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+__device__ __forceinline__ bool ta_mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code,
+                                             unsigned long long limit = TA_WAIT_CYCLES) {
   if (ta_mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   for (unsigned it = 1;; ++it) {
     if (ta_mbar_try_wait(bar, parity)) return true;
     if ((it & 255u) == 0u) {
       if (*abort_flag) return false;
-      if ((unsigned long long)(clock64() - t0) > TA_WAIT_CYCLES) {
+      if ((unsigned long long)(clock64() - t0) > limit) {
         *abort_flag = code;
         atomicCAS(&g_attention_tc_error, 0, code);
         return false;
@@ -51,7 +52,8 @@ __device__ __forceinline__ bool ta_mbar_wait(uint32_t bar, uint32_t parity, vola
 }
 // The same for the single producer and issue threads: they sleep between polls, so that their spinning
 // does not take issue slots from the softmax warps that share their schedulers.
-__device__ __forceinline__ bool ta_mbar_wait_idle(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+__device__ __forceinline__ bool ta_mbar_wait_idle(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code,
+                                                  unsigned long long limit = TA_WAIT_CYCLES) {
   if (ta_mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   for (unsigned it = 1;; ++it) {
@@ -59,13 +61,18 @@ __device__ __forceinline__ bool ta_mbar_wait_idle(uint32_t bar, uint32_t parity,
     if (ta_mbar_try_wait(bar, parity)) return true;
     if ((it & 63u) == 0u) {
       if (*abort_flag) return false;
-      if ((unsigned long long)(clock64() - t0) > TA_WAIT_CYCLES) {
+      if ((unsigned long long)(clock64() - t0) > limit) {
         *abort_flag = code;
         atomicCAS(&g_attention_tc_error, 0, code);
         return false;
       }
     }
   }
+}
+// For a role that gave up: what is in flight gets a while to land before the CTA's memory is given away.
+__device__ __forceinline__ void ta_mbar_drain(uint32_t bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!ta_mbar_try_wait(bar, parity) && (unsigned long long)(clock64() - t0) < TA_WAIT_CYCLES / 8) {}
 }
 __device__ __forceinline__ void ta_tma_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"

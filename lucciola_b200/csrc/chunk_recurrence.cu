@@ -834,15 +834,13 @@ LB_EXPORT long long lb_chunk_recurrence_scratch(int kind, int heads, int dim, in
   return lb::cr_layout(p, kind) * heads;
 }
 
-// The sequences seqs[0 .. num_long - 1] of the step (host array; with seq_tokens[i] tokens each, which must be what cu_tokens
-// says), all their tokens.  `scratch` holds scratch_chunks chunks; more are worked off in turns.  fixed: `decay`; ssm: a, A_log,
-// dt_bias, D; delta: a, b, A_log, dt_bias; hgrn2: k (the gate's input), bias, lower; channels: a (the decays), b.
-LB_EXPORT int lb_chunk_recurrence(int kind, const float* q, long long q_ld, const float* k, long long k_ld, const float* v, long long v_ld,
-                                  const float* a, long long a_ld, const float* b, long long b_ld, const float* A_log, const float* dt_bias,
-                                  const float* D, const float* bias, const float* lower, const float* decay, float* state, float* out,
-                                  long long out_ld, const int* cu_tokens, const int* slots, const int* seqs, const int* seq_tokens,
-                                  int num_long, int heads, int groups, int dim, int vdim, int unit_norm, float q_scale, float unit_eps,
-                                  int act, float* scratch, int scratch_chunks, cudaStream_t stream) {
+namespace lb {
+
+static int run_chunks(int kind, const float* q, long long q_ld, const float* k, long long k_ld, const float* v, long long v_ld, const float* a,
+                      long long a_ld, const float* b, long long b_ld, const float* A_log, const float* dt_bias, const float* D, const float* bias,
+                      const float* lower, const float* decay, float* state, float* out, long long out_ld, const int* cu_tokens, const int* slots,
+                      const int* seqs, const int* seq_tokens, int num_long, int heads, int groups, int dim, int vdim, int unit_norm, float q_scale,
+                      float unit_eps, int act, float* scratch, int scratch_chunks, cudaStream_t stream, int hold, unsigned long long wait_cycles) {
   LB_CHECK_ARG(lb_chunk_recurrence_scratch(kind, heads, dim, vdim) > 0, "chunk_recurrence: kind %d with %d heads of %d x %d", kind, heads, dim, vdim);
   LB_CHECK_ARG(q && k && v && state && out && cu_tokens && slots && seqs && seq_tokens && scratch && scratch_chunks > 0, "chunk_recurrence: null argument");
   LB_CHECK_ARG(groups > 0 && heads % groups == 0, "chunk_recurrence: %d heads are not a multiple of %d groups", heads, groups);
@@ -857,7 +855,7 @@ LB_EXPORT int lb_chunk_recurrence(int kind, const float* q, long long q_ld, cons
   p.A_log = A_log; p.dt_bias = dt_bias; p.D = D; p.bias = bias; p.lower = lower; p.decay = decay;
   p.state = state; p.out = out; p.out_ld = out_ld; p.cu_tokens = cu_tokens; p.slots = slots;
   p.heads = heads; p.groups = groups; p.dim = dim; p.vdim = vdim; p.unit_norm = unit_norm; p.act = act;
-  p.q_scale = q_scale; p.unit_eps = unit_eps; p.scratch = scratch;
+  p.q_scale = q_scale; p.unit_eps = unit_eps; p.scratch = scratch; p.hold = hold; p.wait_cycles = wait_cycles;
   auto aligned = [](const float* x, long long ld) { return (uintptr_t)x % 16 == 0 && ld % 4 == 0; };
   p.vec = dim % 4 == 0 && aligned(q, q_ld) && aligned(k, k_ld) && (kind != lb::CR_CHANNELS || aligned(a, a_ld));
   p.vecv = vdim % 4 == 0 && aligned(v, v_ld);
@@ -886,4 +884,38 @@ LB_EXPORT int lb_chunk_recurrence(int kind, const float* q, long long q_ld, cons
     done += ns;
   }
   return 0;
+}
+
+}  // namespace lb
+
+// The sequences seqs[0 .. num_long - 1] of the step (host array; with seq_tokens[i] tokens each, which must be what cu_tokens
+// says), all their tokens.  `scratch` holds scratch_chunks chunks; more are worked off in turns.  fixed: `decay`; ssm: a, A_log,
+// dt_bias, D; delta: a, b, A_log, dt_bias; hgrn2: k (the gate's input), bias, lower; channels: a (the decays), b.
+LB_EXPORT int lb_chunk_recurrence(int kind, const float* q, long long q_ld, const float* k, long long k_ld, const float* v, long long v_ld,
+                                  const float* a, long long a_ld, const float* b, long long b_ld, const float* A_log, const float* dt_bias,
+                                  const float* D, const float* bias, const float* lower, const float* decay, float* state, float* out,
+                                  long long out_ld, const int* cu_tokens, const int* slots, const int* seqs, const int* seq_tokens,
+                                  int num_long, int heads, int groups, int dim, int vdim, int unit_norm, float q_scale, float unit_eps,
+                                  int act, float* scratch, int scratch_chunks, cudaStream_t stream) {
+  return lb::run_chunks(kind, q, q_ld, k, k_ld, v, v_ld, a, a_ld, b, b_ld, A_log, dt_bias, D, bias, lower, decay, state, out, out_ld, cu_tokens,
+                        slots, seqs, seq_tokens, num_long, heads, groups, dim, vdim, unit_norm, q_scale, unit_eps, act, scratch, scratch_chunks,
+                        stream, 0, lb::CR_WAIT_CYCLES);
+}
+
+// For tests of the give-up paths: the same of at most four chunks, with what `hold` names (CrHold) left out and a wait limit of `wait_cycles`
+// clock cycles.  The first wait that depends on it runs out, the roles of each CTA leave once what they have in flight has landed, its code goes to
+// the error flag (lb_chunk_device_error), no output and, by the wide walk, no state is stored, and the context stays usable.
+LB_EXPORT int lb_chunk_recurrence_wait_test(int kind, const float* q, long long q_ld, const float* k, long long k_ld, const float* v, long long v_ld,
+                                            const float* a, long long a_ld, const float* b, long long b_ld, const float* A_log, const float* dt_bias,
+                                            const float* D, const float* bias, const float* lower, const float* decay, float* state, float* out,
+                                            long long out_ld, const int* cu_tokens, const int* slots, const int* seqs, const int* seq_tokens,
+                                            int num_long, int heads, int groups, int dim, int vdim, int unit_norm, float q_scale, float unit_eps,
+                                            int act, float* scratch, int scratch_chunks, cudaStream_t stream, int hold,
+                                            unsigned long long wait_cycles) {
+  LB_CHECK_ARG(hold > 0 && hold < 32 && wait_cycles > 0 && wait_cycles <= lb::CR_WAIT_CYCLES, "chunk_recurrence_wait_test: hold %d, limit %llu", hold, wait_cycles);
+  LB_CHECK_ARG(num_long == 1 && seq_tokens && seq_tokens[0] <= lb::CR_C * (scratch_chunks < 4 ? scratch_chunks : 4),
+               "chunk_recurrence_wait_test: one sequence of at most four chunks, all of them at once");
+  return lb::run_chunks(kind, q, q_ld, k, k_ld, v, v_ld, a, a_ld, b, b_ld, A_log, dt_bias, D, bias, lower, decay, state, out, out_ld, cu_tokens,
+                        slots, seqs, seq_tokens, num_long, heads, groups, dim, vdim, unit_norm, q_scale, unit_eps, act, scratch, scratch_chunks,
+                        stream, hold, wait_cycles);
 }

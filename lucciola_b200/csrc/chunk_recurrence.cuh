@@ -13,6 +13,12 @@ constexpr int CR_THREADS = 512;
 constexpr int CR_SCAN = 256, CR_WALK = 256;
 constexpr int CR_SEQS = 64;              // sequences a launch
 
+constexpr unsigned long long CR_WAIT_CYCLES = 4000000000ull;     // a bounded wait's limit
+
+// What a launch of lb_chunk_recurrence_wait_test leaves out, so that a wait runs out: the commits of the states' kernel; the copies or the
+// products of the wide walk, of the outputs.
+enum CrHold : int { CR_HOLD_STATES = 1, CR_HOLD_WALK_COPIES = 2, CR_HOLD_WALK = 4, CR_HOLD_OUT_COPIES = 8, CR_HOLD_OUT = 16 };
+
 enum CrKind : int { CR_FIXED = 0, CR_SSM = 1, CR_DELTA = 2, CR_HGRN2 = 3, CR_CHANNELS = 4 };
 
 __host__ __device__ constexpr bool cr_delta(int kind) { return kind == CR_DELTA || kind == CR_CHANNELS; }
@@ -29,6 +35,8 @@ struct ChunkParams {
   int vec, vecv;                         // rows of q, k, a and rows of v in whole aligned 16-byte pieces
   int slot0;                             // first chunk of this launch, counted over the sequences below
   int num_seqs;
+  unsigned long long wait_cycles;        // after this many clock cycles a wait on a barrier gives up
+  int hold;                              // tests of the give-up paths only, CrHold
   int wide;                              // delta rules: the walk of chunk_tcgen05.cu, which wants W and K cut
   float* scratch;                        // per (chunk of this launch, head), the arrays at these offsets
   long long per_head;

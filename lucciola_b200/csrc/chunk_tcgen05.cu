@@ -24,9 +24,10 @@
 
 namespace lb {
 
+static_assert(CR_WAIT_CYCLES == TA_WAIT_CYCLES, "one limit for all waits");
 constexpr int CT_THREADS = 512;                    // that compute
 constexpr int CT_OUT_THREADS = CT_THREADS + 128;   // and, of the outputs, a warp for the products, one for S and U, two for the tokens' numbers
-enum CtError : int { CT_ERR_STATES = 401, CT_ERR_OUT = 410 };
+enum CtError : int { CT_ERR_STATES = 401, CT_ERR_OUT = 410, CW_ERR = 450 };      // and the barrier's number
 // Barriers of the outputs.  The first ones count an arrival of every warp that computes.
 enum CtBar : int {
   CT_READY_QK, CT_READY_Q, CT_READY_A,             // operands are in shared memory
@@ -35,7 +36,7 @@ enum CtBar : int {
   CT_WARP_BARS,
   CT_SCORES = CT_WARP_BARS, CT_STATES = CT_SCORES + 3, CT_OUT = CT_STATES + 3,           // products are done
   CT_FULL_S, CT_FULL_S1, CT_FULL_U,                // S and U have landed
-  CT_READY_G, CT_PLACE, CT_BARS = CT_PLACE + 4
+  CT_READY_G, CT_PLACE, CT_DRAIN = CT_PLACE + 4, CT_BARS
 };
 
 __device__ __forceinline__ void ct_put4(uint8_t* dst, int part, float4 x) {
@@ -124,6 +125,13 @@ __device__ __forceinline__ void ct_sums(uint32_t at, float* out) {
 
 __device__ __forceinline__ void ct_publish() {       // what this thread wrote into shared memory, to the tensor cores
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+// A barrier of `threads` threads that says to all of them whether any came with a value.
+__device__ __forceinline__ bool ct_any(int id, int threads, int value) {
+  uint32_t any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %3, 0;\n\tbarrier.cta.red.or.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(any) : "r"(id), "r"(threads), "r"(value) : "memory");
+  return any != 0;
 }
 __device__ __forceinline__ void ct_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void ct_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -326,7 +334,8 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_states_kernel(const __gri
   const CtOperand U = {ta_smem_u32(Us), UPART, 0, CR_C, 1};
   const int quad = warp & 3, cols = 16 * (warp >> 2);
   uint32_t parity = 0;
-  for (int v0 = 0; v0 < p.vdim; v0 += VT) {
+  bool aborted = false;                            // the same in all threads
+  for (int v0 = 0; v0 < p.vdim && !aborted; v0 += VT) {
     if (v0 > 0) {
       CtRows<VT>::load(vsrc + v0, p.v_ld, c.m, min(VT, p.vdim - v0), p.vecv, tid, u4);
       if (tid == 0) ct_bulk_out_read();
@@ -339,38 +348,44 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_states_kernel(const __gri
     if (tid == 0) ct_bulk_out(mine + p.off_up + v0 / VT * (3 * UPART / 4), ta_smem_u32(Us), 3 * UPART);
     if (tid < VT) reinterpret_cast<int*>(mine)[p.off_f + v0 + tid] = from[tid];
 #pragma unroll 1
-    for (int d0 = 0; d0 < KD; d0 += 64) {
+    for (int d0 = 0; d0 < KD && !aborted; d0 += 64) {
       float x[16];
 #pragma unroll
       for (int ks = 0; ks < 4; ks += 2) {
         if (warp == 0 && elect_one()) {
           const CtOperand K = {ta_smem_u32(Ks) + d0 * 128, KPART, 0, CR_C, 1};   // 64 rows of the state: one block of 64 columns
           ct_product(tmem, 64, ks, 2, U, K, ct_idesc(1, 1, VT, 64));
-          ta_commit(bar);
+          if (!(p.hold & CR_HOLD_STATES)) ta_commit(bar);
         }
         __syncwarp();
-        ta_mbar_wait(bar, parity, &abort_s, CT_ERR_STATES);
+        ta_mbar_wait(bar, parity, &abort_s, CT_ERR_STATES, p.wait_cycles);
         parity ^= 1;
         ct_after_sync();
         const uint32_t at = tmem + ((uint32_t)(32 * quad) << 16) + cols;
         if (ks == 0) ct_sums<2, 64, VT == 64>(at, x);
         else ct_sums<2, 64, VT == 64, true>(at, x);
         ct_before_sync();
-        __syncthreads();                           // the sums are read
+        if (ks == 0) __syncthreads();              // the sums are read
+        else aborted = __syncthreads_or(abort_s);  // and whoever gave up, all leave
         ct_after_sync();
       }
+      const int cols_left = aborted ? 0 : p.v_ld_s - v0;
       constexpr int N = VT == 64 ? 8 : 16;
 #pragma unroll
       for (int i = 0; i < N; ++i) {
         const int v = VT == 128 ? 32 * quad + lane : 16 * quad + (lane >> 2) + 8 * ((i >> 1) & 1);
         const int d = VT == 128 ? i : 8 * (i >> 2) + 2 * (lane & 3) + (i & 1);
-        if (v0 + v < p.v_ld_s) mine[(size_t)(d0 + cols + d) * p.v_ld_s + v0 + v] = from[v] < CR_C ? __int_as_float(0x7fffffff) : x[i];
+        if (v < cols_left) mine[(size_t)(d0 + cols + d) * p.v_ld_s + v0 + v] = from[v] < CR_C ? __int_as_float(0x7fffffff) : x[i];
       }
-      if (abort_s) { d0 = KD; v0 = p.vdim; }
     }
     __syncthreads();                               // from[] is read
   }
   if (tid == 0) ct_bulk_out_read();
+  if (aborted) {                                   // the products that were waited for last
+    if (warp == 0 && elect_one()) ta_commit(bar);
+    __syncwarp();
+    ta_mbar_drain(bar, parity ^ 1u);
+  }
   if (warp == 0) ct_free<256>(tmem);
 }
 
@@ -494,12 +509,17 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
   pdl_wait();
   // Every barrier advances once a (chunk, head) or a tile of columns; bit b of `phases` is the parity this thread waits for next.
   uint32_t phases = 0;
+  // Where one gives up, abort_s is set, and every other wait that is not served gives up as well; a role leaves at the end of the (chunk, head)
+  // or tile in which it did, and nothing is stored.
+  volatile int* const gave_up = &abort_s;
+  bool ok = true;                                  // of the roles that are one thread, or two warps
   auto wait = [&](int b) {
-    ta_mbar_wait(bar + 8 * b, (phases >> b) & 1u, &abort_s, CT_ERR_OUT + b);
+    const bool served = ta_mbar_wait(bar + 8 * b, (phases >> b) & 1u, gave_up, CT_ERR_OUT + b, p.wait_cycles);
     phases ^= 1u << b;
+    return served;
   };
   auto wait_idle = [&](int b) {
-    ta_mbar_wait_idle(bar + 8 * b, (phases >> b) & 1u, &abort_s, CT_ERR_OUT + b);
+    ok &= ta_mbar_wait_idle(bar + 8 * b, (phases >> b) & 1u, gave_up, CT_ERR_OUT + b, p.wait_cycles);
     phases ^= 1u << b;
   };
 
@@ -511,57 +531,69 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
                       oK = {ta_smem_u32(Kp), L::KPART, L::KROWS * 128, L::KROWS, 0}, oX = {ta_smem_u32(Qp), L::XPART, 96 * 128, 96, 0};
       auto steps = [](int pass) { return pass < PASSES - 1 ? STEPS : 2; };
       auto scores = [&](int pass) {
-        if (pass >= 2) wait(CT_FREE_A);
+        if (pass >= 2) ok &= wait(CT_FREE_A);
         ct_after_sync();
         if (ROWS) ct_product(tmem, 48, 0, KD / 16, oX, oK, ct_idesc(0, 0, 128, 48));
         else ct_product(tmem + 256 * (pass & 1), 64, pass * STEPS, steps(pass), oQ, oK, ct_idesc(0, 0, 64, 64));
         ta_commit(bar + 8 * (CT_SCORES + pass));
       };
       auto states = [&](int pass, bool behind_scores) {
-        if (pass < HALVES) wait(CT_FULL_S + pass);
-        if (behind_scores || pass >= 2) wait((PASSES + pass) & 1 ? CT_FREE_S : CT_FREE_A);
+        if (pass < HALVES) ok &= wait(CT_FULL_S + pass);
+        if (behind_scores || pass >= 2) ok &= wait((PASSES + pass) & 1 ? CT_FREE_S : CT_FREE_A);
         ct_after_sync();
         ct_product(tmem + (pass == PASSES - 1 ? 320 : 256 * ((PASSES + pass) & 1)), 64, pass * STEPS, steps(pass), oS, oQ, ct_idesc(1, 0, VT, 64));
         ta_commit(bar + 8 * (CT_STATES + pass));
       };
-      for (int u = blockIdx.x; u < units; u += gridDim.x) {
-        wait(CT_READY_QK);
+      const int have = p.hold & CR_HOLD_OUT ? 0 : units;
+      for (int u = blockIdx.x; u < have && ok; u += gridDim.x) {
+        ok &= wait(CT_READY_QK);
 #pragma unroll 1
         for (int pass = 0; pass < (ROWS ? 1 : PASSES); ++pass) scores(pass);
-        if (ROWS) wait(CT_READY_Q);                // in the place of the scores' operand
-        for (int v0 = 0; v0 < p.vdim; v0 += VT) {
-          if (v0 > 0) wait(CT_FREE_T);
+        if (ROWS) ok &= wait(CT_READY_Q);                // in the place of the scores' operand
+        for (int v0 = 0; v0 < p.vdim && ok; v0 += VT) {
+          if (v0 > 0) ok &= wait(CT_FREE_T);
 #pragma unroll 1
           for (int pass = 0; pass < PASSES; ++pass) states(pass, !ROWS && v0 == 0);
-          wait(CT_FREE_A);
-          wait(CT_FULL_U);
-          if (v0 == 0) wait(CT_READY_A);
+          ok &= wait(CT_FREE_A);
+          ok &= wait(CT_FULL_U);
+          if (v0 == 0) ok &= wait(CT_READY_A);
           ct_after_sync();
           ct_product(tmem, 64, 0, 4, oU, oA, ct_idesc(1, 0, VT, 64));
           ta_commit(bar + 8 * CT_OUT);
         }
       }
+      ta_commit(bar + 8 * CT_DRAIN);               // nobody else may have waited for what was issued last
+      ta_mbar_drain(bar + 8 * CT_DRAIN, 0);
     }
     __syncwarp();
   } else if (warp == CT_THREADS / 32 + 1) {
     // ---- S and U, as soon as their places are free, one thread
     if (elect_one()) {
       bool first = true;
-      for (int u = blockIdx.x; u < units; u += gridDim.x) {
+      int copies[3] = {};                          // asked for so far: the halves of S, U
+      auto copy = [&](int i, uint32_t to, const float* from) {
+        ta_mbar_expect_tx(bar + 8 * (CT_FULL_S + i), 3 * L::UPART);
+        ct_bulk_in(to, from, 3 * L::UPART, bar + 8 * (CT_FULL_S + i));
+        ++copies[i];
+      };
+      const int have = p.hold & CR_HOLD_OUT_COPIES ? 0 : units;
+      for (int u = blockIdx.x; u < have && ok; u += gridDim.x) {
         const float* mine = p.scratch + (size_t)u * p.per_head;
-        for (int v0 = 0; v0 < p.vdim; v0 += VT, first = false) {
+        for (int v0 = 0; v0 < p.vdim && ok; v0 += VT, first = false) {
+#pragma unroll
           for (int i = 0; i < HALVES; ++i) {
             if (!first) wait_idle(CT_STATES + PASSES - HALVES + i);
             if (ROWS && v0 == 0 && i == 0) wait_idle(CT_FREE_R);
-            ta_mbar_expect_tx(bar + 8 * (CT_FULL_S + i), 3 * L::UPART);
-            ct_bulk_in(ta_smem_u32(Sp) + i * 3 * L::UPART, mine + p.off_s + (v0 / VT * HALVES + i) * (3 * L::UPART / 4), 3 * L::UPART, bar + 8 * (CT_FULL_S + i));
+            if (ok) copy(i, ta_smem_u32(Sp) + i * 3 * L::UPART, mine + p.off_s + (v0 / VT * HALVES + i) * (3 * L::UPART / 4));
           }
           if (!first) wait_idle(CT_OUT);
           if (v0 == 0) wait_idle(CT_SCORES + (ROWS ? 0 : PASSES - 1));
-          ta_mbar_expect_tx(bar + 8 * CT_FULL_U, 3 * L::UPART);
-          ct_bulk_in(ta_smem_u32(Kp), mine + p.off_up + v0 / VT * (3 * L::UPART / 4), 3 * L::UPART, bar + 8 * CT_FULL_U);
+          if (ok) copy(2, ta_smem_u32(Kp), mine + p.off_up + v0 / VT * (3 * L::UPART / 4));
         }
       }
+#pragma unroll
+      for (int i = 0; i < 3; ++i)                  // nobody leaves while a copy of its own is in flight
+        if (copies[i] > 0) ta_mbar_drain(bar + 8 * (CT_FULL_S + i), (copies[i] - 1) & 1);
     }
     __syncwarp();
   } else if (warp >= CT_THREADS / 32 + 2) {
@@ -578,7 +610,7 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
     put_place(0);
     put_place(1);
     int n = 0;
-    for (int u = blockIdx.x; u < units; u += gridDim.x, ++n) {
+    for (int u = blockIdx.x; u < units && (!ROWS || ok); u += gridDim.x, ++n) {
       const int buf = n & 1;
       if (n >= 2) wait_idle(CT_FREE_N + buf);      // the one before the one before is through
       put_place(n + 2);
@@ -586,7 +618,7 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
         const ChunkPlace c = cr_place(p, u / p.heads);
         cr_numbers<KIND>(p, c, u % p.heads, gs, ws, j);
         if (n >= 1) wait_idle(CT_FREE_G);
-        asm volatile("bar.sync 2, 64;" ::: "memory");
+        if (ct_any(2, 64, !ok)) break;             // both warps or none
         Product d, all;
         const float w = KIND == CR_SSM ? ws[j] : 1.f;
         float* to = Gs + j;
@@ -621,9 +653,9 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
     // q, then k (and the decays) of the next one: no more than fits beside the operands at a time, or the loads wait for one another
     auto request_q = [&](int u, int n) {
       const int grp = u % p.heads / (p.heads / p.groups);
-      wait(CT_PLACE + (n & 3));
-      c.first = place[2 * (n & 3)];
-      c.m = place[2 * (n & 3) + 1];
+      const bool served = wait(CT_PLACE + (n & 3));
+      c.first = served ? place[2 * (n & 3)] : 0;       // without a place no token is read
+      c.m = served ? place[2 * (n & 3) + 1] : 0;
       QK::load(p.q + (size_t)c.first * p.q_ld + (size_t)grp * p.dim, p.q_ld, c.m, p.dim, p.vec, tid, q4);
     };
     auto request_k = [&](int u) {
@@ -668,6 +700,7 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
       const bool more = u + (int)gridDim.x < units;
       float o[16];
       if constexpr (!ROWS) {
+        if (__any_sync(0xffffffffu, *gave_up)) break;
         QK::put(Qp, L::QPART, tid, q4);
         QK::put(Kp, L::KPART, tid, k4);
         ct_publish();
@@ -710,7 +743,7 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
           *reinterpret_cast<float4*>(Kf + at4) = KIND == CR_HGRN2 ? cr_map(k4[i], [](float g) { return 1.f - g; }) : k4[i];
           *reinterpret_cast<float4*>(Gf + at4) = KIND == CR_HGRN2 ? k4[i] : g4[KIND == CR_CHANNELS ? i : 0];
         }
-        barrier();
+        if (ct_any(1, CT_THREADS, *gave_up)) break;              // all warps or none: they meet again below
         // q G(block's start, i), k G(j, block's end)
         if (part < 8) {
           auto of = [&](const float* m, int t) { return *reinterpret_cast<const float2*>(m + t * KD + ch); };
@@ -831,6 +864,7 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
         ct_sums<2, 64, VT == 64, true>(at + 320, o);
         wait(CT_OUT);
         ct_after_sync();
+        const int m = *gave_up ? 0 : here.m;       // whoever it was: nothing is stored
         float* dst = p.out + (size_t)(here.first + t0) * p.out_ld + (size_t)h * p.vdim + v0 + v;
         const float* skip = KIND == CR_SSM ? p.v + (size_t)(here.first + t0) * p.v_ld + (size_t)h * p.vdim + v0 + v : nullptr;
         const float D = KIND == CR_SSM && p.D ? p.D[h] : 0.f;
@@ -843,7 +877,7 @@ __global__ void __launch_bounds__(CT_OUT_THREADS, 1) chunk_outputs_kernel(const 
             const int dt = VT == 128 ? i : 8 * (i >> 2) + (i & 1), dv = VT == 128 ? 0 : 8 * ((i >> 1) & 1);
             float y = ROWS ? o[i] + x[i - i0] : fmaf(o[i], cs[buf * CR_C + t0 + dt], x[i - i0]);
             if (t0 + dt >= (dv ? bad1 : bad0)) y = __int_as_float(0x7fffffff);
-            if (t0 + dt < here.m && v0 + v + dv < p.vdim) {
+            if (t0 + dt < m && v0 + v + dv < p.vdim) {
               if (KIND == CR_SSM && p.D) y = fmaf(D, skip[dt * p.v_ld + dv], y);
               dst[dt * p.out_ld + dv] = y;
             }
@@ -871,7 +905,7 @@ constexpr int CW_COLS = 16, CW_THREADS = 256;        // that compute; and a warp
 constexpr int CW_PART = CR_C * 128 * 2;              // bytes of a part of W or K
 constexpr int CW_STAGE = 6 * CW_PART;                // W, K
 constexpr int CW_BYTES = 1024 + 2 * CW_STAGE + 128 * 128 + CR_C * 128;
-enum CwBar : int { CW_READY_S, CW_READY_U, CW_WS, CW_KU, CW_FULL_W, CW_FULL_W1, CW_FULL_K, CW_FULL_K1, CW_FREE_W, CW_FREE_W1, CW_FREE_K, CW_FREE_K1, CW_BARS };
+enum CwBar : int { CW_READY_S, CW_READY_U, CW_WS, CW_KU, CW_FULL_W, CW_FULL_W1, CW_FULL_K, CW_FULL_K1, CW_FREE_W, CW_FREE_W1, CW_FREE_K, CW_FREE_K1, CW_DRAIN, CW_BARS };
 
 // The first 16 lanes of the warp's quarter x 8 columns: x[e] is lane l / 4 + 8 (e / 2), column 2 (l % 4) + e % 2.
 __device__ __forceinline__ void ct_ld8_half(uint32_t at, float* x) {
@@ -929,9 +963,10 @@ __global__ void __launch_bounds__(CW_THREADS + 64, 1) chunk_walk_wide_kernel(con
   pdl_wait();
   const size_t stride = (size_t)p.heads * p.per_head;
   float* mine = p.scratch + ((size_t)(first + c_lo - p.slot0) * p.heads + h) * p.per_head;
-  uint32_t phases = 0;                               // parities, as in the outputs
+  uint32_t phases = 0;                               // parities, as in the outputs; and as there, all leave where one gives up
+  bool ok = true;
   auto wait = [&](int b) {
-    ta_mbar_wait(bar + 8 * b, (phases >> b) & 1u, &abort_s, CT_ERR_OUT + CT_BARS + b);
+    ok &= ta_mbar_wait(bar + 8 * b, (phases >> b) & 1u, &abort_s, CW_ERR + b, p.wait_cycles);
     phases ^= 1u << b;
   };
 
@@ -943,7 +978,8 @@ __global__ void __launch_bounds__(CW_THREADS + 64, 1) chunk_walk_wide_kernel(con
         ta_umma(d + 16, ct_desc(left, 1, ks), right, ct_idesc(left.mn, 1, m, 32), 1);
         ta_umma(d + 32, ct_desc(left, 2, ks), right, ct_idesc(left.mn, 1, m, 16), 1);
       };
-      for (int c = c_lo; c < c_hi; ++c) {
+      const int end = p.hold & CR_HOLD_WALK ? c_lo : c_hi;
+      for (int c = c_lo; c < end && ok; ++c) {
         const int buf = (c - c_lo) & 1;
         const uint32_t w_at = ta_smem_u32(base) + buf * CW_STAGE;
         const CtOperand W = {w_at, CW_PART, CR_C * 128, CR_C, 0}, K = {w_at + 3 * CW_PART, CW_PART, 0, CR_C, 1};
@@ -962,21 +998,31 @@ __global__ void __launch_bounds__(CW_THREADS + 64, 1) chunk_walk_wide_kernel(con
         ta_commit(bar + 8 * CW_KU);
         ta_commit(bar + 8 * (CW_FREE_K + buf));
       }
+      ta_commit(bar + 8 * CW_DRAIN);
+      ta_mbar_drain(bar + 8 * CW_DRAIN, 0);
     }
     __syncwarp();
   } else if (warp == CW_THREADS / 32 + 1) {
     if (elect_one()) {
       const float* from = mine;
-      for (int c = c_lo; c < c_hi; ++c, from += stride) {
+      const int end = p.hold & CR_HOLD_WALK_COPIES ? c_lo : c_hi;
+      int copies = 0;                                // W and K of chunk c_lo + i are copies 2 i and 2 i + 1
+      for (int c = c_lo; c < end; ++c, from += stride) {
         const int buf = (c - c_lo) & 1;
         const uint32_t to = ta_smem_u32(base) + buf * CW_STAGE;
         if (c >= c_lo + 2) wait(CW_FREE_W + buf);
+        if (!ok) break;
         ta_mbar_expect_tx(bar + 8 * (CW_FULL_W + buf), 3 * CW_PART);
         ct_bulk_in(to, from + p.off_w, 3 * CW_PART, bar + 8 * (CW_FULL_W + buf));
+        ++copies;
         if (c >= c_lo + 2) wait(CW_FREE_K + buf);
+        if (!ok) break;
         ta_mbar_expect_tx(bar + 8 * (CW_FULL_K + buf), 3 * CW_PART);
         ct_bulk_in(to + 3 * CW_PART, from + p.off_k, 3 * CW_PART, bar + 8 * (CW_FULL_K + buf));
+        ++copies;
       }
+      for (int i = max(0, copies - 4); i < copies; ++i)         // the last four may still be in flight
+        ta_mbar_drain(bar + 8 * ((i & 1 ? CW_FULL_K : CW_FULL_W) + ((i >> 1) & 1)), (i >> 2) & 1);
     }
     __syncwarp();
   } else {
@@ -1024,7 +1070,7 @@ __global__ void __launch_bounds__(CW_THREADS + 64, 1) chunk_walk_wide_kernel(con
     for (int i = 0; i < 8; ++i) s[i] = i < have ? S[i] : 0.f;
     put_state(mine);
     request(mine);
-    for (int c = c_lo; c < c_hi; ++c) {
+    for (int c = c_lo; c < c_hi && __all_sync(0xffffffffu, ok); ++c) {
       const float2 u0 = u_next[0], u1 = u_next[1];
       const float decay = g;
       float* const keep = mine;
@@ -1064,8 +1110,9 @@ __global__ void __launch_bounds__(CW_THREADS + 64, 1) chunk_walk_wide_kernel(con
       for (int i = 0; i < 8; ++i) s[i] = fmaf(decay, s[i], x[i]);
       if (c + 1 < c_hi) put_state(mine);
     }
+    const int keep = *(volatile int*)&abort_s ? 0 : have;              // whoever gave up: the request's state stays as it was
 #pragma unroll
-    for (int i = 0; i < 8; ++i) if (i < have) S[i] = s[i];
+    for (int i = 0; i < 8; ++i) if (i < keep) S[i] = s[i];
   }
   ct_before_sync();
   __syncthreads();

@@ -1,6 +1,9 @@
 """The chunked recurrences where their products' tiles, rings and CTAs change over: value columns in one tile of 64, of 128 and in several,
 more (chunk, head)s than SMs, so that a CTA takes several one behind the other, and a value that is not finite behind the first
-tile of columns; against the plain recurrence in 64 bits (GPU)."""
+tile of columns; against the plain recurrence in 64 bits; and waits that run out (GPU)."""
+import ctypes
+import time
+
 import pytest
 import torch
 
@@ -60,6 +63,50 @@ def test_a_bad_value_in_any_tile_of_columns(kind, token, column):
     beside = torch.arange(heads * vdim, device=DEV) != column
     assert torch.equal(got[:, beside], good[:, beside])
     assert torch.isnan(got[token:, column]).all() and torch.isnan(after[0, 0, :, column]).all()
+
+
+@pytest.mark.parametrize("hold,kind,code", [(1, "fixed", 401), (1, "ssm", 401), (1, "hgrn2", 401), (2, "delta", 450), (2, "channels", 450), (4, "delta", 450), (4, "channels", 450)]
+                         + [(hold, kind, 410) for hold in (8, 16) for kind in KINDS])
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 128), (40, 128, 40), (8, 128, 260), (3, 64, 64)])
+def test_a_wait_that_runs_out(hold, kind, code, heads, dim, vdim, monkeypatch):
+    """Without the products of K^T U (1), the copies (2) or products (4) of the walk, the copies (8) or products (16) of the outputs, and a limit of
+    200 000 cycles, 0.1 ms: the kernel returns, leaves the number of the wait, stores no output and (the walk) no state, with copies in flight or with
+    none, and an ordinary call right after is right.  One (chunk, head) a CTA, more of them than SMs, three tiles of columns, small states."""
+    from lucciola_b200 import ops
+    from lucciola_b200.csrc import library
+    if hold in (2, 4) and dim <= 64:
+        pytest.skip("the walk on the ordinary pipes, which waits for nothing")
+    torch.manual_seed(19)
+    lens = [250]
+    o, step = gentle(kind, 250, heads, heads, dim, vdim), step_of([250], [0])
+    state = 0.3 * torch.randn(1, heads, dim, vdim, device=DEV)
+    want, S = plain(kind, o, state, step, heads, heads, dim, vdim)
+    fn, real = library().lb_chunk_recurrence_wait_test, ops._call
+    fn.argtypes, fn.restype = ops._SIGNATURES["lb_chunk_recurrence"] + [ctypes.c_int, ctypes.c_ulonglong], ctypes.c_int
+    held = []
+
+    def call(name, *args):
+        if name != "lb_chunk_recurrence":
+            return real(name, *args)
+        held.append(fn(*args, hold, 200_000))
+    assert ops.device_error() == 0
+    monkeypatch.setattr(ops, "_call", call)
+    kept = state.clone()
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    got = through_ops(kind, o, kept, step, heads, heads, dim, vdim, True, shifted=False)
+    torch.cuda.synchronize()
+    assert time.perf_counter() - t0 < 1.0                # its limit, not the ordinary two seconds
+    monkeypatch.setattr(ops, "_call", real)
+    assert held == [0]
+    assert code <= ops.device_error() < code + 40 and ops.device_error() == 0
+    if hold >= 8:
+        assert torch.isnan(got).all()
+    if hold in (2, 4):
+        assert torch.equal(kept, state)
+    got = through_ops(kind, o, state, step, heads, heads, dim, vdim, True, shifted=False)
+    assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max() and (state.double() - S).abs().max() <= 1e-5 * S.abs().max()
+    assert ops.device_error() == 0
 
 
 @pytest.mark.parametrize("tokens,channels", [(1, 64), (8, 64), (4096, 260), (1200, 1024)])
