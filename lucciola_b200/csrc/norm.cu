@@ -123,12 +123,19 @@ __global__ void rmsnorm_short_rows_kernel(TO* __restrict__ out, const float* __r
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= num_rows) return;
   const float* r = x + (size_t)row * hidden;
-  float ss = 0.f;
-  for (int j = lane; j < hidden; j += 32) { const float v = r[j]; ss += v * v; }
+  float ss = 0.f, v[8];                            // the first 256 of a row stay in registers; all their loads are under way at once
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = lane + 32 * i < hidden ? r[lane + 32 * i] : 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) ss += v[i] * v[i];
+  for (int j = lane + 256; j < hidden; j += 32) { const float y = r[j]; ss += y * y; }
   ss = warp_sum(ss);
   const float inv = rsqrtf(ss / (float)hidden + eps);
   TO* o = out + (size_t)row * hidden;
-  for (int j = lane; j < hidden; j += 32) o[j] = from_f32<TO>(r[j] * inv * weight[j]);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (lane + 32 * i < hidden) o[lane + 32 * i] = from_f32<TO>(v[i] * inv * weight[lane + 32 * i]);
+  for (int j = lane + 256; j < hidden; j += 32) o[j] = from_f32<TO>(r[j] * inv * weight[j]);
 }
 
 // RMSNorm in groups: the row is cut into `groups` equal consecutive parts and each part is divided by its own
