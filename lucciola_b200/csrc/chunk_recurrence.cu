@@ -786,10 +786,14 @@ static cudaError_t launch_chunks(int kind, const ChunkParams& p, int nslots, cud
     if (p.wide) {
       e = cr_launch_walk(p, nslots, stream);
     } else {
+      // Fewer columns a CTA where those with 32 leave SMs idle.  Of 128 rows CTAs of 16 columns are always more than there are SMs: with
+      // fewer the wide walk runs.
+      constexpr int least = KD == 64 ? 8 : 16;
       int nv = 32;
-      while (nv > 8 && (long long)p.num_seqs * p.heads * ((p.vdim + nv - 1) / nv) < 100) nv /= 2;
-      e = nv == 32 ? launch_chunk_walk<KD, 32>(p, nslots, stream) : nv == 16 ? launch_chunk_walk<KD, 16>(p, nslots, stream)
-                                                                             : launch_chunk_walk<KD, 8>(p, nslots, stream);
+      while (nv > least && (long long)p.num_seqs * p.heads * ((p.vdim + nv - 1) / nv) < 100) nv /= 2;
+      if (nv == 32) e = launch_chunk_walk<KD, 32>(p, nslots, stream);
+      else if (KD == 128 || nv == 16) e = launch_chunk_walk<KD, 16>(p, nslots, stream);
+      else e = launch_chunk_walk<KD, least>(p, nslots, stream);
     }
   } else {
     e = cr_launch_states(kind, p, nslots, stream);
@@ -860,12 +864,14 @@ static int run_chunks(int kind, const float* q, long long q_ld, const float* k, 
   p.vec = dim % 4 == 0 && aligned(q, q_ld) && aligned(k, k_ld) && (kind != lb::CR_CHANNELS || aligned(a, a_ld));
   p.vecv = vdim % 4 == 0 && aligned(v, v_ld);
   lb::cr_layout(p, kind);
+  int sms = 0;
+  if (cudaError_t e = lb::cr_sms(&sms)) { lb::set_error("chunk_recurrence: %s", cudaGetErrorString(e)); return 2; }
   for (int done = 0; done < num_long;) {
     const int ns = num_long - done < lb::CR_SEQS ? num_long - done : lb::CR_SEQS;
     p.num_seqs = ns;
     // The walk on tcgen05 has a CTA for 16 columns and one CTA an SM: where all of them run at once it is the faster (16 heads of 128 x 128,
     // one prompt of 2048 tokens, 92 -> 68 us), in more than one round the one with 32 columns a CTA is (32 heads, two rounds, 136 | 125).
-    p.wide = lb::cr_delta(kind) && dim > 64 && (long long)ns * heads * ((vdim + 15) / 16) <= 148;
+    p.wide = lb::cr_delta(kind) && dim > 64 && (long long)ns * heads * ((vdim + 15) / 16) <= sms;
     if (!p.wide) p.off_k = p.off_w + lb::CR_C * ((dim <= 64 ? 64 : 128) + 4);      // right behind W: one copy
     else p.off_k = p.off_w + lb::CR_C * 128 * 3 / 2;
     p.base[0] = 0;

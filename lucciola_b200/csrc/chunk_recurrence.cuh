@@ -184,6 +184,13 @@ __device__ __forceinline__ void cr_put(uint8_t* at, int part, const Split& x) {
   *reinterpret_cast<uint32_t*>(at + 2 * part) = x.l;
 }
 
+// SMs of the current device.
+inline cudaError_t cr_sms(int* sms) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+}
+
 // chunk_tcgen05.cu: the states before the chunks of the delta rules; K^T U of the other kinds; the outputs.
 cudaError_t cr_launch_walk(const ChunkParams& p, int nslots, cudaStream_t stream);       // delta rules, `wide`
 cudaError_t cr_launch_states(int kind, const ChunkParams& p, int nslots, cudaStream_t stream);

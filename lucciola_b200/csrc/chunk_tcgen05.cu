@@ -1135,10 +1135,8 @@ static cudaError_t launch_outputs(const ChunkParams& p, int nslots, cudaStream_t
   constexpr int bytes = CtOut<KIND, KD, VT>::BYTES;
   static const cudaError_t cfg = ct_allow(chunk_outputs_kernel<KIND, KD, VT>, bytes);
   if (cfg != cudaSuccess) return cfg;
-  int dev = 0, sms = 148;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
+  int sms = 0;
+  if (cudaError_t e = cr_sms(&sms)) return e;
   const int units = nslots * p.heads;
   return launch(chunk_outputs_kernel<KIND, KD, VT>, dim3(units < sms ? units : sms), dim3(CT_OUT_THREADS), bytes, stream, p, units);
 }
@@ -1158,7 +1156,8 @@ cudaError_t cr_launch_states(int kind, const ChunkParams& p, int nslots, cudaStr
   switch (kind) {
     case CR_FIXED: return CT_SIZES(CR_FIXED, launch_states);
     case CR_SSM: return CT_SIZES(CR_SSM, launch_states);
-    default: return CT_SIZES(CR_HGRN2, launch_states);
+    case CR_HGRN2: return CT_SIZES(CR_HGRN2, launch_states);
+    default: return cudaErrorInvalidValue;         // the delta rules' states come from a walk
   }
 }
 cudaError_t cr_launch_outputs(int kind, const ChunkParams& p, int nslots, cudaStream_t stream) {
@@ -1167,7 +1166,8 @@ cudaError_t cr_launch_outputs(int kind, const ChunkParams& p, int nslots, cudaSt
     case CR_SSM: return CT_SIZES(CR_SSM, launch_outputs);
     case CR_DELTA: return CT_SIZES(CR_DELTA, launch_outputs);
     case CR_HGRN2: return CT_SIZES(CR_HGRN2, launch_outputs);
-    default: return CT_SIZES(CR_CHANNELS, launch_outputs);
+    case CR_CHANNELS: return CT_SIZES(CR_CHANNELS, launch_outputs);
+    default: return cudaErrorInvalidValue;
   }
 }
 
