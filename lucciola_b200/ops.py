@@ -658,8 +658,9 @@ def short_conv_step(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bi
 
 # Portions that may go through the chunked form of a recurrence (csrc/chunk_recurrence.cu).
 CHUNK_LEAST = 32
-# Scratch of the chunked form, in floats: more chunks are worked off in turns.
-CHUNK_SCRATCH = 64 << 20
+# Scratch of the chunked form, in floats: more chunks are worked off in turns (16 heads of 128 x 128, 4096 tokens, us with 256 MB | 128 MB: fixed
+# decays 168 | 185, HGRN2 234 | 263, delta rule 371 | 412); and what has to do where the memory for that is not there.
+CHUNK_SCRATCH, CHUNK_SCRATCH_SCANT = 64 << 20, 32 << 20
 _CHUNK_KINDS = {"fixed": 0, "ssm": 1, "delta": 2, "hgrn2": 3, "channels": 4}
 
 # What a step's recurrence costs in us, all launches (B200; fitted to 1400 steps of 1 to 16 equal portions of 32 to 448 tokens or of one to
@@ -764,7 +765,14 @@ def _chunk_recurrence(kind: str, q: tuple, k: tuple, v: tuple, state: torch.Tens
     lens = [step.q_lens[i] for i in long]
     one = _chunk_floats(code, heads, dim, vdim)
     chunks = max(1, min(sum(-(-t // 64) for t in lens), CHUNK_SCRATCH // max(one, 1)))
-    scratch = torch.empty(chunks * one, dtype=torch.float32, device=out.device)
+    try:
+        scratch = torch.empty(chunks * one, dtype=torch.float32, device=out.device)
+    except torch.OutOfMemoryError:
+        fewer = max(1, CHUNK_SCRATCH_SCANT // max(one, 1))
+        if fewer >= chunks:
+            raise
+        chunks = fewer
+        scratch = torch.empty(chunks * one, dtype=torch.float32, device=out.device)
     seqs, tokens = (c_int * n)(*long), (c_int * n)(*lens)
     _call("lb_chunk_recurrence", code, *q, *k, *v, *a, *b, _ptr(A_log), _ptr(dt_bias), _ptr(D), _ptr(bias), _ptr(lower), _ptr(decay), state.data_ptr(),
           out.data_ptr(), out.stride(0), step.cu_tokens.data_ptr(), step.state_slots.data_ptr(), _address(seqs), _address(tokens), n,

@@ -258,6 +258,43 @@ def test_scratch_for_fewer_chunks_and_more_sequences_than_a_launch(kind, monkeyp
     assert (got.double() - want).abs().max() <= 1e-5 * want.abs().max() and (state.double() - S).abs().max() <= 1e-5 * S.abs().max()
 
 
+def test_scratch_where_memory_is_scant(monkeypatch):
+    """Where the allocator has no room for all chunks at once they are worked off in more turns, the same bits; and where there is none for
+    those either, the call fails as any other does that finds no memory."""
+    from lucciola_b200 import ops
+    heads, dim, vdim, T = 32, 128, 128, 1900
+    torch.manual_seed(12)
+    o = operands("hgrn2", T, heads, heads, dim, vdim)
+    state, step = torch.randn(1, heads, dim, vdim, device=DEV), step_of([T], [0])
+    one = 4 * ops._chunk_floats(ops._CHUNK_KINDS["hgrn2"], heads, dim, vdim)
+    assert 4 * ops.CHUNK_SCRATCH_SCANT < 30 * one <= 4 * ops.CHUNK_SCRATCH
+    whole_state = state.clone()
+    whole = through_ops("hgrn2", o, whole_state, step, heads, heads, dim, vdim, True)
+    total = torch.cuda.get_device_properties(0).total_memory
+    rows = 4 * T * heads * (2 * dim + 2 * vdim)            # through_ops lays q, k, v side by side, and the outputs
+    real, turns = ops._call, []
+
+    def call(name, *args):
+        if name == "lb_chunk_recurrence":
+            turns.append(-(-30 // args[-2]))               # of as many chunks as the scratch holds
+        real(name, *args)
+    monkeypatch.setattr(ops, "_call", call)
+    try:
+        for room, fits in ((160 << 20, True), (40 << 20, False)):
+            got_state = state.clone()
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+            torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + rows + room) / total)
+            if fits:
+                got = through_ops("hgrn2", o, got_state, step, heads, heads, dim, vdim, True)
+                assert turns == [2] and torch.equal(got, whole) and torch.equal(got_state, whole_state)
+            else:
+                with pytest.raises(torch.OutOfMemoryError):
+                    through_ops("hgrn2", o, got_state, step, heads, heads, dim, vdim, True)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+
+
 @pytest.mark.parametrize("channels,lens", [(8192, [1]), (260, [1] * 9), (4096, [700, 1, 2, 3, 4, 5, 333]), (1028, [9, 200]), (64, [3000]), (2048, [5, 4, 1, 1, 90])])
 @pytest.mark.parametrize("bias", [False, True])
 def test_short_convolution_of_several_tokens_a_thread(channels, lens, bias):
