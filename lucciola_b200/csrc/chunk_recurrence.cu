@@ -34,10 +34,14 @@
 // bits, 16 places at a time, and the sums from one 16 to the next are ordinary additions: those of single chunks, and the walk where its
 // CTAs run at once, in chunk_tcgen05.cu; here the triangular solve's and the walk in several rounds (see cr_step).  Decays
 // and strengths that are one number a token come out of 64 bits, and their products carry what rounding drops.  Against 64 bits the
-// outputs before the norm are 0.2 to 0.98 times as far off as those of the kernels that walk token by token, over the layers' sizes.
+// outputs before the norm and the states are 0.1 to 0.97 times as far off as those of the kernels that walk token by token, over the layers' sizes
+// and operands (rms; HGRN2's outputs, 0.85 to 0.93, were 0.82 to 0.91 while mma.sync formed them: 7.3e-8 -> 7.6e-8 of the result); with fast
+// decays and operands of random sign HGRN2's outputs are up to 1.07 times as far off, states of channel decays up to 1.22.
 //
 // Measured (B200, all launches, token by token | every product by mma.sync | here): HGRN2, one prompt of 2048 tokens and 16 heads of
-// 128 x 128, 403 | 150 | 124 us; the delta rule 865 | 210 | 177; fixed decays, four prompts of 1654 tokens in all, 341 | 137 | 88.
+// 128 x 128, 403 | 147 | 130 us; the delta rule 865 | 214 | 185; fixed decays, four prompts of 1654 tokens in all, 341 | 137 | 84.  Channel decays, 263
+// (275 by mma.sync); where 256 to 288 (chunk, head)s stand in more walks than run at once (32 heads, 512 tokens: 134 | 139 us; nine portions of 128,
+// 142 | 147) the outputs' second round of CTAs costs them more than their products gain, 1 to 6 %.
 // What bounds the kernels here: mma.sync issues one product every 8 cycles a scheduler on this GPU whatever its type, so the six products
 // of 16 places are worth 1.3 times the ordinary 32-bit pipes; the walk is 32 links of two small products each.
 #include "chunk_recurrence.cuh"

@@ -48,7 +48,8 @@ struct ChunkParams {
   int base[CR_SEQS + 1];                 // its first chunk
 };
 
-// 1 / d and x / d for d = 1 + e^-x >= 1: the approximate reciprocal (off by 1 ulp) and one step on the remainder, which leaves half an ulp;
+// 1 / d and x / d for d = 1 + e^-x >= 1: the approximate reciprocal (off by 1 ulp) and one step on the remainder (Newton's, and Markstein's for
+// the quotient), which leaves half an ulp;
 // a d whose reciprocal is no normal number counts as 2^126.
 __device__ __forceinline__ float cr_reciprocal(float& d) {
   float r;

@@ -13,8 +13,8 @@
 
 namespace lb {
 
-// x / (1 + e^-x) as the approximate reciprocal and one step on the remainder, which leaves half an ulp as a division does at a third of its
-// instructions; a division only where the reciprocal would be no normal number or the remainder no number.
+// x / (1 + e^-x) as the approximate reciprocal and one step on the quotient's remainder (Markstein's), which leaves half an ulp as a division does at a
+// third of its instructions; a division only where the reciprocal would be no normal number or the remainder no number.
 __device__ __forceinline__ bool silu_plain(float x) { return fabsf(x) < 80.f; }
 __device__ __forceinline__ float silu_divided(float x) { return x / (1.f + expf(-x)); }
 __device__ __forceinline__ float silu_near(float x) {

@@ -109,7 +109,8 @@ def test_a_wait_that_runs_out(hold, kind, code, heads, dim, vdim, monkeypatch):
     assert ops.device_error() == 0
 
 
-@pytest.mark.parametrize("tokens,channels", [(1, 64), (8, 64), (4096, 260), (1200, 1024)])
+# a token by itself, and one, two, four and eight tokens a thread
+@pytest.mark.parametrize("tokens,channels", [(1, 64), (8, 64), (3000, 64), (4096, 260), (1200, 1024), (1557, 4096)])
 def test_silu_of_the_short_convolution(tokens, channels):
     """Where the activation changes from the reciprocal to the division (80), around the largest and smallest results and at what is no
     number, alone and four in a word, for every number of tokens a thread: x / (1 + e^-x) within two units in the last place for the

@@ -295,10 +295,10 @@ def test_scratch_where_memory_is_scant(monkeypatch):
         torch.cuda.set_per_process_memory_fraction(1.0)
 
 
-@pytest.mark.parametrize("channels,lens", [(8192, [1]), (260, [1] * 9), (4096, [700, 1, 2, 3, 4, 5, 333]), (1028, [9, 200]), (64, [3000]), (2048, [5, 4, 1, 1, 90])])
+@pytest.mark.parametrize("channels,lens", [(8192, [1]), (260, [1] * 9), (4096, [700, 1, 2, 3, 4, 5, 333]), (4096, [1205, 1, 2, 3, 4, 9, 333]), (1028, [9, 200]), (64, [3000]), (2048, [5, 4, 1, 1, 90])])
 @pytest.mark.parametrize("bias", [False, True])
 def test_short_convolution_of_several_tokens_a_thread(channels, lens, bias):
-    """Portions that start and end anywhere in a thread's tokens, and steps of single tokens with the state in the same launch:
+    """Portions that start and end anywhere in a thread's two, four or eight tokens, and steps of single tokens with the state in the same launch:
     the very sums of the token-a-thread kernel (any taps and alignment), so the same bits."""
     from lucciola_b200 import ops
     torch.manual_seed(6)
