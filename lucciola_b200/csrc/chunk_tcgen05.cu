@@ -14,7 +14,7 @@
 // leave the states and U already cut, in the form in which they are read here by one copy a half.
 //
 // Measured (16 heads of 128 x 128, us, mma.sync with the operands cut by every warp that reads them | here): outputs of 2048 tokens, HGRN2
-// 96 | 81, delta rule 78 | 51; of four prompts of 1654 tokens, fixed decays, 79 | 42; K^T U of these 46 | 31, HGRN2 43 | 30; the scan, which cuts
+// 96 | 83, delta rule 78 | 54; of four prompts of 1654 tokens, fixed decays, 79 | 43; K^T U of these 46 | 28, HGRN2 43 | 27; the scan, which cuts
 // the states now, 10.5 | 13.6.  One prompt of 160 tokens, 8 heads, fixed decays, all launches: 62 | 25.
 // What bounds it: a CTA of the outputs holds 216 KB, so one runs on an SM, and its (chunk, head) takes 10 us: loads of q and k that wait for room
 // beside the operands (3 us), their silu or norm and cutting, and the read-out, around 4 us of products.  With a decay for every
