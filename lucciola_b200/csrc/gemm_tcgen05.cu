@@ -311,9 +311,8 @@ __device__ __forceinline__ float gated_mul(int act, float limit, float g, float 
   return silu_mul(g, u);
 }
 
-// Up to 32 tokens: two sums of the tile (GemmParams::chains).
-template <int BT>
-__host__ __device__ constexpr int tmem_cols() { return BT <= 32 ? 2 * BT : BT; }
+template <int BT, bool TWO>
+__host__ __device__ constexpr int tmem_cols() { return TWO ? 2 * BT : BT < 32 ? 32 : BT; }
 
 template <int BT, int STAGES>
 struct SmemLayout {
@@ -324,7 +323,8 @@ struct SmemLayout {
   static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 1) * 8 + 16;
 };
 
-template <int BT, int STAGES>
+// TWO: GemmParams::chains == 2, the sums of the tile side by side (a kernel of its own: in one with the others it cost each of them 0.1 us).
+template <int BT, int STAGES, bool TWO>
 __global__ void __launch_bounds__(192, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GemmParams p) {
   using L = SmemLayout<BT, STAGES>;
@@ -366,7 +366,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols<BT>()) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols<BT, TWO>()) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -410,10 +410,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc(BT);
       bool ok = true;
-      for (int chain = p.chains == 2 ? 0 : 1, i = 0; ok && chain < 2; ++chain) {
-        const uint32_t acc = p.chains == 2 ? tmem_acc + chain * BT : tmem_acc;
-        const int begin = i, end = chain == 0 ? num_kb / 2 : num_kb;
-        for (; i < end; ++i) {
+      auto sum = [&](int begin, int end, uint32_t acc) {
+        for (int i = begin; i < end && ok; ++i) {
           const int s = i % STAGES;
           ok = mbar_wait(full_bar(s), (i / STAGES) & 1, abort_flag, ERR_FULL_WAIT, p.wait_cycles);
           if (!ok) break;
@@ -427,6 +425,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           }
           umma_commit(empty_bar(s));
         }
+      };
+      if (TWO) {
+        sum(0, num_kb / 2, tmem_acc);
+        sum(num_kb / 2, num_kb, tmem_acc + BT);
+      } else {
+        sum(0, num_kb, tmem_acc);
       }
       if (ok) umma_commit(accum_bar);
     }
@@ -466,7 +470,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       float* part = (direct || via_cluster) ? nullptr : p.workspace + (size_t)split * p.M * p.N;
       float* part_smem = reinterpret_cast<float*>(smem);          // [BT][128]; the stages are drained by now
       float* row_f = part_smem + BT * BM;                         // the rows' norm factors, when the input lacks them
-      if (p.rs.on && direct && p.chains > 1) {
+      if (TWO && p.rs.on && direct) {
         // As where the splits of a cluster are added up, so that the sums are the same either way.
         pdl_wait();
         if (p.swiglu) {
@@ -496,7 +500,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       for (int c = 0; c < BT; c += 16) {
         uint32_t r[16];
         tmem_ld16(taddr + c, r);
-        if (p.chains > 1) {
+        if (TWO) {
           uint32_t r2[16];
           tmem_ld16(taddr + BT + c, r2);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -726,7 +730,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(tmem_cols<BT>()) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(tmem_cols<BT, TWO>()) : "memory");
   }
 }
 
@@ -789,13 +793,13 @@ static bool cached_map(CUtensorMap* out, const void* base, long long rows, long 
   return true;
 }
 
-template <int BT, int STAGES>
+template <int BT, int STAGES, bool TWO = false>
 int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, int splits, cudaStream_t stream) {
   using L = SmemLayout<BT, STAGES>;
   const int smem = L::TOTAL + 1024;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BT, STAGES, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) { set_error("gemm_tcgen05: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e)); return 2; }
     configured = true;
   }
@@ -810,9 +814,9 @@ int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p,
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_pdl_enabled ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BT, STAGES>, mw, mx, p);
+    cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BT, STAGES, TWO>, mw, mx, p);
   } else {
-    launch(gemm_tcgen05_kernel<BT, STAGES>, grid, dim3(192), smem, stream, mw, mx, p);
+    launch(gemm_tcgen05_kernel<BT, STAGES, TWO>, grid, dim3(192), smem, stream, mw, mx, p);
   }
   return 0;
 }
@@ -1524,8 +1528,8 @@ static int launch_prefill(const void* y, int y_dtype, const void* x, const void*
 static int launch_for_tile(int bt, const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, int splits,
                            cudaStream_t stream) {
   switch (bt) {
-    case 16: return launch_tc<16, 6>(mw, mx, p, splits, stream);
-    case 32: return launch_tc<32, 5>(mw, mx, p, splits, stream);
+    case 16: return p.chains == 2 ? launch_tc<16, 6, true>(mw, mx, p, splits, stream) : launch_tc<16, 6>(mw, mx, p, splits, stream);
+    case 32: return p.chains == 2 ? launch_tc<32, 5, true>(mw, mx, p, splits, stream) : launch_tc<32, 5>(mw, mx, p, splits, stream);
     case 64: return launch_tc<64, 4>(mw, mx, p, splits, stream);
     case 128: return launch_tc<128, 3>(mw, mx, p, splits, stream);
     default: return launch_tc<256, 4>(mw, mx, p, splits, stream);
