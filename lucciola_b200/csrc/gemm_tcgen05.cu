@@ -311,8 +311,11 @@ __device__ __forceinline__ float gated_mul(int act, float limit, float g, float 
   return silu_mul(g, u);
 }
 
-template <int BT, bool TWO>
-__host__ __device__ constexpr int tmem_cols() { return TWO ? 2 * BT : BT < 32 ? 32 : BT; }
+// Up to 32 tokens: two sums of the tile (GemmParams::chains).  In one kernel with the products that don't need them they cost each of those up to
+// 0.1 us (the decode benchmark 1737 -> 1727 tokens/s); in a kernel of their own the change from one kernel's instructions to the other's costs 0.4 us
+// (a feed-forward of one token 19.9 -> 20.4, the decoder of 4 layers 2108 -> 2167).
+template <int BT>
+__host__ __device__ constexpr int tmem_cols() { return BT <= 32 ? 2 * BT : BT; }
 
 template <int BT, int STAGES>
 struct SmemLayout {
@@ -323,8 +326,7 @@ struct SmemLayout {
   static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 1) * 8 + 16;
 };
 
-// TWO: GemmParams::chains == 2, the sums of the tile side by side (a kernel of its own: in one with the others it cost each of them 0.1 us).
-template <int BT, int STAGES, bool TWO>
+template <int BT, int STAGES>
 __global__ void __launch_bounds__(192, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GemmParams p) {
   using L = SmemLayout<BT, STAGES>;
@@ -366,7 +368,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols<BT, TWO>()) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols<BT>()) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -410,8 +412,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc(BT);
       bool ok = true;
-      auto sum = [&](int begin, int end, uint32_t acc) {
-        for (int i = begin; i < end && ok; ++i) {
+      for (int chain = p.chains == 2 ? 0 : 1, i = 0; ok && chain < 2; ++chain) {
+        const uint32_t acc = p.chains == 2 ? tmem_acc + chain * BT : tmem_acc;
+        const int begin = i, end = chain == 0 ? num_kb / 2 : num_kb;
+        for (; i < end; ++i) {
           const int s = i % STAGES;
           ok = mbar_wait(full_bar(s), (i / STAGES) & 1, abort_flag, ERR_FULL_WAIT, p.wait_cycles);
           if (!ok) break;
@@ -425,12 +429,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           }
           umma_commit(empty_bar(s));
         }
-      };
-      if (TWO) {
-        sum(0, num_kb / 2, tmem_acc);
-        sum(num_kb / 2, num_kb, tmem_acc + BT);
-      } else {
-        sum(0, num_kb, tmem_acc);
       }
       if (ok) umma_commit(accum_bar);
     }
@@ -470,7 +468,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       float* part = (direct || via_cluster) ? nullptr : p.workspace + (size_t)split * p.M * p.N;
       float* part_smem = reinterpret_cast<float*>(smem);          // [BT][128]; the stages are drained by now
       float* row_f = part_smem + BT * BM;                         // the rows' norm factors, when the input lacks them
-      if (TWO && p.rs.on && direct) {
+      if (p.rs.on && direct && p.chains > 1) {
         // As where the splits of a cluster are added up, so that the sums are the same either way.
         pdl_wait();
         if (p.swiglu) {
@@ -500,7 +498,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       for (int c = 0; c < BT; c += 16) {
         uint32_t r[16];
         tmem_ld16(taddr + c, r);
-        if (TWO) {
+        if (p.chains > 1) {
           uint32_t r2[16];
           tmem_ld16(taddr + BT + c, r2);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -730,7 +728,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(tmem_cols<BT, TWO>()) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(tmem_cols<BT>()) : "memory");
   }
 }
 
@@ -793,13 +791,13 @@ static bool cached_map(CUtensorMap* out, const void* base, long long rows, long 
   return true;
 }
 
-template <int BT, int STAGES, bool TWO = false>
+template <int BT, int STAGES>
 int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, int splits, cudaStream_t stream) {
   using L = SmemLayout<BT, STAGES>;
   const int smem = L::TOTAL + 1024;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BT, STAGES, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) { set_error("gemm_tcgen05: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e)); return 2; }
     configured = true;
   }
@@ -814,9 +812,9 @@ int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p,
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_pdl_enabled ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BT, STAGES, TWO>, mw, mx, p);
+    cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BT, STAGES>, mw, mx, p);
   } else {
-    launch(gemm_tcgen05_kernel<BT, STAGES, TWO>, grid, dim3(192), smem, stream, mw, mx, p);
+    launch(gemm_tcgen05_kernel<BT, STAGES>, grid, dim3(192), smem, stream, mw, mx, p);
   }
   return 0;
 }
@@ -928,7 +926,8 @@ struct PrefillSmemT {
 };
 
 // With PAIR, m_tiles counts pairs of token tiles, num_tiles tiles of 256 tokens, and the grid holds two CTAs a tile slot.
-template <bool PAIR>
+// CUT: GemmParams::chains > 0 (a kernel of its own, since the read-out of several sums takes 206 registers instead of 128).
+template <bool PAIR, bool CUT>
 __global__ void __launch_bounds__(192, 1)
 gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                             const __grid_constant__ CUtensorMap map_w2, GemmParams p, int m_tiles, int num_tiles,
@@ -1067,7 +1066,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
       bool ok = true;
       int s = 0;
       uint32_t turn = 0;
-      const int chains = !PAIR && p.chains > 1 ? p.chains : 1;
+      const int chains = CUT && p.chains > 1 ? p.chains : 1;
       for (int t = 0; t < my_tiles && ok; ++t) {
         const int b = t & 1;
         int m0, n0, bn;
@@ -1100,7 +1099,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
     }
   } else {
     // ---- epilogue: warp w reads lanes (w % 4) * 32 .. + 31, i.e. 32 tokens, 16 features at a time -------------
-    const int quarter = warp & 3, chains = p.chains > 1 ? p.chains : 1;
+    const int quarter = warp & 3, chains = CUT && p.chains > 1 ? p.chains : 1;
     bool ok = true;
     for (int t = 0; t < my_tiles && ok; ++t) {
       int m0, n0, bn;
@@ -1117,12 +1116,12 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
       if (p.rs.on) {
         pdl_wait();
         const int first = m0 + quarter * 32;
-        if (!PAIR && p.chains > 1) {          // where the splits of a cluster are added up: a warp a token
+        if (CUT && chains > 1) {              // where the splits of a cluster are added up: a warp a token
           for (int i = 0; i < 32 && first + i < p.M; ++i) {
             const float f = row_factor_warp(p.rs, first + i, lane);
             if (lane == i) rf = f;
           }
-        } else if (!PAIR && p.chains == 1) {  // in one split: eight threads a token
+        } else if (CUT) {                     // in one split: eight threads a token
           for (int i = 0; i < 32 && first + i < p.M; i += 4) {
             const float f = row_factor_eight(p.rs, first + i + (lane >> 3), p.M, lane & 7);
             const float mine = __shfl_sync(0xffffffffu, f, (lane & 3) * 8);
@@ -1251,7 +1250,7 @@ gemm_tcgen05_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __g
       for (int c = 0; c < bn; c += 16) {
         uint32_t r[16];
         tmem_ld16(taddr + c, r);
-        if (PAIR || chains == 1) {
+        if (!CUT || chains == 1) {
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         } else {
           uint32_t more[4][16];                                  // four sums on their way at a time, added one by one
@@ -1425,7 +1424,7 @@ static void prefill_choose(int M, int N, int K, int swiglu, int force_bn, int pa
   if (use_pair && pair_slots < 0) {
     const int smem_pair = PrefillSmemT<true>::TOTAL + 1024;
     pair_slots = num_sms / 2;
-    if (cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_pair) == cudaSuccess) {
+    if (cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_pair) == cudaSuccess) {
       cudaLaunchConfig_t qc = {};
       qc.gridDim = dim3(2 * (num_sms / 2)); qc.blockDim = dim3(192); qc.dynamicSmemBytes = smem_pair;
       cudaLaunchAttribute qa[1];
@@ -1433,7 +1432,7 @@ static void prefill_choose(int M, int N, int K, int swiglu, int force_bn, int pa
       qa[0].val.clusterDim.x = 2; qa[0].val.clusterDim.y = 1; qa[0].val.clusterDim.z = 1;
       qc.attrs = qa; qc.numAttrs = 1;
       int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, gemm_tcgen05_prefill_kernel<true>, &qc) == cudaSuccess && n > 0 && n < pair_slots) pair_slots = n;
+      if (cudaOccupancyMaxActiveClusters(&n, gemm_tcgen05_prefill_kernel<true, false>, &qc) == cudaSuccess && n > 0 && n < pair_slots) pair_slots = n;
     }
     cudaGetLastError();
   }
@@ -1499,16 +1498,17 @@ static int launch_prefill(const void* y, int y_dtype, const void* x, const void*
   const uintptr_t lowest = (uintptr_t)y | (uintptr_t)(ldy * el);
   const int vec_store = lowest % 32 == 0 ? 2 : lowest % 16 == 0;
   const int smem = (use_pair ? PrefillSmemT<true>::TOTAL : PrefillSmemT<false>::TOTAL) + 1024;
-  static bool configured[2] = {false, false};
-  if (!configured[use_pair]) {
-    cudaError_t e = use_pair ? cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-                             : cudaFuncSetAttribute(gemm_tcgen05_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  auto* const kernel = use_pair ? gemm_tcgen05_prefill_kernel<true, false> : chains > 0 ? gemm_tcgen05_prefill_kernel<false, true> : gemm_tcgen05_prefill_kernel<false, false>;
+  static bool configured[3] = {false, false, false};
+  bool& ready = configured[use_pair ? 0 : chains > 0 ? 1 : 2];
+  if (!ready) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) { set_error("gemm_tcgen05: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e)); return 2; }
-    configured[use_pair] = true;
+    ready = true;
   }
   const int grid = num_tiles < slots ? num_tiles : slots;
   if (!use_pair) {
-    launch(gemm_tcgen05_prefill_kernel<false>, dim3(grid), dim3(192), smem, stream, mx, mw, mw2, p, m_tiles, num_tiles, plan, vec_store);
+    launch(kernel, dim3(grid), dim3(192), smem, stream, mx, mw, mw2, p, m_tiles, num_tiles, plan, vec_store);
     return 0;
   }
   cudaLaunchConfig_t cfg = {};
@@ -1519,7 +1519,7 @@ static int launch_prefill(const void* y, int y_dtype, const void* x, const void*
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = g_pdl_enabled ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, gemm_tcgen05_prefill_kernel<true>, mx, mw, mw2, p, m_tiles, num_tiles, plan, vec_store);
+  cudaLaunchKernelEx(&cfg, kernel, mx, mw, mw2, p, m_tiles, num_tiles, plan, vec_store);
   return 0;
 }
 
@@ -1528,8 +1528,8 @@ static int launch_prefill(const void* y, int y_dtype, const void* x, const void*
 static int launch_for_tile(int bt, const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, int splits,
                            cudaStream_t stream) {
   switch (bt) {
-    case 16: return p.chains == 2 ? launch_tc<16, 6, true>(mw, mx, p, splits, stream) : launch_tc<16, 6>(mw, mx, p, splits, stream);
-    case 32: return p.chains == 2 ? launch_tc<32, 5, true>(mw, mx, p, splits, stream) : launch_tc<32, 5>(mw, mx, p, splits, stream);
+    case 16: return launch_tc<16, 6>(mw, mx, p, splits, stream);
+    case 32: return launch_tc<32, 5>(mw, mx, p, splits, stream);
     case 64: return launch_tc<64, 4>(mw, mx, p, splits, stream);
     case 128: return launch_tc<128, 3>(mw, mx, p, splits, stream);
     default: return launch_tc<256, 4>(mw, mx, p, splits, stream);
